@@ -23,19 +23,30 @@
 // at about 2^-bL max|a| max|b| K.
 //
 // Pipeline: one TMA producer thread, one MMA issuer thread, eight epilogue
-// warps (the tile's accumulators fill the tensor memory, so the epilogue of
-// one tile cannot overlap the MMAs of the next; two warps per lane quarter
-// halve its latency-bound duration).  Per 64-wide K block the producer loads the L slices of the B tile
-// (in 16-row boxes, only the rows of the trajectory's own columns) into one
-// ring stage and the L slices of the A tile into L stages of a second ring; the issuer runs the L(L+1)/2 slice products of the block from
-// shared memory with the MMA width cut to the trajectory's own N, the L - i
-// products of A slice i back to back per 16-wide K step so that A comes from
-// the tensor core's collector buffer after its first read.  The
-// epilogue stages the FP64 tile in shared memory for coalesced stores.  The
-// wide configuration (two B stages, deep A ring) holds one CTA per SM; the
-// compact one (one B stage, L A stages, <= 256 TMEM columns) two.  Every wait
-// is bounded: on expiry the kernel sets an error flag, drains its copies,
-// frees its tensor memory and returns.
+// warps (two per tensor-memory lane quarter).  Per 64-wide K block the producer
+// loads the L slices of the B tile (in 16-row boxes, only the rows of the
+// tile's own nT columns, slice after slice) into one ring stage and the L
+// slices of the A tile into L stages of a second ring.
+//
+// The B slices of a stage are consecutive rows of one operand (slice j at row
+// j nT), and level l's accumulator sits at tensor-memory column l nT, so the
+// products of A slice i with the B slices 0..L-1-i are ONE product with an N of
+// (L - i) nT columns landing on the columns from i nT on.  The issuer runs it
+// as one or two MMAs of up to 256 columns.  An MMA of N columns takes
+// max(N / 2, 32 + N / 4) cycles (it reads 4 KB of A and 32 N bytes of B from
+// shared memory at 128 bytes a cycle; tests/mma_rate.cu), so per-slice MMAs of
+// N = 80 run at 77% of the pipe's rate and those of 128 and more at all of it;
+// there are also 2.3 times fewer of them to issue.  L = 6, N tiles of 80,
+// W = V S of the 512-trajectory batch: 4.19 ms with one MMA per slice pair,
+// 2.52 this way (h2: 0.70 and 0.49, Z: 0.98 and 0.86).
+//
+// The epilogue first turns the accumulators into integers in registers and
+// hands the tensor memory back, then scales and stores, so that only the first
+// part keeps the next tile's MMAs waiting (the accumulators of one tile fill
+// the tensor memory).  The wide configuration (two B stages, deep A ring)
+// holds one CTA per SM; the compact one (one B stage, L A stages, <= 256 TMEM
+// columns) two.  Every wait is bounded: on expiry the kernel sets an error
+// flag, drains its copies, frees its tensor memory and returns.
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -70,38 +81,30 @@ struct FxCfg {
   static_assert(TC_BM * SP * 8 <= RING, "output staging fits the ring");
 };
 
+// ldexp out of line: results outside the normal range (the epilogue is unrolled
+// over a warp's columns, and its instructions have to stay in the cache).
+__device__ __noinline__ double ll_scaled_far(long long T, int e) { return ldexp((double)T, e); }
+
 // T 2^e as a double by integer operations (the FP64 pipes are the scarce
-// resource): round-to-nearest-even when |T| needs more than 53 bits; results
-// outside the normal range go through ldexp.
+// resource): round-to-nearest-even when |T| needs more than 53 bits.
 __device__ __forceinline__ double ll_scaled(long long T, int e) {
-  if (T == 0) return 0.0;
-  const unsigned long long sign = T < 0 ? 0x8000000000000000ull : 0ull;
+  const unsigned long long sign = (unsigned long long)T & 0x8000000000000000ull;
   unsigned long long a = T < 0 ? (unsigned long long)(-T) : (unsigned long long)T;
-  const int msb = 63 - __clzll((long long)a);
-  int ee;  // value = a 2^ee with a in [2^52, 2^53)
-  if (msb > 52) {
-    const int sh = msb - 52;
-    const unsigned long long rem = a & ((1ull << sh) - 1), half = 1ull << (sh - 1);
-    a >>= sh;
-    if (rem > half || (rem == half && (a & 1ull))) a++;
-    ee = e + sh;
-    if (a >> 53) {
-      a >>= 1;
-      ee++;
-    }
-  } else {
-    a <<= (52 - msb);
-    ee = e - (52 - msb);
-  }
-  const int be = ee + 52 + 1023;
-  if (be <= 0 || be >= 2047) return ldexp((double)T, e);
-  return __longlong_as_double((long long)(sign | ((unsigned long long)be << 52) | (a & 0xFFFFFFFFFFFFFull)));
+  if (a == 0) return 0.0;
+  const int lz = __clzll((long long)a);
+  a <<= lz;
+  const unsigned rem = (unsigned)a & 0x7FFu;
+  a >>= 11;  // 53 bits; a rounding carry runs on into the exponent
+  a += (rem > 0x400u || (rem == 0x400u && (a & 1ull))) ? 1ull : 0ull;
+  const int be = e - lz + 1086;  // biased exponent of a 2^(e - lz + 11)
+  if (be <= 0 || be >= 2046) return ll_scaled_far(T, e);
+  return __longlong_as_double((long long)(sign | (((unsigned long long)(be - 1) << 52) + a)));
 }
 
 // One work item of a persistent CTA: trajectory, first output row, first
-// output column, K split.
+// output column and column count (a multiple of 16), K split.
 struct FxTile {
-  int traj, m0, n0, split;
+  int traj, m0, n0, nT, split;
 };
 
 // out[traj][split][M][N] = C (FP64) over the tile list; a persistent CTA takes
@@ -125,7 +128,8 @@ __global__ void __launch_bounds__(32 * (EW + 2), NA_ > 0 ? 2 : 1)
               int kPer, int digitBits, const FxTile* __restrict__ tiles, int nTiles, int* __restrict__ err) {
   using C = FxCfg<BN, L, NA_, NB_>;
   constexpr int NA = C::NA, NB = C::NB;
-  static_assert(EW % 4 == 0 && (CB == 8 || CB == 16) && BN % CB == 0, "epilogue warps / column batch");
+  static_assert(EW % 4 == 0 && CB == 8 && BN % CB == 0, "epilogue warps / column batch");
+  constexpr int NBAT = (BN / CB + EW / 4 - 1) / (EW / 4);  // column batches of one epilogue warp
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* ringA = smem;
@@ -164,10 +168,9 @@ __global__ void __launch_bounds__(32 * (EW + 2), NA_ > 0 ? 2 : 1)
   const uint32_t tmem = tmemSlot;
 
   // per-tile geometry (every role derives the same values)
-  auto geometry = [&](const FxTile& tl, int& M, int& N, int& nT, int& kt0, int& nk) {
+  auto geometry = [&](const FxTile& tl, int& M, int& N, int& kt0, int& nk) {
     int segTiles;
     tc_dims(shp[tl.traj], gemmId, M, N, segTiles);
-    nT = min(BN, (N - tl.n0 + 15) / 16 * 16);
     const int sT = max(1, (segTiles + kPer - 1) / kPer);  // this trajectory's splits
     const int per = (segTiles + sT - 1) / sT;              // <= kPer
     kt0 = tl.split * per;
@@ -180,8 +183,8 @@ __global__ void __launch_bounds__(32 * (EW + 2), NA_ > 0 ? 2 : 1)
       int ta = 0, tb = 0;
       for (int t = blockIdx.x; t < nTiles && !abortFlag; t += gridDim.x) {
         const FxTile tl = tiles[t];
-        int M, N, nT, kt0, nk;
-        geometry(tl, M, N, nT, kt0, nk);
+        int M, N, kt0, nk;
+        geometry(tl, M, N, kt0, nk);
         const TrajShape& T = shp[tl.traj];
         const int aRow0 = aShared ? T.vRow : 0, aCol0 = aShared ? T.vRow - T.gShift : 0;
         const int aZ = aShared ? T.vRoot : tl.traj;
@@ -193,11 +196,11 @@ __global__ void __launch_bounds__(32 * (EW + 2), NA_ > 0 ? 2 : 1)
             break;
           }
           const int x0 = (kt0 + kb) * TC_BK;
-          mbar_expect_tx(&bFull[sb], (uint32_t)(L * nT * TC_BK * 2));
+          mbar_expect_tx(&bFull[sb], (uint32_t)(L * tl.nT * TC_BK * 2));
+          uint8_t* dstB = ringB + sb * C::BG_BYTES;
           for (int j = 0; j < L; j++)
-            for (int r = 0; r < nT; r += 16)
-              tma_load_3d(ringB + sb * C::BG_BYTES + j * C::B_BYTES + r * TC_BK * 2, &tB, &bFull[sb],
-                          j * segPitch + x0, tl.n0 + r, tl.traj);
+            for (int r = 0; r < tl.nT; r += 16, dstB += 16 * TC_BK * 2)
+              tma_load_3d(dstB, &tB, &bFull[sb], j * segPitch + x0, tl.n0 + r, tl.traj);
           tb++;
           issuedB = tb;
           for (int i = 0; i < L; i++) {
@@ -218,17 +221,26 @@ __global__ void __launch_bounds__(32 * (EW + 2), NA_ > 0 ? 2 : 1)
   } else if (warp == EW + 1) {
     if (lane == 0) {
       // MMA issuer: kind::f16, D=F32, A=B=BF16, K-major, M=128; descriptors
-      // advance by address / 16: +2 per 16-wide K step, +B_BYTES/16 per B slice
+      // advance by address / 16: +2 per 16-wide K step, +8 per B row
       const uint64_t bdesc0 = sw128_desc(smem_u32(ringB));
       const uint64_t adesc0 = sw128_desc(smem_u32(ringA));
       int ca = 0, cb = 0, ph = 0;  // ph: accumulator phases (tiles with K work)
       for (int t = blockIdx.x; t < nTiles && !abortFlag; t += gridDim.x) {
         const FxTile tl = tiles[t];
-        int M, N, nT, kt0, nk;
-        geometry(tl, M, N, nT, kt0, nk);
+        int M, N, kt0, nk;
+        geometry(tl, M, N, kt0, nk);
         if (nk == 0) continue;  // the epilogue writes the empty split's zeros
-        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nT >> 3) << 17) |
-                               ((uint32_t)(TC_BM >> 4) << 24);
+        // A slice i covers (L - i) nT columns: one MMA up to 256 of them, else two halves
+        uint32_t id0[L], id1[L], half[L];
+#pragma unroll
+        for (int i = 0; i < L; i++) {
+          const int cols = (L - i) * tl.nT;
+          const int n0 = cols <= 256 ? cols : (cols / 2 + 15) / 16 * 16;
+          const uint32_t base = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TC_BM >> 4) << 24);
+          half[i] = (uint32_t)n0;
+          id0[i] = base | ((uint32_t)(n0 >> 3) << 17);
+          id1[i] = cols > n0 ? base | ((uint32_t)((cols - n0) >> 3) << 17) : 0u;
+        }
         if (ph > 0 && !mbar_wait(&accEmpty, (ph - 1) & 1, &abortFlag)) {  // the epilogue drained TMEM
           abortFlag = 1;
           atomicExch(err, 16);
@@ -261,19 +273,20 @@ __global__ void __launch_bounds__(32 * (EW + 2), NA_ > 0 ? 2 : 1)
             consumedA = ca;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint64_t ad = adesc0 + (uint64_t)((sa * C::A_BYTES) >> 4);
-            // the L - i products of A slice i share each 16-wide K step of A:
-            // issued back to back, A is read from shared memory once per step
-            // and reused from the collector buffer
+            const uint32_t d0 = tmem + (uint32_t)(i * tl.nT), d1 = d0 + half[i];
+            const uint64_t bd1 = bd + 8 * half[i];
+            if (id1[i]) {
+              // both halves of a K step read the same 4 KB of A: the second from the collector
 #pragma unroll
-            for (int k = 0; k < TC_BK / 16; k++) {
-#pragma unroll
-              for (int j = 0; j < L - i; j++) {
-                const int last = L - i - 1;
-                const int coll = last == 0 ? 0 : (j == 0 ? 1 : (j == last ? 3 : 2));
-                umma_bf16_coll(coll, tmem + (uint32_t)((i + j) * BN), ad + 2 * k,
-                               bd + (uint64_t)((j * C::B_BYTES) >> 4) + 2 * k, idesc,
-                               (kb > 0 || i > 0 || k > 0) ? 1u : 0u);
+              for (int k = 0; k < TC_BK / 16; k++) {
+                const uint32_t acc = (kb > 0 || i > 0 || k > 0) ? 1u : 0u;
+                umma_bf16_coll(1, d0, ad + 2 * k, bd + 2 * k, id0[i], acc);
+                umma_bf16_coll(3, d1, ad + 2 * k, bd1 + 2 * k, id1[i], acc);
               }
+            } else {
+#pragma unroll
+              for (int k = 0; k < TC_BK / 16; k++)
+                umma_bf16(d0, ad + 2 * k, bd + 2 * k, id0[i], (kb > 0 || i > 0 || k > 0) ? 1u : 0u);
             }
             umma_commit(&aEmpty[sa]);
           }
@@ -289,19 +302,18 @@ __global__ void __launch_bounds__(32 * (EW + 2), NA_ > 0 ? 2 : 1)
     // epilogue: warp w owns TMEM lanes [32q, 32q+32) = tile rows, q = w % 4
     // (the lane quarter a warp may access), and every (EW/4)-th batch of CB
     // columns starting at batch w / 4
-    const long long base = 1LL << digitBits;
     const int q = warp & 3, cg = warp >> 2;
     int ph = 0;
     for (int t = blockIdx.x; t < nTiles; t += gridDim.x) {
       const FxTile tl = tiles[t];
-      int M, N, nT, kt0, nk;
-      geometry(tl, M, N, nT, kt0, nk);
+      int M, N, kt0, nk;
+      geometry(tl, M, N, kt0, nk);
       double* Oz = batn(out, bs, tl.traj) + (size_t)tl.split * (size_t)M * N;
       const int r = q * 32 + lane, row = tl.m0 + r;
       const bool rowOk = row < M;
       if (nk == 0) {  // empty split: its partial is zero
         if (rowOk && cg == 0)
-          for (int col = tl.n0; col < min(N, tl.n0 + BN); col++) Oz[(size_t)row * N + col] = 0.0;
+          for (int col = tl.n0; col < min(N, tl.n0 + tl.nT); col++) Oz[(size_t)row * N + col] = 0.0;
         continue;
       }
       const bool waited = mbar_wait(&accFull, ph & 1, &abortFlag);
@@ -310,53 +322,65 @@ __global__ void __launch_bounds__(32 * (EW + 2), NA_ > 0 ? 2 : 1)
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      // the level sums of this warp's columns as 64-bit integers
+      long long Tv[NBAT][CB];
+#pragma unroll
+      for (int bt = 0; bt < NBAT; bt++) {
+        const int c = (cg + bt * (EW / 4)) * CB;
+        if (c < tl.nT) {
+          uint32_t acc[L][CB];
+#pragma unroll
+          for (int l = 0; l < L; l++)
+            TMEM_LD_X8(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(l * tl.nT + c), acc[l]);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int j = 0; j < CB; j++) {
+            long long v = 0;
+#pragma unroll
+            for (int l = 0; l < L; l++)
+              v = (long long)((unsigned long long)v << digitBits) + (long long)__float2int_rn(__uint_as_float(acc[l][j]));
+            Tv[bt][j] = v;
+          }
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&accEmpty);
+      ph++;
       const TrajShape& T = shp[tl.traj];
       const int* eA = aShared ? expA + T.vExp : batn(expA, bs, tl.traj);
       const int* eB = batn(expB, bs, tl.traj);
       const int ea = rowOk ? eA[row] - digitBits * (L + 1) : 0;
       unsigned rowMaxEx = 0;
-#pragma unroll 1
-      for (int c = cg * CB; c < nT; c += (EW / 4) * CB) {
-        uint32_t acc[L][CB];
 #pragma unroll
-        for (int l = 0; l < L; l++) {
-          if (CB == 16)
-            TMEM_LD_X16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(l * BN + c), acc[l]);
-          else
-            TMEM_LD_X8(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(l * BN + c), acc[l]);
-        }
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        double v[CB];
+      for (int bt = 0; bt < NBAT; bt++) {
+        const int c = (cg + bt * (EW / 4)) * CB;
+        if (c < tl.nT) {
+          double v[CB];
 #pragma unroll
-        for (int j = 0; j < CB; j++) {
-          const int col = tl.n0 + c + j;
-          unsigned ex = 0;
-          v[j] = 0.0;
-          if (rowOk && col < N) {
-            long long Tv = 0;
-#pragma unroll
-            for (int l = 0; l < L; l++) Tv = Tv * base + (long long)__float2int_rn(__uint_as_float(acc[l][j]));
-            v[j] = ll_scaled(Tv, ea + eB[col]);
-            ex = (unsigned)(__double2hiint(v[j]) >> 20) & 0x7FFu;
+          for (int j = 0; j < CB; j++) {
+            const int col = tl.n0 + c + j;
+            unsigned ex = 0;
+            v[j] = 0.0;
+            if (rowOk && col < N) {
+              v[j] = ll_scaled(Tv[bt][j], ea + eB[col]);
+              ex = (unsigned)(__double2hiint(v[j]) >> 20) & 0x7FFu;
+            }
+            if (maxCol) {
+              unsigned m = __reduce_max_sync(0xffffffffu, ex);
+              if (lane == 0 && m) atomicMax(batn(maxCol, bs, tl.traj) + col, m);
+            }
+            rowMaxEx = max(rowMaxEx, ex);
           }
-          if (maxCol) {
-            unsigned m = __reduce_max_sync(0xffffffffu, ex);
-            if (lane == 0 && m) atomicMax(batn(maxCol, bs, tl.traj) + col, m);
-          }
-          rowMaxEx = max(rowMaxEx, ex);
-        }
-        if (rowOk) {
-          double* dst = Oz + (size_t)row * N + tl.n0 + c;
+          if (rowOk) {
+            double* dst = Oz + (size_t)row * N + tl.n0 + c;
 #pragma unroll
-          for (int j = 0; j < CB; j += 2)
-            if (tl.n0 + c + j < N) *reinterpret_cast<double2*>(dst + j) = make_double2(v[j], v[j + 1]);
+            for (int j = 0; j < CB; j += 2)
+              if (tl.n0 + c + j < N) *reinterpret_cast<double2*>(dst + j) = make_double2(v[j], v[j + 1]);
+          }
         }
       }
       if (maxRow && rowOk && rowMaxEx) atomicMax(batn(maxRow, bs, tl.traj) + row, rowMaxEx);
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&accEmpty);
-      ph++;
     }
   }
   __syncthreads();
@@ -381,10 +405,8 @@ void launch_fx_t(cgpu_ctx* c, const CUtensorMap& ta, const CUtensorMap& tb, doub
                  const int* expB, unsigned* maxRow, unsigned* maxCol, int gemmId, int segPitchA, int segPitch,
                  int aShared, int kPer, int digitBits, const FxTile* tiles, int nTiles, int ctasPerSm, int* err) {
   using C = FxCfg<BN, L, NA_, NB_>;
-  // eight epilogue warps (two per tensor-memory lane quarter); the compact
-  // configuration (two CTAs per SM) loads eight columns per batch to stay
-  // inside half the register file
-  constexpr int EW = 8, CB = NA_ > 0 ? 8 : 16;
+  // eight epilogue warps (two per tensor-memory lane quarter)
+  constexpr int EW = 8, CB = 8;
   auto kern = k_fx_gemm<BN, L, NA_, NB_, EW, CB>;
   static bool attr = false;
   if (!attr) {
@@ -484,17 +506,37 @@ int fx_split_count(int M, int N, int BN, int kTiles, int nb, int digitBits) {
   return (kTiles + per - 1) / per;
 }
 
+// The columns of a trajectory go to ceil(N / bn) tiles of equal width (to 16
+// columns): a full tile and a narrow remainder would take the same MMA columns
+// but issue the remainder's in short MMAs.  The tiles are sorted by their work
+// (K blocks times columns), largest first, so that the CTAs, which take every
+// gridDim-th tile, end together; tiles of one trajectory stay neighbours.
 void* fx_build_tiles(cgpu_ctx* c, int gemmId, int bn, int nSplit, int* nTiles) {
   std::vector<FxTile> v;
+  std::vector<std::pair<long, int>> order;  // (work of the widest tile, trajectory)
   for (int b = 0; b < c->nb; b++) {
+    const TrajShape& S = c->shape_h[b];
+    const int kTiles = gemmId == TC_GEMM_Z ? S.Kp / TC_BK : S.Kg / TC_BK;
+    const int units = ceil_div(gemmId == TC_GEMM_Z ? 2 * S.nOS * S.nOS : 2 * S.nPairs, 16);
+    const int nt = ceil_div(units, bn / 16);
+    order.push_back({-(long)kTiles * ceil_div(units, nt), b});
+  }
+  std::stable_sort(order.begin(), order.end());
+  for (const auto& o : order) {
+    const int b = o.second;
     const TrajShape& S = c->shape_h[b];
     int P2 = 2 * S.nPairs, Q2 = 2 * S.nOS * S.nOS, M, N;
     if (gemmId == TC_GEMM_W) { M = S.nG; N = P2; }
     else if (gemmId == TC_GEMM_Z) { M = S.nG; N = Q2; }
     else { M = P2; N = P2; }
+    const int units = ceil_div(N, 16), nt = ceil_div(units, bn / 16);
     for (int m0 = 0; m0 < M; m0 += TC_BM)
-      for (int n0 = 0; n0 < N; n0 += bn)
-        for (int z = 0; z < nSplit; z++) v.push_back(FxTile{b, m0, n0, z});
+      for (int z = 0; z < nSplit; z++)
+        for (int k = 0, u = 0; k < nt; k++) {
+          const int w = units / nt + (k < units % nt ? 1 : 0);
+          v.push_back(FxTile{b, m0, 16 * u, 16 * w, z});
+          u += w;
+        }
   }
   *nTiles = (int)v.size();
   void* d = nullptr;
