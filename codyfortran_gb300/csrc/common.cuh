@@ -340,7 +340,7 @@ struct cgpu_ctx {
   z_t *basis_d = nullptr, *lw_d = nullptr, *trial_d = nullptr, *work_d = nullptr;
   int maxKrylov = 0;
   int krylovWindow = 0;                       // 0: full re-orthogonalisation; k: last k basis vectors
-  // fixed-point form: every trajectory's grid a contiguous piece of one of a few root grids (same
+  // fixed-point forms: every trajectory's grid a contiguous piece of one of a few root grids (same
   // interaction): one shared interaction matrix per root, rows/columns from fxVRow
   int fxShared = 0, fxKgMax = 0;
   std::vector<int> fxVRow, fxVRoot, fxRoots;  // per trajectory: row offset, root index; per root: trajectory
@@ -366,6 +366,9 @@ struct cgpu_ctx {
   std::string lastError;
   long launches = 0;  // kernels launched by this context (since the last reset)
   MixedBufs* mixed = nullptr;
+  // the contractions as digit slices on the tensor cores: mixed_fx / mixed_fx6, and the FP64 form unless its
+  // digit planes (14 bytes per interaction matrix entry) leave no room for the context (choose_fixed_point)
+  int fxOn = 0;
   z_t* sysTmp_d = nullptr;  // three nG-point vectors of the Sys* entry points (first use)
   McAdjoint* mcAdj = nullptr;  // MCTDHF pulse gradient: checkpoints and work buffers (first use)
   // profiling: CUDA events around every launch of one kernel family
@@ -477,10 +480,12 @@ void launch_build_vint(cgpu_ctx* c);
 size_t zgemm_partial_need(const cgpu_ctx* c);
 // k_mixed.cu
 size_t mixed_layout(cgpu_ctx* c, char* base, size_t off);  // sizes (base == nullptr) or places the buffers
+size_t mixed_outside_bytes(const cgpu_ctx* c);  // device bytes beside the arena (shared interaction slices)
 void mixed_init(cgpu_ctx* c);
 void mixed_free(cgpu_ctx* c);
 int mixed_error(cgpu_ctx* c);
 void launch_correlation_mixed(cgpu_ctx* c, z_t* dOrbs, const z_t* orbs, int wantH2);
+void launch_fill_h2_fx(cgpu_ctx* c, const z_t* orbs);  // FillH2 with the FP64 form's slices (fxOn)
 // Tile tuner hooks of the fixed-point contractions.  A tile table t[9] holds,
 // for W = V S, Z = W R'' and h2 = S^T W in turn: N-tile width, compact (two
 // CTAs per SM) flag, K splits.  fx_tiles_get returns false outside the

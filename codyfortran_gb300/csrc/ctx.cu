@@ -347,10 +347,12 @@ size_t layout(cgpu_ctx* c, char* base) {
   Z(c->h1_d, nO2);
   Z(c->rdm2_d, nO4);
   Z(c->h2_d, nO4);
-  Z(c->S_d, nG * P);
-  Z(c->W_d, nG * P);
-  Z(c->Sfull_d, nG * Q);
-  Z(c->Wfull_d, 2 * nG * Q);
+  if (!c->fxOn) {
+    Z(c->S_d, nG * P);
+    Z(c->W_d, nG * P);
+    Z(c->Sfull_d, nG * Q);
+    Z(c->Wfull_d, 2 * nG * Q);
+  }
   Z(c->Rp_d, Q * Q);
   Z(c->h2s_d, Q * Q);
   Z(c->Mreg_d, Q);
@@ -382,7 +384,7 @@ void put(cgpu_ctx* c, int b, T* dst0, const std::vector<T>& v) {
 }
 
 
-// Fixed-point form of a batch: when every trajectory has the same dense
+// Fixed-point forms of a batch: when every trajectory has the same dense
 // interaction and its grid is a contiguous, bitwise-equal piece of one of a
 // few root grids (FEDVR boxes of different length with the same elements: the
 // grids with an even and with an odd element count on [-n, n] form two
@@ -397,8 +399,7 @@ void detect_shared_interaction(cgpu_ctx* c) {
   c->fxVRoot.assign(n, 0);
   c->fxRoots.clear();
   c->fxKgMax = (c->nG + 63) / 64 * 64;
-  const bool fx = c->precision == CGPU_PREC_MIXED_FX || c->precision == CGPU_PREC_MIXED_FX6;
-  if (!fx || !c->hasInteraction || n < 2) return;
+  if (!c->fxOn || !c->hasInteraction || n < 2) return;
   std::vector<int> order(n);
   for (size_t b = 0; b < n; b++) order[b] = (int)b;
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return c->sys[a].nG > c->sys[b].nG; });
@@ -475,7 +476,6 @@ void build_ctx(cgpu_ctx* c, const cgpu_desc* descs, int nSys) {
     if (descs[b].krylov_window != c->krylovWindow || descs[b].krylov_window < 0)
       throw std::string("krylov_window must be >= 0 and the same for every trajectory of a batch");
   c->nGO = nGO;
-  detect_shared_interaction(c);
   ci_build_work(c);
   c->nS = (c->method == CGPU_METHOD_TDCI) ? c->nC : c->nC + nGO;
   c->minS = minS;
@@ -493,13 +493,34 @@ void build_ctx(cgpu_ctx* c, const cgpu_desc* descs, int nSys) {
     c->lzBlocksHeur = c->lzBlocks;
     c->lzBlocksCap = (int)std::max<size_t>(1, std::min(need, (size_t)2 * c->lzBlocks));
   }
-  c->lzBlocks = c->lzBlocksCap;
-  c->partialCap = std::max({lanczos_partial_need(c), gram_partial_need(c, c->nOS), zgemm_partial_need(c),
-                            (size_t)148});
-  c->lzBlocks = c->lzBlocksHeur;
+  size_t total = 0;
+  auto size_up = [&](int fx) {
+    c->fxOn = fx;
+    detect_shared_interaction(c);
+    c->lzBlocks = c->lzBlocksCap;
+    c->partialCap = std::max({lanczos_partial_need(c), gram_partial_need(c, c->nOS), zgemm_partial_need(c),
+                              (size_t)148});
+    c->lzBlocks = c->lzBlocksHeur;
+    c->bs = layout(c, nullptr);
+    total = c->bs * (size_t)nSys + mixed_outside_bytes(c);
+  };
+  // The contractions run as digit slices in both fixed-point forms.  In the FP64
+  // form they do too (28 slice products on the tensor cores against the FP64
+  // pipe, 12 to 40 times slower on every shape measured), unless only the
+  // FP64-pipe kernels' smaller footprint fits the device.
+  const bool fxForm = d0->precision == CGPU_PREC_MIXED_FX || d0->precision == CGPU_PREC_MIXED_FX6;
+  const bool fp64 = d0->precision == CGPU_PREC_FP64 && c->hasInteraction && c->method != CGPU_METHOD_TDCI;
+  size_up(fxForm || fp64);
+  if (!fxForm && fp64) {
+    size_t freeB = 0, totB = 0;
+    CODY_CUDA(cudaMemGetInfo(&freeB, &totB));
+    if (total + ((size_t)512 << 20) > freeB) {
+      mixed_free(c);
+      size_up(0);
+    }
+  }
   // arena
-  c->bs = layout(c, nullptr);
-  size_t total = c->bs * (size_t)nSys;
+  total = c->bs * (size_t)nSys;
   CODY_CUDA(cudaMalloc(&c->arena, total));
   CODY_CUDA(cudaMemset(c->arena, 0, total));
   CODY_CUDA(cudaDeviceSynchronize());
@@ -1815,7 +1836,8 @@ long cgpu_batch_kernels_per_step(const cgpu_batch* b) { return (b && b->c) ? b->
 long cgpu_batch_launch_count(cgpu_batch* b, int reset) { return (b && b->c) ? cgpu_launch_count(b->c, reset) : -1; }
 
 int cgpu_batch_shared_interactions(const cgpu_batch* b) {
-  return (b && b->c && b->c->fxShared) ? (int)b->c->fxRoots.size() : 0;
+  if (!b || !b->c || b->c->precision == CGPU_PREC_FP64) return 0;  // counts the mixed fixed-point forms' matrices
+  return b->c->fxShared ? (int)b->c->fxRoots.size() : 0;
 }
 
 int cgpu_batch_profile_begin(cgpu_batch* b, int kernel) {

@@ -1,26 +1,31 @@
-// k_fx.cu -- fixed-point split GEMM on tcgen05 tensor cores (the mixed_fx form
-// of the contractions of ApplyCorrelationOp,
-// src/Method/Mb/OrbBased/S_Method_Mb_OrbBased.f90:647-872).
+// k_fx.cu -- fixed-point split GEMM on tcgen05 tensor cores (the FP64 and the
+// mixed_fx forms of the contractions of ApplyCorrelationOp and FillH2,
+// src/Method/Mb/OrbBased/S_Method_Mb_OrbBased.f90:227-329, 647-872).
 //
-// An FP64 operand row x[0..K) is carried as L slices of base-2^b digits under
+// An FP64 operand row x[0..K) is carried as L slices of base-256 digits under
 // one power of two per row:
-//     x[k] ~= 2^e sum_{i<L} d_i[k] 2^(-b(i+1)),   max_k |x[k]| < 2^e,
-//     |d_0| <= 2^b, d_i in [-2^(b-1), 2^(b-1)) for i > 0 (bf16 holds them exactly, b <= 8),
-// i.e. x rounded to bL fractional bits of its row maximum.  The product of an
-// A row and a B row splits into levels l = i + j:
-//     C = 2^(ea + eb) sum_l 2^(-b(l+2)) D_l,   D_l = sum_{i+j=l} sum_k a_i[k] b_j[k].
+//     x[k] ~= 2^e sum_{i<L} d_i[k] 2^(-8(i+1)),   max_k |x[k]| < 2^(e-1),
+//     |d_i| <= 128 (bf16 holds them exactly),
+// i.e. x rounded to 8L - 1 fractional bits of its row maximum.  The product of
+// an A row and a B row splits into levels l = i + j:
+//     C = 2^(ea + eb) sum_l 2^(-8(l+2)) D_l,   D_l = sum_{i+j=l} sum_k a_i[k] b_j[k].
 // Each level has its own FP32 accumulator in tensor memory (L accumulators of
-// BN columns), fed by the slice products of that level.  A slice product is
-// an integer of magnitude <= 2^2b, so D_0 and D_1 stay below 2^24 -- exact in
-// FP32 -- for K <= 2^(24-2b) (b = 6: K <= 4096, 7: 1024, 8: 256; longer
-// contractions are split in K and the FP64 partials summed) and D_2 for
-// K <= 0.8 2^(24-2b); a higher level that passes 2^24 rounds by 2^-24 of a
-// term at least 2^-2b below the result's scale.  The epilogue combines the
-// levels in 64-bit integers (Horner in base 2^b), converts once to FP64 and
-// applies the power-of-two scale, so C is the product of the truncated
-// operands whatever the summation order.  Levels l >= L are not formed; with
-// the operand truncation (2^-(bL+1) of each row maximum) they bound the error
-// at about 2^-bL max|a| max|b| K.
+// nT columns), fed by the slice products of that level.  A slice product is an
+// integer of magnitude <= 2^14, so over a chunk of K = 256 a level sum of l + 1
+// products stays below (l + 1) 2^22: exact in FP32 for the four leading levels
+// whatever the operands, and for the others unless every digit of both rows is
+// at its extreme with one sign (then C itself is 2^6 times its terms and one
+// unit of level 4 is 2^-54 of it).  After every chunk the epilogue adds the
+// level sums to 64-bit integers, so C is the product of the truncated operands
+// whatever the summation order.  Levels l >= L are not formed; with the operand
+// truncation (2^-8L of each row maximum) they bound the error at about
+// 2^-8L max|a| max|b| sqrt(K).
+//
+// L = 4 to 6 serve the mixed_fx / mixed_fx6 forms (their Z operands with
+// max_k |x[k]| < 2^e, |d_0| <= 256: one bit more, K <= 256).  L = 7 (55 bits) is
+// the FP64 form: the FP64 pipe of this GPU does two FMA a cycle and SM
+// (1.2 TFLOP/s), 28 slice products on the tensor cores about 60 TFLOP/s of the
+// same contraction, and the sum of a row rounds once instead of K times.
 //
 // Pipeline: one TMA producer thread, one MMA issuer thread, eight epilogue
 // warps (two per tensor-memory lane quarter).  Per 64-wide K block the producer
@@ -36,17 +41,19 @@
 // max(N / 2, 32 + N / 4) cycles (it reads 4 KB of A and 32 N bytes of B from
 // shared memory at 128 bytes a cycle; tests/mma_rate.cu), so per-slice MMAs of
 // N = 80 run at 77% of the pipe's rate and those of 128 and more at all of it;
-// there are also 2.3 times fewer of them to issue.  L = 6, N tiles of 80,
-// W = V S of the 512-trajectory batch: 4.19 ms with one MMA per slice pair,
-// 2.52 this way (h2: 0.70 and 0.49, Z: 0.98 and 0.86).
+// there are also 2.3 times fewer of them to issue (six 6-bit slices, N = 80,
+// W = V S of the 512-trajectory batch: 4.13 ms with one MMA per slice pair,
+// 2.52 this way).
 //
-// The epilogue first turns the accumulators into integers in registers and
-// hands the tensor memory back, then scales and stores, so that only the first
-// part keeps the next tile's MMAs waiting (the accumulators of one tile fill
-// the tensor memory).  The wide configuration (two B stages, deep A ring)
-// holds one CTA per SM; the compact one (one B stage, L A stages, <= 256 TMEM
-// columns) two.  Every wait is bounded: on expiry the kernel sets an error
-// flag, drains its copies, frees its tensor memory and returns.
+// The epilogue adds the accumulators of a chunk to integers in registers and
+// hands the tensor memory back; scaling and stores follow the tile's last
+// chunk.  Tiles with L nT <= half the tensor-memory columns alternate between
+// the two halves, so that the next chunk's MMAs run during the drain; wider
+// ones wait for it (about 1.5 k of 13 k cycles).  The wide configuration (two B
+// stages, deep A ring) holds one CTA per SM; the compact one (one B stage, L A
+// stages, <= 256 TMEM columns) two.  Every wait is bounded: on expiry the
+// kernel sets an error flag, drains its copies, frees its tensor memory and
+// returns.
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -61,6 +68,8 @@ using namespace tcdev;
 
 constexpr int FX_SMEM_MAX = 232448;
 
+constexpr int FX_CHUNK = 4;  // 64-wide K blocks per accumulation in tensor memory (K = 256)
+
 template <int BN, int L, int NA_, int NB_>
 struct FxCfg {
   static constexpr int A_BYTES = TC_BM * TC_BK * 2;
@@ -71,19 +80,52 @@ struct FxCfg {
   static constexpr int NA = NA_ > 0 ? NA_ : std::min(8, (FX_SMEM_MAX - 2048 - NB * BG_BYTES) / A_BYTES);
   static constexpr int RING = NA * A_BYTES + NB * BG_BYTES;
   static constexpr int SMEM = RING + 1024;
-  static constexpr int SP = BN + 1;  // staged output row pitch (doubles)
   static constexpr uint32_t TMEM_COLS = (L * BN) <= 32 ? 32 : (L * BN) <= 64 ? 64 : (L * BN) <= 128 ? 128
                                         : (L * BN) <= 256 ? 256 : 512;
   static_assert(L * BN <= 512, "tensor memory holds 512 columns");
   static_assert(BN % 16 == 0 && BN >= 16, "N tile: multiple of 16");
-  static_assert(NA >= 2 || NA >= L, "A ring");
+  static_assert(NA >= 2, "A ring");
   static_assert(SMEM + 2048 <= FX_SMEM_MAX, "shared memory");
-  static_assert(TC_BM * SP * 8 <= RING, "output staging fits the ring");
+};
+
+// The level sums of one output over its chunks as integers: T = sum_l D_l
+// 256^(L-1-l).  L <= 5 fits 64 bits (|D_0| <= 2^22 a chunk: below 2^63 for 512
+// chunks, which fx_min_splits keeps); longer ones are held as hi 2^24 + lo.
+template <int L>
+struct FxAcc {
+  static constexpr int LH = L <= 5 ? L : L - 3;  // levels in hi
+  long long hi, lo;
+  __device__ __forceinline__ void clear() { hi = lo = 0; }
+  // levels [l0, l0 + n) of column j
+  template <int N, int CB>
+  __device__ __forceinline__ void add(const uint32_t (&d)[N][CB], int j, int l0, int n) {
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+      if (i >= n) break;
+      const int l = l0 + i, v = __float2int_rn(__uint_as_float(d[i][j]));
+      const int sh = 8 * (l < LH ? LH - 1 - l : L - 1 - l);
+      const long long t = sh > 24 ? (long long)((unsigned long long)(long long)v << sh)
+                                  : (long long)v * (1 << (sh > 24 ? 0 : sh));
+      if (l < LH) hi += t;
+      else lo += t;
+    }
+  }
+  __device__ __forceinline__ double value(int e) const;  // T 2^e
 };
 
 // ldexp out of line: results outside the normal range (the epilogue is unrolled
 // over a warp's columns, and its instructions have to stay in the cache).
 __device__ __noinline__ double ll_scaled_far(long long T, int e) { return ldexp((double)T, e); }
+
+__device__ __noinline__ double ldexp_far(double v, int e) { return ldexp(v, e); }
+
+// v 2^e, exponent arithmetic on the bits where the result is normal.
+__device__ __forceinline__ double d_scaled(double v, int e) {
+  if (v == 0.0) return 0.0;
+  const int be = ((__double2hiint(v) >> 20) & 0x7FF) + e;
+  if (be <= 0 || be >= 2047) return ldexp_far(v, e);
+  return __hiloint2double(__double2hiint(v) + (e << 20), __double2loint(v));
+}
 
 // T 2^e as a double by integer operations (the FP64 pipes are the scarce
 // resource): round-to-nearest-even when |T| needs more than 53 bits.
@@ -101,6 +143,13 @@ __device__ __forceinline__ double ll_scaled(long long T, int e) {
   return __longlong_as_double((long long)(sign | (((unsigned long long)(be - 1) << 52) + a)));
 }
 
+template <int L>
+__device__ __forceinline__ double FxAcc<L>::value(int e) const {
+  // hi and lo are exact as doubles (hi < 2^53 for 128 chunks), so the fma is the one rounding
+  if constexpr (L > 5) return d_scaled(fma((double)hi, 16777216.0, (double)lo), e);
+  else return ll_scaled(hi, e);
+}
+
 // One work item of a persistent CTA: trajectory, first output row, first
 // output column and column count (a multiple of 16), K split.
 struct FxTile {
@@ -110,31 +159,36 @@ struct FxTile {
 // out[traj][split][M][N] = C (FP64) over the tile list; a persistent CTA takes
 // tiles blockIdx.x, blockIdx.x + gridDim.x, ...  Warps 0..EW-1: epilogue (TMEM
 // lanes 32(w%4)..32(w%4)+31, column batches of CB); warp EW: TMA producer;
-// warp EW+1: MMA issuer.  The rings and their
-// phases run on across tiles; the accumulator hand-off uses accFull (MMA ->
-// epilogue) and accEmpty (epilogue -> MMA), so the producer loads the next
-// tile while the epilogue drains the current one.  K splits: a trajectory of
-// segTiles K blocks takes ceil(segTiles / kPer) balanced splits; the tiles of
-// the list beyond them write zero partials.  maxRow/maxCol (unsplit K only):
-// the largest biased exponent of |C| per output row / column.
+// warp EW+1: MMA issuer.  The rings and their phases run on across tiles, so
+// the producer loads the next tile while the epilogue drains the current one.
+// One accumulator phase per chunk, numbered over the CTA's life: phase p signals
+// accFull[p % 2] (MMA -> epilogue) and accEmpty[p % 2] (epilogue -> MMA) and uses
+// the tensor-memory half p % 2 if its tile fits one.  Its MMAs wait for the
+// drain of phase p - 2 (same half), and of p - 1 too where either tile needs
+// both halves.  K splits: a trajectory of segTiles K blocks takes
+// ceil(segTiles / kPer) balanced splits; the tiles of the list beyond them
+// write zero partials.  maxRow/maxCol (unsplit K only): the largest biased
+// exponent of |C| per output row / column.  A row or column whose exponent is
+// FX_EXP_NAN (an operand with an infinity or a NaN) gives NaN.
 // aShared: A is shared by the trajectories (3D map with one plane per root
 // grid); the trajectory's rows start at vRow of plane vRoot, its K range at
 // vRow - gShift, its row exponents at expA[vExp].
-template <int BN, int L, int NA_, int NB_, int EW, int CB>
+template <int BN, int L, int NA_, int NB_, int EW>
 __global__ void __launch_bounds__(32 * (EW + 2), NA_ > 0 ? 2 : 1)
     k_fx_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUtensorMap tB, double* __restrict__ out,
               const int* __restrict__ expA, const int* __restrict__ expB, unsigned* __restrict__ maxRow,
               unsigned* __restrict__ maxCol, TRAJ_ARGS, int gemmId, int segPitchA, int segPitch, int aShared,
-              int kPer, int digitBits, const FxTile* __restrict__ tiles, int nTiles, int* __restrict__ err) {
+              int kPer, const FxTile* __restrict__ tiles, int nTiles, int* __restrict__ err) {
   using C = FxCfg<BN, L, NA_, NB_>;
-  constexpr int NA = C::NA, NB = C::NB;
-  static_assert(EW % 4 == 0 && CB == 8 && BN % CB == 0, "epilogue warps / column batch");
+  constexpr int NA = C::NA, NB = C::NB, CB = 8;
+  static_assert(EW % 4 == 0 && BN % CB == 0, "epilogue warps / column batch");
   constexpr int NBAT = (BN / CB + EW / 4 - 1) / (EW / 4);  // column batches of one epilogue warp
+  constexpr uint32_t HALF = C::TMEM_COLS / 2;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* ringA = smem;
   uint8_t* ringB = smem + NA * C::A_BYTES;
-  __shared__ __align__(8) uint64_t aFull[NA], aEmpty[NA], bFull[NB], bEmpty[NB], accFull, accEmpty, finalBar;
+  __shared__ __align__(8) uint64_t aFull[NA], aEmpty[NA], bFull[NB], bEmpty[NB], accFull[2], accEmpty[2], finalBar;
   __shared__ uint32_t tmemSlot;
   __shared__ volatile int abortFlag;
   __shared__ int consumedA, consumedB, issuedA, issuedB;
@@ -151,8 +205,10 @@ __global__ void __launch_bounds__(32 * (EW + 2), NA_ > 0 ? 2 : 1)
       mbar_init(&bFull[s], 1);
       mbar_init(&bEmpty[s], 1);
     }
-    mbar_init(&accFull, 1);
-    mbar_init(&accEmpty, EW);
+    for (int s = 0; s < 2; s++) {
+      mbar_init(&accFull[s], 1);
+      mbar_init(&accEmpty[s], EW);
+    }
     mbar_init(&finalBar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -224,12 +280,14 @@ __global__ void __launch_bounds__(32 * (EW + 2), NA_ > 0 ? 2 : 1)
       // advance by address / 16: +2 per 16-wide K step, +8 per B row
       const uint64_t bdesc0 = sw128_desc(smem_u32(ringB));
       const uint64_t adesc0 = sw128_desc(smem_u32(ringA));
-      int ca = 0, cb = 0, ph = 0;  // ph: accumulator phases (tiles with K work)
-      for (int t = blockIdx.x; t < nTiles && !abortFlag; t += gridDim.x) {
+      int ca = 0, cb = 0, ph = 0;  // ph: accumulator phases (chunks)
+      bool prevNarrow = true, ok = true;
+      for (int t = blockIdx.x; t < nTiles && !abortFlag && ok; t += gridDim.x) {
         const FxTile tl = tiles[t];
         int M, N, kt0, nk;
         geometry(tl, M, N, kt0, nk);
         if (nk == 0) continue;  // the epilogue writes the empty split's zeros
+        const bool narrow = (uint32_t)(L * tl.nT) <= HALF;
         // A slice i covers (L - i) nT columns: one MMA up to 256 of them, else two halves
         uint32_t id0[L], id1[L], half[L];
 #pragma unroll
@@ -241,14 +299,20 @@ __global__ void __launch_bounds__(32 * (EW + 2), NA_ > 0 ? 2 : 1)
           id0[i] = base | ((uint32_t)(n0 >> 3) << 17);
           id1[i] = cols > n0 ? base | ((uint32_t)((cols - n0) >> 3) << 17) : 0u;
         }
-        if (ph > 0 && !mbar_wait(&accEmpty, (ph - 1) & 1, &abortFlag)) {  // the epilogue drained TMEM
-          abortFlag = 1;
-          atomicExch(err, 16);
-          break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        bool ok = true;
         for (int kb = 0; kb < nk && ok; kb++) {
+          const bool first = kb % FX_CHUNK == 0;
+          if (first) {  // a new phase: its half (or both) drained by the epilogue
+            if ((ph > 1 && !mbar_wait(&accEmpty[ph & 1], ((ph >> 1) - 1) & 1, &abortFlag)) ||
+                (ph > 0 && !(narrow && prevNarrow) &&
+                 !mbar_wait(&accEmpty[(ph - 1) & 1], ((ph - 1) >> 1) & 1, &abortFlag))) {
+              abortFlag = 1;
+              atomicExch(err, 16);
+              ok = false;
+              break;
+            }
+            prevNarrow = narrow;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          }
           const int sb = cb % NB, rb = cb / NB;
           if (!mbar_wait(&bFull[sb], rb & 1, &abortFlag)) {
             abortFlag = 1;
@@ -260,6 +324,7 @@ __global__ void __launch_bounds__(32 * (EW + 2), NA_ > 0 ? 2 : 1)
           consumedB = cb;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint64_t bd = bdesc0 + (uint64_t)((sb * C::BG_BYTES) >> 4);
+          const uint32_t tcol = tmem + (narrow && (ph & 1) ? HALF : 0u);
 #pragma unroll
           for (int i = 0; i < L; i++) {
             const int sa = ca % NA, ra = ca / NA;
@@ -273,28 +338,30 @@ __global__ void __launch_bounds__(32 * (EW + 2), NA_ > 0 ? 2 : 1)
             consumedA = ca;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint64_t ad = adesc0 + (uint64_t)((sa * C::A_BYTES) >> 4);
-            const uint32_t d0 = tmem + (uint32_t)(i * tl.nT), d1 = d0 + half[i];
+            const uint32_t d0 = tcol + (uint32_t)(i * tl.nT), d1 = d0 + half[i];
             const uint64_t bd1 = bd + 8 * half[i];
             if (id1[i]) {
               // both halves of a K step read the same 4 KB of A: the second from the collector
 #pragma unroll
               for (int k = 0; k < TC_BK / 16; k++) {
-                const uint32_t acc = (kb > 0 || i > 0 || k > 0) ? 1u : 0u;
+                const uint32_t acc = (!first || i > 0 || k > 0) ? 1u : 0u;
                 umma_bf16_coll(1, d0, ad + 2 * k, bd + 2 * k, id0[i], acc);
                 umma_bf16_coll(3, d1, ad + 2 * k, bd1 + 2 * k, id1[i], acc);
               }
             } else {
 #pragma unroll
               for (int k = 0; k < TC_BK / 16; k++)
-                umma_bf16(d0, ad + 2 * k, bd + 2 * k, id0[i], (kb > 0 || i > 0 || k > 0) ? 1u : 0u);
+                umma_bf16(d0, ad + 2 * k, bd + 2 * k, id0[i], (!first || i > 0 || k > 0) ? 1u : 0u);
             }
             umma_commit(&aEmpty[sa]);
           }
-          if (ok) umma_commit(&bEmpty[sb]);
+          if (!ok) break;
+          umma_commit(&bEmpty[sb]);
+          if (kb % FX_CHUNK == FX_CHUNK - 1 || kb == nk - 1) {
+            umma_commit(&accFull[ph & 1]);
+            ph++;
+          }
         }
-        if (!ok) break;
-        umma_commit(&accFull);
-        ph++;
       }
       umma_commit(&finalBar);  // arrives when every issued MMA has completed
     }
@@ -316,41 +383,55 @@ __global__ void __launch_bounds__(32 * (EW + 2), NA_ > 0 ? 2 : 1)
           for (int col = tl.n0; col < min(N, tl.n0 + tl.nT); col++) Oz[(size_t)row * N + col] = 0.0;
         continue;
       }
-      const bool waited = mbar_wait(&accFull, ph & 1, &abortFlag);
-      if (__any_sync(0xffffffffu, !waited)) {
+      const bool narrow = (uint32_t)(L * tl.nT) <= HALF;
+      FxAcc<L> T[NBAT][CB];  // the level sums of this warp's columns
+#pragma unroll
+      for (int bt = 0; bt < NBAT; bt++)
+#pragma unroll
+        for (int j = 0; j < CB; j++) T[bt][j].clear();
+      bool waited = true;
+      for (int k0 = 0; k0 < nk; k0 += FX_CHUNK) {
+        waited = mbar_wait(&accFull[ph & 1], (ph >> 1) & 1, &abortFlag);
+        if (__any_sync(0xffffffffu, !waited)) {
+          waited = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t tcol = tmem + ((uint32_t)(q * 32) << 16) + (narrow && (ph & 1) ? HALF : 0u);
+#pragma unroll
+        for (int bt = 0; bt < NBAT; bt++) {
+          const int c = (cg + bt * (EW / 4)) * CB;
+          if (c < tl.nT) {
+            // the levels of hi, then those of lo (registers for one group at a time)
+            constexpr int LH = FxAcc<L>::LH;
+            uint32_t d[LH][CB];
+#pragma unroll
+            for (int l = 0; l < LH; l++) TMEM_LD_X8(tcol + (uint32_t)(l * tl.nT + c), d[l]);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int j = 0; j < CB; j++) T[bt][j].add(d, j, 0, LH);
+            if constexpr (L > LH) {
+#pragma unroll
+              for (int l = LH; l < L; l++) TMEM_LD_X8(tcol + (uint32_t)(l * tl.nT + c), d[l - LH]);
+              asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+              for (int j = 0; j < CB; j++) T[bt][j].add(d, j, LH, L - LH);
+            }
+          }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&accEmpty[ph & 1]);
+        ph++;
+      }
+      if (!waited) {
         if (lane == 0) atomicExch(err, 15);
         break;
       }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      // the level sums of this warp's columns as 64-bit integers
-      long long Tv[NBAT][CB];
-#pragma unroll
-      for (int bt = 0; bt < NBAT; bt++) {
-        const int c = (cg + bt * (EW / 4)) * CB;
-        if (c < tl.nT) {
-          uint32_t acc[L][CB];
-#pragma unroll
-          for (int l = 0; l < L; l++)
-            TMEM_LD_X8(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(l * tl.nT + c), acc[l]);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-          for (int j = 0; j < CB; j++) {
-            long long v = 0;
-#pragma unroll
-            for (int l = 0; l < L; l++)
-              v = (long long)((unsigned long long)v << digitBits) + (long long)__float2int_rn(__uint_as_float(acc[l][j]));
-            Tv[bt][j] = v;
-          }
-        }
-      }
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&accEmpty);
-      ph++;
-      const TrajShape& T = shp[tl.traj];
-      const int* eA = aShared ? expA + T.vExp : batn(expA, bs, tl.traj);
+      const TrajShape& S = shp[tl.traj];
+      const int* eA = aShared ? expA + S.vExp : batn(expA, bs, tl.traj);
       const int* eB = batn(expB, bs, tl.traj);
-      const int ea = rowOk ? eA[row] - digitBits * (L + 1) : 0;
+      const int ea = rowOk ? eA[row] - 8 * (L + 1) : 0;
       unsigned rowMaxEx = 0;
 #pragma unroll
       for (int bt = 0; bt < NBAT; bt++) {
@@ -363,7 +444,9 @@ __global__ void __launch_bounds__(32 * (EW + 2), NA_ > 0 ? 2 : 1)
             unsigned ex = 0;
             v[j] = 0.0;
             if (rowOk && col < N) {
-              v[j] = ll_scaled(Tv[bt][j], ea + eB[col]);
+              const int e = ea + eB[col];
+              v[j] = T[bt][j].value(e);
+              if (e > FX_EXP_NAN / 2) v[j] = __longlong_as_double(0x7FF8000000000000LL);
               ex = (unsigned)(__double2hiint(v[j]) >> 20) & 0x7FFu;
             }
             if (maxCol) {
@@ -403,11 +486,12 @@ __global__ void __launch_bounds__(32 * (EW + 2), NA_ > 0 ? 2 : 1)
 template <int BN, int L, int NA_, int NB_>
 void launch_fx_t(cgpu_ctx* c, const CUtensorMap& ta, const CUtensorMap& tb, double* out, const int* expA,
                  const int* expB, unsigned* maxRow, unsigned* maxCol, int gemmId, int segPitchA, int segPitch,
-                 int aShared, int kPer, int digitBits, const FxTile* tiles, int nTiles, int ctasPerSm, int* err) {
+                 int aShared, int kPer, const FxTile* tiles, int nTiles, int ctasPerSm, int* err) {
   using C = FxCfg<BN, L, NA_, NB_>;
-  // eight epilogue warps (two per tensor-memory lane quarter)
-  constexpr int EW = 8, CB = 8;
-  auto kern = k_fx_gemm<BN, L, NA_, NB_, EW, CB>;
+  // eight epilogue warps (two per tensor-memory lane quarter); sixteen for L >
+  // 5, whose two 64-bit sums per output would not fit the registers of eight
+  constexpr int EW = L > 5 ? 16 : 8;
+  auto kern = k_fx_gemm<BN, L, NA_, NB_, EW>;
   static bool attr = false;
   if (!attr) {
     CODY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
@@ -416,31 +500,11 @@ void launch_fx_t(cgpu_ctx* c, const CUtensorMap& ta, const CUtensorMap& tb, doub
   if (nTiles <= 0) return;
   const int grid = std::min(nTiles, c->numSms * ctasPerSm);
   kern<<<grid, 32 * (EW + 2), C::SMEM, c->stream>>>(ta, tb, out, expA, expB, maxRow, maxCol, TRAJ_PASS(c), gemmId,
-                                                    segPitchA, segPitch, aShared, kPer, digitBits, tiles, nTiles, err);
+                                                    segPitchA, segPitch, aShared, kPer, tiles, nTiles, err);
   CODY_LAUNCHED(c);
 }
 
 }  // namespace
-
-// 64-wide K blocks per split within which the two leading level sums stay
-// exact in FP32: K <= 2^(24-2b).
-static int fx_exact_tiles(int b) { return (1 << (24 - 2 * b)) / TC_BK; }
-
-void fx_plan(int kTiles, int targetBits, int* digitBits, int* slices) {
-  // the widest digits whose exact range holds the whole contraction (an extra
-  // K split costs more in tile epilogues and partial sums than a slice)
-  int b = 8;
-  while (b > 6 && kTiles > fx_exact_tiles(b)) b--;
-  int L = (targetBits + b - 1) / b;
-  // |Horner sum| < K 2^(b(L+1)+1) <= 2^(25+b(L-1)) must stay inside int64
-  while (b > 6 && b * (L - 1) > 38) {
-    b--;
-    L = (targetBits + b - 1) / b;
-  }
-  if (L > 6 || b * (L - 1) > 38) throw std::string("fx_plan: no digit width carries the target bits");
-  *digitBits = b;
-  *slices = L;
-}
 
 // The instantiated N tiles (fx_gemm's cases): L accumulators of BN columns in
 // 512 (wide) or 256 (compact, two CTAs per SM) tensor-memory columns.
@@ -448,10 +512,10 @@ struct FxTileCfg {
   int bn, L;
   bool compact;
 };
-static const FxTileCfg kFxTiles[] = {
-    {32, 4, false}, {64, 4, false}, {80, 4, false}, {96, 4, false}, {128, 4, false}, {32, 5, false},
-    {64, 5, false}, {80, 5, false}, {96, 5, false}, {32, 6, false}, {64, 6, false},  {80, 6, false},
-    {32, 4, true},  {64, 4, true},  {32, 5, true},  {48, 5, true}};
+static const FxTileCfg kFxTiles[] = {{32, 4, false}, {64, 4, false}, {96, 4, false},
+                                     {32, 5, false}, {64, 5, false}, {80, 5, false}, {96, 5, false},
+                                     {32, 6, false}, {64, 6, false}, {64, 7, false}, {32, 4, true},  {64, 4, true},  {32, 5, true},
+                                     {48, 5, true}};
 
 static int fx_max_bn(int L, bool compact) {
   int m = 0;
@@ -474,10 +538,8 @@ bool fx_tile_supported(int bn, int L, bool compact) {
   return false;
 }
 
-int fx_min_splits(int kTiles, int digitBits) {
-  const int exact = fx_exact_tiles(digitBits);
-  return std::max(1, (kTiles + exact - 1) / exact);
-}
+// 512 chunks (K = 131072) keep the integer level sums inside 64 bits.
+int fx_min_splits(int kTiles) { return std::max(1, (kTiles + 512 * FX_CHUNK - 1) / (512 * FX_CHUNK)); }
 
 int fx_normalize_splits(int kTiles, int s) {
   s = std::max(1, std::min(s, kTiles));
@@ -496,14 +558,31 @@ int fx_tile_n(int N, int L, bool compact) {
   return best;
 }
 
-int fx_split_count(int M, int N, int BN, int kTiles, int nb, int digitBits) {
-  long tiles = (long)((M + TC_BM - 1) / TC_BM) * ((N + BN - 1) / BN) * nb;
-  int s = (int)std::max<long>(1, (152 + tiles - 1) / tiles);
-  s = std::min(s, std::max(1, kTiles / 2));
-  const int exact = fx_exact_tiles(digitBits);
-  s = std::max(s, (kTiles + exact - 1) / exact);  // every split inside the exact range of the level sums
-  int per = (kTiles + s - 1) / s;
-  return (kTiles + per - 1) / per;
+// K splits of one GEMM over the context's trajectories.  A batch of more tiles
+// than SMs takes none.  Otherwise the cheapest by this estimate in SM cycles:
+// waves of tiles, each its K blocks at the MMA rate (4 K steps of L (L + 1) / 2
+// slice products of N / 2 cycles) plus about 8000 to fill the pipeline, drain
+// and store; a split adds its FP64 partials, written and read at about 3 KB a
+// cycle, and (reduceExtra) a reduction kernel of about 6000.
+int fx_split_count(int M, int N, int BN, int L, int kTiles, int nb, bool reduceExtra) {
+  const int nt = (N + BN - 1) / BN, nT = ((N + nt - 1) / nt + 15) / 16 * 16;
+  const long tiles = (long)((M + TC_BM - 1) / TC_BM) * nt * nb;
+  const int lo = fx_min_splits(kTiles);
+  if (tiles >= 152) return fx_normalize_splits(kTiles, lo);
+  int best = lo;
+  double bestCost = 1e300;
+  for (int s = lo; s <= std::max(lo, kTiles / 2); s++) {
+    const int per = (kTiles + s - 1) / s;
+    if ((kTiles + per - 1) / per != s) continue;
+    const double wave = (double)((tiles * s + 151) / 152);
+    double cost = wave * (per * 2.0 * L * (L + 1) / 2 * nT * 1.2 + 8000.0);
+    if (s > 1) cost += (reduceExtra ? 6000.0 : 0.0) + 16.0 * s * M * N * nb / 3000.0;
+    if (cost < bestCost) {
+      bestCost = cost;
+      best = s;
+    }
+  }
+  return fx_normalize_splits(kTiles, best);
 }
 
 // The columns of a trajectory go to ceil(N / bn) tiles of equal width (to 16
@@ -545,27 +624,24 @@ void* fx_build_tiles(cgpu_ctx* c, int gemmId, int bn, int nSplit, int* nTiles) {
   return d;
 }
 
-void fx_gemm(cgpu_ctx* c, int L, int digitBits, bool compact, int gemmId, const CUtensorMap& ta,
-             const CUtensorMap& tb, int bn, double* out, const int* expA, const int* expB, unsigned* maxRow,
-             unsigned* maxCol, int segPitchA, int segPitch, int aShared, int nSplit, const void* tiles, int nTiles,
-             int* err) {
+void fx_gemm(cgpu_ctx* c, int L, bool compact, int gemmId, const CUtensorMap& ta, const CUtensorMap& tb, int bn,
+             double* out, const int* expA, const int* expB, unsigned* maxRow, unsigned* maxCol, int segPitchA,
+             int segPitch, int aShared, int nSplit, const void* tiles, int nTiles, int* err) {
   if (segPitch % TC_BK != 0 || segPitchA % TC_BK != 0)
     throw std::string("fx_gemm: segment pitch must be a multiple of 64");
   if (nSplit > 1 && (maxRow || maxCol)) throw std::string("fx_gemm: output maxima need an unsplit K");
   const int kTiles = segPitch / TC_BK, kPer = (kTiles + nSplit - 1) / nSplit;  // K blocks per split
-  if (digitBits < 6 || digitBits > 8 || digitBits * (L - 1) > 38) throw std::string("fx_gemm: digit width");
-  if (kPer > fx_exact_tiles(digitBits)) throw std::string("fx_gemm: K split beyond the exact range of the digits");
+  if (nSplit < fx_min_splits(kTiles)) throw std::string("fx_gemm: K split beyond the range of the level sums");
   const FxTile* tl = (const FxTile*)tiles;
 #define FX_CASE(BN_, L_, NA_, NB_, CMP_)                                                                        \
   if (bn == BN_ && L == L_ && compact == CMP_) {                                                                \
     launch_fx_t<BN_, L_, NA_, NB_>(c, ta, tb, out, expA, expB, maxRow, maxCol, gemmId, segPitchA, segPitch,    \
-                                   aShared, kPer, digitBits, tl, nTiles, CMP_ ? 2 : 1, err);                   \
+                                   aShared, kPer, tl, nTiles, CMP_ ? 2 : 1, err);                              \
     return;                                                                                                     \
   }
-  FX_CASE(32, 4, 0, 2, false) FX_CASE(64, 4, 0, 2, false) FX_CASE(80, 4, 0, 2, false) FX_CASE(96, 4, 0, 2, false)
-  FX_CASE(128, 4, 0, 2, false)
+  FX_CASE(32, 4, 0, 2, false) FX_CASE(64, 4, 0, 2, false) FX_CASE(96, 4, 0, 2, false)
   FX_CASE(32, 5, 0, 2, false) FX_CASE(64, 5, 0, 2, false) FX_CASE(80, 5, 0, 2, false) FX_CASE(96, 5, 0, 2, false)
-  FX_CASE(32, 6, 0, 2, false) FX_CASE(64, 6, 0, 2, false) FX_CASE(80, 6, 0, 2, false)
+  FX_CASE(32, 6, 0, 2, false) FX_CASE(64, 6, 0, 2, false) FX_CASE(64, 7, 0, 2, false)
   FX_CASE(32, 4, 4, 1, true) FX_CASE(64, 4, 4, 1, true)
   FX_CASE(32, 5, 5, 1, true) FX_CASE(48, 5, 5, 1, true)
 #undef FX_CASE

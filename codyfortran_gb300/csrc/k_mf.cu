@@ -1,4 +1,8 @@
-// k_mf.cu -- interaction and mean-field kernels (FP64 form).
+// k_mf.cu -- interaction and mean-field kernels on the FP64 pipe.
+//
+// They serve the bf16x3 / bf16x6 forms' FillH2 and FP64 contexts whose digit
+// planes would not fit the device memory; the other FP64 contexts run the same
+// contractions on the tensor cores (k_mixed.cu, cgpu_ctx::fxOn).
 //
 // The reference loops over unordered orbital pairs and, per pair, runs an
 // O(nG^2) convolution, multiplies the potential onto every orbital and
@@ -560,6 +564,7 @@ void zgemm(cgpu_ctx* c, int mode, const z_t* A, const z_t* B, z_t* C, double sca
 }  // namespace
 
 size_t zgemm_partial_need(const cgpu_ctx* c) {
+  if (c->fxOn) return 0;
   int Q = c->nOS * c->nOS;
   size_t need = 0;
   // ZG_H2 always goes through the partial buffer (scale 1/2); ZG_Z only when split
@@ -628,6 +633,7 @@ void launch_rdm_inverse(cgpu_ctx* c) {
 // ApplyCorrelationOp: dOrbs += contraction; h2 (nO^4) filled when wantH2.
 // Requires rdm1_d / rdm2_d to hold the current RDMs.
 void launch_correlation(cgpu_ctx* c, z_t* dOrbs, const z_t* orbs, int wantH2) {
+  if (c->fxOn) return launch_correlation_mixed(c, dOrbs, orbs, wantH2);
   launch_rdm_inverse(c);
   if (!c->hasInteraction) {
     if (wantH2) {
@@ -655,6 +661,7 @@ void launch_fill_h2(cgpu_ctx* c, const z_t* orbs) {
     batch_zero(c, c->h2_d, sizeof(z_t) * (size_t)c->nO * c->nO * c->nO * c->nO);
     return;
   }
+  if (c->fxOn) return launch_fill_h2_fx(c, orbs);
   launch_pair_potentials(c, orbs);
   expand_pairs(c, orbs, 1);
   h2_from_pairs(c);

@@ -15,16 +15,14 @@
 //   W_p = a_p + i b_p,  X_p = R1 + R2,  Y_p = i (R1 - R2),
 //   R1 = R'[(l,k), q], R2 = R'[(k,l), q] (0 when l = k).
 //
-// The fixed-point form (precision mixed_fx / mixed_fx6) carries every operand
-// row as L base-2^b digit slices under one power of two per row (k_fx.cu) and
-// returns FP64 results whose only error is the operand truncation (at least
-// 30 / 36 bits of each row's maximum): S and V rows for GEMM1, W rows for
-// GEMM2, R'' rows, W columns for GEMM3.  fx_plan picks the digit width b of
-// each contraction length (GEMM1/3: K = nG, GEMM2: K = 2P) and the slice
-// count L = ceil(bits / b).  S carries LS = max(L1, L3) slices: GEMM1 reads
-// the first L1 (dropping balanced digits costs at most half a unit of the
-// last digit kept), GEMM3 L3.  The row exponents of W come from the GEMM1
-// epilogue, or from the reduction of its K splits.
+// The fixed-point forms (FP64, mixed_fx, mixed_fx6) carry every operand row as L
+// base-256 digit slices under one power of two per row (k_fx.cu) and return
+// FP64 results whose only error is the operand truncation (fx_slices: at least 55
+// / 31 / 39 bits of each row's maximum): S and V rows for GEMM1, W rows and R''
+// rows for GEMM2, W columns for GEMM3.  FillH2 (energies) runs GEMM1 and GEMM3 with the
+// seven slices of the FP64 form in all three.  The row exponents of W come from
+// the GEMM1 epilogue, or from the reduction of its K splits.  The bf16x3 /
+// bf16x6 forms keep their own operands (k_tc.cu) and the FP64 pipe's FillH2.
 #include <cuda_bf16.h>
 
 #include <array>
@@ -34,27 +32,34 @@
 #include "common.cuh"
 #include "tc.cuh"
 
+constexpr int FX_L64 = 7;  // slices of the FP64 form (55 bits of each row's maximum)
+
+// One fixed-point GEMM: N-tile width, two-CTAs-per-SM configuration, K splits, its tile list.
+struct FxGemm {
+  int bn = 64, s = 1, nTiles = 0;
+  bool compact = false;
+  void* tiles = nullptr;
+};
+
 struct MixedBufs {
   int terms = 3;            // 3: bf16x3, 6: bf16x6
   int KgMax = 0, KpMax = 0; // segment pitches: the largest padded K of the grid / pair contractions
-  int bn1 = 64, bn2 = 64, bn3 = 64;
-  int s1 = 1, s2 = 1, s3 = 1;  // K splits of the three GEMMs
+  int bn1 = 64, bn2 = 64, bn3 = 64;  // bf16x3 / bf16x6
+  int s1 = 1, s2 = 1, s3 = 1;        // K splits of the three GEMMs (bf16x3 / bf16x6)
   __nv_bfloat16 *VxB = nullptr, *SxA = nullptr, *WxA = nullptr, *WTxB = nullptr, *RxB = nullptr;
   float *P1 = nullptr, *P2 = nullptr, *P3 = nullptr;
-  int* err = nullptr;
+  int* err = nullptr;       // GEMM error flag: page-locked host memory, and its device address
+  volatile int* err_h = nullptr;
   double* Zd = nullptr;     // (nG, Q) complex
   CUtensorMap mV, mS, mSasB, mW, mWT, mR;  // TMA maps (A operands box 128 rows, B operands box BN rows)
-  // fixed-point form (fxBits > 0): digit width / slices of the K = nG
-  // contractions (GEMM1, GEMM3) and of the K = 2P one (GEMM2)
-  int fxBits = 0, b1 = 0, L1 = 0, b2 = 0, L2 = 0;
-  int fxBits3 = 0, L3 = 0, LS = 0;  // GEMM3 target and slices; S carries LS = max(L1, L3) slices
-  bool compact1 = false, compact2 = false, compact3 = false;  // two-CTAs-per-SM configuration per GEMM
-  int sCap1 = 1, sCap2 = 1, sCap3 = 1;  // K splits the FP64 partial buffers hold (the tuner stays within them)
-  // one interaction matrix per root grid (cgpu_ctx::fxShared): slices [root][c->nG][L1 KgBig]
+  // fixed-point forms (L > 0): digit slices of GEMM1 / GEMM3 and of GEMM2 (L2); V
+  // carries FX_L64 slices of which a GEMM reads the first L
+  int L = 0, L2 = 0;
+  FxGemm gW, gZ, gH, gWx, gHx;      // the form's three GEMMs; W and h2 at FX_L64 slices for FillH2
+  int sCapW = 1, sCapZ = 1, sCapH = 1;  // K splits the FP64 partial buffers hold (the tuner stays within them)
+  CUtensorMap mSx, mSxasB, mWTx;    // S and W^T rows at FX_L64 slices
+  // one interaction matrix per root grid (cgpu_ctx::fxShared): slices [root][c->nG][FX_L64 KgBig]
   // and row exponents [root][c->nG], outside the per-trajectory arena
-  // tile lists of the persistent fixed-point GEMMs (device) and their lengths
-  void *tiles1 = nullptr, *tiles2 = nullptr, *tiles3 = nullptr;
-  int nTiles1 = 0, nTiles2 = 0, nTiles3 = 0;
   int KgBig = 0;
   __nv_bfloat16* Vsh = nullptr;
   int* eVsh = nullptr;
@@ -301,86 +306,73 @@ __global__ void k_reduce_H2(z_t* __restrict__ H2s, const PT* __restrict__ P3, in
 
 // ---- fixed-point digit slices -------------------------------------------------
 
-constexpr int FX_LMAX = 8;
+// Slices of the contractions over the grid (L) and over the pairs (L2).  The
+// mixed forms' targets are 30 and 36 bits of the row maxima; at a contraction
+// length of at most 1024 they held 35 and 42 with the 7-bit digits they used to
+// have there (up to 256: 32 and 40), which five or six 8-bit slices keep.
+void fx_slices(int precision, int kTiles, int pTiles, int* L, int* L2) {
+  if (precision == CGPU_PREC_FP64) {
+    *L = *L2 = FX_L64;
+  } else {
+    const int x6 = precision == CGPU_PREC_MIXED_FX6 ? 1 : 0;
+    *L = x6 && kTiles <= 16 ? 6 : 5;
+    *L2 = (pTiles <= 4 ? 4 : 5) + x6;
+  }
+}
 
-// Signed base-2^b digits of x relative to 2^e (|x| < 2^e): X = round(x 2^(bL-e))
-// = sum_i d_i 2^(b(L-1-i)), d_i in [-2^(b-1), 2^(b-1)) for i > 0, |d_0| <= 2^b.
-// Integer operations only (bL <= 52; 32-bit arithmetic when bL <= 30).  With
-// H = 2^(b-1) sum_{k<L-1} 2^(bk), the digits of Y = X + H below the top one
-// are the plain base-2^b digits d_i + 2^(b-1), so every digit is an
-// independent bit field of Y: d_i = field_i(Y) - 2^(b-1), d_0 = Y >> b(L-1)
-// (arithmetic shift).  The balanced representation is unique, so this gives
-// the digits of the carry-by-carry division.
-// BT / LT > 0 fix the digit width / slice count at compile time (constant
-// shifts); 0 takes them from bRt / LRt.
-template <int BT, int LT>
-__device__ __forceinline__ void fx_digits_t(double x, int e, int bRt, int LRt, int (&d)[FX_LMAX]) {
-  const int b = BT > 0 ? BT : bRt, L = LT > 0 ? LT : LRt;
+// Signed base-256 digits of x relative to 2^e (|x| < 2^(e-1), or < 2^e for L < 7): X = round(x 2^(8L-e))
+// = sum_i d_i 2^(8(L-1-i)), d_i in [-128, 128) for i > 0, |d_0| <= 128.
+// Integer operations only.  With H = 128 sum_{k<L-1} 256^k, the digits of Y = X + H
+// below the top one are the plain base-256 digits d_i + 128, so every digit is an
+// independent byte of Y: d_i = byte_i(Y) - 128, d_0 = Y >> 8(L-1) (arithmetic shift).
+// FP64 subnormals (below 2^-1022 of anything) count as zero.
+template <int L>
+__device__ __forceinline__ void fx_digits(double x, int e, int (&d)[L]) {
   const unsigned long long u = (unsigned long long)__double_as_longlong(x);
   const int ex = (int)((u >> 52) & 0x7FF);
   long long X = 0;
   if (ex != 0) {
     const unsigned long long mant = (u & 0xFFFFFFFFFFFFFull) | (1ull << 52);
-    const int sh = 1075 - ex - b * L + e;  // >= 53 - bL > 0 because |x| < 2^e
-    if (sh < 63) X = (long long)((mant + (1ull << (sh - 1))) >> sh);
+    const int sh = 1075 - ex - 8 * L + e;  // >= 54 - 8L because |x| < 2^(e-1) (53 - 8L: < 2^e)
+    if (8 * L > 53 && sh <= 0) X = (long long)(mant << -sh);
+    else if (sh < 63) X = (long long)((mant + (1ull << (sh - 1))) >> sh);
     if (u >> 63) X = -X;
   }
-  const int mask = (1 << b) - 1, half = 1 << (b - 1);
-  if (b * L <= 30) {  // |X| <= 2^30, H < 2^30
-    int H = 0;
-#pragma unroll
-    for (int i = 1; i < FX_LMAX; i++)
-      if (i < L) H = (H << b) | half;
-    const int Y = (int)X + H;
-#pragma unroll
-    for (int i = 1; i < FX_LMAX; i++)
-      if (i < L) d[i] = ((int)((unsigned)Y >> (b * (L - 1 - i))) & mask) - half;
-    d[0] = Y >> (b * (L - 1));
-    return;
-  }
-  long long H = 0;
-#pragma unroll
-  for (int i = 1; i < FX_LMAX; i++)
-    if (i < L) H = (H << b) | half;
+  constexpr long long H = [] {
+    long long h = 0;
+    for (int i = 1; i < L; i++) h = (h << 8) | 128;
+    return h;
+  }();
   const long long Y = X + H;
 #pragma unroll
-  for (int i = 1; i < FX_LMAX; i++)
-    if (i < L) d[i] = ((int)((unsigned long long)Y >> (b * (L - 1 - i))) & mask) - half;
-  d[0] = (int)(Y >> (b * (L - 1)));
+  for (int i = 1; i < L; i++) d[i] = (int)((unsigned long long)Y >> (8 * (L - 1 - i)) & 255) - 128;
+  d[0] = (int)(Y >> (8 * (L - 1)));
 }
 
-// bf16 of an integer |d| <= 256 without a conversion instruction: the FP32
-// magic-number sum 1.5 2^23 + d is exact, subtracting 1.5 2^23 leaves d as an
-// FP32 with at most 9 significant bits, whose upper half is its bf16.
-__device__ __forceinline__ __nv_bfloat16 fx_bf16(int d) {
-  const float f = __int_as_float(0x4B400000 + d) - 12582912.0f;
-  return __ushort_as_bfloat16((unsigned short)(__float_as_uint(f) >> 16));
+// Two integers |d| <= 128 as a bf16 pair without conversion instructions: the
+// FP32 magic-number sum 1.5 2^23 + d is exact, subtracting 1.5 2^23 leaves d as an
+// FP32 with at most 8 significant bits, whose upper half is its bf16.
+__device__ __forceinline__ unsigned fx_bf16x2(int d0, int d1) {
+  const float f0 = __int_as_float(0x4B400000 + d0) - 12582912.0f, f1 = __int_as_float(0x4B400000 + d1) - 12582912.0f;
+  return __byte_perm(__float_as_uint(f0), __float_as_uint(f1), 0x7632);
 }
 
 __device__ __forceinline__ unsigned fx_biased_exp(double v) { return (unsigned)(__double2hiint(v) >> 20) & 0x7FFu; }
-// smallest e with |x| < 2^e for the largest biased exponent m of a row (0: all zero)
-__device__ __forceinline__ int fx_exp(unsigned m) { return m ? (int)m - 1022 : 0; }
-
-__device__ __forceinline__ void fx_digits(double x, int e, int b, int L, int (&d)[FX_LMAX]) {
-  fx_digits_t<0, 0>(x, e, b, L, d);
+// smallest e with |x| < 2^(e-1) (wide: < 2^e) for the largest biased exponent m
+// of a row (0: all zero; 2047: infinity or NaN).  wide is for the pair
+// contractions of the mixed forms (K <= 256: |d_0| <= 256 stays exact).
+__device__ __forceinline__ int fx_exp(unsigned m, bool wide = false) {
+  return m == 0 ? 0 : m == 2047u ? FX_EXP_NAN : (int)m - (wide ? 1022 : 1021);
 }
 
-template <int BT, int LT>
-__device__ __forceinline__ void fx_store_t(__nv_bfloat16* rowBase, size_t pitch, int k, bool valid, double v, int e,
-                                           int bRt, int LRt) {
-  const int L = LT > 0 ? LT : LRt;
-  int d[FX_LMAX];
+// Columns k, k + 1 (k even) of a row's L digit planes, zeros where not valid.
+template <int L>
+__device__ __forceinline__ void fx_store2(__nv_bfloat16* rowBase, size_t pitch, int k, double v0, double v1, int e) {
+  int d0[L], d1[L];
+  fx_digits<L>(v0, e, d0);
+  fx_digits<L>(v1, e, d1);
 #pragma unroll
-  for (int l = 0; l < FX_LMAX; l++) d[l] = 0;
-  if (valid) fx_digits_t<BT, LT>(v, e, bRt, LRt, d);
-#pragma unroll
-  for (int l = 0; l < FX_LMAX; l++)
-    if (l < L) rowBase[(size_t)l * pitch + k] = fx_bf16(d[l]);
-}
-
-__device__ __forceinline__ void fx_store(__nv_bfloat16* rowBase, size_t pitch, int k, bool valid, double v, int e,
-                                         int b, int L) {
-  fx_store_t<0, 0>(rowBase, pitch, k, valid, v, e, b, L);
+  for (int l = 0; l < L; l++) *reinterpret_cast<unsigned*>(rowBase + (size_t)l * pitch + k) = fx_bf16x2(d0[l], d1[l]);
 }
 
 __device__ unsigned fx_block_max(unsigned m) {
@@ -396,31 +388,28 @@ __device__ unsigned fx_block_max(unsigned m) {
   return r;
 }
 
-// One block per row: the row's values in dynamic shared memory, the exponent
-// of its maximum, then the L digit planes: value k at column shift + k, zero
-// elsewhere in [0, Kpad).
-template <int BT = 0, int LT = 0, class F>
-__device__ void fx_row(__nv_bfloat16* rowBase, int* expOut, int K, int Kpad, int pitch, int b, int L, int shift,
-                       F value) {
+// One block per row of K values: the exponent of its maximum, then the L digit
+// planes, zero in [K, Kpad).  The values are staged in dynamic shared memory
+// when `staged`, else formed twice (rows longer than shared memory).
+template <int L, class F>
+__device__ void fx_row(__nv_bfloat16* rowBase, int* expOut, int K, int Kpad, int pitch, int staged, bool wide, F value) {
   extern __shared__ double fxbuf[];
   unsigned m = 0;
   for (int k = threadIdx.x; k < K; k += blockDim.x) {
     const double v = value(k);
-    fxbuf[k] = v;
+    if (staged) fxbuf[k] = v;
     m = max(m, fx_biased_exp(v));
   }
-  const int e = fx_exp(fx_block_max(m));
+  const int e = fx_exp(fx_block_max(m), wide);
   if (threadIdx.x == 0) *expOut = e;
-  for (int k = threadIdx.x; k < Kpad; k += blockDim.x) {
-    const int src = k - shift;
-    const bool valid = src >= 0 && src < K;
-    fx_store_t<BT, LT>(rowBase, pitch, k, valid, valid ? fxbuf[src] : 0.0, e, b, L);
-  }
+  auto at = [&](int k) { return k < K ? (staged ? fxbuf[k] : value(k)) : 0.0; };
+  for (int k = 2 * threadIdx.x; k < Kpad; k += 2 * blockDim.x) fx_store2<L>(rowBase, pitch, k, at(k), at(k + 1), e);
 }
 
+constexpr size_t FX_STAGE_MAX = 200 * 1024;  // shared memory for staged rows; longer rows are formed twice
+
 __global__ void __launch_bounds__(256) k_fx_split_V(__nv_bfloat16* __restrict__ out, int* __restrict__ eV,
-                                                     const double* __restrict__ V, int pitch, int b, int L,
-                                                     TRAJ_ARGS) {
+                                                     const double* __restrict__ V, int pitch, TRAJ_ARGS) {
   const TrajShape& T = shp[blockIdx.z];
   const int g = blockIdx.x, nG = T.nG;
   if (g >= nG) return;
@@ -428,21 +417,23 @@ __global__ void __launch_bounds__(256) k_fx_split_V(__nv_bfloat16* __restrict__ 
   eV = bat(eV, bs);
   V = bat(V, bs);
   const double* row = V + (size_t)g * nG;
-  fx_row(out + (size_t)g * L * pitch, eV + g, nG, T.Kg, pitch, b, L, 0, [&](int k) { return row[k]; });
+  fx_row<FX_L64>(out + (size_t)g * FX_L64 * pitch, eV + g, nG, (nG + 63) / 64 * 64, pitch, 0, false,
+                 [&](int k) { return row[k]; });
 }
 
 // Rows 2p (real part) and 2p + 1 (imaginary part) of S = conj(phi_l) phi_k w
-// over the grid (p = (l, k)), one block per pair: the complex product and the
-// weight in double-float arithmetic (FP32 pipe; ~2^-44 relative, far below the
-// digits' 2^-36 of the row maximum), both rows staged in shared memory, each
-// with the exponent of its own maximum.  Block 0 of a trajectory also clears
-// the W exponent maxima for GEMM1.
-template <int BT, int LT>
+// over the grid (p = (l, k)), one block per pair, both rows staged in shared
+// memory, each with the exponent of its own maximum.  In the mixed forms the
+// complex product and the weight are double-float (FP32 pipe; ~2^-44 relative,
+// below the digits' 2^-31 / 2^-39 of the row maximum); with FX_L64 slices they
+// are FP64, rounded as FillInteractionSrc rounds them.  Block 0 of a trajectory
+// also clears the W exponent maxima for GEMM1.
+template <int L>
 __global__ void __launch_bounds__(256) k_fx_split_S(__nv_bfloat16* __restrict__ out, int* __restrict__ eS,
                                                      unsigned* __restrict__ mWr, unsigned* __restrict__ mWc,
                                                      const z_t* __restrict__ orbs, const double* __restrict__ w,
                                                      const int* __restrict__ pl, const int* __restrict__ pk, int pitch,
-                                                     int b, int L, TRAJ_ARGS) {
+                                                     int staged, TRAJ_ARGS) {
   const TrajShape& T = shp[blockIdx.z];
   const int p = blockIdx.x, nG = T.nG, nP = T.nPairs;
   if (p >= nP) return;
@@ -461,9 +452,9 @@ __global__ void __launch_bounds__(256) k_fx_split_S(__nv_bfloat16* __restrict__ 
   extern __shared__ double fxbuf[];  // [2][pitch]: the real and the imaginary row
   const z_t* a = orbs + (size_t)nG * pl[p];
   const z_t* bo = orbs + (size_t)nG * pk[p];
-  unsigned mr = 0, mi = 0;
-  for (int g = threadIdx.x; g < nG; g += blockDim.x) {
+  auto value = [&](int g) -> z_t {
     const z_t av = a[g], bv = bo[g];
+    if (L == FX_L64) return zscale(zcmul(av, bv), w[g]);
     const float2 ar = df_split(av.x), ai = df_split(av.y), br = df_split(bv.x), bi = df_split(bv.y);
     const float2 wg = df_split(w[g]);
     // conj(a) b = (ar br + ai bi) + i (ar bi - ai br)
@@ -472,11 +463,17 @@ __global__ void __launch_bounds__(256) k_fx_split_S(__nv_bfloat16* __restrict__ 
     float s0 = 0.0f, c0 = 0.0f, s1 = 0.0f, c1 = 0.0f;
     df_mul_acc(s0, c0, re.x, re.y, wg.x, wg.y);
     df_mul_acc(s1, c1, im.x, im.y, wg.x, wg.y);
-    const double vr = df_to_d(make_float2(s0, c0)), vi = df_to_d(make_float2(s1, c1));
-    fxbuf[g] = vr;
-    fxbuf[pitch + g] = vi;
-    mr = max(mr, fx_biased_exp(vr));
-    mi = max(mi, fx_biased_exp(vi));
+    return zmk(df_to_d(make_float2(s0, c0)), df_to_d(make_float2(s1, c1)));
+  };
+  unsigned mr = 0, mi = 0;
+  for (int g = threadIdx.x; g < nG; g += blockDim.x) {
+    const z_t v = value(g);
+    if (staged) {
+      fxbuf[g] = v.x;
+      fxbuf[pitch + g] = v.y;
+    }
+    mr = max(mr, fx_biased_exp(v.x));
+    mi = max(mi, fx_biased_exp(v.y));
   }
   const int er = fx_exp(fx_block_max(mr));
   const int ei = fx_exp(fx_block_max(mi));
@@ -487,19 +484,21 @@ __global__ void __launch_bounds__(256) k_fx_split_S(__nv_bfloat16* __restrict__ 
   __nv_bfloat16* rowR = out + (size_t)(2 * p) * L * pitch;
   __nv_bfloat16* rowI = out + (size_t)(2 * p + 1) * L * pitch;
   const int Kpad = T.Kg, shift = T.gShift;
-  for (int k = threadIdx.x; k < Kpad; k += blockDim.x) {
-    const int src = k - shift;
-    const bool valid = src >= 0 && src < nG;
-    fx_store_t<BT, LT>(rowR, pitch, k, valid, valid ? fxbuf[src] : 0.0, er, b, L);
-    fx_store_t<BT, LT>(rowI, pitch, k, valid, valid ? fxbuf[pitch + src] : 0.0, ei, b, L);
+  auto at = [&](int g) -> z_t {
+    if (g < 0 || g >= nG) return zmk(0.0, 0.0);
+    return staged ? zmk(fxbuf[g], fxbuf[pitch + g]) : value(g);
+  };
+  for (int k = 2 * threadIdx.x; k < Kpad; k += 2 * blockDim.x) {
+    const z_t v0 = at(k - shift), v1 = at(k + 1 - shift);
+    fx_store2<L>(rowR, pitch, k, v0.x, v1.x, er);
+    fx_store2<L>(rowI, pitch, k, v0.y, v1.y, ei);
   }
 }
 
 // Row n = 2q + s of R'' (K = 2p + t), as k_split_R.
-template <int BT, int LT>
+template <int L>
 __global__ void k_fx_split_R(__nv_bfloat16* __restrict__ out, int* __restrict__ eR, const z_t* __restrict__ Rp,
-                             const int* __restrict__ pl, const int* __restrict__ pk, int pitch, int b, int L,
-                             TRAJ_ARGS) {
+                             const int* __restrict__ pl, const int* __restrict__ pk, int pitch, TRAJ_ARGS) {
   const TrajShape& T = shp[blockIdx.z];
   const int n = T.nOS, nP = T.nPairs, Q = n * n;
   const int row = blockIdx.x;
@@ -510,7 +509,7 @@ __global__ void k_fx_split_R(__nv_bfloat16* __restrict__ out, int* __restrict__ 
   pl = bat(pl, bs);
   pk = bat(pk, bs);
   const int q = row >> 1, s = row & 1;
-  fx_row<BT, LT>(out + (size_t)row * L * pitch, eR + row, 2 * nP, T.Kp, pitch, b, L, 0, [&](int k) {
+  fx_row<L>(out + (size_t)row * L * pitch, eR + row, 2 * nP, T.Kp, pitch, 1, L < FX_L64, [&](int k) {
     const int p = k >> 1, t = k & 1;
     const int l = pl[p], kk = pk[p];
     const z_t R1 = Rp[(size_t)(l * n + kk) * Q + q];
@@ -522,7 +521,9 @@ __global__ void k_fx_split_R(__nv_bfloat16* __restrict__ out, int* __restrict__ 
 }
 
 // W = sum of the K-split partials (into slot 0) and the exponent maxima of its
-// rows and columns (used when GEMM1 ran with split K).
+// rows and columns (used when GEMM1 ran with split K).  A maximum is read before
+// it is raised: almost every entry is below it, and an atomic each would queue
+// the whole matrix on 2P + nG words.
 __global__ void k_fx_reduce_W(double* __restrict__ Wd, unsigned* __restrict__ mWr, unsigned* __restrict__ mWc,
                               int nSplit, TRAJ_ARGS) {
   const TrajShape& T = shp[blockIdx.z];
@@ -536,30 +537,29 @@ __global__ void k_fx_reduce_W(double* __restrict__ Wd, unsigned* __restrict__ mW
     for (int z = 0; z < nSplit; z++) v += Wd[(size_t)z * tot + e];
     Wd[e] = v;
     const unsigned ex = fx_biased_exp(v);
-    if (ex) {
-      atomicMax(mWr + e / N, ex);
-      atomicMax(mWc + e % N, ex);
-    }
+    unsigned *r = mWr + e / N, *q = mWc + e % N;
+    if (ex > *(volatile unsigned*)r) atomicMax(r, ex);
+    if (ex > *(volatile unsigned*)q) atomicMax(q, ex);
   }
 }
 
-// W (FP64 [nG][2P]) to WxA (rows g, K = 2P: b2/L2 digits) and WTxB (rows n,
-// K = nG at columns gShift + g: b1/L3 digits) planes, with the row exponents
-// eWr[g] / eWc[n].  One block per 32-row strip of W, walking the trajectory's
-// own K = 2P columns in 32 x 32 tiles transposed through shared memory.
-// B1/L3T, B2/L2T > 0: the digit plans fixed at compile time (0: run-time b1, L3, b2, L2).
-template <int B1, int L3T, int B2, int L2T>
+// W (FP64 [nG][2P]) to WxA (rows g, K = 2P, L2 digits; null: not wanted) and WTxB
+// (rows n, K = nG at columns gShift + g, L digits) planes, with the row
+// exponents eWr[g] / eWc[n].  One block per 64 x 64 tile (columns of WTxB by
+// columns of W), transposed through shared memory; a lane forms two adjacent
+// columns of a plane, so that the digits leave as 128-byte rows.
+constexpr int FW_T = 64;
+template <int L, int L2>
 __global__ void __launch_bounds__(256) k_fx_split_W(__nv_bfloat16* __restrict__ WxA, __nv_bfloat16* __restrict__ WTxB,
                                                      int* __restrict__ eWr, int* __restrict__ eWc,
                                                      const double* __restrict__ Wd, const unsigned* __restrict__ mWr,
-                                                     const unsigned* __restrict__ mWc, int pitchP, int pitchG, int b1,
-                                                     int L3rt, int b2, int L2rt, TRAJ_ARGS) {
-  const int L3 = L3T > 0 ? L3T : L3rt, L2 = L2T > 0 ? L2T : L2rt;
-  __shared__ double tile[SW_T][SW_T + 1];
+                                                     const unsigned* __restrict__ mWc, int pitchP, int pitchG,
+                                                     TRAJ_ARGS) {
+  __shared__ double tile[FW_T][FW_T + 1];
   const TrajShape& T = shp[blockIdx.z];
-  const int nG = T.nG, N2P = 2 * T.nPairs, KpP = T.Kp, KpG = T.Kg;
-  const int g0 = blockIdx.x * SW_T;
-  if (g0 >= KpG) return;
+  const int nG = T.nG, N2P = 2 * T.nPairs, KpP = T.Kp, KpG = T.Kg, sh = T.gShift;
+  const int c0 = blockIdx.x * FW_T, n0 = blockIdx.y * FW_T;
+  if (c0 >= KpG || n0 >= KpP) return;
   WxA = bat(WxA, bs);
   WTxB = bat(WTxB, bs);
   eWr = bat(eWr, bs);
@@ -567,33 +567,26 @@ __global__ void __launch_bounds__(256) k_fx_split_W(__nv_bfloat16* __restrict__ 
   Wd = bat(Wd, bs);
   mWr = bat(mWr, bs);
   mWc = bat(mWc, bs);
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
-  const int sh = T.gShift;
-  for (int n0 = 0; n0 < KpP; n0 += SW_T) {
-    if (n0 > 0) __syncthreads();  // the previous tile has been read
-    for (int r = ty; r < SW_T; r += 8) {
-      const int g = g0 + r, n = n0 + tx;
-      const bool valid = g < nG && n < N2P;
-      const double v = valid ? Wd[(size_t)g * N2P + n] : 0.0;
-      tile[r][tx] = v;
-      if (g < nG) {
-        const int e = fx_exp(mWr[g]);
-        if (n == 0) eWr[g] = e;
-        fx_store_t<B2, L2T>(WxA + (size_t)g * L2 * pitchP, pitchP, n, valid, v, e, b2, L2);
-      }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int i = threadIdx.x; i < FW_T * FW_T; i += 256) {
+    const int r = i / FW_T, c = i % FW_T, g = c0 + r - sh, n = n0 + c;
+    tile[r][c] = (g >= 0 && g < nG && n < N2P) ? Wd[(size_t)g * N2P + n] : 0.0;
+  }
+  __syncthreads();
+  if (WxA)
+    for (int r = warp; r < FW_T; r += 8) {
+      const int g = c0 + r - sh;
+      if (g < 0 || g >= nG) continue;
+      const int e = fx_exp(mWr[g], L2 < FX_L64);
+      if (n0 == 0 && lane == 0) eWr[g] = e;
+      fx_store2<L2>(WxA + (size_t)g * L2 * pitchP, pitchP, n0 + 2 * lane, tile[r][2 * lane], tile[r][2 * lane + 1], e);
     }
-    __syncthreads();
-    for (int r = ty; r < SW_T; r += 8) {
-      const int n = n0 + r, g = g0 + tx, col = g + sh;
-      if (n < N2P && col < KpG) {
-        const int e = fx_exp(mWc[n]);
-        if (g == 0) eWc[n] = e;
-        fx_store_t<B1, L3T>(WTxB + (size_t)n * L3 * pitchG, pitchG, col, g < nG, tile[tx][r], e, b1, L3);
-      }
-      if (n < N2P && g0 == 0)  // columns before the shifted grid
-        for (int cz = tx; cz < sh; cz += 32)
-          fx_store_t<B1, L3T>(WTxB + (size_t)n * L3 * pitchG, pitchG, cz, false, 0.0, 0, b1, L3);
-    }
+  for (int r = warp; r < FW_T; r += 8) {
+    const int n = n0 + r;
+    if (n >= N2P) break;
+    const int e = fx_exp(mWc[n]);
+    if (c0 == 0 && lane == 0) eWc[n] = e;
+    fx_store2<L>(WTxB + (size_t)n * L * pitchG, pitchG, c0 + 2 * lane, tile[2 * lane][r], tile[2 * lane + 1][r], e);
   }
 }
 
@@ -608,49 +601,44 @@ size_t take(size_t& off, size_t bytes) {
 // Sizes (base == nullptr) or places (base = the arena) the mixed-form buffers of
 // one trajectory block starting at byte offset `off`; returns the end offset.
 size_t mixed_layout(cgpu_ctx* c, char* base, size_t off) {
-  if (c->precision == CGPU_PREC_FP64 || !c->hasInteraction) return off;
+  if ((c->precision == CGPU_PREC_FP64 && !c->fxOn) || !c->hasInteraction) return off;
   if (!c->mixed) c->mixed = new MixedBufs();
   MixedBufs* m = c->mixed;
-  m->fxBits = c->precision == CGPU_PREC_MIXED_FX ? 30 : c->precision == CGPU_PREC_MIXED_FX6 ? 36 : 0;
-  m->fxBits3 = m->fxBits;
   m->terms = c->precision == CGPU_PREC_MIXED_X6 ? 6 : 3;
   int nG = c->nG, nP = c->nPairs, Q = c->nOS * c->nOS, T = m->terms;
   m->KgMax = (nG + 63) / 64 * 64;
   m->KpMax = (2 * nP + 63) / 64 * 64;
   typedef __nv_bfloat16 bf;
-  if (m->fxBits) {
+  if (c->fxOn) {
     m->KgMax = c->fxKgMax;  // includes the K-tile offsets of a shared interaction matrix
-    // digit widths from the longest contraction of the batch (K = nG, K = 2P)
-    fx_plan(m->KgMax / 64, m->fxBits, &m->b1, &m->L1);
-    int b3 = 0;
-    fx_plan(m->KgMax / 64, m->fxBits3, &b3, &m->L3);
-    if (b3 != m->b1) throw std::string("mixed_fx: GEMM1 and GEMM3 share the S digits");
-    m->LS = std::max(m->L1, m->L3);
-    fx_plan(m->KpMax / 64, m->fxBits, &m->b2, &m->L2);
-    const int L1 = m->L1, L2 = m->L2;
-    m->compact2 = c->nb > 1 && fx_compact_ok(L2);
-    m->bn1 = fx_tile_n(2 * nP, L1, false);
-    m->bn2 = fx_tile_n(2 * Q, L2, m->compact2);
-    m->bn3 = fx_tile_n(2 * nP, m->L3, false);
-    m->s1 = fx_split_count(nG, 2 * nP, m->bn1, m->KgMax / 64, c->nb, m->b1);
-    m->s2 = fx_split_count(nG, 2 * Q, m->bn2, m->KpMax / 64, c->nb, m->b2);
-    m->s3 = fx_split_count(2 * nP, 2 * nP, m->bn3, m->KgMax / 64, c->nb, m->b1);
-    // partial buffers: a single system holds twice the heuristic's K splits
-    // (room for the tile tuner), a batch exactly the heuristic's
-    const int grow = c->nb == 1 ? 2 : 1;
-    m->sCap1 = std::min(m->s1 * grow, m->KgMax / 64);
-    m->sCap2 = std::min(m->s2 * grow, m->KpMax / 64);
-    m->sCap3 = std::min(m->s3 * grow, m->KgMax / 64);
+    const int kg = m->KgMax / 64, kp = m->KpMax / 64;
+    fx_slices(c->precision, kg, kp, &m->L, &m->L2);
+    const int L = m->L, L2 = m->L2;
+    auto plan = [&](FxGemm& g, int Lg, int M, int N, int kTiles, bool compact, bool extra) {
+      g.compact = compact;
+      g.bn = fx_tile_n(N, Lg, compact);
+      g.s = fx_split_count(M, N, g.bn, Lg, kTiles, c->nb, extra);
+    };
+    plan(m->gW, L, nG, 2 * nP, kg, false, true);
+    plan(m->gZ, L2, nG, 2 * Q, kp, c->nb > 1 && fx_compact_ok(L2), true);
+    plan(m->gH, L, 2 * nP, 2 * nP, kg, false, false);
+    plan(m->gWx, FX_L64, nG, 2 * nP, kg, false, true);
+    plan(m->gHx, FX_L64, 2 * nP, 2 * nP, kg, false, false);
+    // partial buffers: a single system of a tunable form holds twice the
+    // heuristic's K splits (room for the tile tuner), else exactly the heuristic's
+    const int grow = c->nb == 1 && L != FX_L64 ? 2 : 1;
+    m->sCapW = std::max(std::min(m->gW.s * grow, kg), m->gWx.s);
+    m->sCapZ = std::min(m->gZ.s * grow, kp);
+    m->sCapH = std::max(std::min(m->gH.s * grow, kg), m->gHx.s);
     const size_t perTrajV = c->fxShared ? 0 : 1;
-    size_t oV = take(off, perTrajV * sizeof(bf) * (size_t)nG * L1 * m->KgMax);
-    size_t oS = take(off, sizeof(bf) * (size_t)2 * nP * m->LS * m->KgMax);
+    size_t oV = take(off, perTrajV * sizeof(bf) * (size_t)nG * FX_L64 * m->KgMax);
+    size_t oS = take(off, sizeof(bf) * (size_t)2 * nP * FX_L64 * m->KgMax);
     size_t oW = take(off, sizeof(bf) * (size_t)nG * L2 * m->KpMax);
-    size_t oWT = take(off, sizeof(bf) * (size_t)2 * nP * m->L3 * m->KgMax);
+    size_t oWT = take(off, sizeof(bf) * (size_t)2 * nP * FX_L64 * m->KgMax);
     size_t oR = take(off, sizeof(bf) * (size_t)2 * Q * L2 * m->KpMax);
-    size_t oWd = take(off, sizeof(double) * (size_t)m->sCap1 * nG * 2 * nP);
-    size_t oZp = take(off, m->sCap2 > 1 ? sizeof(double) * (size_t)m->sCap2 * nG * 2 * Q : 0);
-    size_t oGd = take(off, sizeof(double) * (size_t)m->sCap3 * 2 * nP * 2 * nP);
-    size_t oE = take(off, sizeof(int));
+    size_t oWd = take(off, sizeof(double) * (size_t)m->sCapW * nG * 2 * nP);
+    size_t oZp = take(off, m->sCapZ > 1 ? sizeof(double) * (size_t)m->sCapZ * nG * 2 * Q : 0);
+    size_t oGd = take(off, sizeof(double) * (size_t)m->sCapH * 2 * nP * 2 * nP);
     size_t oZ = take(off, sizeof(double) * (size_t)2 * nG * Q);
     size_t oeV = take(off, perTrajV * sizeof(int) * (size_t)nG);
     size_t oeS = take(off, sizeof(int) * (size_t)2 * nP);
@@ -666,9 +654,8 @@ size_t mixed_layout(cgpu_ctx* c, char* base, size_t off) {
       m->WTxB = (bf*)(base + oWT);
       m->RxB = (bf*)(base + oR);
       m->Wd = (double*)(base + oWd);
-      m->Zp = m->sCap2 > 1 ? (double*)(base + oZp) : nullptr;
+      m->Zp = m->sCapZ > 1 ? (double*)(base + oZp) : nullptr;
       m->Gd = (double*)(base + oGd);
-      m->err = (int*)(base + oE);
       m->Zd = (double*)(base + oZ);
       m->eV = perTrajV ? (int*)(base + oeV) : nullptr;
       m->eS = (int*)(base + oeS);
@@ -696,7 +683,6 @@ size_t mixed_layout(cgpu_ctx* c, char* base, size_t off) {
   size_t o1 = take(off, sizeof(float) * (size_t)m->s1 * nG * 2 * nP);
   size_t o2 = take(off, sizeof(float) * (size_t)m->s2 * nG * 2 * Q);
   size_t o3 = take(off, sizeof(float) * (size_t)m->s3 * 2 * nP * 2 * nP);
-  size_t oE = take(off, sizeof(int));
   size_t oZ = take(off, sizeof(double) * (size_t)2 * nG * Q);
   if (base) {
     m->VxB = (bf*)(base + oV);
@@ -707,18 +693,25 @@ size_t mixed_layout(cgpu_ctx* c, char* base, size_t off) {
     m->P1 = (float*)(base + o1);
     m->P2 = (float*)(base + o2);
     m->P3 = (float*)(base + o3);
-    m->err = (int*)(base + oE);
     m->Zd = (double*)(base + oZ);
   }
   return off;
 }
 
+size_t mixed_outside_bytes(const cgpu_ctx* c) {
+  if (!c->fxOn || !c->fxShared) return 0;
+  const size_t kgBig = (c->nG + 63) / 64 * 64;
+  return c->fxRoots.size() * (size_t)c->nG * (FX_L64 * kgBig * sizeof(__nv_bfloat16) + sizeof(int));
+}
+
 void mixed_free(cgpu_ctx* c) {
   if (c->mixed) {
-    if (c->mixed->Vsh) cudaFree(c->mixed->Vsh);
-    if (c->mixed->eVsh) cudaFree(c->mixed->eVsh);
-    for (void* p : {c->mixed->tiles1, c->mixed->tiles2, c->mixed->tiles3})
-      if (p) cudaFree(p);
+    MixedBufs* m = c->mixed;
+    if (m->Vsh) cudaFree(m->Vsh);
+    if (m->eVsh) cudaFree(m->eVsh);
+    for (FxGemm* g : {&m->gW, &m->gZ, &m->gH, &m->gWx, &m->gHx})
+      if (g->tiles) cudaFree(g->tiles);
+    if (m->err_h) cudaFreeHost((void*)m->err_h);
   }
   delete c->mixed;  // the other buffers belong to the arena
   c->mixed = nullptr;
@@ -728,78 +721,85 @@ void mixed_free(cgpu_ctx* c) {
 void mixed_init(cgpu_ctx* c) {
   MixedBufs* m = c->mixed;
   if (!m) return;
-  int T = m->terms, pG = T * m->KgMax, pP = T * m->KpMax, pS = pG, pWT = pG;
-  if (m->fxBits) {
-    pG = m->L1 * m->KgMax;   // V: K = nG slices
-    pS = m->LS * m->KgMax;   // S (GEMM1 reads the first L1 slices, GEMM3 L3)
-    pWT = m->L3 * m->KgMax;  // W columns for GEMM3
-    pP = m->L2 * m->KpMax;   // W, R: K = 2P slices
+  {
+    void* h = nullptr;
+    CODY_CUDA(cudaHostAlloc(&h, sizeof(int), cudaHostAllocMapped));
+    *(int*)h = 0;
+    m->err_h = (volatile int*)h;
+    CODY_CUDA(cudaHostGetDevicePointer((void**)&m->err, h, 0));
   }
-  size_t nGK = (size_t)c->nG * m->KgMax;
-  if (m->fxBits && c->fxShared) {
-    // each root trajectory's interaction matrix, sliced once for the batch
-    const int nR = (int)c->fxRoots.size();
-    m->KgBig = (c->nG + 63) / 64 * 64;
-    const size_t plane = (size_t)c->nG * m->L1 * m->KgBig;  // elements per root
-    CODY_CUDA(cudaMalloc(&m->Vsh, sizeof(__nv_bfloat16) * plane * nR));
-    CODY_CUDA(cudaMalloc(&m->eVsh, sizeof(int) * (size_t)c->nG * nR));
-    CODY_CUDA(cudaMemsetAsync(m->Vsh, 0, sizeof(__nv_bfloat16) * plane * nR, c->stream));
-    for (int r = 0; r < nR; r++) {
-      const int root = c->fxRoots[r], nGb = c->sys[root].nG;
-      const double* Vb = (const double*)((const char*)c->Vint_d + (size_t)root * c->bs);
-      k_fx_split_V<<<dim3(nGb, 1, 1), 256, sizeof(double) * m->KgBig, c->stream>>>(
-          m->Vsh + plane * r, m->eVsh + (size_t)c->nG * r, Vb, m->KgBig, m->b1, m->L1, c->shape_d + root, 0);
+  const int P2 = 2 * c->nPairs, Q2 = 2 * c->nOS * c->nOS;
+  if (m->L) {
+    const int L = m->L, pV = FX_L64 * m->KgMax, pG = L * m->KgMax, pP = m->L2 * m->KpMax;
+    if (c->fxShared) {
+      // each root trajectory's interaction matrix, sliced once for the batch
+      const int nR = (int)c->fxRoots.size();
+      m->KgBig = (c->nG + 63) / 64 * 64;
+      const size_t plane = (size_t)c->nG * FX_L64 * m->KgBig;  // elements per root
+      CODY_CUDA(cudaMalloc(&m->Vsh, sizeof(__nv_bfloat16) * plane * nR));
+      CODY_CUDA(cudaMalloc(&m->eVsh, sizeof(int) * (size_t)c->nG * nR));
+      CODY_CUDA(cudaMemsetAsync(m->Vsh, 0, sizeof(__nv_bfloat16) * plane * nR, c->stream));
+      for (int r = 0; r < nR; r++) {
+        const int root = c->fxRoots[r], nGb = c->sys[root].nG;
+        const double* Vb = (const double*)((const char*)c->Vint_d + (size_t)root * c->bs);
+        k_fx_split_V<<<dim3(nGb, 1, 1), 256, 0, c->stream>>>(m->Vsh + plane * r, m->eVsh + (size_t)c->nG * r, Vb,
+                                                             m->KgBig, c->shape_d + root, 0);
+        CODY_LAUNCHED(c);
+      }
+      m->mVsh = tc_make_map_planes(m->Vsh, c->nG, FX_L64 * m->KgBig, 128, nR, sizeof(__nv_bfloat16) * plane);
+    } else {
+      k_fx_split_V<<<dim3(c->nG, 1, c->nb), 256, 0, c->stream>>>(m->VxB, m->eV, c->Vint_d, m->KgMax, TRAJ_PASS(c));
       CODY_LAUNCHED(c);
+      m->mV = tc_make_map(c, m->VxB, c->nG, pV, 128);
     }
-    m->mVsh = tc_make_map_planes(m->Vsh, c->nG, m->L1 * m->KgBig, 128, nR, sizeof(__nv_bfloat16) * plane);
-  } else if (m->fxBits)
-    k_fx_split_V<<<dim3(c->nG, 1, c->nb), 256, sizeof(double) * m->KgMax, c->stream>>>(m->VxB, m->eV, c->Vint_d,
-                                                                                     m->KgMax, m->b1, m->L1,
-                                                                                     TRAJ_PASS(c));
-  else
-    k_split_V<<<bgrid(c, ew_blocks(c, nGK)), 256, 0, c->stream>>>(m->VxB, c->Vint_d, m->KgMax, T, TRAJ_PASS(c));
-  CODY_LAUNCHED(c);
-  int P2 = 2 * c->nPairs, Q2 = 2 * c->nOS * c->nOS;
-  if (m->VxB) m->mV = tc_make_map(c, m->VxB, c->nG, pG, 128);
-  // the fixed-point GEMM loads its B operands in 16-row boxes
-  m->mS = tc_make_map(c, m->SxA, P2, pS, m->fxBits ? 16 : m->bn1);
-  m->mW = tc_make_map(c, m->WxA, c->nG, pP, 128);
-  m->mR = tc_make_map(c, m->RxB, Q2, pP, m->fxBits ? 16 : m->bn2);
-  m->mSasB = tc_make_map(c, m->SxA, P2, pS, 128);
-  if (m->fxBits) {
-    m->tiles1 = fx_build_tiles(c, TC_GEMM_W, m->bn1, m->s1, &m->nTiles1);
-    m->tiles2 = fx_build_tiles(c, TC_GEMM_Z, m->bn2, m->s2, &m->nTiles2);
-    m->tiles3 = fx_build_tiles(c, TC_GEMM_H2, m->bn3, m->s3, &m->nTiles3);
+    // A operands in 128-row boxes, B operands in 16-row boxes
+    m->mS = tc_make_map(c, m->SxA, P2, pG, 16);
+    m->mSasB = tc_make_map(c, m->SxA, P2, pG, 128);
+    m->mSx = tc_make_map(c, m->SxA, P2, pV, 16);
+    m->mSxasB = tc_make_map(c, m->SxA, P2, pV, 128);
+    m->mWT = tc_make_map(c, m->WTxB, P2, pG, 16);
+    m->mWTx = tc_make_map(c, m->WTxB, P2, pV, 16);
+    m->mW = tc_make_map(c, m->WxA, c->nG, pP, 128);
+    m->mR = tc_make_map(c, m->RxB, Q2, pP, 16);
+    auto tiles = [&](FxGemm& g, int id) { g.tiles = fx_build_tiles(c, id, g.bn, g.s, &g.nTiles); };
+    tiles(m->gW, TC_GEMM_W);
+    tiles(m->gZ, TC_GEMM_Z);
+    tiles(m->gH, TC_GEMM_H2);
+    tiles(m->gWx, TC_GEMM_W);
+    tiles(m->gHx, TC_GEMM_H2);
+  } else {
+    const int T = m->terms, pG = T * m->KgMax, pP = T * m->KpMax;
+    k_split_V<<<bgrid(c, ew_blocks(c, (size_t)c->nG * m->KgMax)), 256, 0, c->stream>>>(m->VxB, c->Vint_d, m->KgMax, T,
+                                                                                    TRAJ_PASS(c));
+    CODY_LAUNCHED(c);
+    m->mV = tc_make_map(c, m->VxB, c->nG, pG, 128);
+    m->mS = tc_make_map(c, m->SxA, P2, pG, m->bn1);
+    m->mW = tc_make_map(c, m->WxA, c->nG, pP, 128);
+    m->mR = tc_make_map(c, m->RxB, Q2, pP, m->bn2);
+    m->mSasB = tc_make_map(c, m->SxA, P2, pG, 128);
+    m->mWT = tc_make_map(c, m->WTxB, P2, pG, m->bn3);
   }
-  m->mWT = tc_make_map(c, m->WTxB, P2, pWT, m->fxBits ? 16 : m->bn3);
   CODY_CUDA(cudaStreamSynchronize(c->stream));
 }
 
-int mixed_error(cgpu_ctx* c) {
-  if (!c->mixed) return 0;
-  int e = 0;
-  CODY_CUDA(cudaMemcpy(&e, c->mixed->err, sizeof(int), cudaMemcpyDeviceToHost));
-  return e;
-}
+// The kernels set the flag in host memory, so reading it after a
+// synchronisation costs nothing.
+int mixed_error(cgpu_ctx* c) { return c->mixed && c->mixed->err_h ? *c->mixed->err_h : 0; }
 
 // The three fixed-point contractions with their K-split reductions, on the
 // operands the digit splits left in the arena (one call = one launch of the
-// GEMM, plus the reduction when K is split).
+// GEMM, plus the reduction when K is split).  exact: FX_L64 slices (FillH2).
 // W = V S (pair potentials; row / column exponent maxima for the W split).
-static void fx_run_W(cgpu_ctx* c) {
+static void fx_run_W(cgpu_ctx* c, bool exact) {
   MixedBufs* m = c->mixed;
   const int nG = c->nG, nP = c->nPairs;
-  const bool one = m->s1 == 1;
-  if (c->fxShared)
-    fx_gemm(c, m->L1, m->b1, m->compact1, TC_GEMM_W, m->mVsh, m->mS, m->bn1, m->Wd, m->eVsh, m->eS,
-            one ? m->mWr : nullptr, one ? m->mWc : nullptr, m->KgBig, m->KgMax, 1, m->s1, m->tiles1, m->nTiles1,
-            m->err);
-  else
-    fx_gemm(c, m->L1, m->b1, m->compact1, TC_GEMM_W, m->mV, m->mS, m->bn1, m->Wd, m->eV, m->eS,
-            one ? m->mWr : nullptr, one ? m->mWc : nullptr, m->KgMax, m->KgMax, 0, m->s1, m->tiles1, m->nTiles1,
-            m->err);
+  const FxGemm& g = exact ? m->gWx : m->gW;
+  const bool one = g.s == 1;
+  fx_gemm(c, exact ? FX_L64 : m->L, g.compact, TC_GEMM_W, c->fxShared ? m->mVsh : m->mV, exact ? m->mSx : m->mS, g.bn,
+          m->Wd, c->fxShared ? m->eVsh : m->eV, m->eS, one ? m->mWr : nullptr, one ? m->mWc : nullptr,
+          c->fxShared ? m->KgBig : m->KgMax, m->KgMax, c->fxShared, g.s, g.tiles, g.nTiles, m->err);
   if (!one) {
-    k_fx_reduce_W<<<bgrid(c, ew_blocks(c, (size_t)nG * 2 * nP)), 256, 0, c->stream>>>(m->Wd, m->mWr, m->mWc, m->s1,
+    k_fx_reduce_W<<<bgrid(c, ew_blocks(c, (size_t)nG * 2 * nP)), 256, 0, c->stream>>>(m->Wd, m->mWr, m->mWc, g.s,
                                                                                    TRAJ_PASS(c));
     CODY_LAUNCHED(c);
   }
@@ -809,84 +809,90 @@ static void fx_run_W(cgpu_ctx* c) {
 static void fx_run_Z(cgpu_ctx* c) {
   MixedBufs* m = c->mixed;
   const int nG = c->nG, Q = c->nOS * c->nOS;
-  fx_gemm(c, m->L2, m->b2, m->compact2, TC_GEMM_Z, m->mW, m->mR, m->bn2, m->s2 > 1 ? m->Zp : m->Zd, m->eWr, m->eR,
-          nullptr, nullptr, m->KpMax, m->KpMax, 0, m->s2, m->tiles2, m->nTiles2, m->err);
-  if (m->s2 > 1) {
-    k_reduce_Z<<<bgrid(c, ew_blocks(c, (size_t)nG * Q)), 256, 0, c->stream>>>((z_t*)m->Zd, m->Zp, m->s2,
-                                                                        TRAJ_PASS(c));
+  const FxGemm& g = m->gZ;
+  fx_gemm(c, m->L2, g.compact, TC_GEMM_Z, m->mW, m->mR, g.bn, g.s > 1 ? m->Zp : m->Zd, m->eWr, m->eR, nullptr, nullptr,
+          m->KpMax, m->KpMax, 0, g.s, g.tiles, g.nTiles, m->err);
+  if (g.s > 1) {
+    k_reduce_Z<<<bgrid(c, ew_blocks(c, (size_t)nG * Q)), 256, 0, c->stream>>>((z_t*)m->Zd, m->Zp, g.s, TRAJ_PASS(c));
     CODY_LAUNCHED(c);
   }
 }
 
 // G = S^T W (h2) and its reduction into the spatial h2 block.
-static void fx_run_H2(cgpu_ctx* c) {
+static void fx_run_H2(cgpu_ctx* c, bool exact) {
   MixedBufs* m = c->mixed;
   const int Q = c->nOS * c->nOS;
-  fx_gemm(c, m->L3, m->b1, m->compact3, TC_GEMM_H2, m->mSasB, m->mWT, m->bn3, m->Gd, m->eS, m->eWc, nullptr, nullptr,
-          m->KgMax, m->KgMax, 0, m->s3, m->tiles3, m->nTiles3, m->err);
-  k_reduce_H2<<<bgrid(c, ew_blocks(c, (size_t)Q * Q)), 256, 0, c->stream>>>(c->h2s_d, m->Gd, m->s3, c->pidx_d,
+  const FxGemm& g = exact ? m->gHx : m->gH;
+  fx_gemm(c, exact ? FX_L64 : m->L, g.compact, TC_GEMM_H2, exact ? m->mSxasB : m->mSasB, exact ? m->mWTx : m->mWT, g.bn,
+          m->Gd, m->eS, m->eWc, nullptr, nullptr, m->KgMax, m->KgMax, 0, g.s, g.tiles, g.nTiles, m->err);
+  k_reduce_H2<<<bgrid(c, ew_blocks(c, (size_t)Q * Q)), 256, 0, c->stream>>>(c->h2s_d, m->Gd, g.s, c->pidx_d,
                                                                       TRAJ_PASS(c));
   CODY_LAUNCHED(c);
 }
 
 // ---- tile tuner hooks ---------------------------------------------------------
+// The FP64 form has one tile width and is not tuned.
+static bool fx_tunable(const cgpu_ctx* c) { return c->mixed && c->mixed->L && c->precision != CGPU_PREC_FP64; }
 
 bool fx_tiles_get(const cgpu_ctx* c, int* t) {
+  if (!fx_tunable(c)) return false;
   const MixedBufs* m = c->mixed;
-  if (!m || !m->fxBits) return false;
-  const int v[9] = {m->bn1, m->compact1, m->s1, m->bn2, m->compact2, m->s2, m->bn3, m->compact3, m->s3};
-  for (int i = 0; i < 9; i++) t[i] = v[i];
+  int i = 0;
+  for (const FxGemm* g : {&m->gW, &m->gZ, &m->gH}) {
+    t[i++] = g->bn;
+    t[i++] = g->compact;
+    t[i++] = g->s;
+  }
   return true;
 }
 
-// Slices, digit width, K blocks, split capacity and output columns of GEMM g.
-static void fx_gemm_plan(const cgpu_ctx* c, int g, int& L, int& b, int& kTiles, int& cap, int& N) {
+// K blocks, split capacity and output columns of GEMM g.
+static void fx_gemm_plan(const cgpu_ctx* c, int g, int& kTiles, int& cap, int& N) {
   const MixedBufs* m = c->mixed;
-  if (g == TC_GEMM_W) { L = m->L1; b = m->b1; kTiles = m->KgMax / 64; cap = m->sCap1; N = 2 * c->nPairs; }
-  else if (g == TC_GEMM_Z) { L = m->L2; b = m->b2; kTiles = m->KpMax / 64; cap = m->sCap2; N = 2 * c->nOS * c->nOS; }
-  else { L = m->L3; b = m->b1; kTiles = m->KgMax / 64; cap = m->sCap3; N = 2 * c->nPairs; }
+  if (g == TC_GEMM_W) { kTiles = m->KgMax / 64; cap = m->sCapW; N = 2 * c->nPairs; }
+  else if (g == TC_GEMM_Z) { kTiles = m->KpMax / 64; cap = m->sCapZ; N = 2 * c->nOS * c->nOS; }
+  else { kTiles = m->KgMax / 64; cap = m->sCapH; N = 2 * c->nPairs; }
 }
 
 void fx_tiles_set(cgpu_ctx* c, const int* t) {
   MixedBufs* m = c->mixed;
-  if (!m || !m->fxBits) throw std::string("tiles: not a fixed-point context");
-  int bn[3], sp[3];
-  bool cm[3];
+  if (!fx_tunable(c)) throw std::string("tiles: not a fixed-point context");
+  int sp[3];
   for (int g = 0; g < 3; g++) {
-    int L, b, kTiles, cap, N;
-    fx_gemm_plan(c, g, L, b, kTiles, cap, N);
-    bn[g] = t[3 * g];
-    cm[g] = t[3 * g + 1] != 0;
-    if (!fx_tile_supported(bn[g], L, cm[g])) throw std::string("tiles: no fixed-point GEMM configuration for that tile");
+    int kTiles, cap, N;
+    fx_gemm_plan(c, g, kTiles, cap, N);
+    if (!fx_tile_supported(t[3 * g], g == TC_GEMM_Z ? m->L2 : m->L, t[3 * g + 1] != 0))
+      throw std::string("tiles: no fixed-point GEMM configuration for that tile");
     if (t[3 * g + 2] < 1 || t[3 * g + 2] > kTiles) throw std::string("tiles: K split count outside 1..K blocks");
     sp[g] = fx_normalize_splits(kTiles, t[3 * g + 2]);
     // every split keeps at least two K blocks, as the set-up heuristic does
-    if (sp[g] < fx_min_splits(kTiles, b) || sp[g] > cap || (sp[g] > 1 && sp[g] > kTiles / 2))
-      throw std::string("tiles: K split outside the exact range of the digits or the partial buffers");
+    if (sp[g] < fx_min_splits(kTiles) || sp[g] > cap || (sp[g] > 1 && sp[g] > kTiles / 2))
+      throw std::string("tiles: K split outside the range of the level sums or the partial buffers");
   }
-  void** lists[3] = {&m->tiles1, &m->tiles2, &m->tiles3};
-  int* counts[3] = {&m->nTiles1, &m->nTiles2, &m->nTiles3};
   CODY_CUDA(cudaStreamSynchronize(c->stream));
+  FxGemm* gm[3] = {&m->gW, &m->gZ, &m->gH};
   for (int g = 0; g < 3; g++) {
-    if (*lists[g]) CODY_CUDA(cudaFree(*lists[g]));
-    *lists[g] = fx_build_tiles(c, g, bn[g], sp[g], counts[g]);
+    FxGemm& G = *gm[g];
+    if (G.tiles) CODY_CUDA(cudaFree(G.tiles));
+    G.tiles = nullptr;
+    G.tiles = fx_build_tiles(c, g, t[3 * g], sp[g], &G.nTiles);
+    G.bn = t[3 * g];
+    G.compact = t[3 * g + 1] != 0;
+    G.s = sp[g];
   }
-  m->bn1 = bn[0]; m->compact1 = cm[0]; m->s1 = sp[0];
-  m->bn2 = bn[1]; m->compact2 = cm[1]; m->s2 = sp[1];
-  m->bn3 = bn[2]; m->compact3 = cm[2]; m->s3 = sp[2];
 }
 
 void fx_tile_candidates(const cgpu_ctx* c, int g, std::vector<std::array<int, 3>>& out) {
   out.clear();
-  if (!c->mixed || !c->mixed->fxBits) return;
-  int L, b, kTiles, cap, N;
-  fx_gemm_plan(c, g, L, b, kTiles, cap, N);
+  if (!fx_tunable(c)) return;
+  int kTiles, cap, N;
+  fx_gemm_plan(c, g, kTiles, cap, N);
   std::vector<std::pair<int, bool>> cfgs;
-  fx_tile_configs(L, cfgs);
+  fx_tile_configs(g == TC_GEMM_Z ? c->mixed->L2 : c->mixed->L, cfgs);
   std::vector<int> splits;
   for (int s : {1, 2, 3, 4, cap}) {
     int v = fx_normalize_splits(kTiles, s);
-    if (v >= fx_min_splits(kTiles, b) && v <= cap && (v == 1 || v <= kTiles / 2) &&
+    if (v >= fx_min_splits(kTiles) && v <= cap && (v == 1 || v <= kTiles / 2) &&
         std::find(splits.begin(), splits.end(), v) == splits.end())
       splits.push_back(v);
   }
@@ -898,9 +904,9 @@ void fx_tile_candidates(const cgpu_ctx* c, int g, std::vector<std::array<int, 3>
 
 double fx_time_contraction(cgpu_ctx* c, int g, int reps) {
   auto run = [&]() {
-    if (g == TC_GEMM_W) fx_run_W(c);
+    if (g == TC_GEMM_W) fx_run_W(c, false);
     else if (g == TC_GEMM_Z) fx_run_Z(c);
-    else fx_run_H2(c);
+    else fx_run_H2(c, false);
   };
   run();
   cudaEvent_t e0, e1;
@@ -918,48 +924,62 @@ double fx_time_contraction(cgpu_ctx* c, int g, int reps) {
   return ms / reps;
 }
 
-// The fixed-point form of the three contractions.
-void correlation_fx(cgpu_ctx* c, z_t* dOrbs, const z_t* orbs, int wantH2) {
+// S rows as L digit slices, W = V S, W columns as L and (wantW) rows as L2 digit slices.
+template <int L, int L2>
+static void fx_potentials(cgpu_ctx* c, const z_t* orbs, bool exact, bool wantW) {
   MixedBufs* m = c->mixed;
-  const int nG = c->nG, nP = c->nPairs, n = c->nOS, Q = n * n;
-  z_t* Z = (z_t*)m->Zd;
-  {
-    ProfScope prof(c, CGPU_KERNEL_PAIR_POTENTIALS);
-    auto split_s = k_fx_split_S<0, 0>;
-    if (m->b1 == 6 && m->LS == 6) split_s = k_fx_split_S<6, 6>;
-    else if (m->b1 == 6 && m->LS == 5) split_s = k_fx_split_S<6, 5>;
-    const size_t shS = 2 * sizeof(double) * m->KgMax;
-    if (shS > 48 * 1024)
-      CODY_CUDA(cudaFuncSetAttribute(split_s, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shS));
-    split_s<<<dim3(nP, 1, c->nb), 256, shS, c->stream>>>(
-        m->SxA, m->eS, m->mWr, m->mWc, orbs, c->w_d, c->pairL_d, c->pairK_d, m->KgMax, m->b1, m->LS, TRAJ_PASS(c));
-    CODY_LAUNCHED(c);
-    fx_run_W(c);
-    dim3 gw(ceil_div(m->KgMax, SW_T), 1, c->nb);
-    // the digit plans of the two fixed-point forms on long grids, compiled in
-    auto split_w = k_fx_split_W<0, 0, 0, 0>;
-    if (m->b1 == 6 && m->L3 == 6 && m->b2 == 8 && m->L2 == 5) split_w = k_fx_split_W<6, 6, 8, 5>;
-    else if (m->b1 == 6 && m->L3 == 5 && m->b2 == 8 && m->L2 == 4) split_w = k_fx_split_W<6, 5, 8, 4>;
-    split_w<<<gw, 256, 0, c->stream>>>(m->WxA, m->WTxB, m->eWr, m->eWc, m->Wd, m->mWr, m->mWc, m->KpMax, m->KgMax,
-                                       m->b1, m->L3, m->b2, m->L2, TRAJ_PASS(c));
-    CODY_LAUNCHED(c);
-  }
+  ProfScope prof(c, CGPU_KERNEL_PAIR_POTENTIALS);
+  const size_t need = 2 * sizeof(double) * m->KgMax;
+  const int staged = need <= FX_STAGE_MAX;
+  if (staged && need > 48 * 1024)
+    CODY_CUDA(cudaFuncSetAttribute(k_fx_split_S<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need));
+  k_fx_split_S<L><<<dim3(c->nPairs, 1, c->nb), 256, staged ? need : 0, c->stream>>>(
+      m->SxA, m->eS, m->mWr, m->mWc, orbs, c->w_d, c->pairL_d, c->pairK_d, m->KgMax, staged, TRAJ_PASS(c));
+  CODY_LAUNCHED(c);
+  fx_run_W(c, exact);
+  dim3 gw(m->KgMax / FW_T, m->KpMax / FW_T, c->nb);
+  k_fx_split_W<L, L2><<<gw, 256, 0, c->stream>>>(wantW ? m->WxA : nullptr, m->WTxB, m->eWr, m->eWc, m->Wd, m->mWr,
+                                                 m->mWc, m->KpMax, m->KgMax, TRAJ_PASS(c));
+  CODY_LAUNCHED(c);
+}
+
+// The fixed-point forms of the three contractions.
+template <int L, int L2>
+static void correlation_fx_t(cgpu_ctx* c, z_t* dOrbs, const z_t* orbs, int wantH2) {
+  MixedBufs* m = c->mixed;
+  const int Q = c->nOS * c->nOS;
+  fx_potentials<L, L2>(c, orbs, false, true);
   {
     ProfScope prof(c, CGPU_KERNEL_CORRELATION);
-    auto split_r = k_fx_split_R<0, 0>;
-    if (m->b2 == 8 && m->L2 == 5) split_r = k_fx_split_R<8, 5>;
-    else if (m->b2 == 8 && m->L2 == 4) split_r = k_fx_split_R<8, 4>;
-    split_r<<<dim3(2 * Q, 1, c->nb), 64, sizeof(double) * m->KpMax, c->stream>>>(
-        m->RxB, m->eR, c->Rp_d, c->pairL_d, c->pairK_d, m->KpMax, m->b2, m->L2, TRAJ_PASS(c));
+    k_fx_split_R<L2><<<dim3(2 * Q, 1, c->nb), 64, sizeof(double) * m->KpMax, c->stream>>>(
+        m->RxB, m->eR, c->Rp_d, c->pairL_d, c->pairK_d, m->KpMax, TRAJ_PASS(c));
     CODY_LAUNCHED(c);
     fx_run_Z(c);
-    launch_corr_epilogue(c, dOrbs, orbs, Z);
+    launch_corr_epilogue(c, dOrbs, orbs, (z_t*)m->Zd);
   }
   if (wantH2) {
     ProfScope prof(c, CGPU_KERNEL_H2);
-    fx_run_H2(c);
+    fx_run_H2(c, false);
     launch_h2_layout(c);
   }
+}
+
+static void correlation_fx(cgpu_ctx* c, z_t* dOrbs, const z_t* orbs, int wantH2) {
+  const int L = c->mixed->L, L2 = c->mixed->L2;
+  if (L == FX_L64) return correlation_fx_t<FX_L64, FX_L64>(c, dOrbs, orbs, wantH2);
+  if (L == 5 && L2 == 4) return correlation_fx_t<5, 4>(c, dOrbs, orbs, wantH2);
+  if (L == 5 && L2 == 5) return correlation_fx_t<5, 5>(c, dOrbs, orbs, wantH2);
+  if (L == 5 && L2 == 6) return correlation_fx_t<5, 6>(c, dOrbs, orbs, wantH2);
+  if (L == 6 && L2 == 5) return correlation_fx_t<6, 5>(c, dOrbs, orbs, wantH2);
+  if (L == 6 && L2 == 6) return correlation_fx_t<6, 6>(c, dOrbs, orbs, wantH2);
+  throw std::string("internal: no kernels for this slice plan");
+}
+
+void launch_fill_h2_fx(cgpu_ctx* c, const z_t* orbs) {
+  fx_potentials<FX_L64, FX_L64>(c, orbs, true, false);
+  ProfScope prof(c, CGPU_KERNEL_H2);
+  fx_run_H2(c, true);
+  launch_h2_layout(c);
 }
 
 // ApplyCorrelationOp in the mixed form: dOrbs += rho^-1 rho2 W phi; h2 (FP64 nO^4) when wantH2.
@@ -974,7 +994,7 @@ void launch_correlation_mixed(cgpu_ctx* c, z_t* dOrbs, const z_t* orbs, int want
   }
   MixedBufs* m = c->mixed;
   int nG = c->nG, nP = c->nPairs, n = c->nOS, Q = n * n, T = m->terms;
-  if (m->fxBits) return correlation_fx(c, dOrbs, orbs, wantH2);
+  if (m->L) return correlation_fx(c, dOrbs, orbs, wantH2);
   {
     ProfScope prof(c, CGPU_KERNEL_PAIR_POTENTIALS);
     k_split_S<<<bgrid(c, ew_blocks(c, (size_t)2 * nP * m->KgMax)), 256, 0, c->stream>>>(

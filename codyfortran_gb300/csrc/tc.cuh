@@ -24,9 +24,11 @@ CUtensorMap tc_make_map(const cgpu_ctx* c, const __nv_bfloat16* base, int rowsMa
 void tc_gemm(cgpu_ctx* c, int gemmId, const CUtensorMap& ta, const CUtensorMap& tb, int bn, float* P, int terms,
              int segPitch, int nSplit, int Mmax, int Nmax, int* err);
 
+// Row exponent of an operand row that holds an infinity or a NaN.
+constexpr int FX_EXP_NAN = 1 << 20;
 // Fixed-point slice GEMM (k_fx.cu): out[traj][split][M][N] (FP64) = A B^T (the
 // B map with 16-row boxes, the A map with 128-row boxes) for
-// operands carried as L base-2^digitBits digit slices (K segments of
+// operands carried as L base-256 digit slices (K segments of
 // segPitchA / segPitch elements) with row exponents expA / expB; maxRow /
 // maxCol (unsplit K only) receive the largest biased exponent of |C| per row /
 // column.  compact: the two-CTAs-per-SM configuration (small K).  aShared: A
@@ -34,22 +36,15 @@ void tc_gemm(cgpu_ctx* c, int gemmId, const CUtensorMap& ta, const CUtensorMap& 
 // nSplit: K splits of the longest contraction (segPitch / 64 K blocks, kPer
 // blocks per split); a trajectory of fewer K blocks takes only the splits its
 // own K needs, balanced, and its remaining partials are written as zeros.
-void fx_gemm(cgpu_ctx* c, int L, int digitBits, bool compact, int gemmId, const CUtensorMap& ta,
-             const CUtensorMap& tb, int bn, double* out, const int* expA, const int* expB, unsigned* maxRow,
-             unsigned* maxCol, int segPitchA, int segPitch, int aShared, int nSplit, const void* tiles, int nTiles,
-             int* err);
+void fx_gemm(cgpu_ctx* c, int L, bool compact, int gemmId, const CUtensorMap& ta, const CUtensorMap& tb, int bn,
+             double* out, const int* expA, const int* expB, unsigned* maxRow, unsigned* maxCol, int segPitchA,
+             int segPitch, int aShared, int nSplit, const void* tiles, int nTiles, int* err);
 // Device list of the fixed-point GEMM's tiles (trajectory, row, column, K split) of the
 // context for an N tile of bn columns: only tiles inside a trajectory's output.
 void* fx_build_tiles(cgpu_ctx* c, int gemmId, int bn, int nSplit, int* nTiles);
 // 3D TMA map over an explicit [planes][rowsMax][pitch] bf16 tensor (planes planeBytes apart).
 CUtensorMap tc_make_map_planes(const __nv_bfloat16* base, int rowsMax, int pitch, int boxRows, int planes,
                                size_t planeBytes);
-// Digit width (6..8 bits) and slice count carrying at least targetBits
-// fractional bits for a contraction of kTiles 64-wide K blocks: the widest
-// digits whose two leading level sums stay exact in FP32 over the whole K
-// (K <= 2^(24-2b)) and whose epilogue sum of the levels stays inside int64
-// (b (L-1) <= 38).
-void fx_plan(int kTiles, int targetBits, int* digitBits, int* slices);
 // N-tile width for N output columns and L slices (wide: L * BN <= 512, compact: <= 256).
 int fx_tile_n(int N, int L, bool compact);
 // Whether a compact configuration exists for L slices.
@@ -57,13 +52,13 @@ bool fx_compact_ok(int L);
 // The instantiated (N tile width, compact) configurations for L slices.
 void fx_tile_configs(int L, std::vector<std::pair<int, bool>>& out);
 bool fx_tile_supported(int bn, int L, bool compact);
-// Fewest K splits that keep every split inside the exact range of the digits.
-int fx_min_splits(int kTiles, int digitBits);
+// Fewest K splits that keep the level sums of every split inside their integers.
+int fx_min_splits(int kTiles);
 // The split count fx_gemm runs for a request of s splits (balanced K blocks per split).
 int fx_normalize_splits(int kTiles, int s);
-// K splits of the fixed-point GEMM: about one wave of 152 SMs, and every split
-// inside the exact range of the level sums at digitBits (2^(24-2b) K).
-int fx_split_count(int M, int N, int BN, int kTiles, int nb, int digitBits);
+// K splits of the fixed-point GEMM for kTiles 64-wide K blocks (reduceExtra:
+// the partials need a reduction kernel of their own).
+int fx_split_count(int M, int N, int BN, int L, int kTiles, int nb, bool reduceExtra);
 
 // ---- device helpers shared by the tcgen05 kernels (TMA, mbarriers, MMA, TMEM) ----
 namespace tcdev {
