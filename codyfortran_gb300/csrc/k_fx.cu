@@ -29,9 +29,13 @@
 //
 // Pipeline: one TMA producer thread, one MMA issuer thread, eight epilogue
 // warps (two per tensor-memory lane quarter).  Per 64-wide K block the producer
-// loads the L slices of the B tile (in 16-row boxes, only the rows of the
-// tile's own nT columns, slice after slice) into one ring stage and the L
-// slices of the A tile into L stages of a second ring.
+// loads the L slices of the B tile (only the rows of the tile's own nT columns,
+// slice after slice) into one ring stage and the L slices of the A tile into L
+// stages of a second ring.  A TMA instruction costs its thread about 100 cycles
+// (measured: 16 KB per stage in one box 5.8 TB/s over all SMs, in eight boxes
+// 3.1), so the B group is one instruction: a 4D box of 64 columns, nT rows, L
+// slices, from the map made for that nT (in 16-row boxes, W = V S of the
+// 512-trajectory batch in the 39-bit form 2.48 ms, this way 2.25).
 //
 // The B slices of a stage are consecutive rows of one operand (slice j at row
 // j nT), and level l's accumulator sits at tensor-memory column l nT, so the
@@ -62,6 +66,21 @@
 #include "common.cuh"
 #include "tc.cuh"
 
+// B operand [nb][rowsMax][L][pitch] as 4D maps (column, row, slice, trajectory)
+// with boxes of 64 columns, 16 (i + 1) rows and all L slices.
+FxMaps fx_make_maps(const cgpu_ctx* c, const __nv_bfloat16* base, int rowsMax, int pitch, int L) {
+  FxMaps f;
+  for (int i = 0; i < FX_MAPS; i++) {
+    const unsigned long long dims[4] = {(unsigned long long)pitch, (unsigned long long)rowsMax, (unsigned long long)L,
+                                        (unsigned long long)c->nb};
+    const unsigned long long strides[3] = {(unsigned long long)pitch * L * 2, (unsigned long long)pitch * 2,
+                                           c->nb > 1 ? c->bs : (unsigned long long)pitch * L * 2 * rowsMax};
+    const unsigned box[4] = {tcdev::TC_BK, 16u * (i + 1), (unsigned)L, 1};
+    f.m[i] = tc_encode_map(base, 4, dims, strides, box);
+  }
+  return f;
+}
+
 namespace {
 
 using namespace tcdev;
@@ -83,7 +102,7 @@ struct FxCfg {
   static constexpr uint32_t TMEM_COLS = (L * BN) <= 32 ? 32 : (L * BN) <= 64 ? 64 : (L * BN) <= 128 ? 128
                                         : (L * BN) <= 256 ? 256 : 512;
   static_assert(L * BN <= 512, "tensor memory holds 512 columns");
-  static_assert(BN % 16 == 0 && BN >= 16, "N tile: multiple of 16");
+  static_assert(BN % 16 == 0 && BN >= 16 && BN <= 16 * FX_MAPS, "N tile: multiple of 16 with a B map");
   static_assert(NA >= 2, "A ring");
   static_assert(SMEM + 2048 <= FX_SMEM_MAX, "shared memory");
 };
@@ -175,10 +194,10 @@ struct FxTile {
 // vRow - gShift, its row exponents at expA[vExp].
 template <int BN, int L, int NA_, int NB_, int EW>
 __global__ void __launch_bounds__(32 * (EW + 2), NA_ > 0 ? 2 : 1)
-    k_fx_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUtensorMap tB, double* __restrict__ out,
+    k_fx_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ FxMaps tB, double* __restrict__ out,
               const int* __restrict__ expA, const int* __restrict__ expB, unsigned* __restrict__ maxRow,
-              unsigned* __restrict__ maxCol, TRAJ_ARGS, int gemmId, int segPitchA, int segPitch, int aShared,
-              int kPer, const FxTile* __restrict__ tiles, int nTiles, int* __restrict__ err) {
+              unsigned* __restrict__ maxCol, TRAJ_ARGS, int gemmId, int segPitchA, int aShared, int kPer,
+              const FxTile* __restrict__ tiles, int nTiles, int* __restrict__ err) {
   using C = FxCfg<BN, L, NA_, NB_>;
   constexpr int NA = C::NA, NB = C::NB, CB = 8;
   static_assert(EW % 4 == 0 && BN % CB == 0, "epilogue warps / column batch");
@@ -235,7 +254,7 @@ __global__ void __launch_bounds__(32 * (EW + 2), NA_ > 0 ? 2 : 1)
 
   if (warp == EW) {
     if (lane == 0) {
-      // TMA producer: per K block the L B slices (16-row boxes of the tile's rows), then the L A slices
+      // TMA producer: per K block the L B slices of the tile's rows, then the L A slices
       int ta = 0, tb = 0;
       for (int t = blockIdx.x; t < nTiles && !abortFlag; t += gridDim.x) {
         const FxTile tl = tiles[t];
@@ -253,10 +272,7 @@ __global__ void __launch_bounds__(32 * (EW + 2), NA_ > 0 ? 2 : 1)
           }
           const int x0 = (kt0 + kb) * TC_BK;
           mbar_expect_tx(&bFull[sb], (uint32_t)(L * tl.nT * TC_BK * 2));
-          uint8_t* dstB = ringB + sb * C::BG_BYTES;
-          for (int j = 0; j < L; j++)
-            for (int r = 0; r < tl.nT; r += 16, dstB += 16 * TC_BK * 2)
-              tma_load_3d(dstB, &tB, &bFull[sb], j * segPitch + x0, tl.n0 + r, tl.traj);
+          tma_load_4d(ringB + sb * C::BG_BYTES, &tB.m[tl.nT / 16 - 1], &bFull[sb], x0, tl.n0, 0, tl.traj);
           tb++;
           issuedB = tb;
           for (int i = 0; i < L; i++) {
@@ -484,9 +500,9 @@ __global__ void __launch_bounds__(32 * (EW + 2), NA_ > 0 ? 2 : 1)
 }
 
 template <int BN, int L, int NA_, int NB_>
-void launch_fx_t(cgpu_ctx* c, const CUtensorMap& ta, const CUtensorMap& tb, double* out, const int* expA,
-                 const int* expB, unsigned* maxRow, unsigned* maxCol, int gemmId, int segPitchA, int segPitch,
-                 int aShared, int kPer, const FxTile* tiles, int nTiles, int ctasPerSm, int* err) {
+void launch_fx_t(cgpu_ctx* c, const CUtensorMap& ta, const FxMaps& tb, double* out, const int* expA,
+                 const int* expB, unsigned* maxRow, unsigned* maxCol, int gemmId, int segPitchA, int aShared, int kPer,
+                 const FxTile* tiles, int nTiles, int ctasPerSm, int* err) {
   using C = FxCfg<BN, L, NA_, NB_>;
   // eight epilogue warps (two per tensor-memory lane quarter); sixteen for L >
   // 5, whose two 64-bit sums per output would not fit the registers of eight
@@ -500,7 +516,7 @@ void launch_fx_t(cgpu_ctx* c, const CUtensorMap& ta, const CUtensorMap& tb, doub
   if (nTiles <= 0) return;
   const int grid = std::min(nTiles, c->numSms * ctasPerSm);
   kern<<<grid, 32 * (EW + 2), C::SMEM, c->stream>>>(ta, tb, out, expA, expB, maxRow, maxCol, TRAJ_PASS(c), gemmId,
-                                                    segPitchA, segPitch, aShared, kPer, tiles, nTiles, err);
+                                                    segPitchA, aShared, kPer, tiles, nTiles, err);
   CODY_LAUNCHED(c);
 }
 
@@ -624,7 +640,7 @@ void* fx_build_tiles(cgpu_ctx* c, int gemmId, int bn, int nSplit, int* nTiles) {
   return d;
 }
 
-void fx_gemm(cgpu_ctx* c, int L, bool compact, int gemmId, const CUtensorMap& ta, const CUtensorMap& tb, int bn,
+void fx_gemm(cgpu_ctx* c, int L, bool compact, int gemmId, const CUtensorMap& ta, const FxMaps& tb, int bn,
              double* out, const int* expA, const int* expB, unsigned* maxRow, unsigned* maxCol, int segPitchA,
              int segPitch, int aShared, int nSplit, const void* tiles, int nTiles, int* err) {
   if (segPitch % TC_BK != 0 || segPitchA % TC_BK != 0)
@@ -635,8 +651,8 @@ void fx_gemm(cgpu_ctx* c, int L, bool compact, int gemmId, const CUtensorMap& ta
   const FxTile* tl = (const FxTile*)tiles;
 #define FX_CASE(BN_, L_, NA_, NB_, CMP_)                                                                        \
   if (bn == BN_ && L == L_ && compact == CMP_) {                                                                \
-    launch_fx_t<BN_, L_, NA_, NB_>(c, ta, tb, out, expA, expB, maxRow, maxCol, gemmId, segPitchA, segPitch,    \
-                                   aShared, kPer, tl, nTiles, CMP_ ? 2 : 1, err);                              \
+    launch_fx_t<BN_, L_, NA_, NB_>(c, ta, tb, out, expA, expB, maxRow, maxCol, gemmId, segPitchA, aShared,     \
+                                   kPer, tl, nTiles, CMP_ ? 2 : 1, err);                              \
     return;                                                                                                     \
   }
   FX_CASE(32, 4, 0, 2, false) FX_CASE(64, 4, 0, 2, false) FX_CASE(96, 4, 0, 2, false)

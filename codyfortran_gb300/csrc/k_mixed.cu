@@ -57,7 +57,8 @@ struct MixedBufs {
   int L = 0, L2 = 0;
   FxGemm gW, gZ, gH, gWx, gHx;      // the form's three GEMMs; W and h2 at FX_L64 slices for FillH2
   int sCapW = 1, sCapZ = 1, sCapH = 1;  // K splits the FP64 partial buffers hold (the tuner stays within them)
-  CUtensorMap mSx, mSxasB, mWTx;    // S and W^T rows at FX_L64 slices
+  FxMaps bS, bWT, bR, bSx, bWTx;    // B operands (x: at FX_L64 slices)
+  CUtensorMap mSxasB;               // S rows as the A operand at FX_L64 slices
   // one interaction matrix per root grid (cgpu_ctx::fxShared): slices [root][c->nG][FX_L64 KgBig]
   // and row exponents [root][c->nG], outside the per-trajectory arena
   int KgBig = 0;
@@ -752,15 +753,14 @@ void mixed_init(cgpu_ctx* c) {
       CODY_LAUNCHED(c);
       m->mV = tc_make_map(c, m->VxB, c->nG, pV, 128);
     }
-    // A operands in 128-row boxes, B operands in 16-row boxes
-    m->mS = tc_make_map(c, m->SxA, P2, pG, 16);
     m->mSasB = tc_make_map(c, m->SxA, P2, pG, 128);
-    m->mSx = tc_make_map(c, m->SxA, P2, pV, 16);
     m->mSxasB = tc_make_map(c, m->SxA, P2, pV, 128);
-    m->mWT = tc_make_map(c, m->WTxB, P2, pG, 16);
-    m->mWTx = tc_make_map(c, m->WTxB, P2, pV, 16);
     m->mW = tc_make_map(c, m->WxA, c->nG, pP, 128);
-    m->mR = tc_make_map(c, m->RxB, Q2, pP, 16);
+    m->bS = fx_make_maps(c, m->SxA, P2, m->KgMax, L);
+    m->bSx = fx_make_maps(c, m->SxA, P2, m->KgMax, FX_L64);
+    m->bWT = fx_make_maps(c, m->WTxB, P2, m->KgMax, L);
+    m->bWTx = fx_make_maps(c, m->WTxB, P2, m->KgMax, FX_L64);
+    m->bR = fx_make_maps(c, m->RxB, Q2, m->KpMax, m->L2);
     auto tiles = [&](FxGemm& g, int id) { g.tiles = fx_build_tiles(c, id, g.bn, g.s, &g.nTiles); };
     tiles(m->gW, TC_GEMM_W);
     tiles(m->gZ, TC_GEMM_Z);
@@ -795,7 +795,7 @@ static void fx_run_W(cgpu_ctx* c, bool exact) {
   const int nG = c->nG, nP = c->nPairs;
   const FxGemm& g = exact ? m->gWx : m->gW;
   const bool one = g.s == 1;
-  fx_gemm(c, exact ? FX_L64 : m->L, g.compact, TC_GEMM_W, c->fxShared ? m->mVsh : m->mV, exact ? m->mSx : m->mS, g.bn,
+  fx_gemm(c, exact ? FX_L64 : m->L, g.compact, TC_GEMM_W, c->fxShared ? m->mVsh : m->mV, exact ? m->bSx : m->bS, g.bn,
           m->Wd, c->fxShared ? m->eVsh : m->eV, m->eS, one ? m->mWr : nullptr, one ? m->mWc : nullptr,
           c->fxShared ? m->KgBig : m->KgMax, m->KgMax, c->fxShared, g.s, g.tiles, g.nTiles, m->err);
   if (!one) {
@@ -810,7 +810,7 @@ static void fx_run_Z(cgpu_ctx* c) {
   MixedBufs* m = c->mixed;
   const int nG = c->nG, Q = c->nOS * c->nOS;
   const FxGemm& g = m->gZ;
-  fx_gemm(c, m->L2, g.compact, TC_GEMM_Z, m->mW, m->mR, g.bn, g.s > 1 ? m->Zp : m->Zd, m->eWr, m->eR, nullptr, nullptr,
+  fx_gemm(c, m->L2, g.compact, TC_GEMM_Z, m->mW, m->bR, g.bn, g.s > 1 ? m->Zp : m->Zd, m->eWr, m->eR, nullptr, nullptr,
           m->KpMax, m->KpMax, 0, g.s, g.tiles, g.nTiles, m->err);
   if (g.s > 1) {
     k_reduce_Z<<<bgrid(c, ew_blocks(c, (size_t)nG * Q)), 256, 0, c->stream>>>((z_t*)m->Zd, m->Zp, g.s, TRAJ_PASS(c));
@@ -823,7 +823,7 @@ static void fx_run_H2(cgpu_ctx* c, bool exact) {
   MixedBufs* m = c->mixed;
   const int Q = c->nOS * c->nOS;
   const FxGemm& g = exact ? m->gHx : m->gH;
-  fx_gemm(c, exact ? FX_L64 : m->L, g.compact, TC_GEMM_H2, exact ? m->mSxasB : m->mSasB, exact ? m->mWTx : m->mWT, g.bn,
+  fx_gemm(c, exact ? FX_L64 : m->L, g.compact, TC_GEMM_H2, exact ? m->mSxasB : m->mSasB, exact ? m->bWTx : m->bWT, g.bn,
           m->Gd, m->eS, m->eWc, nullptr, nullptr, m->KgMax, m->KgMax, 0, g.s, g.tiles, g.nTiles, m->err);
   k_reduce_H2<<<bgrid(c, ew_blocks(c, (size_t)Q * Q)), 256, 0, c->stream>>>(c->h2s_d, m->Gd, g.s, c->pidx_d,
                                                                       TRAJ_PASS(c));

@@ -218,24 +218,38 @@ CUtensorMap tc_make_map(const cgpu_ctx* c, const __nv_bfloat16* base, int rowsMa
   return tc_make_map_planes(base, rowsMax, pitch, boxRows, c->nb, c->bs);
 }
 
-CUtensorMap tc_make_map_planes(const __nv_bfloat16* base, int rowsMax, int pitch, int boxRows, int planes,
-                               size_t planeBytes) {
+CUtensorMap tc_encode_map(const __nv_bfloat16* base, int rank, const unsigned long long* dims,
+                          const unsigned long long* strides, const unsigned* box) {
   ensure_encode();
-  if (planes > 1 && planeBytes % 16 != 0) throw std::string("tensor map: bad alignment");
-  if (planes == 1) planeBytes = (size_t)pitch * 2 * (size_t)rowsMax;
-  if ((uintptr_t)base % 16 != 0 || pitch % TC_BK != 0 || planeBytes % 16 != 0)
-    throw std::string("tensor map: bad alignment");
+  cuuint64_t d[5], st[4];
+  cuuint32_t bx[5], es[5];
+  for (int i = 0; i < rank; i++) {
+    d[i] = dims[i];
+    bx[i] = box[i];
+    es[i] = 1;
+    if (i + 1 < rank) {
+      st[i] = strides[i];
+      if (st[i] % 16 != 0) throw std::string("tensor map: bad alignment");
+    }
+  }
+  if ((uintptr_t)base % 16 != 0) throw std::string("tensor map: bad alignment");
   CUtensorMap m;
   std::memset(&m, 0, sizeof(m));
-  cuuint64_t dims[3] = {(cuuint64_t)pitch, (cuuint64_t)rowsMax, (cuuint64_t)planes};
-  cuuint64_t strides[2] = {(cuuint64_t)pitch * 2, (cuuint64_t)planeBytes};
-  cuuint32_t box[3] = {(cuuint32_t)TC_BK, (cuuint32_t)boxRows, 1};
-  cuuint32_t es[3] = {1, 1, 1};
-  CUresult r = g_encode(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<__nv_bfloat16*>(base), dims, strides, box,
-                        es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  CUresult r = g_encode(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<__nv_bfloat16*>(base), d, st, bx, es,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) throw std::string("cuda: cuTensorMapEncodeTiled failed");
   return m;
+}
+
+CUtensorMap tc_make_map_planes(const __nv_bfloat16* base, int rowsMax, int pitch, int boxRows, int planes,
+                               size_t planeBytes) {
+  if (planes == 1) planeBytes = (size_t)pitch * 2 * (size_t)rowsMax;
+  if (pitch % TC_BK != 0) throw std::string("tensor map: bad alignment");
+  const unsigned long long dims[3] = {(unsigned long long)pitch, (unsigned long long)rowsMax, (unsigned long long)planes};
+  const unsigned long long strides[2] = {(unsigned long long)pitch * 2, (unsigned long long)planeBytes};
+  const unsigned box[3] = {TC_BK, (unsigned)boxRows, 1};
+  return tc_encode_map(base, 3, dims, strides, box);
 }
 
 void tc_gemm(cgpu_ctx* c, int gemmId, const CUtensorMap& ta, const CUtensorMap& tb, int bn, float* P, int terms,

@@ -26,9 +26,17 @@ void tc_gemm(cgpu_ctx* c, int gemmId, const CUtensorMap& ta, const CUtensorMap& 
 
 // Row exponent of an operand row that holds an infinity or a NaN.
 constexpr int FX_EXP_NAN = 1 << 20;
+// The TMA maps of a fixed-point B operand, one per tile width 16, 32, ...
+constexpr int FX_MAPS = 6;
+struct FxMaps {
+  CUtensorMap m[FX_MAPS];
+};
+FxMaps fx_make_maps(const cgpu_ctx* c, const __nv_bfloat16* base, int rowsMax, int pitch, int L);
+// A bf16 tensor map (128-byte swizzle) of `rank` dimensions; strides in bytes from the second dimension on.
+CUtensorMap tc_encode_map(const __nv_bfloat16* base, int rank, const unsigned long long* dims,
+                          const unsigned long long* strides, const unsigned* box);
 // Fixed-point slice GEMM (k_fx.cu): out[traj][split][M][N] (FP64) = A B^T (the
-// B map with 16-row boxes, the A map with 128-row boxes) for
-// operands carried as L base-256 digit slices (K segments of
+// A map with 128-row boxes) for operands carried as L base-256 digit slices (K segments of
 // segPitchA / segPitch elements) with row exponents expA / expB; maxRow /
 // maxCol (unsplit K only) receive the largest biased exponent of |C| per row /
 // column.  compact: the two-CTAs-per-SM configuration (small K).  aShared: A
@@ -36,7 +44,7 @@ constexpr int FX_EXP_NAN = 1 << 20;
 // nSplit: K splits of the longest contraction (segPitch / 64 K blocks, kPer
 // blocks per split); a trajectory of fewer K blocks takes only the splits its
 // own K needs, balanced, and its remaining partials are written as zeros.
-void fx_gemm(cgpu_ctx* c, int L, bool compact, int gemmId, const CUtensorMap& ta, const CUtensorMap& tb, int bn,
+void fx_gemm(cgpu_ctx* c, int L, bool compact, int gemmId, const CUtensorMap& ta, const FxMaps& tb, int bn,
              double* out, const int* expA, const int* expB, unsigned* maxRow, unsigned* maxCol, int segPitchA,
              int segPitch, int aShared, int nSplit, const void* tiles, int nTiles, int* err);
 // Device list of the fixed-point GEMM's tiles (trajectory, row, column, K split) of the
@@ -120,6 +128,15 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, u
       "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::
           "r"(smem_u32(dst)),
       "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar))
+      : "memory");
+}
+
+__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1,
+                                            int c2, int c3) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::
+          "r"(smem_u32(dst)),
+      "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(bar))
       : "memory");
 }
 
