@@ -322,8 +322,7 @@ struct cgpu_ctx {
   z_t *Rp_d = nullptr;                        // (nOS^2, nOS^2) correlation matrix
   z_t *h2s_d = nullptr;                       // (nOS^2, nOS^2) spatial h2 block
   z_t *Mreg_d = nullptr;                      // (nOS, nOS)
-  z_t *Uprev_d = nullptr;                     // (nOS, nOS) natural orbitals of the previous rho^-1 call
-  z_t *r1s_d = nullptr;                       // spin-summed spatial rdm1
+  z_t *Uprev_d = nullptr;                     // (nOS, nOS) natural orbitals of the previous occupations call
   z_t *r2s_d = nullptr;                       // spin-summed spatial rdm2 (nOS^2 x nOS^2)
   // reductions / scratch
   z_t* partial_d = nullptr;
@@ -474,6 +473,7 @@ void launch_pair_potentials(cgpu_ctx* c, const z_t* orbs);
 void launch_correlation(cgpu_ctx* c, z_t* dOrbs, const z_t* orbs, int wantH2);
 void launch_fill_h2(cgpu_ctx* c, const z_t* orbs);
 void launch_rdm_inverse(cgpu_ctx* c);
+void launch_rdm_occupations(cgpu_ctx* c);
 void launch_corr_epilogue(cgpu_ctx* c, z_t* dOrbs, const z_t* orbs, const z_t* Z);
 void launch_h2_layout(cgpu_ctx* c);
 void launch_build_vint(cgpu_ctx* c);

@@ -357,7 +357,6 @@ size_t layout(cgpu_ctx* c, char* base) {
   Z(c->h2s_d, Q * Q);
   Z(c->Mreg_d, Q);
   Z(c->Uprev_d, Q);
-  Z(c->r1s_d, Q);
   Z(c->r2s_d, Q * Q);
   Z(c->gram_d, Q);
   Z(c->orbTmp_d, nG * n);
@@ -1109,7 +1108,7 @@ void observables(cgpu_ctx* c, const double* tHost, double* out) {
   }
   c->useStepTime = 0;
   const bool occ = c->method != CGPU_METHOD_TDCI && c->nOS <= 32;
-  if (occ) launch_rdm_inverse(c);
+  if (occ) launch_rdm_occupations(c);
   launch_norm_dipole(c, c->state_d);
   std::vector<double> rows((size_t)c->nb * 64);
   CODY_CUDA(cudaMemcpy2DAsync(rows.data(), 64 * sizeof(double), c->scal_d, c->bs, 64 * sizeof(double), c->nb,

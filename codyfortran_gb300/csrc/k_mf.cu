@@ -18,7 +18,7 @@
 //   h2[(i1,j1),(l2,k2)] = 1/2 sum_g S[g,(i1,j1)] W[g,(l2,k2)]  (ZGEMM^T, FillH2Block)
 //
 // plus the regularised inverse of the one-body RDM (RdmDiagonalize_Rdm1 +
-// regInvMat, :722-754) by a parallel cyclic Jacobi eigensolver in one CTA.
+// regInvMat, :722-754).
 // Every kernel covers all trajectories of the context (blockIdx.z).
 #include <algorithm>
 
@@ -246,8 +246,8 @@ __global__ void k_split_reduce(z_t* __restrict__ C, const z_t* __restrict__ P, i
 }
 
 // ---------------------------------------------------------------------------
-// Regularised inverse of the spin-summed one-body RDM (one CTA per trajectory).
-// Parallel cyclic Jacobi (round-robin pairing), complex Hermitian n <= 32.
+// Natural occupations: eigenvalues of the spin-summed one-body RDM (one CTA per
+// trajectory).  Parallel cyclic Jacobi (round-robin pairing), complex Hermitian n <= 32.
 // ---------------------------------------------------------------------------
 constexpr int JB_MAX = 32;
 
@@ -256,22 +256,18 @@ constexpr int JB_MAX = 32;
 // is nearly diagonal between consecutive evaluations, so it converges in a few
 // sweeps; Uprev V is stored for the next call.  Uprev is re-orthonormalised
 // (one modified Gram-Schmidt pass) on load so rounding cannot accumulate.
-// The result Mreg = U f(n) U^H depends only on rho (to rounding).
-__global__ void __launch_bounds__(512) k_rdm_inverse(z_t* __restrict__ Mreg, z_t* __restrict__ r1s,
-                                                     const z_t* __restrict__ rdm1, z_t* __restrict__ Uprev,
-                                                     double* __restrict__ occ, TRAJ_ARGS) {
+// The eigenvalues depend only on rho (to rounding).
+__global__ void __launch_bounds__(512) k_rdm_occupations(const z_t* __restrict__ rdm1, z_t* __restrict__ Uprev,
+                                                         double* __restrict__ occ, TRAJ_ARGS) {
   extern __shared__ z_t jsm[];
   const TrajShape& T = shp[blockIdx.z];
   const int nO = T.nO, n = T.nOS, restricted = T.restricted;
-  const double reg = T.regEps;
-  Mreg = bat(Mreg, bs);
-  r1s = bat(r1s, bs);
   rdm1 = bat(rdm1, bs);
   Uprev = bat(Uprev, bs);
   z_t(*A)[JB_MAX + 1] = reinterpret_cast<z_t(*)[JB_MAX + 1]>(jsm);
   z_t(*V)[JB_MAX + 1] = reinterpret_cast<z_t(*)[JB_MAX + 1]>(jsm + JB_MAX * (JB_MAX + 1));
   z_t(*U)[JB_MAX + 1] = reinterpret_cast<z_t(*)[JB_MAX + 1]>(jsm + 2 * JB_MAX * (JB_MAX + 1));
-  __shared__ double rc[JB_MAX / 2], rs[JB_MAX / 2], ev[JB_MAX];
+  __shared__ double rc[JB_MAX / 2], rs[JB_MAX / 2];
   __shared__ z_t rph[JB_MAX / 2];
   __shared__ int rp[JB_MAX / 2], rq[JB_MAX / 2];
   __shared__ double offs, diags;
@@ -281,7 +277,6 @@ __global__ void __launch_bounds__(512) k_rdm_inverse(z_t* __restrict__ Mreg, z_t
     z_t v = rdm1[i + (size_t)nO * j];
     if (restricted) v = zadd(v, rdm1[(n + i) + (size_t)nO * (n + j)]);
     A[i][j] = v;
-    r1s[e] = v;
     U[i][j] = Uprev[i + (size_t)n * j];
   }
   __syncthreads();
@@ -333,15 +328,20 @@ __global__ void __launch_bounds__(512) k_rdm_inverse(z_t* __restrict__ Mreg, z_t
   int ne = (n + 1) & ~1;
   int half = ne / 2;
   for (int sweep = 0; sweep < 30; sweep++) {
-    if (tid == 0) {
+    if (tid < 32) {  // row sums by lane, then a fixed-order tree
       double off = 0.0, dg = 0.0;
-      for (int j = 0; j < n; j++)
-        for (int i = 0; i < n; i++) {
-          double a2 = A[i][j].x * A[i][j].x + A[i][j].y * A[i][j].y;
-          if (i == j) dg += a2; else off += a2;
-        }
-      offs = off;
-      diags = dg;
+      for (int i = 0; i < n && tid < n; i++) {
+        double a2 = A[i][tid].x * A[i][tid].x + A[i][tid].y * A[i][tid].y;
+        if (i == tid) dg += a2; else off += a2;
+      }
+      for (int o = 16; o > 0; o >>= 1) {
+        off += __shfl_xor_sync(0xffffffffu, off, o);
+        dg += __shfl_xor_sync(0xffffffffu, dg, o);
+      }
+      if (tid == 0) {
+        offs = off;
+        diags = dg;
+      }
     }
     __syncthreads();
     if (offs <= 1e-28 * (diags + offs) || offs == 0.0) break;  // rounding floor is ~1e-32
@@ -412,31 +412,106 @@ __global__ void __launch_bounds__(512) k_rdm_inverse(z_t* __restrict__ Mreg, z_t
       __syncthreads();
     }
   }
-  // eigenvalues, eigenvectors U_new = U V (into A), stored for the next call
+  // eigenvalues; eigenvectors U V, stored for the next call
   occ = bat(occ, bs);
-  for (int e = tid; e < n; e += blockDim.x) {
-    ev[e] = A[e][e].x;
-    occ[e] = ev[e];  // natural occupations (eigenvalues of the spin-summed rho1, unsorted)
-  }
-  __syncthreads();
+  for (int e = tid; e < n; e += blockDim.x) occ[e] = A[e][e].x;
   for (int e = tid; e < n * n; e += blockDim.x) {
     int i = e % n, j = e / n;
     z_t s = zmk(0.0, 0.0);
     for (int k = 0; k < n; k++) zfma(s, U[i][k], V[k][j]);
-    A[i][j] = s;
     Uprev[i + (size_t)n * j] = s;
   }
-  __syncthreads();
-  // Mreg(k1,j1) = sum_j U(k1,j) n_j/(n_j^2+reg) conj(U(j1,j))
+}
+
+// Mreg = U f(n) U^H, f(n) = n / (n^2 + eps), without the eigenvectors: with s =
+// sqrt(eps), f(n) = Re 1 / (n + i s), so Mreg is the Hermitian part of
+// (rho + i s)^-1, one n x n complex inverse.  Its error, about 2^-53 ||rho|| /
+// |n_k + i s| in the component of an occupation n_k, is the one that an
+// eigenvalue's absolute error gives f(n_k).  Gauss-Jordan in shared memory with
+// partial pivoting: per column, warp 0 finds the pivot, swaps the rows and
+// scales the pivot row, then the block updates (4 n^2 FP64 FMA a column at two a
+// cycle: the FP64 pipe and n pivot chains of about 600 cycles bound it).  The
+// Jacobi sweeps (k_rdm_occupations) take 4 n^3 FMA each and several of them:
+// 437 -> 23 us at n = 16, 303 -> 18 in a batch of 24 with n <= 12.
+__global__ void __launch_bounds__(256) k_rdm_inverse(z_t* __restrict__ Mreg, const z_t* __restrict__ rdm1,
+                                                     TRAJ_ARGS) {
+  __shared__ z_t A[JB_MAX][JB_MAX + 1];
+  __shared__ z_t row[JB_MAX], col[JB_MAX];
+  __shared__ int perm[JB_MAX];
+  const TrajShape& T = shp[blockIdx.z];
+  const int nO = T.nO, n = T.nOS, restricted = T.restricted, tid = threadIdx.x;
+  const double s = sqrt(T.regEps);
+  Mreg = bat(Mreg, bs);
+  rdm1 = bat(rdm1, bs);
+  auto rho = [&](int i, int j) {
+    z_t v = rdm1[i + (size_t)nO * j];
+    if (restricted) v = zadd(v, rdm1[(n + i) + (size_t)nO * (n + j)]);
+    return v;
+  };
   for (int e = tid; e < n * n; e += blockDim.x) {
-    int k1 = e % n, j1 = e / n;
-    z_t acc = zmk(0.0, 0.0);
-    for (int j = 0; j < n; j++) {
-      double occ = ev[j];
-      double f = occ / (occ * occ + reg);
-      zfma(acc, zscale(A[k1][j], f), zconj(A[j1][j]));
+    const int i = e % n, j = e / n;
+    const z_t v = rho(i, j);
+    A[i][j] = i == j ? zmk(v.x, s) : v;
+  }
+  if (tid < n) perm[tid] = tid;
+  __syncthreads();
+  for (int k = 0; k < n; k++) {
+    if (tid < 32) {
+      const int l = tid;
+      z_t ck = l < n ? A[l][k] : zmk(0.0, 0.0);
+      // pivot: the largest |re| + |im| at or below the diagonal, by its FP32 size (any near-largest entry serves)
+      float mag = l >= k && l < n ? fabsf((float)ck.x) + fabsf((float)ck.y) : -1.0f;
+      int p = l;
+      for (int o = 16; o > 0; o >>= 1) {
+        const float m2 = __shfl_xor_sync(0xffffffffu, mag, o);
+        const int p2 = __shfl_xor_sync(0xffffffffu, p, o);
+        if (m2 > mag || (m2 == mag && p2 < p)) {
+          mag = m2;
+          p = p2;
+        }
+      }
+      if (!(mag >= 0.0f) || p < k || p >= n) p = k;  // NaN entries: any pivot, the result is NaN
+      const z_t a = A[p][k];
+      const double d = 1.0 / fma(a.x, a.x, a.y * a.y);
+      const z_t inv = zmk(a.x * d, -a.y * d);
+      __syncwarp();  // every lane has read A[p][k] and column k
+      if (l < n) {
+        const z_t t = A[p][l], u = A[k][l];
+        row[l] = l == k ? inv : zmul(t, inv);
+        if (p != k) A[p][l] = u;
+        // column k as the update reads it: the old row k now sits in row p
+        col[l] = l == p ? A[k][k] : ck;
+        if (p == k) col[l] = ck;
+      }
+      if (l == 0 && p != k) {
+        const int q = perm[k];
+        perm[k] = perm[p];
+        perm[p] = q;
+      }
     }
-    Mreg[e] = acc;
+    __syncthreads();
+    for (int e = tid; e < n * n; e += blockDim.x) {
+      const int i = e / n, j = e - i * n;
+      if (i == k) {
+        A[k][j] = row[j];
+      } else {
+        z_t v = j == k ? zmk(0.0, 0.0) : A[i][j];
+        const z_t c = col[i], r = row[j];
+        v.x = fma(-c.x, r.x, fma(c.y, r.y, v.x));
+        v.y = fma(-c.x, r.y, fma(-c.y, r.x, v.y));
+        A[i][j] = v;
+      }
+    }
+    __syncthreads();
+  }
+  // A holds (P B)^-1: column r of it is column perm[r] of B^-1
+  __shared__ int at[JB_MAX];
+  if (tid < n) at[perm[tid]] = tid;
+  __syncthreads();
+  for (int e = tid; e < n * n; e += blockDim.x) {
+    const int i = e % n, j = e / n;
+    const z_t v = A[i][at[j]], w = A[j][at[i]];
+    Mreg[e] = zmk(0.5 * (v.x + w.x), 0.5 * (v.y - w.y));
   }
 }
 
@@ -603,18 +678,25 @@ static void h2_from_pairs(cgpu_ctx* c) {
   launch_h2_layout(c);
 }
 
+void launch_rdm_occupations(cgpu_ctx* c) {
+  ProfScope prof(c, CGPU_KERNEL_RDM_INVERSE);
+  if (c->nOS > JB_MAX) throw std::string("natural occupations: more than 32 stored orbitals is not supported");
+  constexpr size_t jsmem = 3 * sizeof(z_t) * JB_MAX * (JB_MAX + 1);
+  static bool attr = false;
+  if (!attr) {
+    CODY_CUDA(cudaFuncSetAttribute(k_rdm_occupations, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jsmem));
+    attr = true;
+  }
+  k_rdm_occupations<<<bgrid(c, 1), 512, jsmem, c->stream>>>(c->rdm1_d, c->Uprev_d, c->scal_d + CODY_SCAL_OCC,
+                                                            TRAJ_PASS(c));
+  CODY_LAUNCHED(c);
+}
+
 void launch_rdm_inverse(cgpu_ctx* c) {
   ProfScope prof(c, CGPU_KERNEL_RDM_INVERSE);
   int n = c->nOS;
   if (n > JB_MAX) throw std::string("ApplyCorrelationOp: more than 32 stored orbitals is not supported");
-  constexpr size_t jsmem = 3 * sizeof(z_t) * JB_MAX * (JB_MAX + 1);
-  static bool attr = false;
-  if (!attr) {
-    CODY_CUDA(cudaFuncSetAttribute(k_rdm_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jsmem));
-    attr = true;
-  }
-  k_rdm_inverse<<<bgrid(c, 1), 512, jsmem, c->stream>>>(c->Mreg_d, c->r1s_d, c->rdm1_d, c->Uprev_d,
-                                                        c->scal_d + CODY_SCAL_OCC, TRAJ_PASS(c));
+  k_rdm_inverse<<<bgrid(c, 1), 256, 0, c->stream>>>(c->Mreg_d, c->rdm1_d, TRAJ_PASS(c));
   CODY_LAUNCHED(c);
   size_t Q = (size_t)n * n;
   if (c->fuseLayouts)

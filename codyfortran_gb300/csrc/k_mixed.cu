@@ -765,8 +765,10 @@ void mixed_init(cgpu_ctx* c) {
     tiles(m->gW, TC_GEMM_W);
     tiles(m->gZ, TC_GEMM_Z);
     tiles(m->gH, TC_GEMM_H2);
-    tiles(m->gWx, TC_GEMM_W);
-    tiles(m->gHx, TC_GEMM_H2);
+    if (L != FX_L64) {  // the FP64 form's FillH2 uses its own gW, gH
+      tiles(m->gWx, TC_GEMM_W);
+      tiles(m->gHx, TC_GEMM_H2);
+    }
   } else {
     const int T = m->terms, pG = T * m->KgMax, pP = T * m->KpMax;
     k_split_V<<<bgrid(c, ew_blocks(c, (size_t)c->nG * m->KgMax)), 256, 0, c->stream>>>(m->VxB, c->Vint_d, m->KgMax, T,
@@ -793,7 +795,7 @@ int mixed_error(cgpu_ctx* c) { return c->mixed && c->mixed->err_h ? *c->mixed->e
 static void fx_run_W(cgpu_ctx* c, bool exact) {
   MixedBufs* m = c->mixed;
   const int nG = c->nG, nP = c->nPairs;
-  const FxGemm& g = exact ? m->gWx : m->gW;
+  const FxGemm& g = exact && m->L != FX_L64 ? m->gWx : m->gW;
   const bool one = g.s == 1;
   fx_gemm(c, exact ? FX_L64 : m->L, g.compact, TC_GEMM_W, c->fxShared ? m->mVsh : m->mV, exact ? m->bSx : m->bS, g.bn,
           m->Wd, c->fxShared ? m->eVsh : m->eV, m->eS, one ? m->mWr : nullptr, one ? m->mWc : nullptr,
@@ -822,7 +824,7 @@ static void fx_run_Z(cgpu_ctx* c) {
 static void fx_run_H2(cgpu_ctx* c, bool exact) {
   MixedBufs* m = c->mixed;
   const int Q = c->nOS * c->nOS;
-  const FxGemm& g = exact ? m->gHx : m->gH;
+  const FxGemm& g = exact && m->L != FX_L64 ? m->gHx : m->gH;
   fx_gemm(c, exact ? FX_L64 : m->L, g.compact, TC_GEMM_H2, exact ? m->mSxasB : m->mSasB, exact ? m->bWTx : m->bWT, g.bn,
           m->Gd, m->eS, m->eWc, nullptr, nullptr, m->KgMax, m->KgMax, 0, g.s, g.tiles, g.nTiles, m->err);
   k_reduce_H2<<<bgrid(c, ew_blocks(c, (size_t)Q * Q)), 256, 0, c->stream>>>(c->h2s_d, m->Gd, g.s, c->pidx_d,
