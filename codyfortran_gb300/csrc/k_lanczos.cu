@@ -482,6 +482,7 @@ __global__ void __launch_bounds__(LZ_THREADS) k_lz3_dot(z_t* __restrict__ part, 
   const TrajShape& S = shp[blockIdx.z];
   lz = bat(lz, bs);
   if (lz[LZ_DONE] != 0.0) return;
+  part = bat(part, bs);
   vCur = bat(vCur, bs);
   w = bat(w, bs);
   m = bat(m, bs);
