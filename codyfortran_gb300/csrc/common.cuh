@@ -216,6 +216,28 @@ struct TrajShape {
   CiView view;
 };
 
+// Laser field E(t): sin^2 pulse (pattern of src/SysPotential/Ylm/CoulombLaser/
+// S_SysPotential_Ylm_CoulombLaser.f90:60-83) or piecewise-constant samples.
+__device__ inline double field_amplitude_dev(const LaserDev& L, double t) {
+  if (L.kind == CGPU_LASER_SIN2) {
+    if (L.omega <= 0.0) return 0.0;
+    const double PI = 3.14159265358979323846264338327950288;
+    double duration = 2.0 * PI * L.nCycles / L.omega;
+    double tRel = t - L.tStart;
+    if (tRel < 0.0 || tRel > duration) return 0.0;
+    double env = sin(PI * tRel / duration);
+    env = env * env;
+    return L.E0 * env * cos(L.omega * (tRel - 0.5 * duration) + L.cep);
+  }
+  if (L.kind == CGPU_LASER_SAMPLED) {
+    double u = (t - L.sampleT0) / L.sampleDt;
+    long n = (long)floor(u + 1e-9);
+    if (n < 0 || n >= L.nSamples) return 0.0;
+    return L.samples[n];
+  }
+  return 0.0;
+}
+
 // Pointer p of trajectory 0 moved to the trajectory of this block.
 template <class T>
 __device__ __forceinline__ T* bat(T* p, size_t bs) {
@@ -345,6 +367,14 @@ struct cgpu_ctx {
   std::vector<int> fxVRow, fxVRoot, fxRoots;  // per trajectory: row offset, root index; per root: trajectory
   double* lz_d = nullptr;   // Lanczos scalars: alpha, beta, dots, phi, flags
   double* lz_h = nullptr;   // pinned mirror (trajectory 0)
+  // k_sil.cu: blocks of the one-launch SIL (0: not used), the largest piece of a block
+  int silBlocks = 0, silCap = 0;
+  void* silBlk_d = nullptr;
+  z_t* silPart_d = nullptr;
+  unsigned* silBar_d = nullptr;
+  // page-locked host words that kernels write: [0] error of a bounded wait, [1] warnings of the last adaptive SIL
+  volatile int* flags_h = nullptr;
+  int* flags_d = nullptr;
   // TDCI static data
   z_t* tdciOrbs_d = nullptr;
   // stream / graph
@@ -527,8 +557,15 @@ void launch_lanczos_update(cgpu_ctx* c, int j, int maxDim, int pass1Blocks = 0);
 void launch_lanczos_tail(cgpu_ctx* c, int j, double dt, int evalExp);  // j = 0: use the device mDim
 void launch_lanczos_combine(cgpu_ctx* c, z_t* out, const z_t* start);
 void launch_lz_set(cgpu_ctx* c, int idx, double v);
+// k_sil.cu: SIL on OrbsLin in one launch (silBlocks > 0), on c->metric_d; the
+// exponential of the launch-per-pass form
+void sil_init(cgpu_ctx* c);
+void sil_free(cgpu_ctx* c);
+void launch_sil(cgpu_ctx* c, z_t* state, double t, double dt, int K, double tol, int maxRestarts);
+void launch_lz_expsub(cgpu_ctx* c, int j, double dt);
 size_t lanczos_partial_need(const cgpu_ctx* c);
 #define CODY_LZ_BETA 64
+#define CODY_LZ_PHI 256
 #define CODY_LZ_S 400
 #define CODY_LZ_ERR 385
 #define CODY_LZ_MDIM 386

@@ -598,12 +598,22 @@ void build_ctx(cgpu_ctx* c, const cgpu_desc* descs, int nSys) {
   c->stageOff = so;
   CODY_CUDA(cudaMemcpy(c->stageOff_d, so.data(), sizeof(long) * (nSys + 1), cudaMemcpyHostToDevice));
   mixed_init(c);
+  sil_init(c);
+  {
+    void* h = nullptr;
+    CODY_CUDA(cudaHostAlloc(&h, sizeof(int) * 2, cudaHostAllocMapped));
+    c->flags_h = (volatile int*)h;
+    c->flags_h[0] = c->flags_h[1] = 0;
+    CODY_CUDA(cudaHostGetDevicePointer((void**)&c->flags_d, h, 0));
+  }
   CODY_CUDA(cudaMallocHost(&c->lz_h, sizeof(double) * 512));
   CODY_CUDA(cudaDeviceSynchronize());
 }
 
 void free_ctx(cgpu_ctx* c) {
   mixed_free(c);
+  sil_free(c);
+  if (c->flags_h) cudaFreeHost((void*)c->flags_h);
   mc_adjoint_free(c);
   if (c->stepGraph) cudaGraphExecDestroy(c->stepGraph);
   for (cudaEvent_t e : c->profEvents) cudaEventDestroy(e);
@@ -706,6 +716,8 @@ void euler_device(cgpu_ctx* c, int which, int imag, z_t* state, double t0, doubl
   launch_axpby(c, state, c->dstate_d, zmk(t1 - t0, 0.0), zmk(1.0, 0.0), VSEL_STATE);
 }
 
+void sync(cgpu_ctx* c);
+
 // One PerformLanczosStep from start (device) into out (may be start itself).
 // Returns converged (adaptive) or -1 (not checked).
 int lanczos_pass(cgpu_ctx* c, int which, double tBase, double dt, int maxDim, double tol, double* errOut,
@@ -748,14 +760,23 @@ int lanczos_pass(cgpu_ctx* c, int which, double tBase, double dt, int maxDim, do
 }
 
 // SIL Integrate (src/IntegratorList/Sil/S_IntegratorList_Sil.f90:114-177) on a device state.
+// Returns the passes that did not converge (wantWarnings; else it may return before they are known).
 int sil_device(cgpu_ctx* c, int which, z_t* state, double t0, double t1, int krylovDim, double tol, int maxRestarts,
-               const double* metric_d) {
+               const double* metric_d, bool wantWarnings = false) {
   const double zeroThreshold = 1.0e-14;
   if (std::fabs(t1 - t0) <= zeroThreshold) return 0;
   int maxDim = std::max(1, std::min(krylovDim, c->minS));
   if (maxDim > c->maxKrylov) throw std::string("SIL: krylovDim exceeds the context's max_krylov");
   c->metric_d = const_cast<double*>(metric_d);
   int warnings = 0;
+  if (tol > 0.0 && c->nb > 1) throw std::string("SIL: adaptive (tolerance > 0) steps need a single system");
+  if (which == CGPU_TD_ORBS_LIN && c->silBlocks > 0) {
+    launch_sil(c, state, t0, t1 - t0, maxDim, tol, maxRestarts);
+    if (!(tol > 0.0)) return 1;
+    if (!wantWarnings) return 0;
+    sync(c);
+    return c->flags_h[1];
+  }
   if (!(tol > 0.0)) {
     // fixed order: one pass, no acceptance test; the basis holds the start
     // vector, so the pass reads and overwrites the state in place (the
@@ -1044,6 +1065,7 @@ std::string traj_prefix(const char* dir, int b, bool create) {
 
 void sync(cgpu_ctx* c) {
   CODY_CUDA(cudaStreamSynchronize(c->stream));
+  if (c->flags_h && c->flags_h[0]) throw std::string("SIL: a bounded wait between blocks expired");
   if (c->mixed && mixed_error(c)) throw std::string("tensor-core GEMM: a bounded mbarrier wait expired");
 }
 
@@ -1445,7 +1467,7 @@ int cgpu_integrate_sil(cgpu_ctx* c, int which, cgpu_complex* state, double t0, d
     CODY_CUDA(cudaMemcpyAsync(c->metricUser_d, metric, sizeof(double) * c->nS, cudaMemcpyHostToDevice, c->stream));
     m = c->metricUser_d;
   }
-  int w = sil_device(c, which, c->state_d, t0, t1, krylov_dim, tolerance, max_restarts, m);
+  int w = sil_device(c, which, c->state_d, t0, t1, krylov_dim, tolerance, max_restarts, m, warnings != nullptr);
   if (warnings) *warnings = w;
   down(c, state, c->state_d, c->nS);
   sync(c);

@@ -1,4 +1,4 @@
-// k_lanczos.cu -- short-iterative-Lanczos kernels
+// k_lanczos.cu -- short-iterative-Lanczos kernels, one launch per pass
 // (PerformLanczosStep / EvaluateExpInSubspace / MetricDot,
 //  src/IntegratorList/Sil/S_IntegratorList_Sil.f90:184-310).
 //
@@ -20,6 +20,9 @@
 // per-block partials in a fixed order, re-summed identically by every
 // consumer block.
 //
+// This form serves batches of more trajectories than SMs and Krylov steps of
+// derivatives other than the one-body part; the others run in k_sil.cu.
+//
 // Device scalar block lz[] (doubles):
 #include <algorithm>
 
@@ -40,7 +43,9 @@ constexpr int LZ_DT = 389;      // dt of the current sub-step
 constexpr int LZ_BREAKJ = 390;  // iteration at which breakdown happened
 constexpr int LZ_S = 400;       // scale of basis slot k: v_(k+1) = s_k u_k  [400, 433)
 constexpr int LZ_SMAX = 33;
-static_assert(LZ_S == CODY_LZ_S && LZ_BETA == CODY_LZ_BETA && LZ_DONE == CODY_LZ_DONE, "Lanczos scalar slots");
+static_assert(LZ_S == CODY_LZ_S && LZ_BETA == CODY_LZ_BETA && LZ_DONE == CODY_LZ_DONE && LZ_PHI == CODY_LZ_PHI &&
+                  LZ_ALPHA == 0,
+              "Lanczos scalar slots");
 
 constexpr int LZ_THREADS = 256;
 
@@ -266,117 +271,6 @@ __global__ void k_lz_mark_done(double* lz, int j, size_t bs) {
   lz = bat(lz, bs);
   if (lz[LZ_DONE] == 0.0 && lz[LZ_BREAKJ] == (double)j) lz[LZ_DONE] = 1.0;
 }
-
-// EvaluateExpInSubspace: phi = exp(-i dt T_m) e1 for the m x m Lanczos
-// tridiagonal T_m and the error estimate beta_m |phi_m|.  The reference
-// diagonalises T_m (DSYEV) and forms U exp(-i dt L) U^T e1; the same vector is
-// computed here without an eigensolver, by the Chebyshev (Jacobi-Anger)
-// expansion of the exponential (Tal-Ezer & Kosloff, J. Chem. Phys. 81, 3967 (1984)):
-//   T' = (T - c)/R with spectrum in [-1, 1] (Gershgorin bounds),
-//   exp(-i z x) = J_0(z) + 2 sum_k (-i)^k J_k(z) T_k(x),  z = dt R,
-//   phi = exp(-i dt c) sum_k a_k q_k,  q_0 = e1, q_1 = T' e1, q_{k+1} = 2 T' q_k - q_{k-1}.
-// The Bessel values J_k(z) come from Miller's backward recurrence normalised
-// by J_0 + 2 sum J_2k = 1.  The series is summed until the coefficients fall
-// below 1e-17 relative, i.e. to machine precision.  One warp, lane i = row i (m <= 32).
-__global__ void k_lz_expsub(double* __restrict__ lz, int mFixed, double dt, double tol, size_t bs) {
-  constexpr int KMAX = 1200;
-  lz = bat(lz, bs);
-  __shared__ double J[KMAX + 2];
-  __shared__ int nTerms;
-  int lane = threadIdx.x;
-  int m = mFixed > 0 ? mFixed : (int)lz[LZ_MDIM];
-  if (m > 32) m = 32;
-  if (m < 1) return;
-  double a = (lane < m) ? lz[LZ_ALPHA + lane] : 0.0;
-  double bl = (lane >= 1 && lane < m) ? lz[LZ_BETA + lane - 1] : 0.0;  // beta_{i-1}: couples i-1, i
-  double br = (lane + 1 < m) ? lz[LZ_BETA + lane] : 0.0;               // beta_i:   couples i, i+1
-  double lo = (lane < m) ? a - fabs(bl) - fabs(br) : 1e300;
-  double hi = (lane < m) ? a + fabs(bl) + fabs(br) : -1e300;
-  for (int o = 16; o > 0; o >>= 1) {
-    lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-    hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-  }
-  double c = 0.5 * (hi + lo);
-  double R = 0.5 * (hi - lo);
-  R = R * (1.0 + 1e-12) + 1e-300;
-  double z = fabs(dt) * R;
-  double sgn = dt >= 0.0 ? 1.0 : -1.0;  // exp(-i dt T) with dt < 0 is the complex conjugate series
-  if (lane == 0) {
-    int K = (int)(1.5 * z + 40.0);
-    if (K > KMAX - 20) K = KMAX - 20;
-    if (z < 1e-300) {
-      J[0] = 1.0;
-      for (int k = 1; k <= K; k++) J[k] = 0.0;
-    } else {
-      int N = K + 20;
-      double jp = 0.0, jc = 1e-280, norm = 0.0;
-      for (int k = N; k >= 1; k--) {
-        double jm = (2.0 * k / z) * jc - jp;  // J_{k-1}
-        jp = jc;
-        jc = jm;
-        if (k - 1 <= K) J[k - 1] = jc;
-        if (k - 1 >= 1 && ((k - 1) & 1) == 0) norm += 2.0 * jc;
-        if (fabs(jc) > 1e250) {  // rescale to keep the recurrence finite
-          double s = 1e-250;
-          jc *= s;
-          jp *= s;
-          norm *= s;
-          for (int q = k - 1; q <= K && q <= N; q++) J[q] *= s;
-        }
-      }
-      norm += jc;  // J_0
-      for (int k = 0; k <= K; k++) J[k] /= norm;
-    }
-    int n = K;  // |J_k(z)| <= 1, so an absolute cut-off is relative to the largest term
-    while (n > 1 && fabs(J[n]) < 1e-18 && n > z) n--;
-    nTerms = n;
-  }
-  __syncwarp();
-  int K = nTerms;
-  double inv = 1.0 / R;
-  double ta = (a - c) * inv, tl = bl * inv, tr = br * inv;
-  // q_0 = e1, q_1 = T' e1
-  double qm = (lane == 0) ? 1.0 : 0.0;
-  double qlm = __shfl_up_sync(0xffffffffu, qm, 1);
-  double qrm = __shfl_down_sync(0xffffffffu, qm, 1);
-  double q = ta * qm + tl * (lane >= 1 ? qlm : 0.0) + tr * (lane + 1 < m ? qrm : 0.0);
-  if (lane >= m) q = 0.0;
-  double pr = J[0] * qm, pi = 0.0;
-  // a_k = 2 (-i)^k J_k: k = 1 -> -2i J_1
-  pi += -2.0 * J[1] * q;
-  for (int k = 2; k <= K; k++) {
-    double ql = __shfl_up_sync(0xffffffffu, q, 1);
-    double qr = __shfl_down_sync(0xffffffffu, q, 1);
-    double qn = 2.0 * (ta * q + tl * (lane >= 1 ? ql : 0.0) + tr * (lane + 1 < m ? qr : 0.0)) - qm;
-    if (lane >= m) qn = 0.0;
-    qm = q;
-    q = qn;
-    double co = 2.0 * J[k];
-    switch (k & 3) {
-      case 0: pr += co * q; break;   // (-i)^k = 1
-      case 1: pi -= co * q; break;   // -i
-      case 2: pr -= co * q; break;   // -1
-      default: pi += co * q; break;  // +i
-    }
-  }
-  pi *= sgn;
-  // phase exp(-i dt c)
-  double sn, cs;
-  sincos(dt * c, &sn, &cs);
-  double fr = cs * pr + sn * pi;
-  double fi = cs * pi - sn * pr;
-  if (lane < m) {
-    lz[LZ_PHI + 2 * lane] = fr;
-    lz[LZ_PHI + 2 * lane + 1] = fi;
-  }
-  if (lane == m - 1) {
-    double err = lz[LZ_BETA + m - 1] * sqrt(fr * fr + fi * fi);
-    if (lz[LZ_BREAKJ] == (double)m) err = 0.0;
-    lz[LZ_ERR] = err;
-    (void)tol;
-  }
-}
-
 
 // out = nrm * sum_{j < mDim} phi_j s_j V_j   (or out = in when the start vector had zero norm)
 // DF: the sum in double-float arithmetic on the orbital entries (the
@@ -728,8 +622,7 @@ void launch_lanczos_update(cgpu_ctx* c, int j, int maxDim, int pass1Blocks) {
 void launch_lanczos_tail(cgpu_ctx* c, int j, double dt, int evalExp) {
   ProfScope prof(c, CGPU_KERNEL_VECTOR);
   if (!evalExp) return;
-  k_lz_expsub<<<bgrid(c, 1), 32, 0, c->stream>>>(c->lz_d, j, dt, 0.0, c->bs);
-  CODY_LAUNCHED(c);
+  launch_lz_expsub(c, j, dt);
 }
 
 void launch_lanczos_combine(cgpu_ctx* c, z_t* out, const z_t* start) {

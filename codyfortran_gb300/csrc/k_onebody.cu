@@ -27,28 +27,6 @@ constexpr int RED_BLOCKS = 148;  // partial-sum blocks for grid reductions (one 
 // multiplies orbs[g+d].  One CTA covers OB_THREADS grid points of one orbital;
 // the tile and its halo are staged in shared memory.
 // ---------------------------------------------------------------------------
-// Laser field E(t): sin^2 pulse (pattern of src/SysPotential/Ylm/CoulombLaser/
-// S_SysPotential_Ylm_CoulombLaser.f90:60-83) or piecewise-constant samples.
-__device__ double field_amplitude_dev(const LaserDev& L, double t) {
-  if (L.kind == CGPU_LASER_SIN2) {
-    if (L.omega <= 0.0) return 0.0;
-    const double PI = 3.14159265358979323846264338327950288;
-    double duration = 2.0 * PI * L.nCycles / L.omega;
-    double tRel = t - L.tStart;
-    if (tRel < 0.0 || tRel > duration) return 0.0;
-    double env = sin(PI * tRel / duration);
-    env = env * env;
-    return L.E0 * env * cos(L.omega * (tRel - 0.5 * duration) + L.cep);
-  }
-  if (L.kind == CGPU_LASER_SAMPLED) {
-    double u = (t - L.sampleT0) / L.sampleDt;
-    long n = (long)floor(u + 1e-9);
-    if (n < 0 || n >= L.nSamples) return 0.0;
-    return L.samples[n];
-  }
-  return 0.0;
-}
-
 // Eout (one slot per trajectory) = E(*tBase + tOff) for every trajectory.
 __global__ void k_field(double* __restrict__ Eout, TRAJ_ARGS, const double* __restrict__ tBase, double tOff) {
   Eout = bat(Eout, bs);
