@@ -368,7 +368,8 @@ struct cgpu_ctx {
   double* lz_d = nullptr;   // Lanczos scalars: alpha, beta, dots, phi, flags
   double* lz_h = nullptr;   // pinned mirror (trajectory 0)
   // k_sil.cu: blocks of the one-launch SIL (0: not used), the largest piece of a block
-  int silBlocks = 0, silCap = 0;
+  int silGroup = 0, silCap = 0;
+  bool silFits = false;
   void* silBlk_d = nullptr;
   z_t* silPart_d = nullptr;
   unsigned* silBar_d = nullptr;
@@ -557,12 +558,26 @@ void launch_lanczos_update(cgpu_ctx* c, int j, int maxDim, int pass1Blocks = 0);
 void launch_lanczos_tail(cgpu_ctx* c, int j, double dt, int evalExp);  // j = 0: use the device mDim
 void launch_lanczos_combine(cgpu_ctx* c, z_t* out, const z_t* start);
 void launch_lz_set(cgpu_ctx* c, int idx, double v);
-// k_sil.cu: SIL on OrbsLin in one launch (silBlocks > 0), on c->metric_d; the
+// k_sil.cu: SIL on OrbsLin in one launch (silGroup > 0, silFits), on c->metric_d; the
 // exponential of the launch-per-pass form
 void sil_init(cgpu_ctx* c);
 void sil_free(cgpu_ctx* c);
 void launch_sil(cgpu_ctx* c, z_t* state, double t, double dt, int K, double tol, int maxRestarts);
 void launch_lz_expsub(cgpu_ctx* c, int j, double dt);
+// One fixed-order pass of a single system and its reverse, for the pulse
+// gradient: what the pass leaves behind (V: K state vectors, last: one, the
+// others 32 entries, norm one, parts 32 x SIL_KEEP_PARTS), and sil_spill entries of work
+// space where that is not 0.
+constexpr int SIL_KEEP_PARTS = 256;
+struct SilKeep {
+  int K;
+  z_t *V, *last, *phi, *parts, *spill;
+  double *alpha, *beta, *norm;
+};
+size_t sil_spill(const cgpu_ctx* c);
+void sil_check(cgpu_ctx* c);  // after a synchronisation: throws if a wait between blocks expired
+void launch_sil_keep(cgpu_ctx* c, const z_t* start, z_t* out, double E, double dt, const SilKeep& k);
+void launch_sil_vjp(cgpu_ctx* c, const z_t* obar, z_t* sbar, double E, double dt, const SilKeep& k, double* grad);
 size_t lanczos_partial_need(const cgpu_ctx* c);
 #define CODY_LZ_BETA 64
 #define CODY_LZ_PHI 256

@@ -770,7 +770,7 @@ int sil_device(cgpu_ctx* c, int which, z_t* state, double t0, double t1, int kry
   c->metric_d = const_cast<double*>(metric_d);
   int warnings = 0;
   if (tol > 0.0 && c->nb > 1) throw std::string("SIL: adaptive (tolerance > 0) steps need a single system");
-  if (which == CGPU_TD_ORBS_LIN && c->silBlocks > 0) {
+  if (which == CGPU_TD_ORBS_LIN && c->silGroup > 0 && c->silFits) {
     launch_sil(c, state, t0, t1 - t0, maxDim, tol, maxRestarts);
     if (!(tol > 0.0)) return 1;
     if (!wantWarnings) return 0;
@@ -1065,7 +1065,7 @@ std::string traj_prefix(const char* dir, int b, bool create) {
 
 void sync(cgpu_ctx* c) {
   CODY_CUDA(cudaStreamSynchronize(c->stream));
-  if (c->flags_h && c->flags_h[0]) throw std::string("SIL: a bounded wait between blocks expired");
+  sil_check(c);
   if (c->mixed && mixed_error(c)) throw std::string("tensor-core GEMM: a bounded mbarrier wait expired");
 }
 

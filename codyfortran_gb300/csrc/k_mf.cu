@@ -23,6 +23,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "reginv.cuh"
 
 namespace {
 
@@ -423,94 +424,31 @@ __global__ void __launch_bounds__(512) k_rdm_occupations(const z_t* __restrict__
   }
 }
 
-// Mreg = U f(n) U^H, f(n) = n / (n^2 + eps), without the eigenvectors: with s =
-// sqrt(eps), f(n) = Re 1 / (n + i s), so Mreg is the Hermitian part of
-// (rho + i s)^-1, one n x n complex inverse.  Its error, about 2^-53 ||rho|| /
-// |n_k + i s| in the component of an occupation n_k, is the one that an
-// eigenvalue's absolute error gives f(n_k).  Gauss-Jordan in shared memory with
-// partial pivoting: per column, warp 0 finds the pivot, swaps the rows and
-// scales the pivot row, then the block updates (4 n^2 FP64 FMA a column at two a
-// cycle: the FP64 pipe and n pivot chains of about 600 cycles bound it).  The
-// Jacobi sweeps (k_rdm_occupations) take 4 n^3 FMA each and several of them:
-// 437 -> 23 us at n = 16, 303 -> 18 in a batch of 24 with n <= 12.
+// Mreg = U f(n) U^H, f(n) = n / (n^2 + eps), without the eigenvectors: the
+// Hermitian part of (rho + i sqrt(eps))^-1 (reginv.cuh).  Its error, about 2^-53
+// ||rho|| / |n_k + i s| in the component of an occupation n_k, is the one that an
+// eigenvalue's absolute error gives f(n_k).  4 n^2 FP64 FMA a column at two a cycle
+// and n pivot chains of about 600 cycles bound it.  The Jacobi sweeps
+// (k_rdm_occupations) take 4 n^3 FMA each and several of them: 437 -> 23 us at n =
+// 16, 303 -> 18 in a batch of 24 with n <= 12.
 __global__ void __launch_bounds__(256) k_rdm_inverse(z_t* __restrict__ Mreg, const z_t* __restrict__ rdm1,
                                                      TRAJ_ARGS) {
-  __shared__ z_t A[JB_MAX][JB_MAX + 1];
-  __shared__ z_t row[JB_MAX], col[JB_MAX];
-  __shared__ int perm[JB_MAX];
+  __shared__ RegInvScratch R;
   const TrajShape& T = shp[blockIdx.z];
-  const int nO = T.nO, n = T.nOS, restricted = T.restricted, tid = threadIdx.x;
+  const int nO = T.nO, n = T.nOS, tid = threadIdx.x;
   const double s = sqrt(T.regEps);
   Mreg = bat(Mreg, bs);
   rdm1 = bat(rdm1, bs);
-  auto rho = [&](int i, int j) {
+  for (int e = tid; e < n * n; e += blockDim.x) {
+    const int i = e % n, j = e / n;
     z_t v = rdm1[i + (size_t)nO * j];
-    if (restricted) v = zadd(v, rdm1[(n + i) + (size_t)nO * (n + j)]);
-    return v;
-  };
-  for (int e = tid; e < n * n; e += blockDim.x) {
-    const int i = e % n, j = e / n;
-    const z_t v = rho(i, j);
-    A[i][j] = i == j ? zmk(v.x, s) : v;
+    if (T.restricted) v = zadd(v, rdm1[(n + i) + (size_t)nO * (n + j)]);
+    R.A[i][j] = i == j ? zmk(v.x, s) : v;
   }
-  if (tid < n) perm[tid] = tid;
   __syncthreads();
-  for (int k = 0; k < n; k++) {
-    if (tid < 32) {
-      const int l = tid;
-      z_t ck = l < n ? A[l][k] : zmk(0.0, 0.0);
-      // pivot: the largest |re| + |im| at or below the diagonal, by its FP32 size (any near-largest entry serves)
-      float mag = l >= k && l < n ? fabsf((float)ck.x) + fabsf((float)ck.y) : -1.0f;
-      int p = l;
-      for (int o = 16; o > 0; o >>= 1) {
-        const float m2 = __shfl_xor_sync(0xffffffffu, mag, o);
-        const int p2 = __shfl_xor_sync(0xffffffffu, p, o);
-        if (m2 > mag || (m2 == mag && p2 < p)) {
-          mag = m2;
-          p = p2;
-        }
-      }
-      if (!(mag >= 0.0f) || p < k || p >= n) p = k;  // NaN entries: any pivot, the result is NaN
-      const z_t a = A[p][k];
-      const double d = 1.0 / fma(a.x, a.x, a.y * a.y);
-      const z_t inv = zmk(a.x * d, -a.y * d);
-      __syncwarp();  // every lane has read A[p][k] and column k
-      if (l < n) {
-        const z_t t = A[p][l], u = A[k][l];
-        row[l] = l == k ? inv : zmul(t, inv);
-        if (p != k) A[p][l] = u;
-        // column k as the update reads it: the old row k now sits in row p
-        col[l] = l == p ? A[k][k] : ck;
-        if (p == k) col[l] = ck;
-      }
-      if (l == 0 && p != k) {
-        const int q = perm[k];
-        perm[k] = perm[p];
-        perm[p] = q;
-      }
-    }
-    __syncthreads();
-    for (int e = tid; e < n * n; e += blockDim.x) {
-      const int i = e / n, j = e - i * n;
-      if (i == k) {
-        A[k][j] = row[j];
-      } else {
-        z_t v = j == k ? zmk(0.0, 0.0) : A[i][j];
-        const z_t c = col[i], r = row[j];
-        v.x = fma(-c.x, r.x, fma(c.y, r.y, v.x));
-        v.y = fma(-c.x, r.y, fma(-c.y, r.x, v.y));
-        A[i][j] = v;
-      }
-    }
-    __syncthreads();
-  }
-  // A holds (P B)^-1: column r of it is column perm[r] of B^-1
-  __shared__ int at[JB_MAX];
-  if (tid < n) at[perm[tid]] = tid;
-  __syncthreads();
+  reg_invert(R, n);
   for (int e = tid; e < n * n; e += blockDim.x) {
-    const int i = e % n, j = e / n;
-    const z_t v = A[i][at[j]], w = A[j][at[i]];
+    const z_t v = R.inv(e % n, e / n), w = R.inv(e / n, e % n);
     Mreg[e] = zmk(0.5 * (v.x + w.x), 0.5 * (v.y - w.y));
   }
 }

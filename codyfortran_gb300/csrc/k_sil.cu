@@ -27,12 +27,14 @@
 // The groups' blocks wait on one another, so the launch is cooperative (at most
 // one block per SM) and every wait is bounded.
 #include <algorithm>
+#include <cstring>
 
 #include "common.cuh"
 
 namespace {
 
 constexpr int SIL_K = 32;
+constexpr int SIL_PART = SIL_K + 8;            // partial sums of a block
 constexpr int SIL_MIN = 32;                    // smallest piece worth a block of its own
 constexpr size_t SIL_SMEM = 200 * 1024;
 constexpr long long SIL_WAIT = 4000000000LL;   // cycles after which a barrier gives up
@@ -111,8 +113,14 @@ __device__ __forceinline__ double warp_sum4(double v0, double v1, double v2, dou
 // the lanes, the normalisation is a warp sum, a Chebyshev term costs four FMA, and
 // both recurrences start where (z/2)^n / n!, a bound on |J_n|, falls below 1e-19
 // (52 -> 10 us at K = 16).  jb: 1216 doubles of shared memory.
-__device__ void lz_expsub_warp(const double* alpha, const double* beta, int m, double dt, double* jb, double& fr,
-                               double& fi) {
+//
+// lz_series_warp: centre c, radius R, last term K and the coefficients jb[0] = J_0,
+// jb[k] = 2 J_k of the series of exp(-i dt/n T); PARTS (the pulse gradient): n > 1
+// where |dt| R is above LZ_PART, so that jb holds every term.
+constexpr double LZ_PART = 700.0;
+template <bool PARTS>
+__device__ void lz_series_warp(const double* alpha, const double* beta, int m, double dt, double* jb, double& c,
+                               double& R, int& K, int& n) {
   constexpr int KMAX = 1180;
   const int lane = threadIdx.x & 31;
   const double a = lane < m ? alpha[lane] : 0.0;
@@ -123,8 +131,12 @@ __device__ void lz_expsub_warp(const double* alpha, const double* beta, int m, d
     lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
     hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
   }
-  const double c = 0.5 * (hi + lo), R = 0.5 * (hi - lo) * (1.0 + 1e-12) + 1e-300, z = fabs(dt) * R;
-  int K = 1;  // last term of the series
+  c = 0.5 * (hi + lo);
+  R = 0.5 * (hi - lo) * (1.0 + 1e-12) + 1e-300;
+  n = 1;
+  if (PARTS) n = (int)fmin(fmax(ceil(fabs(dt) * R / LZ_PART), 1.0), (double)SIL_KEEP_PARTS);
+  const double z = PARTS ? fabs(dt) * R / n : fabs(dt) * R;
+  K = 1;
   if (z >= 1e-300) {
     // log2 of (z/2)^n / n! below -64
     const float l2 = log2f((float)fmin(z, 1e30) * 0.5f);
@@ -168,17 +180,79 @@ __device__ void lz_expsub_warp(const double* alpha, const double* beta, int m, d
     for (int k = lane; k <= K; k += 32) jb[k] *= k == 0 ? inv : 2.0 * inv;
   }
   __syncwarp();
-  // 2 T' and the recurrence; a_k = 2 (-i)^k J_k: 1, -i, -1, i in turn
-  const double iR = 2.0 / R, ta = (a - c) * iR, tl = bl * iR, tr = br * iR;
-  double qm = lane == 0 ? 1.0 : 0.0, q;
-  {
-    const double ql = __shfl_up_sync(0xffffffffu, qm, 1), qr = __shfl_down_sync(0xffffffffu, qm, 1);
-    q = 0.5 * fma(ta, qm, fma(tl, ql, tr * qr));
+}
+
+// The tridiagonal 2 T' of a series, a lane a row.
+struct LzRow {
+  double ta, tl, tr;
+  __device__ LzRow(const double* alpha, const double* beta, int m, double c, double iR) {
+    const int lane = threadIdx.x & 31;
+    ta = lane < m ? (alpha[lane] - c) * iR : 0.0;
+    tl = lane >= 1 && lane < m ? beta[lane - 1] * iR : 0.0;
+    tr = lane + 1 < m ? beta[lane] * iR : 0.0;
   }
+  __device__ double mul(double v, double minus) const {  // 2 T' v - minus
+    const double l = __shfl_up_sync(0xffffffffu, v, 1), r = __shfl_down_sync(0xffffffffu, v, 1);
+    return fma(ta, v, fma(tl, l, fma(tr, r, -minus)));
+  }
+};
+
+// The parts after one another, on a complex vector; parts: the vector at the start of
+// each, 32 entries a part (may be null).
+__device__ __noinline__ z_t lz_expsub_parts(LzRow T, const double* jb, int K, int n, double dt, double c,
+                                            z_t* parts) {
+  const int lane = threadIdx.x & 31;
+  double vr = lane == 0 ? 1.0 : 0.0, vi = 0.0, sn, cs;
+  sincos(dt / n * c, &sn, &cs);
+  for (int s = 0; s < n; s++) {
+    if (parts) parts[32 * s + lane] = zmk(vr, vi);
+    double mr = vr, mi = vi, qr = 0.5 * T.mul(vr, 0.0), qi = 0.5 * T.mul(vi, 0.0);
+    double er = jb[0] * vr, ei = jb[0] * vi, orr = jb[1] * qr, oi = jb[1] * qi;  // even terms; odd terms without -i
+    for (int k = 2; k <= K; k++) {
+      const double nr = T.mul(qr, mr), ni = T.mul(qi, mi);
+      mr = qr;
+      mi = qi;
+      qr = nr;
+      qi = ni;
+      const double co = (k & 2) == 0 ? jb[k] : -jb[k];
+      if (k & 1) {
+        orr = fma(co, qr, orr);
+        oi = fma(co, qi, oi);
+      } else {
+        er = fma(co, qr, er);
+        ei = fma(co, qi, ei);
+      }
+    }
+    if (dt < 0.0) {
+      orr = -orr;
+      oi = -oi;
+    }
+    const double pr = er + oi, pi = ei - orr;
+    vr = cs * pr + sn * pi;
+    vi = cs * pi - sn * pr;
+  }
+  return zmk(vr, vi);
+}
+
+template <bool PARTS>
+__device__ void lz_expsub_warp(const double* alpha, const double* beta, int m, double dt, double* jb, double& fr,
+                               double& fi, z_t* parts = nullptr) {
+  const int lane = threadIdx.x & 31;
+  double c, R;
+  int K, n;
+  lz_series_warp<PARTS>(alpha, beta, m, dt, jb, c, R, K, n);
+  const LzRow T(alpha, beta, m, c, 2.0 / R);
+  if (PARTS && n > 1) {
+    const z_t v = lz_expsub_parts(T, jb, K, n, dt, c, parts);
+    fr = v.x;
+    fi = v.y;
+    return;
+  }
+  // a_k = 2 (-i)^k J_k: 1, -i, -1, i in turn
+  double qm = lane == 0 ? 1.0 : 0.0, q = 0.5 * T.mul(qm, 0.0);
   double pr = jb[0] * qm, pi = -jb[1] * q;
   for (int k = 2; k <= K; k++) {
-    const double ql = __shfl_up_sync(0xffffffffu, q, 1), qr = __shfl_down_sync(0xffffffffu, q, 1);
-    const double qn = fma(ta, q, fma(tl, ql, fma(tr, qr, -qm)));
+    const double qn = T.mul(q, qm);
     qm = q;
     q = qn;
     const double co = (k & 2) == 0 ? jb[k] : -jb[k];  // k mod 4 = 0: 1, 1: -i, 2: -1, 3: i
@@ -192,9 +266,69 @@ __device__ void lz_expsub_warp(const double* alpha, const double* beta, int m, d
   fi = cs * pi - sn * pr;
 }
 
+// Co-states of alpha and beta (lane i: alpha_i, beta_i) from that of phi (lane i:
+// yb, in the convention dL = Re sum conj(yb) dphi): the reverse of the Chebyshev
+// recurrence, part by part from the last.  With the series' coefficients a_k (and
+// the phase) and the co-states conj(a_k) yb of the terms q_k,
+//   l_k = conj(a_k) yb + 2 T' l_{k+1} - l_{k+2},
+//   T'bar = l_1 q_0^T + sum_{k>1} 2 l_k q_{k-1}^T,  q_0bar = conj(a_0) yb + T' l_1 - l_2,
+// the q_k run back by q_{k-1} = 2 T' q_k - q_{k+1}.  c and R are constants of the
+// expansion: phi does not depend on them.
+__device__ void lz_expsub_vjp_warp(const double* alpha, const double* beta, int m, double dt, double* jb, z_t yb,
+                                   const z_t* parts, double& abar, double& bbar) {
+  const int lane = threadIdx.x & 31;
+  double c, R;
+  int K, n;
+  lz_series_warp<true>(alpha, beta, m, dt, jb, c, R, K, n);
+  const double iR = 2.0 / R;
+  const LzRow T(alpha, beta, m, c, iR);
+  double sn, cs;
+  sincos(dt / n * c, &sn, &cs);
+  double sa = 0.0, sb = 0.0;
+  for (int s = n - 1; s >= 0; s--) {
+    const z_t v = s == 0 ? zmk(lane == 0 ? 1.0 : 0.0, 0.0) : parts[32 * s + lane];
+    double mr = v.x, mi = v.y, qr = 0.5 * T.mul(mr, 0.0), qi = 0.5 * T.mul(mi, 0.0);  // q_0, q_1
+    for (int k = 2; k <= K; k++) {
+      const double nr = T.mul(qr, mr), ni = T.mul(qi, mi);
+      mr = qr;
+      mi = qi;
+      qr = nr;
+      qi = ni;
+    }
+    // f = conj(phase) yb; conj((-i)^k) f: f, i f, -f, -i f in turn (conjugate series: the odd ones negated)
+    const double f0 = fma(yb.x, cs, -yb.y * sn), f1 = fma(yb.x, sn, yb.y * cs), od = dt < 0.0 ? -1.0 : 1.0;
+    double l1r = 0.0, l1i = 0.0, l2r = 0.0, l2i = 0.0;  // l_{k+1}, l_{k+2}
+    for (int k = K; k >= 1; k--) {                      // q = q_k, qm = q_{k-1}
+      const double co = ((k & 2) ? -jb[k] : jb[k]) * ((k & 1) ? od : 1.0);
+      const double gr = (k & 1) ? -f1 : f0, gi = (k & 1) ? f0 : f1;
+      const double lr = fma(co, gr, T.mul(l1r, l2r)), li = fma(co, gi, T.mul(l1i, l2i));
+      l2r = l1r;
+      l2i = l1i;
+      l1r = lr;
+      l1i = li;
+      const double h = k == 1 ? 0.5 : 1.0;
+      const double nlr = __shfl_down_sync(0xffffffffu, lr, 1), nli = __shfl_down_sync(0xffffffffu, li, 1);
+      const double nqr = __shfl_down_sync(0xffffffffu, mr, 1), nqi = __shfl_down_sync(0xffffffffu, mi, 1);
+      sa = fma(h, fma(lr, mr, li * mi), sa);
+      sb = fma(h, fma(lr, nqr, fma(li, nqi, fma(nlr, mr, nli * mi))), sb);
+      if (k > 1) {
+        const double pr = T.mul(mr, qr), pi = T.mul(mi, qi);  // q_{k-2}
+        qr = mr;
+        qi = mi;
+        mr = pr;
+        mi = pi;
+      }
+    }
+    yb = zmk(fma(jb[0], f0, 0.5 * T.mul(l1r, 2.0 * l2r)), fma(jb[0], f1, 0.5 * T.mul(l1i, 2.0 * l2i)));
+  }
+  abar = lane < m ? sa * iR : 0.0;
+  bbar = lane + 1 < m ? sb * iR : 0.0;
+}
+
 namespace {
 
 struct SilArgs {
+  const z_t* start;  // the vector to propagate, and its result (may be the same)
   z_t *state, *w0, *w1, *basis;
   size_t ldv;
   const double *m, *T, *V0, *x;
@@ -210,20 +344,29 @@ struct SilArgs {
   int* flags;      // host memory: [0] error, [1] warnings of trajectory 0
   int cap, smemV;  // entries of the largest piece; basis vectors in shared memory
   int pt;          // threads per entry (4 where the pieces leave most of the block idle, else 1)
+  // for the pulse gradient: a given field value, and what its reverse pass reads
+  double E;
+  SilKeep keep;
 };
+
+// MODE: a propagation, the pass kept for its reverse, the same with the vectors in
+// global memory.
+constexpr int SIL_STEP = 0, SIL_KEPT = 1, SIL_SPILLED = 2;
 
 // SIL_T threads a block: 256 for the small pieces (four threads an entry), whose
 // iteration is a chain of latencies; 512 where the basis fits shared memory; 1024
 // where it is read from L2 (10 helium steps 10.1 / 10.6 / 11.9 ms with 256 / 512 /
 // 1024, 2801 x 16 points 462 / 414 / 488 us, a scan of 24 8.78 / 8.37 / 8.13 ms).
-template <int SIL_T>
+template <int SIL_T, int MODE = SIL_STEP>
 __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
   constexpr int SIL_W = SIL_T / 32;
+  constexpr bool KEEP = MODE != SIL_STEP;
   const SilBlock B = A.blk[blockIdx.x];
   const TrajShape& S = shp[B.traj];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int nG = S.nG, band = S.band, nd = 2 * band + 1, nC = S.nC, cap = A.cap;
   z_t* state = batn(A.state, bs, B.traj);
+  const z_t* start = batn(A.start, bs, B.traj);
   z_t* wb[2] = {batn(A.w0, bs, B.traj), batn(A.w1, bs, B.traj)};
   z_t* basis = batn(A.basis, bs, B.traj);
   const double* m = batn(A.m, bs, B.traj);
@@ -231,13 +374,14 @@ __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
   const double* V0 = batn(A.V0, bs, B.traj);
   const double* x = batn(A.x, bs, B.traj);
   const int* btOf = batn(A.btOf, bs, B.traj);
-  constexpr int PS = SIL_K + 2;
+  constexpr int PS = SIL_PART;
   z_t* part = A.part + (size_t)(blockIdx.x - B.rank) * PS;  // the group's partials
   z_t* mine = part + (size_t)B.rank * PS;
   unsigned* bar = A.bar + 2 * B.traj;
   unsigned target = 0;
 
-  extern __shared__ z_t sm[];
+  extern __shared__ z_t smDyn[];
+  z_t* sm = MODE == SIL_SPILLED ? A.keep.spill + blockIdx.x * (size_t)(3 * cap + 2 * band) : smDyn;
   z_t* vt = sm;                          // v_j with its halo: entries l0 - band .. l1 + band
   z_t* w = vt + cap + 2 * band;
   z_t* mw = w + cap;                     // m w
@@ -372,20 +516,20 @@ __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
     double q = 0.0;
     for (int e = tid; e < cnt; e += SIL_T) {
       const size_t i = vidx(S, l0 + e);
-      const z_t v = state[i];
+      const z_t v = start[i];
       q = fma(m[i], fma(v.x, v.x, v.y * v.y), q);
     }
     // the field takes a few microseconds of FP64 on one lane: beside the norm
     auto field = [&]() {
       if (tid == SIL_T - 1)
-        shE = S.hasPot ? field_amplitude_dev(S.laser, *batn(A.tBase, bs, B.traj) + tCur + 0.5 * dtS) : 0.0;
+        shE = KEEP ? A.E : S.hasPot ? field_amplitude_dev(S.laser, *batn(A.tBase, bs, B.traj) + tCur + 0.5 * dtS) : 0.0;
     };
     field();
     publish(q, SIL_K + 1);
     if (!(ok = barrier())) break;
     gather(SIL_K + 1, 1);
     const double nrm = sqrt(coef[0].x);
-    if (nrm <= SIL_ZERO) {  // nothing to propagate: the state stays
+    if (nrm <= SIL_ZERO && !KEEP) {  // nothing to propagate: the state stays
       conv = true;
     } else {
       for (;;) {
@@ -396,7 +540,7 @@ __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
         }
         const double E = shE;
         double inv = 1.0 / nrm, bPrev = 0.0;
-        const z_t* src = state;
+        const z_t* src = start;
         int mDim = A.K;
         for (int j = 1; j <= A.K; j++) {
           // v_j and its halo
@@ -406,7 +550,10 @@ __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
             z_t v = zmk(0.0, 0.0);
             if (l >= 0 && l < S.nS) v = zscale(__ldcg(src + vidx(S, l)), inv);
             vt[t] = v;
-            if (t >= band && t < band + cnt) vec(j - 1, t - band) = v;
+            if (t >= band && t < band + cnt) {
+              vec(j - 1, t - band) = v;
+              if (KEEP && A.smemV) A.keep.V[A.ldv * (j - 1) + vidx(S, l)] = v;
+            }
           }
           __syncthreads();
           double h2 = 0.0;
@@ -424,7 +571,7 @@ __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
                 h.x = fma(cf, vv[d].x, h.x);
                 h.y = fma(cf, vv[d].y, h.y);
               }
-              if (S.hasPot && eq == pt - 1) {
+              if ((S.hasPot || KEEP) && eq == pt - 1) {
                 const double p = fma(E, x[g], V0[g]);
                 h.x = fma(p, vv[band].x, h.x);
                 h.y = fma(p, vv[band].y, h.y);
@@ -473,13 +620,13 @@ __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
             alpha[j - 1] = a;
             beta[j - 1] = be;
           }
-          const bool broke = be <= SIL_ZERO;
+          const bool broke = be <= SIL_ZERO && !KEEP;  // the kept pass runs over all orders
           const bool last = broke || j == A.K;
           if (A.tol > 0.0 || last) {
             __syncthreads();
             if (wid == 0) {
               double fr, fi;
-              lz_expsub_warp(alpha, beta, j, dtS, jb, fr, fi);
+              lz_expsub_warp<KEEP>(alpha, beta, j, dtS, jb, fr, fi, KEEP && B.rank == 0 ? A.keep.parts : nullptr);
               if (lane < j) phi[lane] = zmk(fr, fi);
               if (lane == j - 1) errEst = broke ? 0.0 : be * sqrt(fr * fr + fi * fi);
             }
@@ -500,6 +647,15 @@ __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
             z_t acc = zmk(0.0, 0.0);
             for (int k = 0; k < mDim; k++) zfma(acc, vec(k, e), phi[k]);
             state[vidx(S, l0 + e)] = zscale(acc, nrm);
+          }
+          if (KEEP) {
+            for (int e = tid; e < cnt; e += SIL_T) A.keep.last[l0 + e] = w[e];
+            if (B.rank == 0 && tid < A.K) {
+              A.keep.alpha[tid] = alpha[tid];
+              A.keep.beta[tid] = beta[tid];
+              A.keep.phi[tid] = phi[tid];
+              if (tid == 0) *A.keep.norm = nrm;
+            }
           }
           break;
         }
@@ -529,12 +685,206 @@ size_t sil_smem(int cap, int band, int K, bool smemV) {
 
 }  // namespace
 
+namespace {
+
+struct SilVjpArgs {
+  SilKeep k;
+  const z_t* obar;
+  const double *m, *T, *V0, *x;
+  z_t *sbar, *vb0, *vb1;
+  double *grad, E, dt;
+  z_t* part;
+  unsigned* bar;
+  int cap, nBlk;
+  int* flags;
+};
+
+// The reverse of one kept pass: sbar = (d out / d start)^H obar, grad += the field
+// part, differentiating the three-term recurrence (its re-orthogonalisation is the
+// identity in exact arithmetic).  With r_j = H v_j - beta_{j-1} v_{j-1} - alpha_j v_j =
+// beta_j v_{j+1} the reverse step of order j is local in the vectors once two sums
+// over the previous one are known:
+//   bb = bbar_j - <vbar_{j+1}, v_{j+1}> / beta_j,   rbar = vbar_{j+1} / beta_j + bb m v_{j+1},
+//   ab = abar_j - <vbar_{j+1}, v_j> / beta_j,       wbar_j = rbar + ab m v_j,
+//   vbar_j = ||s|| conj(phi_j) obar - beta_j wbar_{j+1} - alpha_j rbar + ab m (r_j + alpha_j v_j) + H^T wbar_j,
+// with bbar_j reduced by <wbar_{j+1}, v_j>, so there is one barrier per order.  A
+// block forms wbar on its halo itself.  12 orders, 501 x 8 points: 1200 us as
+// launches per operation, 148 here.
+template <bool SPILL>
+__global__ void __launch_bounds__(256, 1) k_sil_vjp(const SilVjpArgs A, TRAJ_ARGS) {
+  constexpr int T = 256, W = T / 32;
+  const TrajShape& S = shp[0];
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, rank = blockIdx.x;
+  const int nG = S.nG, band = S.band, nd = 2 * band + 1, nC = S.nC, nS = S.nS, K = A.k.K;
+  constexpr int PS = SIL_PART;
+  z_t* mine = A.part + (size_t)rank * PS;
+  unsigned target = 0;
+  extern __shared__ z_t smDyn[];
+  z_t* sm = SPILL ? A.k.spill + rank * (size_t)(3 * A.cap + 2 * band) : smDyn;
+  z_t* wh = sm;                       // wbar_j with its halo
+  z_t* vbj = wh + A.cap + 2 * band;   // vbar of the last order
+  z_t* wPrev = vbj + A.cap;           // wbar of the last order
+  __shared__ z_t coef[SIL_K + 1], phi[SIL_K];
+  __shared__ double alpha[SIL_K], beta[SIL_K], abar[SIL_K], bbar[SIL_K], red[4][W], jb[1216];
+  const int per = (nS + A.nBlk - 1) / A.nBlk, l0 = min(nS, rank * per), cnt = min(nS, l0 + per) - l0;
+  auto barrier = [&]() {
+    target += A.nBlk;
+    return group_barrier(A.bar, target, A.nBlk, A.flags);
+  };
+  auto gather = [&](int s0, int n) {
+    for (int k = wid; k < n; k += W) {
+      double x0 = 0.0, y0 = 0.0;
+      for (int b = lane; b < A.nBlk; b += 32) {
+        const z_t p = __ldcg(A.part + (size_t)b * PS + s0 + k);
+        x0 += p.x;
+        y0 += p.y;
+      }
+      const double x = warp_sum2(x0, y0);
+      if ((lane & 15) == 0) reinterpret_cast<double*>(coef)[2 * k + (lane >> 4)] = x;
+    }
+    __syncthreads();
+  };
+  if (tid < K) {
+    alpha[tid] = A.k.alpha[tid];
+    beta[tid] = A.k.beta[tid];
+    phi[tid] = A.k.phi[tid];
+  }
+  const double nrm = *A.k.norm;
+  bool ok = true;
+  // phibar_j = ||s|| <v_j, obar> (no metric)
+  for (int k = wid; k < K; k += W) {
+    const z_t* v = A.k.V + (size_t)nS * k + l0;
+    double ax = 0.0, ay = 0.0;
+    for (int e = lane; e < cnt; e += 32) {
+      const z_t a = v[e], b = A.obar[l0 + e];
+      ax = fma(a.x, b.x, fma(a.y, b.y, ax));
+      ay = fma(a.x, b.y, fma(-a.y, b.x, ay));
+    }
+    const double x = warp_sum2(ax, ay);
+    if ((lane & 15) == 0) reinterpret_cast<double*>(mine)[2 * k + (lane >> 4)] = x;
+  }
+  ok = barrier();
+  double nbar = 0.0, gx = 0.0;
+  if (ok) {
+    gather(0, K);
+    for (int j = 0; j < K; j++) nbar += coef[j].x * phi[j].x + coef[j].y * phi[j].y;
+    if (wid == 0) {
+      const z_t yb = lane < K ? zscale(coef[lane], nrm) : zmk(0.0, 0.0);
+      double a, b;
+      lz_expsub_vjp_warp(alpha, beta, K, A.dt, jb, yb, A.k.parts, a, b);
+      if (lane < K) {
+        abar[lane] = a;
+        bbar[lane] = b;
+      }
+    }
+    __syncthreads();
+  }
+  double d1 = 0.0, e1 = 0.0, f1 = 0.0;  // <vbar_{j+1}, v_{j+1}>, <vbar_{j+1}, v_j>, <wbar_{j+1}, v_j>
+  for (int j = K - 1; ok && j >= 0; j--) {
+    const bool last = j == K - 1;
+    const double be = beta[j], al = alpha[j];
+    const double bb = last ? 0.0 : bbar[j] - f1 - d1 / be, ab = last ? abar[j] : abar[j] - e1 / be, ib = 1.0 / be;
+    const z_t* vj = A.k.V + (size_t)nS * j;
+    const z_t* vn = last ? A.k.last : vj + nS;
+    const z_t* vbn = (j & 1) ? A.vb0 : A.vb1;  // vbar_{j+1}, published by the previous order
+    z_t* vbo = (j & 1) ? A.vb1 : A.vb0;
+    for (int t = tid; t < cnt + 2 * band; t += T) {
+      const int l = l0 - band + t;
+      z_t wv = zmk(0.0, 0.0);
+      if (l >= 0 && l < nS) {
+        const double mi = A.m[l];
+        wv = zscale(vj[l], ab * mi);
+        if (!last) {
+          const z_t r = zadd(zscale(__ldcg(vbn + l), ib), zscale(vn[l], bb * mi));
+          wv = zadd(wv, r);
+        }
+      }
+      wh[t] = wv;
+    }
+    __syncthreads();
+    double s0 = 0.0, s1 = 0.0, s2 = 0.0;
+    for (int e = tid; e < cnt; e += T) {
+      const int l = l0 + e;
+      const z_t v = vj[l], n = vn[l], wv = wh[band + e], ob = A.obar[l];
+      const double mi = A.m[l];
+      z_t o = zscale(zcmul(phi[j], ob), nrm);
+      // ab m (r + alpha v): r = beta_j v_{j+1}, or the kept residual of the last order
+      const double rs = last ? 1.0 : be;
+      o.x = fma(ab * mi, fma(rs, n.x, al * v.x), o.x);
+      o.y = fma(ab * mi, fma(rs, n.y, al * v.y), o.y);
+      if (!last) {
+        const z_t vb = vbj[e], wp = wPrev[e];
+        o.x = fma(-be, wp.x, fma(-al, fma(ib, vb.x, bb * mi * n.x), o.x));
+        o.y = fma(-be, wp.y, fma(-al, fma(ib, vb.y, bb * mi * n.y), o.y));
+      }
+      if (l >= nC) {
+        const int r = l - nC, g = r % nG;
+        const double p = fma(A.E, A.x[g], A.V0[g]);
+        o.x = fma(p, wv.x, o.x);
+        o.y = fma(p, wv.y, o.y);
+        // row gg of T at column g is T[2 band - d][gg]
+        for (int d = max(0, band - g); d < min(nd, nG - g + band); d++) {
+          const double cf = __ldg(A.T + (size_t)(nd - 1 - d) * nG + (g - band + d));
+          const z_t q = wh[e + d];
+          o.x = fma(cf, q.x, o.x);
+          o.y = fma(cf, q.y, o.y);
+        }
+        gx = fma(A.x[g], fma(wv.x, v.x, wv.y * v.y), gx);
+      }
+      vbj[e] = o;
+      wPrev[e] = wv;
+      vbo[l] = o;
+      s0 = fma(o.x, v.x, fma(o.y, v.y, s0));
+      if (j > 0) {
+        const z_t p = vj[l - nS];
+        s1 = fma(o.x, p.x, fma(o.y, p.y, s1));
+        s2 = fma(wv.x, p.x, fma(wv.y, p.y, s2));
+      }
+    }
+    // block sums of s0, s1, s2 and, at the end, gx
+    const double x = warp_sum4(s0, s1, s2, j == 0 ? gx : 0.0);
+    if ((lane & 7) == 0) red[lane >> 3][wid] = x;
+    __syncthreads();
+    if (tid < 4) {
+      double t = 0.0;
+      for (int i = 0; i < W; i++) t += red[tid][i];
+      mine[SIL_K + 4 * (j & 1) + tid] = zmk(t, 0.0);  // a slow block may still read the last order's
+    }
+    if (!(ok = barrier())) break;
+    gather(SIL_K + 4 * (j & 1), 4);
+    d1 = coef[0].x;
+    e1 = coef[1].x;
+    f1 = coef[2].x;
+    __syncthreads();
+  }
+  if (ok) {
+    const double nb = nbar - d1 / nrm;
+    for (int e = tid; e < cnt; e += T) {
+      const int l = l0 + e;
+      const z_t v = A.k.V[l];
+      A.sbar[l] = zadd(zscale(vbj[e], 1.0 / nrm), zscale(v, nb * A.m[l]));
+    }
+    if (rank == 0 && tid == 0 && A.grad) *A.grad += coef[3].x;
+  }
+  if (tid == 0 && A.nBlk > 1 && atomicAdd(A.bar + 1, 1u) == (unsigned)A.nBlk - 1) {
+    A.bar[0] = 0u;
+    A.bar[1] = 0u;
+    __threadfence();
+  }
+}
+
+}  // namespace
+
+static const void* const sil_kernels[2][3] = {
+    {(const void*)k_sil<256>, (const void*)k_sil<512>, (const void*)k_sil<1024>},
+    {(const void*)k_sil<256, SIL_KEPT>, (const void*)k_sil<512, SIL_KEPT>, (const void*)k_sil<1024, SIL_KEPT>}};
+
 // Shares the SMs out to the trajectories in proportion to their state sizes (at
 // least one block each, none with less than SIL_MIN entries).  Left off where
-// the trajectories outnumber the SMs or a piece would not fit a block's shared
-// memory: there the launch-per-pass form fills the chip.
+// the trajectories outnumber the SMs, and not used for the propagation where a piece
+// does not fit a block's shared memory: there the launch-per-pass form fills the chip.
 void sil_init(cgpu_ctx* c) {
-  c->silBlocks = 0;
+  c->silGroup = 0;
   if (c->method == CGPU_METHOD_TDCI || c->nb > c->numSms) return;
   std::vector<SilBlock> v;
   double total = 0.0;
@@ -549,16 +899,21 @@ void sil_init(cgpu_ctx* c) {
     for (int r = 0; r < n; r++) v.push_back(SilBlock{b, r, n});
     cap = std::max(cap, (nS + n - 1) / n);
   }
-  if (sil_smem(cap, c->band, 0, false) > SIL_SMEM) return;
   CODY_CUDA(cudaMalloc(&c->silBlk_d, sizeof(SilBlock) * v.size()));
   CODY_CUDA(cudaMemcpy(c->silBlk_d, v.data(), sizeof(SilBlock) * v.size(), cudaMemcpyHostToDevice));
-  CODY_CUDA(cudaMalloc(&c->silPart_d, sizeof(z_t) * v.size() * (SIL_K + 2)));
+  CODY_CUDA(cudaMalloc(&c->silPart_d, sizeof(z_t) * v.size() * SIL_PART));
   CODY_CUDA(cudaMalloc(&c->silBar_d, sizeof(unsigned) * 2 * c->nb));
   CODY_CUDA(cudaMemset(c->silBar_d, 0, sizeof(unsigned) * 2 * c->nb));
-  for (const void* k : {(const void*)k_sil<256>, (const void*)k_sil<512>, (const void*)k_sil<1024>})
+  for (const void* k : {sil_kernels[0][0], sil_kernels[0][1], sil_kernels[0][2], sil_kernels[1][0], sil_kernels[1][1],
+                        sil_kernels[1][2], (const void*)k_sil_vjp<false>})
     CODY_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SIL_SMEM));
-  c->silBlocks = (int)v.size();
+  c->silGroup = (int)v.size();
   c->silCap = cap;
+  c->silFits = sil_smem(cap, c->band, 0, false) <= SIL_SMEM;
+}
+
+void sil_check(cgpu_ctx* c) {
+  if (c->flags_h && c->flags_h[0]) throw std::string("SIL: a bounded wait between blocks expired");
 }
 
 void sil_free(cgpu_ctx* c) {
@@ -566,10 +921,10 @@ void sil_free(cgpu_ctx* c) {
     if (p) cudaFree(p);
 }
 
-// SIL on OrbsLin from t over dt on a state (all trajectories), in place.
-void launch_sil(cgpu_ctx* c, z_t* state, double t, double dt, int K, double tol, int maxRestarts) {
-  ProfScope prof(c, CGPU_KERNEL_LANCZOS);
+static SilArgs sil_args(cgpu_ctx* c, const z_t* start, z_t* state, double dt, int K) {
   SilArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.start = start;
   a.state = state;
   a.w0 = c->lw_d;
   a.w1 = c->work_d;
@@ -583,22 +938,80 @@ void launch_sil(cgpu_ctx* c, z_t* state, double t, double dt, int K, double tol,
   a.blk = (const SilBlock*)c->silBlk_d;
   a.part = c->silPart_d;
   a.bar = c->silBar_d;
-  a.tBase = (c->inCapture || c->useStepTime) ? c->stepT_d : c->zero_d;
-  a.tOff = c->inCapture ? t - c->captureT0 : t;
+  a.tBase = c->zero_d;
   a.dt = dt;
   a.K = K;
   a.window = c->krylovWindow;
-  a.tol = tol;
-  a.maxRestarts = maxRestarts;
   a.flags = c->flags_d;
   a.cap = c->silCap;
   a.smemV = sil_smem(c->silCap, c->band, K, true) <= SIL_SMEM;
-  const int T = 4 * c->silCap <= 256 ? 256 : a.smemV ? 512 : 1024;
+  return a;
+}
+
+static void sil_launch(cgpu_ctx* c, SilArgs& a, int mode) {
+  const int T = mode == SIL_SPILLED ? 1024 : 4 * c->silCap <= 256 ? 256 : a.smemV ? 512 : 1024;
   a.pt = T == 256 ? 4 : 1;
   void* args[] = {&a, (void*)&c->shape_d, (void*)&c->bs};
-  const void* kern = T == 256 ? (const void*)k_sil<256> : T == 512 ? (const void*)k_sil<512> : (const void*)k_sil<1024>;
-  CODY_CUDA(cudaLaunchCooperativeKernel(kern, dim3(c->silBlocks), dim3(T), args,
-                                        sil_smem(c->silCap, c->band, K, a.smemV), c->stream));
+  const int i = T == 256 ? 0 : T == 512 ? 1 : 2;
+  const void* kern = mode == SIL_SPILLED ? (const void*)k_sil<1024, SIL_SPILLED> : sil_kernels[mode][i];
+  CODY_CUDA(cudaLaunchCooperativeKernel(kern, dim3(c->silGroup), dim3(T), args,
+                                        mode == SIL_SPILLED ? 0 : sil_smem(c->silCap, c->band, a.K, a.smemV),
+                                        c->stream));
+  CODY_LAUNCHED(c);
+}
+
+// SIL on OrbsLin from t over dt on a state (all trajectories), in place.
+void launch_sil(cgpu_ctx* c, z_t* state, double t, double dt, int K, double tol, int maxRestarts) {
+  ProfScope prof(c, CGPU_KERNEL_LANCZOS);
+  SilArgs a = sil_args(c, state, state, dt, K);
+  a.m = c->metric_d;
+  a.tBase = (c->inCapture || c->useStepTime) ? c->stepT_d : c->zero_d;
+  a.tOff = c->inCapture ? t - c->captureT0 : t;
+  a.tol = tol;
+  a.maxRestarts = maxRestarts;
+  sil_launch(c, a, SIL_STEP);
+}
+
+size_t sil_spill(const cgpu_ctx* c) {
+  return c->silFits ? 0 : (size_t)c->silGroup * (3 * (size_t)c->silCap + 2 * c->band);
+}
+
+// One fixed-order pass exp(-i dt h(E)) from start into out in the grid metric (a
+// single system), keeping what its reverse needs.
+void launch_sil_keep(cgpu_ctx* c, const z_t* start, z_t* out, double E, double dt, const SilKeep& k) {
+  SilArgs a = sil_args(c, start, out, dt, k.K);
+  a.m = c->metricW_d;
+  a.window = 0;
+  a.E = E;
+  a.keep = k;
+  if (!a.smemV) a.basis = k.V;
+  sil_launch(c, a, k.spill ? SIL_SPILLED : SIL_KEPT);
+}
+
+// sbar may be obar; grad may be null.
+void launch_sil_vjp(cgpu_ctx* c, const z_t* obar, z_t* sbar, double E, double dt, const SilKeep& k, double* grad) {
+  SilVjpArgs a;
+  a.k = k;
+  a.obar = obar;
+  a.m = c->metricW_d;
+  a.T = c->T_d;
+  a.V0 = c->V0_d;
+  a.x = c->x_d;
+  a.sbar = sbar;
+  a.vb0 = c->lw_d;
+  a.vb1 = c->work_d;
+  a.grad = grad;
+  a.E = E;
+  a.dt = dt;
+  a.part = c->silPart_d;
+  a.bar = c->silBar_d;
+  a.cap = c->silCap;
+  a.nBlk = c->silGroup;
+  a.flags = c->flags_d;
+  void* args[] = {&a, (void*)&c->shape_d, (void*)&c->bs};
+  const void* kern = k.spill ? (const void*)k_sil_vjp<true> : (const void*)k_sil_vjp<false>;
+  CODY_CUDA(cudaLaunchCooperativeKernel(kern, dim3(c->silGroup), dim3(256), args,
+                                        k.spill ? 0 : sil_smem(c->silCap, c->band, 0, false), c->stream));
   CODY_LAUNCHED(c);
 }
 
@@ -609,7 +1022,7 @@ __global__ void k_lz_expsub(double* __restrict__ lz, int mFixed, double dt, size
   if (m > 32) m = 32;
   if (m < 1) return;
   double fr, fi;
-  lz_expsub_warp(lz, lz + CODY_LZ_BETA, m, dt, jb, fr, fi);
+  lz_expsub_warp<false>(lz, lz + CODY_LZ_BETA, m, dt, jb, fr, fi);
   const int lane = threadIdx.x;
   if (lane < m) {
     lz[CODY_LZ_PHI + 2 * lane] = fr;
