@@ -156,10 +156,10 @@ struct CiTables {
   int* dCode;
   int8_t* dFac;
   int* rankTab;        // (nBodies+1) x (nOrbs+1) additive rank table
-  // the same excitations grouped by orbital code (for the RDM gathers):
-  // code q has value xCode[q] and edges [xStart[q], xStart[q+1]) with
-  // source / target configuration (0-based) and sign
-  int nSc, nDc;        // distinct singles / doubles codes
+  // the same excitations grouped by orbital code (for the RDM gathers), the
+  // codes up to their adjoints: code q has value xCode[q] and edges
+  // [xStart[q], xStart[q+1]) with source / target configuration (0-based) and sign
+  int nSc, nDc;        // distinct singles / doubles codes kept
   int *sxCode, *sxStart, *sxSrc, *sxDst;
   int8_t* sxFac;
   int *dxCode, *dxStart, *dxSrc, *dxDst;
@@ -278,7 +278,7 @@ struct SysHost {
   CiTables tab[CODY_MAX_BT] = {};
   CiView view = {};
   // host copies for the work lists: connections per configuration, code-list starts
-  std::vector<int> hsN[CODY_MAX_BT], hdN[CODY_MAX_BT], hsxStart[CODY_MAX_BT], hdxStart[CODY_MAX_BT];
+  std::vector<int> hsN[CODY_MAX_BT], hdN[CODY_MAX_BT], hsxCode[CODY_MAX_BT], hsxStart[CODY_MAX_BT], hdxStart[CODY_MAX_BT];
 };
 
 // One block's share of a CI kernel: trajectory and task range [t0, t1).
@@ -308,6 +308,7 @@ struct cgpu_ctx {
   // CI work lists (blocks balanced by the number of terms; see ci_build_work)
   CiWork *applyWork_d = nullptr, *rdmWork_d = nullptr, *pairWork_d = nullptr;
   int nApplyWork = 0, nRdmWork = 0, nPairWork = 0;
+  int ciPairLanes = 1;  // threads of a pair of singles codes (k_ci_rdm_pairs)
   int ciSmem = 0;                 // bytes of shared memory for a CI vector (0: read it from global memory)
   int hasInteraction = 0, anyLaser = 0;
   // packed host states <-> the arena (batched upload / download)

@@ -137,6 +137,16 @@ __device__ __forceinline__ z_t warp_sum(z_t a) {
   return a;
 }
 
+// Sum over groups of `lanes` lanes (a power of two up to 32), to each of them
+__device__ __forceinline__ z_t lane_sum(z_t a, int lanes) {
+  const unsigned all = lanes == 32 ? 0xffffffffu : ((1u << lanes) - 1u) << (threadIdx.x & 31 & ~(lanes - 1));
+  for (int o = lanes >> 1; o > 0; o >>= 1) {
+    a.x += __shfl_xor_sync(all, a.x, o);
+    a.y += __shfl_xor_sync(all, a.y, o);
+  }
+  return a;
+}
+
 // The CI vector of the block's trajectory: staged in shared memory when it fits
 // (random gathers of C then hit shared memory), else read from global memory.
 __device__ __forceinline__ const z_t* stage_coeffs(const z_t* __restrict__ Cg, int nC, z_t* sm, int useSmem) {
@@ -356,13 +366,27 @@ __device__ __forceinline__ int rest_base(const CiView& v, int r, int b1, int b2)
   return I;
 }
 
+// The code of the adjoint excitation: creation and destruction orbitals exchanged.
+__host__ __device__ __forceinline__ int adjoint_code(int oc, int nO, int doubles) {
+  int o = oc - 1;
+  const int j = o % nO, i = o / nO % nO;
+  if (!doubles) return j * nO + i + 1;
+  o /= nO * nO;
+  return ((o % nO * nO + o / nO) * nO + j) * nO + i + 1;
+}
+
 // RDMs (ApplyH1FillRdm1 / ApplyH2FillRdm2, S_Coeffs_Generic.f90:103-319) as
 // gathers: rdmLin(oc) = sum over the excitations (I -> J) with orbital code
 // oc of f conj(C_J) C_I.  Every entry has exactly one writer, so there are no
-// atomics.  k_ci_rdm_codes: one warp per code of one body type (singles ->
+// atomics.  The adjoint code has the same excitations reversed, with the same
+// signs, so its entry is the conjugate: only the codes oc <= adjoint(oc) are
+// summed, which halves the FP64 work that bounds these kernels (8008
+// configurations of 6 in 16 orbitals: 105 us with every code, 55 now; the pairs of
+// a batch of 24 145 and 95).  k_ci_rdm_codes: one warp per code of one body type (singles ->
 // rdm1, doubles -> rdm2), lanes over the code's excitations (and over the
 // configurations of the other body types); k_ci_rdm_pairs: one thread per pair
-// of singles codes of two body types (the inter-body-type part of rdm2).
+// of singles codes of two body types (the inter-body-type part of rdm2), which
+// also takes the pair with the second code's adjoint.
 __global__ void k_ci_rdm_codes(const z_t* __restrict__ C0, z_t* __restrict__ r1Lin0, z_t* __restrict__ r2Lin0,
                                TRAJ_ARGS, const CiWork* __restrict__ work, int useSmem, int want1, int want2) {
   extern __shared__ z_t csm[];
@@ -413,12 +437,17 @@ __global__ void k_ci_rdm_codes(const z_t* __restrict__ C0, z_t* __restrict__ r1L
       }
     }
     acc = warp_sum(acc);
-    if (lane == 0) (kind == 0 ? r1Lin : r2Lin)[kind == 0 ? v.sxCode[b][q] : v.dxCode[b][q]] = acc;
+    if (lane == 0) {
+      const int oc = kind == 0 ? v.sxCode[b][q] : v.dxCode[b][q], adj = adjoint_code(oc, v.nO, kind);
+      z_t* out = kind == 0 ? r1Lin : r2Lin;
+      out[oc] = acc;
+      if (adj != oc) out[adj] = zconj(acc);
+    }
   }
 }
 
 __global__ void k_ci_rdm_pairs(const z_t* __restrict__ C0, z_t* __restrict__ r2Lin0, TRAJ_ARGS,
-                               const CiWork* __restrict__ work, int useSmem) {
+                               const CiWork* __restrict__ work, int useSmem, int lanes) {
   extern __shared__ z_t csm[];
   const CiWork wk = work[blockIdx.x];
   const int tb = wk.traj;
@@ -426,7 +455,8 @@ __global__ void k_ci_rdm_pairs(const z_t* __restrict__ C0, z_t* __restrict__ r2L
   const z_t* C = stage_coeffs(batn(C0, bs, tb), v.nC, csm, useSmem);
   z_t* r2Lin = batn(r2Lin0, bs, tb);
   const int nO2 = v.nO * v.nO;
-  for (int task = wk.t0 + threadIdx.x; task < wk.t1; task += blockDim.x) {
+  const int gl = threadIdx.x & (lanes - 1), nq = blockDim.x / lanes;
+  for (int task = wk.t0 + threadIdx.x / lanes; task < wk.t1; task += nq) {
     int q = task, b1 = 0, b2 = 1;
     for (;;) {
       int seg = v.nSc[b1] * v.nSc[b2];
@@ -441,21 +471,42 @@ __global__ void k_ci_rdm_pairs(const z_t* __restrict__ C0, z_t* __restrict__ r2L
     int nRest = v.nC / (v.nConf[b1] * v.nConf[b2]);
     const int *src1 = v.sxSrc[b1], *dst1 = v.sxDst[b1], *src2 = v.sxSrc[b2], *dst2 = v.sxDst[b2];
     const int8_t *fac1 = v.sxFac[b1], *fac2 = v.sxFac[b2];
+    const int c1 = v.sxCode[b1][q1], c2 = v.sxCode[b2][q2];
+    const int a1 = adjoint_code(c1, v.nO, 0), a2 = adjoint_code(c2, v.nO, 0);
+    const bool both = a1 != c1 && a2 != c2;
     z_t acc = zmk(0.0, 0.0);
-    for (int e1 = s1; e1 < s1 + n1; e1++) {
-      int i1 = src1[e1] * st1, j1 = dst1[e1] * st1;
-      bool g1 = fac1[e1] < 0;
+    z_t alt = zmk(0.0, 0.0);
+    // term t = (excitations k1, k2) = (t / n2, t % n2), advanced by `lanes` terms without divisions
+    const int dq = lanes / n2, dr = lanes - dq * n2;
+    int k1 = gl / n2, k2 = gl - k1 * n2;
 #pragma unroll 4
-      for (int e2 = s2; e2 < s2 + n2; e2++) {
-        int i2 = src2[e2] * st2, j2 = dst2[e2] * st2;
-        bool neg = g1 != (fac2[e2] < 0);
-        for (int r = 0; r < nRest; r++) {
-          int base = nRest == 1 ? 0 : rest_base(v, r, b1, b2);
-          zcfma(acc, C[base + j1 + j2], zsign(C[base + i1 + i2], neg));
-        }
+    for (int t = gl; t < n1 * n2; t += lanes) {
+      const int e1 = s1 + k1, e2 = s2 + k2;
+      const int i1 = src1[e1] * st1, j1 = dst1[e1] * st1, i2 = src2[e2] * st2, j2 = dst2[e2] * st2;
+      const bool neg = (fac1[e1] < 0) != (fac2[e2] < 0);
+      for (int r = 0; r < nRest; r++) {
+        int base = nRest == 1 ? 0 : rest_base(v, r, b1, b2);
+        zcfma(acc, C[base + j1 + j2], zsign(C[base + i1 + i2], neg));
+        if (both) zcfma(alt, C[base + j1 + i2], zsign(C[base + i1 + j2], neg));
+      }
+      k1 += dq;
+      k2 += dr;
+      if (k2 >= n2) {
+        k2 -= n2;
+        k1++;
       }
     }
-    r2Lin[(v.sxCode[b1][q1] - 1) * nO2 + v.sxCode[b2][q2]] = acc;
+    if (lanes > 1) {
+      acc = lane_sum(acc, lanes);
+      alt = lane_sum(alt, lanes);
+      if (gl > 0) continue;
+    }
+    r2Lin[(c1 - 1) * nO2 + c2] = acc;
+    if (a1 != c1 || a2 != c2) r2Lin[(a1 - 1) * nO2 + a2] = zconj(acc);
+    if (both) {
+      r2Lin[(c1 - 1) * nO2 + a2] = alt;
+      r2Lin[(a1 - 1) * nO2 + c2] = zconj(alt);
+    }
   }
 }
 
@@ -517,12 +568,18 @@ __global__ void __launch_bounds__(CI_RDM_THREADS, 2) k_ci_rdm_codes_df(const z_t
       }
     }
     acc = zdf_warp_sum(acc);
-    if (lane == 0) (kind == 0 ? r1Lin : r2Lin)[kind == 0 ? v.sxCode[b][q] : v.dxCode[b][q]] = zdf_to_z(acc);
+    if (lane == 0) {
+      const int oc = kind == 0 ? v.sxCode[b][q] : v.dxCode[b][q], adj = adjoint_code(oc, v.nO, kind);
+      z_t* out = kind == 0 ? r1Lin : r2Lin;
+      const z_t r = zdf_to_z(acc);
+      out[oc] = r;
+      if (adj != oc) out[adj] = zconj(r);
+    }
   }
 }
 
 __global__ void __launch_bounds__(CI_PAIR_THREADS, 2) k_ci_rdm_pairs_df(const z_t* __restrict__ C0, z_t* __restrict__ r2Lin0, TRAJ_ARGS,
-                                  const CiWork* __restrict__ work) {
+                                  const CiWork* __restrict__ work, int lanes) {
   extern __shared__ float4 cdf[];
   const CiWork wk = work[blockIdx.x];
   const int tb = wk.traj;
@@ -533,7 +590,8 @@ __global__ void __launch_bounds__(CI_PAIR_THREADS, 2) k_ci_rdm_pairs_df(const z_
   const float4* C = cdf;
   z_t* r2Lin = batn(r2Lin0, bs, tb);
   const int nO2 = v.nO * v.nO;
-  for (int task = wk.t0 + threadIdx.x; task < wk.t1; task += blockDim.x) {
+  const int gl = threadIdx.x & (lanes - 1), nq = blockDim.x / lanes;
+  for (int task = wk.t0 + threadIdx.x / lanes; task < wk.t1; task += nq) {
     int q = task, b1 = 0, b2 = 1;
     for (;;) {
       int seg = v.nSc[b1] * v.nSc[b2];
@@ -548,21 +606,43 @@ __global__ void __launch_bounds__(CI_PAIR_THREADS, 2) k_ci_rdm_pairs_df(const z_
     int nRest = v.nC / (v.nConf[b1] * v.nConf[b2]);
     const int *src1 = v.sxSrc[b1], *dst1 = v.sxDst[b1], *src2 = v.sxSrc[b2], *dst2 = v.sxDst[b2];
     const int8_t *fac1 = v.sxFac[b1], *fac2 = v.sxFac[b2];
+    const int c1 = v.sxCode[b1][q1], c2 = v.sxCode[b2][q2];
+    const int a1 = adjoint_code(c1, v.nO, 0), a2 = adjoint_code(c2, v.nO, 0);
+    const bool both = a1 != c1 && a2 != c2;
     zdf_acc acc = {0.0f, 0.0f, 0.0f, 0.0f};
-    for (int e1 = s1; e1 < s1 + n1; e1++) {
-      int i1 = src1[e1] * st1, j1 = dst1[e1] * st1;
-      bool g1 = fac1[e1] < 0;
+    zdf_acc alt = {0.0f, 0.0f, 0.0f, 0.0f};
+    // term t = (excitations k1, k2) = (t / n2, t % n2), advanced by `lanes` terms without divisions
+    const int dq = lanes / n2, dr = lanes - dq * n2;
+    int k1 = gl / n2, k2 = gl - k1 * n2;
 #pragma unroll 4
-      for (int e2 = s2; e2 < s2 + n2; e2++) {
-        int i2 = src2[e2] * st2, j2 = dst2[e2] * st2;
-        bool neg = g1 != (fac2[e2] < 0);
-        for (int r = 0; r < nRest; r++) {
-          int base = nRest == 1 ? 0 : rest_base(v, r, b1, b2);
-          zdf_cfma(acc, C[base + j1 + j2], C[base + i1 + i2], neg);
-        }
+    for (int t = gl; t < n1 * n2; t += lanes) {
+      const int e1 = s1 + k1, e2 = s2 + k2;
+      const int i1 = src1[e1] * st1, j1 = dst1[e1] * st1, i2 = src2[e2] * st2, j2 = dst2[e2] * st2;
+      const bool neg = (fac1[e1] < 0) != (fac2[e2] < 0);
+      for (int r = 0; r < nRest; r++) {
+        int base = nRest == 1 ? 0 : rest_base(v, r, b1, b2);
+        zdf_cfma(acc, C[base + j1 + j2], C[base + i1 + i2], neg);
+        if (both) zdf_cfma(alt, C[base + j1 + i2], C[base + i1 + j2], neg);
+      }
+      k1 += dq;
+      k2 += dr;
+      if (k2 >= n2) {
+        k2 -= n2;
+        k1++;
       }
     }
-    r2Lin[(v.sxCode[b1][q1] - 1) * nO2 + v.sxCode[b2][q2]] = zdf_to_z(acc);
+    z_t ra = zdf_to_z(acc), rb = zdf_to_z(alt);
+    if (lanes > 1) {
+      ra = lane_sum(ra, lanes);
+      rb = lane_sum(rb, lanes);
+      if (gl > 0) continue;
+    }
+    r2Lin[(c1 - 1) * nO2 + c2] = ra;
+    if (a1 != c1 || a2 != c2) r2Lin[(a1 - 1) * nO2 + a2] = zconj(ra);
+    if (both) {
+      r2Lin[(c1 - 1) * nO2 + a2] = rb;
+      r2Lin[(a1 - 1) * nO2 + c2] = zconj(rb);
+    }
   }
 }
 
@@ -668,10 +748,11 @@ __global__ void k_unfold_rdm2(z_t* __restrict__ rdm2, const z_t* __restrict__ li
 }
 
 // Groups an excitation table (maxConn x nConf, on the device) by orbital code:
-// distinct codes ascending, edges of one code in table order.
-void group_by_code(int nConf, int maxConn, const int* nConn_d, const int* exc_d, const int* code_d,
+// distinct codes oc <= adjoint(oc) ascending, edges of one code in table order.
+void group_by_code(int nO, int doubles, int nConf, int maxConn, const int* nConn_d, const int* exc_d, const int* code_d,
                    const int8_t* fac_d, int& nCodes, int*& xCode, int*& xStart, int*& xSrc, int*& xDst,
-                   int8_t*& xFac, std::vector<int>& nHost, std::vector<int>& startHost) {
+                   int8_t*& xFac, std::vector<int>& nHost, std::vector<int>& codeHost,
+                   std::vector<int>& startHost) {
   std::vector<int> n(nConf), exc((size_t)maxConn * nConf), code((size_t)maxConn * nConf);
   std::vector<int8_t> fac((size_t)maxConn * nConf);
   CODY_CUDA(cudaMemcpy(n.data(), nConn_d, sizeof(int) * nConf, cudaMemcpyDeviceToHost));
@@ -679,25 +760,36 @@ void group_by_code(int nConf, int maxConn, const int* nConn_d, const int* exc_d,
   CODY_CUDA(cudaMemcpy(code.data(), code_d, sizeof(int) * code.size(), cudaMemcpyDeviceToHost));
   CODY_CUDA(cudaMemcpy(fac.data(), fac_d, fac.size(), cudaMemcpyDeviceToHost));
   std::vector<int> codes;
-  size_t E = 0;
-  for (int c = 0; c < nConf; c++) E += n[c];
-  codes.reserve(E);
   for (int c = 0; c < nConf; c++)
-    for (int k = 0; k < n[c]; k++) codes.push_back(code[(size_t)maxConn * c + k]);
+    for (int k = 0; k < n[c]; k++) {
+      const int oc = code[(size_t)maxConn * c + k];
+      if (oc <= adjoint_code(oc, nO, doubles)) codes.push_back(oc);
+    }
+  const size_t E = codes.size();
   std::sort(codes.begin(), codes.end());
   codes.erase(std::unique(codes.begin(), codes.end()), codes.end());
   nCodes = (int)codes.size();
   std::vector<int> start(nCodes + 1, 0), src(std::max<size_t>(E, 1)), dst(std::max<size_t>(E, 1));
   std::vector<int8_t> f(std::max<size_t>(E, 1));
-  auto slot = [&](int oc) { return (int)(std::lower_bound(codes.begin(), codes.end(), oc) - codes.begin()); };
+  // place of a code, -1 for those left out
+  auto slot = [&](int oc) {
+    return oc > adjoint_code(oc, nO, doubles)
+               ? -1
+               : (int)(std::lower_bound(codes.begin(), codes.end(), oc) - codes.begin());
+  };
   for (int c = 0; c < nConf; c++)
-    for (int k = 0; k < n[c]; k++) start[slot(code[(size_t)maxConn * c + k]) + 1]++;
+    for (int k = 0; k < n[c]; k++) {
+      const int q = slot(code[(size_t)maxConn * c + k]);
+      if (q >= 0) start[q + 1]++;
+    }
   for (int q = 0; q < nCodes; q++) start[q + 1] += start[q];
   std::vector<int> fill(start.begin(), start.end() - 1);
   for (int c = 0; c < nConf; c++)
     for (int k = 0; k < n[c]; k++) {
       size_t at = (size_t)maxConn * c + k;
-      int e = fill[slot(code[at])]++;
+      const int q = slot(code[at]);
+      if (q < 0) continue;
+      int e = fill[q]++;
       src[e] = c;
       dst[e] = exc[at] - 1;
       f[e] = fac[at];
@@ -714,6 +806,7 @@ void group_by_code(int nConf, int maxConn, const int* nConn_d, const int* exc_d,
   upload(xDst, dst);
   upload(xFac, f);
   nHost = n;
+  codeHost = codes;
   startHost = start;
 }
 
@@ -795,10 +888,11 @@ void ci_build_tables(cgpu_ctx* c, SysHost& s) {
       if (kind == 0) t.maxS = mx; else t.maxD = mx;
     }
     CODY_CUDA(cudaStreamSynchronize(c->stream));  // the tables are written on the context stream
-    group_by_code(t.nConf, std::max(t.maxS, 1), t.sN, t.sExc, t.sCode, t.sFac, t.nSc, t.sxCode, t.sxStart, t.sxSrc,
-                  t.sxDst, t.sxFac, s.hsN[b], s.hsxStart[b]);
-    group_by_code(t.nConf, std::max(t.maxD, 1), t.dN, t.dExc, t.dCode, t.dFac, t.nDc, t.dxCode, t.dxStart, t.dxSrc,
-                  t.dxDst, t.dxFac, s.hdN[b], s.hdxStart[b]);
+    std::vector<int> dCodeHost;
+    group_by_code(s.nO, 0, t.nConf, std::max(t.maxS, 1), t.sN, t.sExc, t.sCode, t.sFac, t.nSc, t.sxCode, t.sxStart, t.sxSrc,
+                  t.sxDst, t.sxFac, s.hsN[b], s.hsxCode[b], s.hsxStart[b]);
+    group_by_code(s.nO, 1, t.nConf, std::max(t.maxD, 1), t.dN, t.dExc, t.dCode, t.dFac, t.nDc, t.dxCode, t.dxStart, t.dxSrc,
+                  t.dxDst, t.dxFac, s.hdN[b], dCodeHost, s.hdxStart[b]);
     CiView& v = s.view;
     v.nSc[b] = t.nSc;
     v.nDc[b] = t.nDc;
@@ -849,10 +943,12 @@ void ci_build_work(cgpu_ctx* c) {
     for (int b1 = 0; b1 < v.nBt; b1++)
       for (int b2 = b1 + 1; b2 < v.nBt; b2++) {
         long nRest = v.nC / ((long)v.nConf[b1] * v.nConf[b2]);
+        auto diag = [&](int b, int q) { return adjoint_code(s.hsxCode[b][q], s.nO, 0) == s.hsxCode[b][q]; };
         for (int q1 = 0; q1 < v.nSc[b1]; q1++)
           for (int q2 = 0; q2 < v.nSc[b2]; q2++)
             pw[t].push_back(1 + (long)(s.hsxStart[b1][q1 + 1] - s.hsxStart[b1][q1]) *
-                                    (s.hsxStart[b2][q2 + 1] - s.hsxStart[b2][q2]) * nRest);
+                                    (s.hsxStart[b2][q2 + 1] - s.hsxStart[b2][q2]) * nRest *
+                                    (diag(b1, q1) || diag(b2, q2) ? 1 : 2));
       }
     for (long w : rw[t]) rTot += w;
     for (long w : pw[t]) pTot += w;
@@ -872,19 +968,27 @@ void ci_build_work(cgpu_ctx* c) {
       }
     }
   };
-  // a block holds at least ~8 configurations (one per warp) / ~CI_PAIR_THREADS RDM pair tasks (one per
-  // thread) on average
+  // a block holds at least ~8 configurations (one per warp) / ~CI_PAIR_THREADS / ciPairLanes RDM pair
+  // tasks on average
   long nConfTot = 0, nTaskTot = 0, nPairTot = 0;
   for (int t = 0; t < c->nb; t++) {
     nConfTot += (long)aw[t].size();
     nTaskTot += (long)rw[t].size();
     nPairTot += (long)pw[t].size();
   }
+  // Lanes a pair: as many as bring the pairs to 512 threads an SM, with eight products each at
+  // least, so that the sum over the lanes (4 FP64 adds a step) does not outweigh them.  2025 pairs
+  // of 64 terms: 48 us with one lane, 16 with 16; 100 pairs of one term 6.5 with one, 14 with 32; a
+  // batch of 77000 95 with one, 121 with four.
+  c->ciPairLanes = 1;
+  while (c->ciPairLanes < 32 && nPairTot * c->ciPairLanes < 512L * c->numSms &&
+         16 * c->ciPairLanes <= pTot / std::max(1L, nPairTot))
+    c->ciPairLanes *= 2;
   cut(aw, std::max({64L, aTot / (8 * 152), (long)(CI_APPLY_THREADS / 32) * aTot / std::max(1L, nConfTot)}), 1 << 20,
       apply);
   cut(rw, std::max({64L, rTot / (8 * 152), (long)(CI_RDM_THREADS / 32) * rTot / std::max(1L, nTaskTot)}), 1 << 20,
       rdm);
-  cut(pw, std::max({64L, pTot / (8 * 152), (long)CI_PAIR_THREADS * pTot / std::max(1L, nPairTot)}), 1 << 20, pairs);
+  cut(pw, std::max({64L, pTot / (8 * 152), (long)CI_PAIR_THREADS / c->ciPairLanes * pTot / std::max(1L, nPairTot)}), 1 << 20, pairs);
   c->nApplyWork = (int)apply.size();
   c->nRdmWork = (int)rdm.size();
   c->nPairWork = (int)pairs.size();
@@ -937,10 +1041,10 @@ void launch_ci_rdm(cgpu_ctx* c, const z_t* C, int want1, int want2) {
   if (want2 && c->nPairWork > 0) {
     if (df)
       k_ci_rdm_pairs_df<<<c->nPairWork, CI_PAIR_THREADS, c->ciSmem, c->stream>>>(C, c->rdm2Lin_d, TRAJ_PASS(c),
-                                                                              c->pairWork_d);
+                                                                              c->pairWork_d, c->ciPairLanes);
     else
       k_ci_rdm_pairs<<<c->nPairWork, CI_PAIR_THREADS, c->ciSmem, c->stream>>>(C, c->rdm2Lin_d, TRAJ_PASS(c),
-                                                                              c->pairWork_d, c->ciSmem > 0);
+                                                                              c->pairWork_d, c->ciSmem > 0, c->ciPairLanes);
     CODY_LAUNCHED(c);
   }
   if (want1) {
