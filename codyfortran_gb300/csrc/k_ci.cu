@@ -30,6 +30,8 @@ constexpr int CI_RDM_THREADS = 512;
 // threads of an H.C block (one configuration per warp): with 55 registers per
 // thread two 512-thread blocks fit an SM, 32 warps sharing two staged CI vectors
 constexpr int CI_APPLY_THREADS = 512;
+// threads of the FP64 forms' blocks (the codes, H.C)
+constexpr int CI_FP64_THREADS = 256;
 
 __device__ __forceinline__ unsigned long long bitmask_below(int p) {  // bits [0, p)
   return p >= 64 ? ~0ULL : ((1ULL << p) - 1ULL);
@@ -206,6 +208,34 @@ __global__ void k_ci_apply(const z_t* __restrict__ C0, z_t* __restrict__ dC0, co
         int n2 = v.sN[b2][c2 - 1];
         size_t col2 = (size_t)v.maxS[b2] * (c2 - 1);
         int st2 = v.stride[b2];
+        if (n1 <= 32 && n2 <= 32) {
+          // the n1 x n2 pairs over all lanes, as in k_ci_apply_df: 22 x 22 pairs are 16 FP64 steps
+          // instead of 22 on 22 lanes (a batch of 24: 299 -> 249 us)
+          int p1 = 0, e1 = 0, p2 = 0, e2 = 0;
+          if (lane < n1) {
+            p1 = ((v.sCode[b][col1 + lane] - 1) * nO2) * 2 + (v.sFac[b][col1 + lane] < 0);
+            e1 = (v.sExc[b][col1 + lane] - c) * st;
+          }
+          if (lane < n2) {
+            p2 = v.sCode[b2][col2 + lane] * 2 + (v.sFac[b2][col2 + lane] < 0);
+            e2 = (v.sExc[b2][col2 + lane] - c2) * st2;
+          }
+          const int total = n1 * n2, q = 32 / n2, r = 32 - q * n2;
+          int k1 = lane / n2, k2 = lane - k1 * n2;
+#pragma unroll 2
+          for (int base = 0; base < total; base += 32) {
+            const int a1 = __shfl_sync(0xffffffffu, p1, k1 & 31), x1 = __shfl_sync(0xffffffffu, e1, k1 & 31);
+            const int a2 = __shfl_sync(0xffffffffu, p2, k2), x2 = __shfl_sync(0xffffffffu, e2, k2);
+            if (base + lane < total)
+              zfma(acc, h2Lin[(a1 >> 1) + (a2 >> 1)], zsign(C[I - 1 + x1 + x2], ((a1 ^ a2) & 1) != 0));
+            k1 += q;
+            k2 += r;
+            if (k2 >= n2) {
+              k2 -= n2;
+              k1++;
+            }
+          }
+        } else
         for (int k2b = 0; k2b < n2; k2b += 32) {
           int k2 = k2b + lane;
           bool has2 = k2 < n2;
@@ -968,8 +998,9 @@ void ci_build_work(cgpu_ctx* c) {
       }
     }
   };
-  // a block holds at least ~8 configurations (one per warp) / ~CI_PAIR_THREADS / ciPairLanes RDM pair
-  // tasks on average
+  // a block holds at least ~aWarps configurations (one per warp; twice as many cost H.C of 8008
+  // configurations 84 us instead of 71) / ~16 codes / ~CI_PAIR_THREADS / ciPairLanes RDM pair tasks on
+  // average
   long nConfTot = 0, nTaskTot = 0, nPairTot = 0;
   for (int t = 0; t < c->nb; t++) {
     nConfTot += (long)aw[t].size();
@@ -984,7 +1015,9 @@ void ci_build_work(cgpu_ctx* c) {
   while (c->ciPairLanes < 32 && nPairTot * c->ciPairLanes < 512L * c->numSms &&
          16 * c->ciPairLanes <= pTot / std::max(1L, nPairTot))
     c->ciPairLanes *= 2;
-  cut(aw, std::max({64L, aTot / (8 * 152), (long)(CI_APPLY_THREADS / 32) * aTot / std::max(1L, nConfTot)}), 1 << 20,
+  const bool df = c->ciDf && sizeof(z_t) * (size_t)c->nC <= 72 * 1024;
+  const long aWarps = (df ? CI_APPLY_THREADS : CI_FP64_THREADS) / 32;
+  cut(aw, std::max({64L, aTot / (8 * 152), aWarps * aTot / std::max(1L, nConfTot)}), 1 << 20,
       apply);
   cut(rw, std::max({64L, rTot / (8 * 152), (long)(CI_RDM_THREADS / 32) * rTot / std::max(1L, nTaskTot)}), 1 << 20,
       rdm);
@@ -1019,7 +1052,7 @@ void launch_ci_apply(cgpu_ctx* c, const z_t* C, z_t* dC, int useH1, int useH2) {
                                                                             TRAJ_PASS(c), c->applyWork_d, useH1,
                                                                             useH2);
   else
-    k_ci_apply<<<c->nApplyWork, 256, c->ciSmem, c->stream>>>(C, dC, c->h1Lin_d, c->h2Lin_d, TRAJ_PASS(c),
+    k_ci_apply<<<c->nApplyWork, CI_FP64_THREADS, c->ciSmem, c->stream>>>(C, dC, c->h1Lin_d, c->h2Lin_d, TRAJ_PASS(c),
                                                             c->applyWork_d, c->ciSmem > 0, useH1, useH2);
   CODY_LAUNCHED(c);
 }
@@ -1034,7 +1067,7 @@ void launch_ci_rdm(cgpu_ctx* c, const z_t* C, int want1, int want2) {
       k_ci_rdm_codes_df<<<c->nRdmWork, CI_RDM_THREADS, c->ciSmem, c->stream>>>(C, c->rdm1Lin_d, c->rdm2Lin_d, TRAJ_PASS(c),
                                                                     c->rdmWork_d, want1, want2);
     else
-      k_ci_rdm_codes<<<c->nRdmWork, 256, c->ciSmem, c->stream>>>(C, c->rdm1Lin_d, c->rdm2Lin_d, TRAJ_PASS(c),
+      k_ci_rdm_codes<<<c->nRdmWork, CI_FP64_THREADS, c->ciSmem, c->stream>>>(C, c->rdm1Lin_d, c->rdm2Lin_d, TRAJ_PASS(c),
                                                                  c->rdmWork_d, c->ciSmem > 0, want1, want2);
     CODY_LAUNCHED(c);
   }
