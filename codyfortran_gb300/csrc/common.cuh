@@ -349,6 +349,7 @@ struct cgpu_ctx {
   z_t *r2s_d = nullptr;                       // spin-summed spatial rdm2 (nOS^2 x nOS^2)
   // reductions / scratch
   z_t* partial_d = nullptr;
+  unsigned* gramCount_d = nullptr;            // blocks of a single system's Gram sum that have arrived
   size_t partialCap = 0;                      // complex entries per trajectory
   int lzBlocks = 148;                         // blocks per trajectory of the Lanczos reductions
   int lzBlocksHeur = 148, lzBlocksCap = 148;  // the set-up heuristic's count and the most the partials hold

@@ -597,6 +597,8 @@ void build_ctx(cgpu_ctx* c, const cgpu_desc* descs, int nSys) {
   for (int b = 0; b < nSys; b++) so[b + 1] = so[b] + c->sys[b].nS;
   c->stageOff = so;
   CODY_CUDA(cudaMemcpy(c->stageOff_d, so.data(), sizeof(long) * (nSys + 1), cudaMemcpyHostToDevice));
+  CODY_CUDA(cudaMalloc(&c->gramCount_d, sizeof(unsigned)));
+  CODY_CUDA(cudaMemset(c->gramCount_d, 0, sizeof(unsigned)));
   mixed_init(c);
   sil_init(c);
   {
@@ -629,7 +631,8 @@ void free_ctx(cgpu_ctx* c) {
     if (s.samples_d) cudaFree(s.samples_d);
   }
   void* ptrs[] = {c->arena,      c->shape_d,     c->metricUser_d, c->stageOff_d, c->stage_d,
-                  c->tStage_d,    c->applyWork_d, c->rdmWork_d,    c->pairWork_d,  c->sysTmp_d};
+                  c->tStage_d,    c->applyWork_d, c->rdmWork_d,    c->pairWork_d,  c->sysTmp_d,
+                  c->gramCount_d};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (c->lz_h) cudaFreeHost(c->lz_h);

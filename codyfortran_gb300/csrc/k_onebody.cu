@@ -324,26 +324,73 @@ __device__ __forceinline__ bool gram_cols(const TrajShape& S, int group, int& c0
 }
 
 // ---------------------------------------------------------------------------
-// Weighted Gram partials: part[blk][i + n*j] = sum_{g in chunks of blk}
-//   conj(A[g, c0+i]) * B[g, c0+j] * w[g]
+// Weighted Gram matrix: G[i + n j] = scale sum_g conj(A[g, c0+i]) B[g, c0+j] w[g],
+// in row chunks per block.  A single system's few small partials (nn entries from
+// nBlk blocks, nn nBlk <= GR_LAST) are summed by the block that arrives last, in block
+// order; more of them, and a batch's, by k_gram_final's warp per entry (a batch of 512
+// lost 2 ms a step to the blocks' counters).  4 x 4 entries over 501 points: 10.4 us
+// and another 4.1 in k_gram_final when 16 threads summed a chunk's 32 rows in one
+// chain, 9.2 now.  16 x 16 over 2801 points, where the FP64 pipe bounds the sums: 18.5
+// us in 88 chunks, 13.3 in one for each SM.
 // ---------------------------------------------------------------------------
-constexpr int GR_CHUNK = 32;
+constexpr int GR_CHUNK = 32, GR_CHUNK_MIN = 8;
 constexpr int GR_PER_THREAD = 16;  // 256 threads x 16 = 4096 = 64^2 Gram entries
+constexpr int GR_THREADS = 256;
+constexpr int GR_LAST = 4096;
 
-__global__ void k_gram_partial(z_t* __restrict__ part, const z_t* __restrict__ A, const z_t* __restrict__ B,
-                               const double* __restrict__ w, TRAJ_ARGS, int group, int chunk) {
+// Lanes (a power of two up to 32) that share an entry of nn <= GR_THREADS.
+__device__ __forceinline__ int gram_lanes(int nn) {
+  int r = 1;
+  while (r < 32 && 2 * r * nn <= GR_THREADS) r *= 2;
+  return r;
+}
+__device__ __forceinline__ z_t gram_lane_sum(z_t s, int lanes) {
+  for (int o = 1; o < lanes; o <<= 1) {
+    s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+    s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+  }
+  return s;
+}
+
+// After a block has written its partials: the last of them sums (count: zero, and
+// zero again afterwards).
+__device__ void gram_last(z_t* G, const z_t* part, int nn, double scale, unsigned* count) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicInc(count, gridDim.x - 1) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const int nBlk = gridDim.x, L = gram_lanes(nn), ln = threadIdx.x % L;
+  for (int e0 = 0; e0 < nn; e0 += GR_THREADS / L) {
+    const int e = e0 + threadIdx.x / L;
+    z_t s = zmk(0.0, 0.0);
+    if (e < nn)
+      for (int b = ln; b < nBlk; b += L) s = zadd(s, __ldcg(part + (size_t)b * nn + e));
+    s = gram_lane_sum(s, L);
+    if (e < nn && ln == 0) G[e] = zscale(s, scale);
+  }
+}
+
+// count: arrivals (null: partials only)
+__global__ void __launch_bounds__(GR_THREADS) k_gram_partial(z_t* __restrict__ G, z_t* __restrict__ part,
+                                                             const z_t* __restrict__ A, const z_t* __restrict__ B,
+                                                             const double* __restrict__ w, TRAJ_ARGS, int group,
+                                                             int chunk, double scale, unsigned* __restrict__ count) {
   extern __shared__ z_t sh[];
   const TrajShape& S = shp[blockIdx.z];
   int c0, n;
   if (!gram_cols(S, group, c0, n)) return;
   const int nG = S.nG;
+  G = bat(G, bs);
   part = bat(part, bs);
   A = bat(A, bs);
   B = bat(B, bs);
   w = bat(w, bs);
   z_t* sa = sh;                 // chunk x n
   z_t* sb = sh + chunk * n;     // chunk x n
-  int nn = n * n;
+  const int nn = n * n, L = gram_lanes(nn), ln = threadIdx.x % L;
   z_t acc[GR_PER_THREAD];
   for (int q = 0; q < GR_PER_THREAD; q++) acc[q] = zmk(0.0, 0.0);
   for (int r0 = blockIdx.x * chunk; r0 < nG; r0 += gridDim.x * chunk) {
@@ -363,11 +410,11 @@ __global__ void k_gram_partial(z_t* __restrict__ part, const z_t* __restrict__ A
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < GR_PER_THREAD; q++) {
-      int e = threadIdx.x + q * blockDim.x;
+      int e = (threadIdx.x + q * GR_THREADS) / L;
       if (e >= nn) break;
       int ii = e % n, jj = e / n;
       z_t s = acc[q];
-      for (int r = 0; r < chunk; r++) {
+      for (int r = ln; r < chunk; r += L) {
         z_t a = sa[r * n + ii], b = sb[r * n + jj];
         s.x += a.x * b.x + a.y * b.y;
         s.y += a.x * b.y - a.y * b.x;
@@ -375,12 +422,18 @@ __global__ void k_gram_partial(z_t* __restrict__ part, const z_t* __restrict__ A
       acc[q] = s;
     }
   }
+  const bool one = count && gridDim.x == 1;
 #pragma unroll
   for (int q = 0; q < GR_PER_THREAD; q++) {
-    int e = threadIdx.x + q * blockDim.x;
-    if (e >= nn) break;
-    part[(size_t)blockIdx.x * nn + e] = acc[q];
+    if (q * GR_THREADS >= nn * L) break;
+    const int e = (threadIdx.x + q * GR_THREADS) / L;
+    const z_t s = gram_lane_sum(acc[q], L);
+    if (e < nn && ln == 0) {
+      if (one) G[e] = zscale(s, scale);
+      else part[(size_t)blockIdx.x * nn + e] = s;
+    }
   }
+  if (count && !one) gram_last(G, part, nn, scale, count);
 }
 
 // one warp per Gram entry, lanes over the block partials (fixed order); G is n x n
@@ -753,7 +806,14 @@ unsigned vec_blocks(const cgpu_ctx* c, size_t n) {
   return (unsigned)std::max<size_t>(1, std::min(b, cap));
 }
 
-int gram_chunk(int n) { return std::max(1, std::min(GR_CHUNK, 1024 / std::max(n, 1))); }  // <= 32 KB shared
+// Rows of a block: at most 32 KB of tiles; a single system's in the FP64 form, whose
+// pipe is the bound, cut to a chunk per SM.
+int gram_chunk(const cgpu_ctx* c, int n) {
+  int chunk = std::max(1, std::min(GR_CHUNK, 1024 / std::max(n, 1)));
+  if (c->nb == 1 && !c->ciDf)
+    chunk = std::min(chunk, std::max(GR_CHUNK_MIN, (c->nG + c->numSms - 1) / c->numSms));
+  return chunk;
+}
 
 int gram_blocks(const cgpu_ctx* c, int chunk) {
   int nBlk = std::min(RED_BLOCKS, (c->nG + chunk - 1) / chunk);
@@ -773,13 +833,16 @@ void check_partial(const cgpu_ctx* c, size_t need) {
 // The weighted Gram partials in double-float arithmetic (the fixed-point forms):
 // the chunk of A and w B staged as double-floats, every term conj(a) b an
 // error-free FP32 product with two-sum accumulation, FP64 partials out.
-__global__ void k_gram_partial_df(z_t* __restrict__ part, const z_t* __restrict__ A, const z_t* __restrict__ B,
-                                  const double* __restrict__ w, TRAJ_ARGS, int group, int chunk) {
+__global__ void __launch_bounds__(GR_THREADS) k_gram_partial_df(z_t* __restrict__ G, z_t* __restrict__ part,
+                                                                const z_t* __restrict__ A, const z_t* __restrict__ B,
+                                                                const double* __restrict__ w, TRAJ_ARGS, int group,
+                                                                int chunk, double scale, unsigned* __restrict__ count) {
   extern __shared__ float4 shg[];
   const TrajShape& S = shp[blockIdx.z];
   int c0, n;
   if (!gram_cols(S, group, c0, n)) return;
   const int nG = S.nG;
+  G = bat(G, bs);
   part = bat(part, bs);
   A = bat(A, bs);
   B = bat(B, bs);
@@ -845,30 +908,28 @@ __global__ void k_gram_partial_df(z_t* __restrict__ part, const z_t* __restrict_
       }
       part[(size_t)blockIdx.x * nn + threadIdx.x] = zdf_to_z(t);
     }
-    return;
-  }
+  } else {
 #pragma unroll
-  for (int q = 0; q < GR_PER_THREAD; q++) {
-    int e = threadIdx.x + q * blockDim.x;
-    if (e >= nn) break;
-    part[(size_t)blockIdx.x * nn + e] = zdf_to_z(acc[q]);
+    for (int q = 0; q < GR_PER_THREAD; q++) {
+      int e = threadIdx.x + q * blockDim.x;
+      if (e >= nn) break;
+      part[(size_t)blockIdx.x * nn + e] = zdf_to_z(acc[q]);
+    }
   }
+  if (count) gram_last(G, part, nn, scale, count);
 }
 
 void launch_gram(cgpu_ctx* c, z_t* G, const z_t* A, const z_t* B, int group, int nMax, double scale) {
-  int chunk = gram_chunk(nMax);
-  int nBlk = gram_blocks(c, chunk);
+  const int chunk = gram_chunk(c, nMax), nBlk = gram_blocks(c, chunk);
   check_partial(c, (size_t)nBlk * nMax * nMax);
   size_t sh = 2 * sizeof(z_t) * chunk * nMax;
-  int threads = 256;
-  if (nMax * nMax > GR_PER_THREAD * threads) throw std::string("launch_gram: more than 64 orbitals");
-  if (c->ciDf)
-    k_gram_partial_df<<<bgrid(c, nBlk), threads, sh, c->stream>>>(c->partial_d, A, B, c->w_d, TRAJ_PASS(c), group,
-                                                                  chunk);
-  else
-    k_gram_partial<<<bgrid(c, nBlk), threads, sh, c->stream>>>(c->partial_d, A, B, c->w_d, TRAJ_PASS(c), group,
-                                                               chunk);
+  if (nMax * nMax > GR_PER_THREAD * GR_THREADS) throw std::string("launch_gram: more than 64 orbitals");
+  unsigned* count = c->nb == 1 && nMax * nMax * nBlk <= GR_LAST ? c->gramCount_d : nullptr;
+  auto part = c->ciDf ? k_gram_partial_df : k_gram_partial;
+  part<<<bgrid(c, nBlk), GR_THREADS, sh, c->stream>>>(G, c->partial_d, A, B, c->w_d, TRAJ_PASS(c), group, chunk, scale,
+                                                      count);
   CODY_LAUNCHED(c);
+  if (count) return;
   k_gram_final<<<bgrid(c, ceil_div((size_t)nMax * nMax * 32, 256)), 256, 0, c->stream>>>(G, c->partial_d, nBlk,
                                                                                          TRAJ_PASS(c), group, scale);
   CODY_LAUNCHED(c);
@@ -884,7 +945,7 @@ int max_group_size(const cgpu_ctx* c, int g) {
 }  // namespace
 
 size_t gram_partial_need(const cgpu_ctx* c, int n) {
-  int chunk = gram_chunk(n);
+  int chunk = gram_chunk(c, n);
   return (size_t)gram_blocks(c, chunk) * n * n;
 }
 
