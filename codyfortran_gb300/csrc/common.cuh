@@ -349,6 +349,7 @@ struct cgpu_ctx {
   z_t *r2s_d = nullptr;                       // spin-summed spatial rdm2 (nOS^2 x nOS^2)
   // reductions / scratch
   z_t* partial_d = nullptr;
+  z_t* partialC_d = nullptr;  // of the coefficients' projector (148 entries)
   unsigned* gramCount_d = nullptr;            // blocks of a single system's Gram sum that have arrived
   size_t partialCap = 0;                      // complex entries per trajectory
   int lzBlocks = 148;                         // blocks per trajectory of the Lanczos reductions
@@ -382,6 +383,9 @@ struct cgpu_ctx {
   z_t* tdciOrbs_d = nullptr;
   // stream / graph
   cudaStream_t stream = nullptr;
+  // the branches of the equation of motion beside `stream` (ctx.cu: td_device)
+  cudaStream_t side[2] = {nullptr, nullptr};
+  cudaEvent_t branchEv[5] = {};
   cudaGraphExec_t stepGraph = nullptr;
   double graphDt = 0;
   int graphKrylov = 0, graphMetric = -1, graphKernels = 0, graphProf = 0;
@@ -518,7 +522,13 @@ void mixed_init(cgpu_ctx* c);
 void mixed_free(cgpu_ctx* c);
 int mixed_error(cgpu_ctx* c);
 void launch_correlation_mixed(cgpu_ctx* c, z_t* dOrbs, const z_t* orbs, int wantH2);
-void launch_fill_h2_fx(cgpu_ctx* c, const z_t* orbs);  // FillH2 with the FP64 form's slices (fxOn)
+void launch_fill_h2_fx(cgpu_ctx* c, const z_t* orbs);
+bool fx_ready(const cgpu_ctx* c);
+void launch_fx_potentials(cgpu_ctx* c, const z_t* orbs);
+void launch_fx_split_R(cgpu_ctx* c);
+void launch_fx_Z(cgpu_ctx* c);
+void launch_fx_epilogue(cgpu_ctx* c, z_t* dOrbs, const z_t* orbs);
+void launch_fx_h2(cgpu_ctx* c);  // FillH2 with the FP64 form's slices (fxOn)
 // Tile tuner hooks of the fixed-point contractions.  A tile table t[9] holds,
 // for W = V S, Z = W R'' and h2 = S^T W in turn: N-tile width, compact (two
 // CTAs per SM) flag, K splits.  fx_tiles_get returns false outside the

@@ -372,6 +372,7 @@ size_t layout(cgpu_ctx* c, char* base) {
   Z(c->basis_d, nS * (size_t)c->maxKrylov);
   if (c->method == CGPU_METHOD_TDCI) Z(c->tdciOrbs_d, nG * n);
   Z(c->partial_d, c->partialCap);
+  Z(c->partialC_d, 148);
   off = mixed_layout(c, base, off);
   return (off + 1023) & ~(size_t)1023;
 }
@@ -448,6 +449,8 @@ void build_ctx(cgpu_ctx* c, const cgpu_desc* descs, int nSys) {
   c->ciDf = (c->precision == CGPU_PREC_MIXED_FX || c->precision == CGPU_PREC_MIXED_FX6) ? 1 : 0;
   c->hasInteraction = d0->has_interaction ? 1 : 0;
   CODY_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
+  for (cudaStream_t& s : c->side) CODY_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+  for (cudaEvent_t& e : c->branchEv) CODY_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   {
     int dev = 0;
     CODY_CUDA(cudaGetDevice(&dev));
@@ -636,6 +639,10 @@ void free_ctx(cgpu_ctx* c) {
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (c->lz_h) cudaFreeHost(c->lz_h);
+  for (cudaEvent_t e : c->branchEv)
+    if (e) cudaEventDestroy(e);
+  for (cudaStream_t s : c->side)
+    if (s) cudaStreamDestroy(s);
   if (c->stream) cudaStreamDestroy(c->stream);
 }
 
@@ -676,15 +683,72 @@ void td_device(cgpu_ctx* c, int which, z_t* out, const z_t* in, double t, z_t po
     explicit FuseScope(cgpu_ctx* cc) : c(cc), prev(cc->fuseLayouts) { c->fuseLayouts = 1; }
     ~FuseScope() { c->fuseLayouts = prev; }
   } fuse(c);
-  launch_ci_rdm(c, C, 1, 1);
-  if (which == CGPU_TD_FULL) {
-    launch_onebody(c, dOrbs, orbs, t, zmk(1.0, 0.0), 0);
-    launch_fill_h1_from(c, orbs, dOrbs, c->h1_d);
-  } else {
-    launch_onebody(c, c->orbTmp_d, orbs, t, zmk(1.0, 0.0), 0);
-    launch_fill_h1_from(c, orbs, c->orbTmp_d, c->h1_d);
-    batch_zero(c, dOrbs, sizeof(z_t) * nGO);
+  auto oneBody = [&]() {
+    if (which == CGPU_TD_FULL) {
+      launch_onebody(c, dOrbs, orbs, t, zmk(1.0, 0.0), 0);
+      launch_fill_h1_from(c, orbs, dOrbs, c->h1_d);
+    } else {
+      launch_onebody(c, c->orbTmp_d, orbs, t, zmk(1.0, 0.0), 0);
+      launch_fill_h1_from(c, orbs, c->orbTmp_d, c->h1_d);
+      batch_zero(c, dOrbs, sizeof(z_t) * nGO);
+    }
+  };
+  if (fx_ready(c) && !c->profTarget) {
+    // Three branches: the pair potentials, Z and the orbitals on the context's
+    // stream; the density matrices and rho^-1 rho2, which Z needs, beside the
+    // potentials; the one-body part, then (after the potentials) h2 and the
+    // coefficients beside Z.  A small system's launches are latencies, and the
+    // density matrices' and H.C's FP64 fills the SMs beside the tensor cores: in one
+    // row and here, 10 helium steps 9.33 / 6.63 ms, a trimer step 3.69 / 3.20, a scan
+    // of 24 7.57 / 6.25, one fx6 derivative 373 / 215 us; a scan of 512 unchanged.
+    // partial_d and gram_d are the one-body branch's up to its event, then the
+    // orbitals'; the coefficients' projector has partials of its own.  A profile of one
+    // kernel family keeps the row.
+    enum { START, DENSITY, ONEBODY, POTENTIALS, COEFFS };
+    auto record = [&](int e) { CODY_CUDA(cudaEventRecord(c->branchEv[e], c->stream)); };
+    auto wait = [&](int e) { CODY_CUDA(cudaStreamWaitEvent(c->stream, c->branchEv[e], 0)); };
+    struct OnStream {
+      cgpu_ctx* c;
+      cudaStream_t prev;
+      OnStream(cgpu_ctx* cc, cudaStream_t s) : c(cc), prev(cc->stream) { c->stream = s; }
+      ~OnStream() { c->stream = prev; }
+    };
+    record(START);
+    launch_fx_potentials(c, orbs);
+    record(POTENTIALS);
+    {
+      OnStream on(c, c->side[0]);
+      wait(START);
+      launch_ci_rdm(c, C, 1, 1);
+      launch_rdm_inverse(c);
+      launch_fx_split_R(c);
+      record(DENSITY);
+    }
+    {
+      OnStream on(c, c->side[1]);
+      wait(START);
+      oneBody();
+      launch_fold_h1(c);
+      batch_zero(c, dC, sizeof(z_t) * c->nC);
+      record(ONEBODY);
+      wait(POTENTIALS);
+      launch_fx_h2(c);
+      launch_fold_h2(c);
+      launch_ci_apply(c, C, dC, 1, 1);
+      launch_project_coeffs(c, dC, C);
+      record(COEFFS);
+    }
+    wait(DENSITY);
+    launch_fx_Z(c);
+    wait(ONEBODY);
+    launch_fx_epilogue(c, dOrbs, orbs);
+    launch_project_orbs(c, dOrbs, orbs);
+    wait(COEFFS);
+    if (!unit) launch_scale(c, out, f, VSEL_STATE);
+    return;
   }
+  launch_ci_rdm(c, C, 1, 1);
+  oneBody();
   if (c->precision == CGPU_PREC_FP64) launch_correlation(c, dOrbs, orbs, 1);
   else launch_correlation_mixed(c, dOrbs, orbs, 1);
   launch_fold_h1(c);

@@ -945,36 +945,61 @@ static void fx_potentials(cgpu_ctx* c, const z_t* orbs, bool exact, bool wantW) 
   CODY_LAUNCHED(c);
 }
 
-// The fixed-point forms of the three contractions.
-template <int L, int L2>
-static void correlation_fx_t(cgpu_ctx* c, z_t* dOrbs, const z_t* orbs, int wantH2) {
+// Calls f<L, L2>() of the context's slice plan.
+template <class F>
+static void fx_plan(const cgpu_ctx* c, F f) {
+  const int L = c->mixed->L, L2 = c->mixed->L2;
+  if (L == FX_L64) return f(std::integral_constant<int, FX_L64>(), std::integral_constant<int, FX_L64>());
+  if (L == 5 && L2 == 4) return f(std::integral_constant<int, 5>(), std::integral_constant<int, 4>());
+  if (L == 5 && L2 == 5) return f(std::integral_constant<int, 5>(), std::integral_constant<int, 5>());
+  if (L == 5 && L2 == 6) return f(std::integral_constant<int, 5>(), std::integral_constant<int, 6>());
+  if (L == 6 && L2 == 5) return f(std::integral_constant<int, 6>(), std::integral_constant<int, 5>());
+  if (L == 6 && L2 == 6) return f(std::integral_constant<int, 6>(), std::integral_constant<int, 6>());
+  throw std::string("internal: no kernels for this slice plan");
+}
+
+// The pieces of the correlation in the fixed-point forms, for callers that place
+// them on several streams: the pair potentials; the digits of rho^-1 rho2 (after
+// launch_rdm_inverse); Z from both, dOrbs += its contraction with the orbitals; h2
+// from the potentials.
+bool fx_ready(const cgpu_ctx* c) { return c->fxOn && c->mixed && c->mixed->L > 0 && c->hasInteraction; }
+
+void launch_fx_potentials(cgpu_ctx* c, const z_t* orbs) {
+  fx_plan(c, [&](auto L, auto L2) { fx_potentials<L(), L2()>(c, orbs, false, true); });
+}
+
+void launch_fx_split_R(cgpu_ctx* c) {
+  ProfScope prof(c, CGPU_KERNEL_CORRELATION);
   MixedBufs* m = c->mixed;
-  const int Q = c->nOS * c->nOS;
-  fx_potentials<L, L2>(c, orbs, false, true);
-  {
-    ProfScope prof(c, CGPU_KERNEL_CORRELATION);
-    k_fx_split_R<L2><<<dim3(2 * Q, 1, c->nb), 64, sizeof(double) * m->KpMax, c->stream>>>(
+  fx_plan(c, [&](auto, auto L2) {
+    k_fx_split_R<L2()><<<dim3(2 * c->nOS * c->nOS, 1, c->nb), 64, sizeof(double) * m->KpMax, c->stream>>>(
         m->RxB, m->eR, c->Rp_d, c->pairL_d, c->pairK_d, m->KpMax, TRAJ_PASS(c));
-    CODY_LAUNCHED(c);
-    fx_run_Z(c);
-    launch_corr_epilogue(c, dOrbs, orbs, (z_t*)m->Zd);
-  }
-  if (wantH2) {
-    ProfScope prof(c, CGPU_KERNEL_H2);
-    fx_run_H2(c, false);
-    launch_h2_layout(c);
-  }
+  });
+  CODY_LAUNCHED(c);
+}
+
+void launch_fx_Z(cgpu_ctx* c) {
+  ProfScope prof(c, CGPU_KERNEL_CORRELATION);
+  fx_run_Z(c);
+}
+
+void launch_fx_epilogue(cgpu_ctx* c, z_t* dOrbs, const z_t* orbs) {
+  ProfScope prof(c, CGPU_KERNEL_CORRELATION);
+  launch_corr_epilogue(c, dOrbs, orbs, (z_t*)c->mixed->Zd);
+}
+
+void launch_fx_h2(cgpu_ctx* c) {
+  ProfScope prof(c, CGPU_KERNEL_H2);
+  fx_run_H2(c, false);
+  launch_h2_layout(c);
 }
 
 static void correlation_fx(cgpu_ctx* c, z_t* dOrbs, const z_t* orbs, int wantH2) {
-  const int L = c->mixed->L, L2 = c->mixed->L2;
-  if (L == FX_L64) return correlation_fx_t<FX_L64, FX_L64>(c, dOrbs, orbs, wantH2);
-  if (L == 5 && L2 == 4) return correlation_fx_t<5, 4>(c, dOrbs, orbs, wantH2);
-  if (L == 5 && L2 == 5) return correlation_fx_t<5, 5>(c, dOrbs, orbs, wantH2);
-  if (L == 5 && L2 == 6) return correlation_fx_t<5, 6>(c, dOrbs, orbs, wantH2);
-  if (L == 6 && L2 == 5) return correlation_fx_t<6, 5>(c, dOrbs, orbs, wantH2);
-  if (L == 6 && L2 == 6) return correlation_fx_t<6, 6>(c, dOrbs, orbs, wantH2);
-  throw std::string("internal: no kernels for this slice plan");
+  launch_fx_potentials(c, orbs);
+  launch_fx_split_R(c);
+  launch_fx_Z(c);
+  launch_fx_epilogue(c, dOrbs, orbs);
+  if (wantH2) launch_fx_h2(c);
 }
 
 void launch_fill_h2_fx(cgpu_ctx* c, const z_t* orbs) {

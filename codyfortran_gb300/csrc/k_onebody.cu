@@ -1021,10 +1021,9 @@ void launch_project_orbs(cgpu_ctx* c, z_t* dOrbs, const z_t* orbs) {
 void launch_project_coeffs(cgpu_ctx* c, z_t* dC, const z_t* C) {
   ProfScope prof(c, CGPU_KERNEL_PROJECTORS);
   int nBlk = coeff_blocks(c);
-  check_partial(c, nBlk);
-  k_dot_partial<<<bgrid(c, nBlk), 256, 0, c->stream>>>(c->partial_d, C, dC, TRAJ_PASS(c));
+  k_dot_partial<<<bgrid(c, nBlk), 256, 0, c->stream>>>(c->partialC_d, C, dC, TRAJ_PASS(c));
   CODY_LAUNCHED(c);
-  k_project_coeffs_apply<<<bgrid(c, vec_blocks(c, c->nC)), 256, 0, c->stream>>>(dC, C, c->partial_d, nBlk,
+  k_project_coeffs_apply<<<bgrid(c, vec_blocks(c, c->nC)), 256, 0, c->stream>>>(dC, C, c->partialC_d, nBlk,
                                                                                   TRAJ_PASS(c));
   CODY_LAUNCHED(c);
 }
