@@ -350,7 +350,7 @@ struct cgpu_ctx {
   // reductions / scratch
   z_t* partial_d = nullptr;
   z_t* partialC_d = nullptr;  // of the coefficients' projector (148 entries)
-  unsigned* gramCount_d = nullptr;            // blocks of a single system's Gram sum that have arrived
+  unsigned* gramCount_d = nullptr;            // blocks of a single system's sum (Gram, energy) that have arrived
   size_t partialCap = 0;                      // complex entries per trajectory
   int lzBlocks = 148;                         // blocks per trajectory of the Lanczos reductions
   int lzBlocksHeur = 148, lzBlocksCap = 148;  // the set-up heuristic's count and the most the partials hold

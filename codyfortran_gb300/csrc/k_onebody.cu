@@ -14,6 +14,8 @@
 // trajectories of the context (blockIdx.z).
 #include <algorithm>
 
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 namespace {
@@ -714,9 +716,104 @@ __global__ void k_mgs2(z_t* __restrict__ f, const double* __restrict__ w, TRAJ_A
   }
 }
 
+// The same by a cluster per trajectory: each of its MG_CTAS blocks holds a piece of
+// the grid of all columns in shared memory, and every warp sends its partial of a
+// dot product to all of them, so that a projection costs one cluster barrier and two
+// warp sums.  One block spends most of a projection in the FP64 adds of its 32 warps'
+// sums, a warp instruction of which holds a sub-partition for 64 cycles: 4 orbitals of
+// 501 points 99 us with k_mgs2, 37 here.
+constexpr int MG_CTAS = 8, MG_THREADS = 128, MG_WARPS = MG_THREADS / 32;
+static_assert(MG_CTAS * MG_WARPS == 32, "one slot a lane");
+constexpr size_t MG_SMEM = 200 * 1024;
+
+size_t mgs_smem(int nG, int n) {
+  const size_t per = (nG + MG_CTAS - 1) / MG_CTAS;
+  return per * (sizeof(z_t) * n + sizeof(double));
+}
+
+// Sums of re and im over the warp: re in lanes 0..15, im in lanes 16..31.
+__device__ __forceinline__ double mg_warp_sum(z_t v) {
+  const bool u = threadIdx.x & 16;
+  double x = u ? v.y : v.x;
+  x += __shfl_xor_sync(0xffffffffu, u ? v.x : v.y, 16);
+  for (int o = 8; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
+}
+
+__global__ void __cluster_dims__(MG_CTAS, 1, 1) __launch_bounds__(MG_THREADS)
+    k_mgs2_cluster(z_t* __restrict__ f, const double* __restrict__ w, TRAJ_ARGS, int c0, int n, int* status) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  extern __shared__ z_t col[];  // [n][per], then the weights
+  __shared__ z_t red[2][32];
+  const TrajShape& S = shp[blockIdx.z];
+  const int nG = S.nG, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, rank = blockIdx.x;
+  f = bat(f, bs);
+  w = bat(w, bs);
+  status = bat(status, bs);
+  if (c0 + n > S.nOS) n = max(0, S.nOS - c0);
+  const int per = (nG + MG_CTAS - 1) / MG_CTAS, l0 = min(nG, rank * per), cnt = min(nG, l0 + per) - l0;
+  double* wt = reinterpret_cast<double*>(col + (size_t)n * per);
+  for (int g = tid; g < cnt; g += MG_THREADS) {
+    wt[g] = w[l0 + g];
+    for (int i = 0; i < n; i++) col[(size_t)i * per + g] = f[(size_t)nG * (c0 + i) + l0 + g];
+  }
+  cluster.sync();  // every block runs before another writes to it
+  int par = 0;
+  // sum over the cluster, to every thread
+  auto total = [&](z_t v) {
+    const double x = mg_warp_sum(v);
+    if ((lane & 15) < MG_CTAS) {
+      z_t* to = cluster.map_shared_rank(&red[par][rank * MG_WARPS + wid], lane & 15);
+      (lane < 16 ? to->x : to->y) = x;
+    }
+    cluster.sync();
+    const double y = mg_warp_sum(red[par][lane]);
+    par ^= 1;
+    return zmk(__shfl_sync(0xffffffffu, y, 0), __shfl_sync(0xffffffffu, y, 16));
+  };
+  for (int i = 0; i < n; i++) {
+    z_t* b = col + (size_t)i * per;
+    for (int pass = 0; pass < 2; pass++)
+      for (int j = 0; j < i; j++) {
+        const z_t* a = col + (size_t)j * per;
+        z_t s = zmk(0.0, 0.0);
+        for (int g = tid; g < cnt; g += MG_THREADS) {
+          const z_t p = a[g], q = b[g];
+          const double wg = wt[g];
+          s.x += (p.x * q.x + p.y * q.y) * wg;
+          s.y += (p.x * q.y - p.y * q.x) * wg;
+        }
+        const z_t o = total(s);
+        for (int g = tid; g < cnt; g += MG_THREADS) {
+          const z_t p = a[g];
+          z_t q = b[g];
+          q.x -= p.x * o.x - p.y * o.y;
+          q.y -= p.x * o.y + p.y * o.x;
+          b[g] = q;
+        }
+      }
+    z_t s = zmk(0.0, 0.0);
+    for (int g = tid; g < cnt; g += MG_THREADS) s.x += (b[g].x * b[g].x + b[g].y * b[g].y) * wt[g];
+    const double nrm = total(s).x;
+    if (rank == 0 && tid == 0 && !(nrm > 0.0)) *status = 1;
+    const double sq = sqrt(nrm);
+    for (int g = tid; g < cnt; g += MG_THREADS) {
+      const z_t q = zmk(b[g].x / sq, b[g].y / sq);
+      b[g] = q;
+      f[(size_t)nG * (c0 + i) + l0 + g] = q;
+    }
+  }
+  cluster.sync();  // no block leaves while another may still write to it
+}
+
 // E = Re[ sum h1(k,l) rho1(l,k) + sum h2(k1,k2,l1,l2) rho2(l1,l2,k1,k2) ]
-__global__ void k_energy(double* out, const z_t* __restrict__ h1, const z_t* __restrict__ r1,
-                         const z_t* __restrict__ h2, const z_t* __restrict__ r2, TRAJ_ARGS) {
+// A single system's terms over several blocks, whose sums the last to arrive adds in
+// block order (part, count; 65536 terms of 16 spin orbitals: 73 us in one block, 11 in
+// 64).
+__global__ void k_energy(double* out, z_t* __restrict__ part, unsigned* __restrict__ count, const z_t* __restrict__ h1,
+                         const z_t* __restrict__ r1, const z_t* __restrict__ h2, const z_t* __restrict__ r2,
+                         TRAJ_ARGS) {
   const TrajShape& S = shp[blockIdx.z];
   const size_t nO = S.nO;
   out = bat(out, bs);
@@ -726,16 +823,30 @@ __global__ void k_energy(double* out, const z_t* __restrict__ h1, const z_t* __r
   r2 = bat(r2, bs);
   z_t s = zmk(0.0, 0.0);
   size_t n2 = nO * nO;
-  for (size_t e = threadIdx.x; e < n2; e += blockDim.x) {
-    size_t k = e % nO, l = e / nO;
-    zfma(s, h1[k + nO * l], r1[l + nO * k]);
-  }
-  for (size_t e = threadIdx.x; e < n2 * n2; e += blockDim.x) {
+  if (blockIdx.x == 0)
+    for (size_t e = threadIdx.x; e < n2; e += blockDim.x) {
+      size_t k = e % nO, l = e / nO;
+      zfma(s, h1[k + nO * l], r1[l + nO * k]);
+    }
+  for (size_t e = threadIdx.x + (size_t)blockIdx.x * blockDim.x; e < n2 * n2; e += (size_t)blockDim.x * gridDim.x) {
     size_t kk = e % n2, ll = e / n2;  // kk = (k1,k2), ll = (l1,l2)
     zfma(s, h2[kk + n2 * ll], r2[ll + n2 * kk]);
   }
   s = block_sum(s);
-  if (threadIdx.x == 0) *out = s.x;
+  if (threadIdx.x == 0) {
+    if (gridDim.x == 1) {
+      *out = s.x;
+      return;
+    }
+    part[blockIdx.x] = s;
+    __threadfence();
+    if (atomicInc(count, gridDim.x - 1) == gridDim.x - 1) {
+      __threadfence();
+      double t = 0.0;
+      for (unsigned b = 0; b < gridDim.x; b++) t += __ldcg(part + b).x;
+      *out = t;
+    }
+  }
 }
 
 // out[:, i] = x * orbs[:, i] (dipole operator on the orbitals)
@@ -1069,7 +1180,15 @@ void launch_rk_stage(cgpu_ctx* c, z_t* inc, z_t* tmp, const z_t* state, const z_
 
 void launch_orthonormalize(cgpu_ctx* c, z_t* orbs, int col0, int nCols, int resetStatus) {
   if (resetStatus) batch_zero(c, c->scal_d, sizeof(int));
-  k_mgs2<<<bgrid(c, 1), 1024, 0, c->stream>>>(orbs, c->w_d, TRAJ_PASS(c), col0, nCols, (int*)c->scal_d);
+  const size_t sh = mgs_smem(c->nG, nCols);
+  if (sh <= MG_SMEM) {
+    if (sh > 48 * 1024)
+      CODY_CUDA(cudaFuncSetAttribute(k_mgs2_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh));
+    k_mgs2_cluster<<<bgrid(c, MG_CTAS), MG_THREADS, sh, c->stream>>>(orbs, c->w_d, TRAJ_PASS(c), col0, nCols,
+                                                                     (int*)c->scal_d);
+  } else {
+    k_mgs2<<<bgrid(c, 1), 1024, 0, c->stream>>>(orbs, c->w_d, TRAJ_PASS(c), col0, nCols, (int*)c->scal_d);
+  }
   CODY_LAUNCHED(c);
 }
 
@@ -1079,12 +1198,14 @@ void launch_norm_dipole(cgpu_ctx* c, const z_t* state) {
                                                                                     TRAJ_PASS(c));
   CODY_LAUNCHED(c);
   launch_fill_h1_from(c, orbs, c->orbTmp_d, c->h1_d);  // h1 <- dipole matrix
-  k_norm_dipole<<<bgrid(c, 1), 256, 0, c->stream>>>(c->scal_d, state, c->h1_d, c->rdm1_d, TRAJ_PASS(c));
+  k_norm_dipole<<<bgrid(c, 1), c->nC > 2048 ? 1024 : 256, 0, c->stream>>>(c->scal_d, state, c->h1_d, c->rdm1_d, TRAJ_PASS(c));
   CODY_LAUNCHED(c);
 }
 
 void launch_energy(cgpu_ctx* c, double* out_d) {
-  k_energy<<<bgrid(c, 1), 1024, 0, c->stream>>>(out_d, c->h1_d, c->rdm1_d, c->h2_d, c->rdm2_d, TRAJ_PASS(c));
+  const size_t n4 = (size_t)c->nO * c->nO * c->nO * c->nO;
+  const unsigned nBlk = c->nb > 1 ? 1 : (unsigned)std::max<size_t>(1, std::min<size_t>(64, n4 / 1024));
+  k_energy<<<bgrid(c, nBlk), 1024, 0, c->stream>>>(out_d, c->partial_d, c->gramCount_d, c->h1_d, c->rdm1_d, c->h2_d, c->rdm2_d, TRAJ_PASS(c));
   CODY_LAUNCHED(c);
 }
 
