@@ -606,6 +606,17 @@ size_t lanczos_partial_need(const cgpu_ctx* c);
     if (e_ != cudaSuccess) throw std::string(#call) + ": " + cudaGetErrorString(e_);                  \
   } while (0)
 
+// The branches' events, and launches on another stream than the context's.
+enum { BR_START, BR_DENSITY, BR_ONEBODY, BR_POTENTIALS, BR_COEFFS };
+inline void branch_record(cgpu_ctx* c, int e) { CODY_CUDA(cudaEventRecord(c->branchEv[e], c->stream)); }
+inline void branch_wait(cgpu_ctx* c, int e) { CODY_CUDA(cudaStreamWaitEvent(c->stream, c->branchEv[e], 0)); }
+struct BranchStream {
+  cgpu_ctx* c;
+  cudaStream_t prev;
+  BranchStream(cgpu_ctx* ctx, cudaStream_t s) : c(ctx), prev(ctx->stream) { c->stream = s; }
+  ~BranchStream() { c->stream = prev; }
+};
+
 #define CODY_LAUNCHED(c) \
   do {                   \
     (c)->launches++;     \

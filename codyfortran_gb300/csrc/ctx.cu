@@ -704,46 +704,39 @@ void td_device(cgpu_ctx* c, int which, z_t* out, const z_t* in, double t, z_t po
     // partial_d and gram_d are the one-body branch's up to its event, then the
     // orbitals'; the coefficients' projector has partials of its own.  A profile of one
     // kernel family keeps the row.
-    enum { START, DENSITY, ONEBODY, POTENTIALS, COEFFS };
-    auto record = [&](int e) { CODY_CUDA(cudaEventRecord(c->branchEv[e], c->stream)); };
-    auto wait = [&](int e) { CODY_CUDA(cudaStreamWaitEvent(c->stream, c->branchEv[e], 0)); };
-    struct OnStream {
-      cgpu_ctx* c;
-      cudaStream_t prev;
-      OnStream(cgpu_ctx* cc, cudaStream_t s) : c(cc), prev(cc->stream) { c->stream = s; }
-      ~OnStream() { c->stream = prev; }
-    };
-    record(START);
+    auto record = [&](int e) { branch_record(c, e); };
+    auto wait = [&](int e) { branch_wait(c, e); };
+    record(BR_START);
     launch_fx_potentials(c, orbs);
-    record(POTENTIALS);
+    record(BR_POTENTIALS);
     {
-      OnStream on(c, c->side[0]);
-      wait(START);
+      BranchStream on(c, c->side[0]);
+      wait(BR_START);
       launch_ci_rdm(c, C, 1, 1);
       launch_rdm_inverse(c);
       launch_fx_split_R(c);
-      record(DENSITY);
+      record(BR_DENSITY);
     }
     {
-      OnStream on(c, c->side[1]);
-      wait(START);
+      BranchStream on(c, c->side[1]);
+      wait(BR_START);
       oneBody();
       launch_fold_h1(c);
       batch_zero(c, dC, sizeof(z_t) * c->nC);
-      record(ONEBODY);
-      wait(POTENTIALS);
+      record(BR_ONEBODY);
+      wait(BR_POTENTIALS);
       launch_fx_h2(c);
       launch_fold_h2(c);
       launch_ci_apply(c, C, dC, 1, 1);
       launch_project_coeffs(c, dC, C);
-      record(COEFFS);
+      record(BR_COEFFS);
     }
-    wait(DENSITY);
+    wait(BR_DENSITY);
     launch_fx_Z(c);
-    wait(ONEBODY);
+    wait(BR_ONEBODY);
     launch_fx_epilogue(c, dOrbs, orbs);
     launch_project_orbs(c, dOrbs, orbs);
-    wait(COEFFS);
+    wait(BR_COEFFS);
     if (!unit) launch_scale(c, out, f, VSEL_STATE);
     return;
   }
