@@ -6,17 +6,18 @@
 // The launch-per-pass form (k_lanczos.cu) spends seven launches and five passes
 // over the vectors on every Krylov iteration.  Here each trajectory has a group
 // of blocks, every block owns a contiguous piece of its state vector, and an
-// iteration is two phases between barriers of the group:
-//   A  h = H v_j on the piece (halo of `band` points from the neighbours),
-//      partials of the dots with the basis vectors and of ||h||^2;
-//   B  h -= sum_k c_k v_k from the summed partials, ||.||^2 partials, h published
-//      for the neighbours' next halo.
-// v_{j+1} = h / beta_j is formed where it is read.  The piece, its metric and
-// (where they fit) its basis vectors stay in shared memory.  Every block sums
-// the same partials in the same order and evaluates exp(-i dt T) e1 itself, so
-// all of them take the same decisions: second Gram-Schmidt pass, breakdown,
-// convergence, halving of the step.  An adaptive integration therefore runs to
-// its end without the host.
+// iteration has one barrier of the group.  With w_j = beta_{j-1} v_j not yet normalised,
+//   before it  g = H w_j on the piece, published for the neighbours' halo of `band`
+//              points; partials of <v_k, g>, <w_j, g>, ||g||^2 and ||w_j||^2;
+//   after it   beta_{j-1} = ||w_j||, v_j = w_j / beta_{j-1}, h = g / beta_{j-1},
+//              w_{j+1} = h - sum_k c_k v_k on the piece and on its halo, whose basis
+//              vectors every block keeps.
+// The second Gram-Schmidt pass (its own barrier) is decided by ||h||^2 - sum |c_k|^2;
+// the norms in T are always sums over the vectors.  The piece, its metric and (where they
+// fit) its basis vectors stay in shared memory.  Every block sums the same partials in
+// the same order and evaluates exp(-i dt T) e1 itself, so all of them take the same
+// decisions: second pass, breakdown, convergence, halving of the step.  An adaptive
+// integration therefore runs to its end without the host.
 //
 // FP64 throughout, also for the mixed forms: up to one group block per SM the
 // FP64 pipe is not the bound of this kernel (44 to 100 FMA an entry and
@@ -34,7 +35,7 @@
 namespace {
 
 constexpr int SIL_K = 32;
-constexpr int SIL_PART = SIL_K + 8;            // partial sums of a block
+constexpr int SIL_PART = SIL_K + 8;            // partial sums of a block (two sets)
 constexpr int SIL_MIN = 32;                    // smallest piece worth a block of its own
 constexpr size_t SIL_SMEM = 200 * 1024;
 constexpr long long SIL_WAIT = 4000000000LL;   // cycles after which a barrier gives up
@@ -327,6 +328,11 @@ __device__ void lz_expsub_vjp_warp(const double* alpha, const double* beta, int 
 
 namespace {
 
+// Vectors of a block: w_j with its halo, g, m g, the basis on the halo and (smemV) on the piece.
+__host__ __device__ __forceinline__ size_t sil_entries(int cap, int band, int K, bool smemV) {
+  return (size_t)cap * (3 + (smemV ? K : 0)) + 2 * (size_t)band * (1 + K);
+}
+
 struct SilArgs {
   const z_t* start;  // the vector to propagate, and its result (may be the same)
   z_t *state, *w0, *w1, *basis;
@@ -374,20 +380,21 @@ __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
   const double* V0 = batn(A.V0, bs, B.traj);
   const double* x = batn(A.x, bs, B.traj);
   const int* btOf = batn(A.btOf, bs, B.traj);
-  constexpr int PS = SIL_PART;
-  z_t* part = A.part + (size_t)(blockIdx.x - B.rank) * PS;  // the group's partials
-  z_t* mine = part + (size_t)B.rank * PS;
+  constexpr int PS = 2 * SIL_PART;
+  z_t* part0 = A.part + (size_t)(blockIdx.x - B.rank) * PS;  // the group's partials, two sets in turn:
+  int set = 0;                                               // a slow block may still read the last one
   unsigned* bar = A.bar + 2 * B.traj;
   unsigned target = 0;
 
   extern __shared__ z_t smDyn[];
-  z_t* sm = MODE == SIL_SPILLED ? A.keep.spill + blockIdx.x * (size_t)(3 * cap + 2 * band) : smDyn;
-  z_t* vt = sm;                          // v_j with its halo: entries l0 - band .. l1 + band
-  z_t* w = vt + cap + 2 * band;
-  z_t* mw = w + cap;                     // m w
-  z_t* V = mw + cap;                     // [K][cap] when smemV
-  __shared__ z_t coef[SIL_K + 1];
-  __shared__ double alpha[SIL_K], beta[SIL_K], red[SIL_W], jb[1216], errEst, shE;
+  z_t* sm = MODE == SIL_SPILLED ? A.keep.spill + blockIdx.x * sil_entries(cap, band, SIL_K, false) : smDyn;
+  z_t* vt = sm;                          // w_j with its halo: entries l0 - band .. l1 + band
+  z_t* g = vt + cap + 2 * band;          // H w_j
+  z_t* mw = g + cap;                     // m g
+  z_t* Vh = mw + cap;                    // [K][2 band]: the basis on the halo
+  z_t* V = Vh + 2 * band * A.K;          // [K][cap] when smemV
+  __shared__ z_t coef[SIL_K + 2];
+  __shared__ double alpha[SIL_K], beta[SIL_K], red[2 * SIL_W], jb[1216], errEst, shE, shBe, shInv, shN0, shN1;
   __shared__ z_t phi[SIL_K];
 
   const int per = (S.nS + B.n - 1) / B.n, l0 = min(S.nS, B.rank * per), cnt = min(S.nS, l0 + per) - l0;
@@ -396,14 +403,17 @@ __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
     target += B.n;
     return group_barrier(bar, target, B.n, A.flags);
   };
-  // sums over the group of partial slots [s0, s0 + n), one or two slots a warp, into coef[0..n)
+  auto mine = [&]() { return part0 + (size_t)B.rank * PS + set * SIL_PART; };
+  // after a barrier: sums over the group of the partial slots [0, n), one or two slots a
+  // warp, into coef[0..n); the next partials go to the other set
   double* cf = reinterpret_cast<double*>(coef);
-  auto gather = [&](int s0, int n) {
+  auto gather = [&](int n) {
+    const z_t* part = part0 + set * SIL_PART;
     if (n <= SIL_W) {
       if (wid < n) {
         double x0 = 0.0, y0 = 0.0;
         for (int b = lane; b < B.n; b += 32) {
-          const z_t p = __ldcg(part + (size_t)b * PS + s0 + wid);
+          const z_t p = __ldcg(part + (size_t)b * PS + wid);
           x0 += p.x;
           y0 += p.y;
         }
@@ -414,8 +424,8 @@ __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
       for (int k = 2 * wid; k < n; k += 2 * SIL_W) {
         double x0 = 0.0, y0 = 0.0, x1 = 0.0, y1 = 0.0;
         for (int b = lane; b < B.n; b += 32) {
-          const z_t* r = part + (size_t)b * PS + s0 + k;
-          const z_t p = __ldcg(r), q = __ldcg(r + 1);  // slot k + 1 exists (PS slots a block)
+          const z_t* r = part + (size_t)b * PS + k;
+          const z_t p = __ldcg(r), q = __ldcg(r + 1);  // slot k + 1 exists (SIL_PART slots a set)
           x0 += p.x;
           y0 += p.y;
           x1 += q.x;
@@ -425,17 +435,20 @@ __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
         if ((lane & 7) == 0 && k + (lane >> 4) < n) cf[2 * k + (lane >> 3)] = x;
       }
     }
+    set ^= 1;
     __syncthreads();
   };
-  // partials of <v_k, w>_m for k in [b0, b1) into slots 0..
-  auto dots = [&](int b0, int b1) {
-    double* out = reinterpret_cast<double*>(mine);
-    if (b1 - b0 <= SIL_W) {
-      const int k = b0 + wid;
-      if (k < b1) {
+  // entry e of vector k of a dots call: basis vector b0 + k, or w_j itself after the n0 of them
+  auto dot_vec = [&](int b0, int n0, int k, int e) { return k < n0 ? vec(b0 + k, e) : vt[band + e]; };
+  // partials of <v_k, .> with mw for k in [b0, b0 + n0) and, with self, w_j into slots 0..
+  auto dots = [&](int b0, int n0, int self) {
+    double* out = reinterpret_cast<double*>(mine());
+    const int n = n0 + self;
+    if (n <= SIL_W) {
+      if (wid < n) {
         double ax = 0.0, ay = 0.0;
         for (int e = lane; e < cnt; e += 32) {
-          const z_t v = vec(k, e), u = mw[e];
+          const z_t v = dot_vec(b0, n0, wid, e), u = mw[e];
           ax = fma(v.x, u.x, fma(v.y, u.y, ax));
           ay = fma(v.x, u.y, fma(-v.y, u.x, ay));
         }
@@ -443,30 +456,29 @@ __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
         if ((lane & 15) == 0) out[2 * wid + (lane >> 4)] = x;
       }
     } else {
-      for (int k = b0 + 2 * wid; k < b1; k += 2 * SIL_W) {
+      for (int k = 2 * wid; k < n; k += 2 * SIL_W) {
         double ax = 0.0, ay = 0.0, bx = 0.0, by = 0.0;
-        const int k1 = min(k + 1, b1 - 1);
+        const int k1 = min(k + 1, n - 1);
         for (int e = lane; e < cnt; e += 32) {
-          const z_t v = vec(k, e), t = vec(k1, e), u = mw[e];
+          const z_t v = dot_vec(b0, n0, k, e), t = dot_vec(b0, n0, k1, e), u = mw[e];
           ax = fma(v.x, u.x, fma(v.y, u.y, ax));
           ay = fma(v.x, u.y, fma(-v.y, u.x, ay));
           bx = fma(t.x, u.x, fma(t.y, u.y, bx));
           by = fma(t.x, u.y, fma(-t.y, u.x, by));
         }
         const double x = warp_sum4(ax, ay, bx, by);
-        if ((lane & 7) == 0 && k + (lane >> 4) < b1) out[2 * (k - b0) + (lane >> 3)] = x;
+        if ((lane & 7) == 0 && k + (lane >> 4) < n) out[2 * k + (lane >> 3)] = x;
       }
     }
   };
-  // block sum of q into the real part of slot `slot` (warps to shared memory, then warp 0)
-  auto publish = [&](double q, int slot) {
-    q = warp_sum(q);
-    if (lane == 0) red[wid] = q;
+  // block sums of p and q into the real and imaginary part of a slot (also orders mw)
+  auto publish = [&](double p, double q, int slot) {
+    const double x = warp_sum2(p, q);
+    if ((lane & 15) == 0) red[2 * wid + (lane >> 4)] = x;
     __syncthreads();
     if (wid == 0) {
-      double x = lane < SIL_W ? red[lane] : 0.0;
-      for (int o = SIL_W / 2; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-      if (lane == 0) mine[slot] = zmk(x, 0.0);
+      const double y = warp_sum2(lane < SIL_W ? red[2 * lane] : 0.0, lane < SIL_W ? red[2 * lane + 1] : 0.0);
+      if ((lane & 15) == 0) reinterpret_cast<double*>(mine() + slot)[lane >> 4] = y;
     }
   };
   const int pt = A.pt, eq = tid % pt, e0 = tid / pt, eStep = SIL_T / pt;
@@ -478,196 +490,207 @@ __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
     }
     return r;
   };
-  // w -= sum coef_k v_{b0+k}; w published in out; its norm partial in the last slot
-  auto subtract = [&](int b0, int n, z_t* out) {
-    double q = 0.0;
-    for (int eb = 0; eb < cnt; eb += eStep) {
-      const int e = eb + e0;
+  // vt = from - sum_k coef_k v_{b0 + k} on the piece and its halo (first: from = gIn inv, and
+  // coef_{n0} v with v = vt inv, which becomes basis vector b0 + n0; else from = vt)
+  auto subtract = [&](int b0, int n0, bool first, double inv, const z_t* gIn) {
+    for (int qb = 0; qb < cnt + 2 * band; qb += eStep) {  // the piece (its accesses aligned), then the halo
+      const int e = qb + e0, hh = e - cnt;
+      const bool own = e < cnt;
+      const int t = own ? band + e : hh < band ? hh : cnt + hh, l = l0 - band + t;
+      const bool in = e < cnt + 2 * band && l >= 0 && l < S.nS;
       z_t r = zmk(0.0, 0.0);
-      if (e < cnt) {
-        if (eq == 0) r = w[e];
-        for (int k = eq; k < n; k += pt) {
-          const z_t v = vec(b0 + k, e), c = coef[k];
+      if (in) {
+        if (eq == 0) r = first ? zscale(own ? g[e] : __ldcg(gIn + vidx(S, l)), inv) : vt[t];
+        for (int k = eq; k < n0; k += pt) {
+          const z_t v = own ? vec(b0 + k, e) : Vh[2 * band * (b0 + k) + hh], c = coef[k];
+          r.x = fma(-c.x, v.x, fma(c.y, v.y, r.x));
+          r.y = fma(-c.x, v.y, fma(-c.y, v.x, r.y));
+        }
+        if (first && eq == n0 % pt) {
+          const z_t v = zscale(vt[t], inv), c = coef[n0];
+          if (own) {
+            vec(b0 + n0, e) = v;
+            if (KEEP && A.smemV) A.keep.V[A.ldv * (b0 + n0) + vidx(S, l)] = v;
+          } else {
+            Vh[2 * band * (b0 + n0) + hh] = v;
+          }
           r.x = fma(-c.x, v.x, fma(c.y, v.y, r.x));
           r.y = fma(-c.x, v.y, fma(-c.y, v.x, r.y));
         }
       }
       r = entry_sum(r);
-      if (e < cnt && eq == 0) {
-        const size_t i = vidx(S, l0 + e);
-        const z_t u = zscale(r, m[i]);
-        w[e] = r;
-        mw[e] = u;
-        out[i] = r;
-        q = fma(u.x, r.x, fma(u.y, r.y, q));
-      }
+      if (in && eq == 0) vt[t] = r;
     }
-    publish(q, SIL_K + 1);
   };
 
   double tCur = A.tOff, rem = A.dt;
-  int warnings = 0;
+  int warnings = 0, it = 0;
   bool ok = true;
   while (ok && fabs(rem) > SIL_ZERO) {
-    double dtS = rem;
+    double dtS = rem, nrm = 0.0;
     int restarts = 0;
     bool conv = false;
-    // ||state||
-    double q = 0.0;
-    for (int e = tid; e < cnt; e += SIL_T) {
-      const size_t i = vidx(S, l0 + e);
-      const z_t v = start[i];
-      q = fma(m[i], fma(v.x, v.x, v.y * v.y), q);
-    }
-    // the field takes a few microseconds of FP64 on one lane: beside the norm
-    auto field = [&]() {
+    for (;;) {
+      __syncthreads();
+      // w_1 and its halo; the field takes a few microseconds of FP64 on one lane beside it
       if (tid == SIL_T - 1)
         shE = KEEP ? A.E : S.hasPot ? field_amplitude_dev(S.laser, *batn(A.tBase, bs, B.traj) + tCur + 0.5 * dtS) : 0.0;
-    };
-    field();
-    publish(q, SIL_K + 1);
-    if (!(ok = barrier())) break;
-    gather(SIL_K + 1, 1);
-    const double nrm = sqrt(coef[0].x);
-    if (nrm <= SIL_ZERO && !KEEP) {  // nothing to propagate: the state stays
-      conv = true;
-    } else {
-      for (;;) {
-        if (restarts > 0) {
-          __syncthreads();
-          field();
-          __syncthreads();
-        }
-        const double E = shE;
-        double inv = 1.0 / nrm, bPrev = 0.0;
-        const z_t* src = start;
-        int mDim = A.K;
-        for (int j = 1; j <= A.K; j++) {
-          // v_j and its halo
-          __syncthreads();
-          for (int t = tid; t < cnt + 2 * band; t += SIL_T) {
-            const int l = l0 - band + t;
-            z_t v = zmk(0.0, 0.0);
-            if (l >= 0 && l < S.nS) v = zscale(__ldcg(src + vidx(S, l)), inv);
-            vt[t] = v;
-            if (t >= band && t < band + cnt) {
-              vec(j - 1, t - band) = v;
-              if (KEEP && A.smemV) A.keep.V[A.ldv * (j - 1) + vidx(S, l)] = v;
-            }
-          }
-          __syncthreads();
-          double h2 = 0.0;
-          for (int eb = 0; eb < cnt; eb += eStep) {
-            const int e = eb + e0, l = l0 + e;
-            z_t h = zmk(0.0, 0.0);
-            if (e < cnt && l >= nC) {  // the coefficients do not move
-              const int r = l - nC, i = r / nG, g = r - i * nG;
-              const double* Tb = T + (size_t)(S.restricted ? 0 : btOf[i]) * nd * nG + g;
-              const z_t* vv = vt + e;
-              const int d0 = max(0, band - g), d1 = min(nd, nG - g + band);  // inside the orbital
-              for (int d = eq; d < d1; d += pt) {
-                if (d < d0) continue;
-                const double cf = __ldg(Tb + (size_t)d * nG);
-                h.x = fma(cf, vv[d].x, h.x);
-                h.y = fma(cf, vv[d].y, h.y);
-              }
-              if ((S.hasPot || KEEP) && eq == pt - 1) {
-                const double p = fma(E, x[g], V0[g]);
-                h.x = fma(p, vv[band].x, h.x);
-                h.y = fma(p, vv[band].y, h.y);
-              }
-            }
-            if (e < cnt && eq == 0 && A.window == 1 && j > 1) {  // three-term recurrence
-              const z_t v = vec(j - 2, e);
-              h.x = fma(-bPrev, v.x, h.x);
-              h.y = fma(-bPrev, v.y, h.y);
-            }
-            h = entry_sum(h);
-            if (e < cnt && eq == 0) {
-              const z_t u = zscale(h, m[vidx(S, l)]);
-              w[e] = h;
-              mw[e] = u;
-              h2 = fma(u.x, h.x, fma(u.y, h.y, h2));
-            }
-          }
-          const int b0 = A.window > 0 ? max(0, j - A.window) : 0, nv = j - b0;
-          publish(h2, nv);  // also orders mw before the dots
-          dots(b0, j);
-          if (!(ok = barrier())) break;
-          gather(0, nv + 1);
-          const double a = coef[nv - 1].x, n0 = coef[nv].x;
-          if (A.window == 1) {
-            __syncthreads();
-            if (tid == 0) coef[0].y = 0.0;
-            __syncthreads();
-          }
-          subtract(b0, nv, wb[j & 1]);
-          if (!(ok = barrier())) break;
-          gather(SIL_K + 1, 1);
-          double n1 = coef[0].x;
-          if (n1 <= SIL_ETA2 * n0) {  // most of h cancelled: project once more
-            __syncthreads();
-            dots(b0, j);
-            if (!(ok = barrier())) break;
-            gather(0, nv);
-            subtract(b0, nv, wb[j & 1]);
-            if (!(ok = barrier())) break;
-            gather(SIL_K + 1, 1);
-            n1 = coef[0].x;
-          }
-          const double be = sqrt(n1);
-          if (tid == 0) {
-            alpha[j - 1] = a;
-            beta[j - 1] = be;
-          }
-          const bool broke = be <= SIL_ZERO && !KEEP;  // the kept pass runs over all orders
-          const bool last = broke || j == A.K;
-          if (A.tol > 0.0 || last) {
-            __syncthreads();
-            if (wid == 0) {
-              double fr, fi;
-              lz_expsub_warp<KEEP>(alpha, beta, j, dtS, jb, fr, fi, KEEP && B.rank == 0 ? A.keep.parts : nullptr);
-              if (lane < j) phi[lane] = zmk(fr, fi);
-              if (lane == j - 1) errEst = broke ? 0.0 : be * sqrt(fr * fr + fi * fi);
-            }
-            __syncthreads();
-            conv = errEst <= A.tol;
-            if ((A.tol > 0.0 && conv) || last) {
-              mDim = j;
-              break;
-            }
-          }
-          src = wb[j & 1];
-          inv = 1.0 / be;
-          bPrev = be;
-        }
-        if (!ok) break;
-        if (conv || !(A.tol > 0.0) || fabs(dtS) <= SIL_ZERO || restarts >= A.maxRestarts) {
-          for (int e = tid; e < cnt; e += SIL_T) {
-            z_t acc = zmk(0.0, 0.0);
-            for (int k = 0; k < mDim; k++) zfma(acc, vec(k, e), phi[k]);
-            state[vidx(S, l0 + e)] = zscale(acc, nrm);
-          }
-          if (KEEP) {
-            for (int e = tid; e < cnt; e += SIL_T) A.keep.last[l0 + e] = w[e];
-            if (B.rank == 0 && tid < A.K) {
-              A.keep.alpha[tid] = alpha[tid];
-              A.keep.beta[tid] = beta[tid];
-              A.keep.phi[tid] = phi[tid];
-              if (tid == 0) *A.keep.norm = nrm;
-            }
-          }
-          break;
-        }
-        dtS = 0.5 * dtS;
-        restarts++;
+      for (int t = tid; t < cnt + 2 * band; t += SIL_T) {
+        const int l = l0 - band + t;
+        vt[t] = l >= 0 && l < S.nS ? __ldcg(start + vidx(S, l)) : zmk(0.0, 0.0);
       }
+      __syncthreads();
+      const double E = shE;
+      int mDim = A.K;
+      for (int j = 1; j <= A.K; j++, it++) {
+        z_t* gOut = wb[it & 1];
+        if (j > 1) __syncthreads();
+        double h2 = 0.0, n2 = 0.0;
+        for (int eb = 0; eb < cnt; eb += eStep) {
+          const int e = eb + e0, l = l0 + e;
+          z_t h = zmk(0.0, 0.0);
+          if (e < cnt && l >= nC) {  // the coefficients do not move
+            const int r = l - nC, i = r / nG, x0 = r - i * nG;
+            const double* Tb = T + (size_t)(S.restricted ? 0 : btOf[i]) * nd * nG + x0;
+            const z_t* vv = vt + e;
+            const int d0 = max(0, band - x0), d1 = min(nd, nG - x0 + band);  // inside the orbital
+            for (int d = eq; d < d1; d += pt) {
+              if (d < d0) continue;
+              const double c = __ldg(Tb + (size_t)d * nG);
+              h.x = fma(c, vv[d].x, h.x);
+              h.y = fma(c, vv[d].y, h.y);
+            }
+            if ((S.hasPot || KEEP) && eq == pt - 1) {
+              const double p = fma(E, x[x0], V0[x0]);
+              h.x = fma(p, vv[band].x, h.x);
+              h.y = fma(p, vv[band].y, h.y);
+            }
+          }
+          h = entry_sum(h);
+          if (e < cnt && eq == 0) {
+            const size_t i = vidx(S, l);
+            const double mi = m[i];
+            const z_t u = zscale(h, mi), v = vt[band + e];
+            g[e] = h;
+            mw[e] = u;
+            gOut[i] = h;
+            h2 = fma(u.x, h.x, fma(u.y, h.y, h2));
+            n2 = fma(mi, fma(v.x, v.x, v.y * v.y), n2);
+          }
+        }
+        // the window's vectors; the three-term recurrence takes v_{j-1} too, for ||h||^2 and its beta
+        const int b0 = A.window > 0 ? max(0, j - (A.window == 1 ? 2 : A.window)) : 0, n0 = j - 1 - b0;
+        publish(h2, n2, n0 + 1);  // also orders mw before the dots
+        dots(b0, n0, 1);
+        if (!(ok = barrier())) break;
+        gather(n0 + 2);
+        if (wid == 0) {  // beta_{j-1} and the coefficients against normalised vectors
+          const double be = sqrt(coef[n0 + 1].y), inv = 1.0 / be;
+          z_t c = lane <= n0 ? zscale(coef[lane], lane < n0 ? inv : inv * inv) : zmk(0.0, 0.0);
+          double q0 = coef[n0 + 1].x * (inv * inv);
+          __syncwarp();
+          if (A.window == 1) {
+            c.y = 0.0;
+            if (n0 == 1) {  // h = H v_j - beta_{j-1} v_{j-1}
+              const double cp = __shfl_sync(0xffffffffu, c.x, 0);
+              q0 += be * (be - 2.0 * cp);
+              if (lane == 0) c.x = be;
+            }
+          }
+          const double sq = A.window == 1 && lane < n0 ? 0.0 : fma(c.x, c.x, c.y * c.y);
+          const double q1 = q0 - warp_sum(sq);
+          if (lane <= n0) coef[lane] = c;
+          if (lane == n0) alpha[j - 1] = c.x;
+          if (lane == 0) {
+            if (j > 1) beta[j - 2] = be;
+            shBe = be;
+            shInv = inv;
+            shN0 = q0;
+            shN1 = q1;
+          }
+        }
+        __syncthreads();
+        if (j == 1) {
+          nrm = shBe;
+          if (nrm <= SIL_ZERO && !KEEP) {  // nothing to propagate: the state stays
+            conv = true;
+            mDim = 0;
+            it++;
+            break;
+          }
+        }
+        double n1 = shN1;
+        subtract(b0, n0, true, shInv, gOut);
+        if (n1 <= SIL_ETA2 * shN0) {  // most of h cancelled: project once more
+          __syncthreads();
+          double q = 0.0;
+          for (int e = tid; e < cnt; e += SIL_T) {
+            const z_t v = vt[band + e], u = zscale(v, m[vidx(S, l0 + e)]);
+            mw[e] = u;
+            q = fma(u.x, v.x, fma(u.y, v.y, q));
+          }
+          const int p0 = A.window > 0 ? max(0, j - A.window) : 0, np = j - p0;
+          publish(q, 0.0, np);
+          dots(p0, np, 0);
+          if (!(ok = barrier())) break;
+          gather(np + 1);
+          if (wid == 0) {
+            const z_t c = lane < np ? coef[lane] : zmk(0.0, 0.0);
+            const double q1 = coef[np].x - warp_sum(fma(c.x, c.x, c.y * c.y));
+            if (lane == 0) shN1 = q1;
+          }
+          subtract(p0, np, false, 0.0, nullptr);
+          __syncthreads();
+          n1 = shN1;
+        }
+        const double be = sqrt(fmax(n1, 0.0));
+        const bool broke = be <= SIL_ZERO && !KEEP;  // the kept pass runs over all orders
+        const bool last = broke || j == A.K;
+        if (A.tol > 0.0 || last) {
+          __syncthreads();
+          if (wid == 0) {
+            if (lane == 0) beta[j - 1] = be;
+            double fr, fi;
+            lz_expsub_warp<KEEP>(alpha, beta, j, dtS, jb, fr, fi, KEEP && B.rank == 0 ? A.keep.parts : nullptr);
+            if (lane < j) phi[lane] = zmk(fr, fi);
+            if (lane == j - 1) errEst = broke ? 0.0 : be * sqrt(fr * fr + fi * fi);
+          }
+          __syncthreads();
+          conv = errEst <= A.tol;
+          if ((A.tol > 0.0 && conv) || last) {
+            mDim = j;
+            it++;
+            break;
+          }
+        }
+      }
+      if (!ok || mDim == 0) break;
+      if (conv || !(A.tol > 0.0) || fabs(dtS) <= SIL_ZERO || restarts >= A.maxRestarts) {
+        for (int e = tid; e < cnt; e += SIL_T) {
+          z_t acc = zmk(0.0, 0.0);
+          for (int k = 0; k < mDim; k++) zfma(acc, vec(k, e), phi[k]);
+          state[vidx(S, l0 + e)] = zscale(acc, nrm);
+        }
+        if (KEEP) {
+          for (int e = tid; e < cnt; e += SIL_T) A.keep.last[l0 + e] = vt[band + e];
+          if (B.rank == 0 && tid < A.K) {
+            A.keep.alpha[tid] = alpha[tid];
+            A.keep.beta[tid] = beta[tid];
+            A.keep.phi[tid] = phi[tid];
+            if (tid == 0) *A.keep.norm = nrm;
+          }
+        }
+        break;
+      }
+      dtS = 0.5 * dtS;
+      restarts++;
     }
     if (!ok) break;
     if (!conv) warnings++;
     if (!(A.tol > 0.0)) break;  // fixed order: one pass over the whole step
     tCur += dtS;
     rem -= dtS;
+    if (fabs(rem) > SIL_ZERO) ok = barrier();  // the neighbours' pieces of the new start
   }
   if (tid == 0) {
     if (B.traj == 0 && B.rank == 0) A.flags[1] = A.tol > 0.0 ? warnings : 1;
@@ -679,9 +702,7 @@ __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
   }
 }
 
-size_t sil_smem(int cap, int band, int K, bool smemV) {
-  return sizeof(z_t) * ((size_t)cap * (3 + (smemV ? K : 0)) + 2 * band);
-}
+size_t sil_smem(int cap, int band, int K, bool smemV) { return sizeof(z_t) * sil_entries(cap, band, K, smemV); }
 
 }  // namespace
 
@@ -901,7 +922,7 @@ void sil_init(cgpu_ctx* c) {
   }
   CODY_CUDA(cudaMalloc(&c->silBlk_d, sizeof(SilBlock) * v.size()));
   CODY_CUDA(cudaMemcpy(c->silBlk_d, v.data(), sizeof(SilBlock) * v.size(), cudaMemcpyHostToDevice));
-  CODY_CUDA(cudaMalloc(&c->silPart_d, sizeof(z_t) * v.size() * SIL_PART));
+  CODY_CUDA(cudaMalloc(&c->silPart_d, sizeof(z_t) * v.size() * 2 * SIL_PART));
   CODY_CUDA(cudaMalloc(&c->silBar_d, sizeof(unsigned) * 2 * c->nb));
   CODY_CUDA(cudaMemset(c->silBar_d, 0, sizeof(unsigned) * 2 * c->nb));
   for (const void* k : {sil_kernels[0][0], sil_kernels[0][1], sil_kernels[0][2], sil_kernels[1][0], sil_kernels[1][1],
@@ -909,7 +930,7 @@ void sil_init(cgpu_ctx* c) {
     CODY_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SIL_SMEM));
   c->silGroup = (int)v.size();
   c->silCap = cap;
-  c->silFits = sil_smem(cap, c->band, 0, false) <= SIL_SMEM;
+  c->silFits = sil_smem(cap, c->band, SIL_K, false) <= SIL_SMEM;
 }
 
 void sil_check(cgpu_ctx* c) {
@@ -973,7 +994,7 @@ void launch_sil(cgpu_ctx* c, z_t* state, double t, double dt, int K, double tol,
 }
 
 size_t sil_spill(const cgpu_ctx* c) {
-  return c->silFits ? 0 : (size_t)c->silGroup * (3 * (size_t)c->silCap + 2 * c->band);
+  return c->silFits ? 0 : (size_t)c->silGroup * sil_entries(c->silCap, c->band, SIL_K, false);
 }
 
 // One fixed-order pass exp(-i dt h(E)) from start into out in the grid metric (a
