@@ -944,6 +944,10 @@ void check_partial(const cgpu_ctx* c, size_t need) {
 // The weighted Gram partials in double-float arithmetic (the fixed-point forms):
 // the chunk of A and w B staged as double-floats, every term conj(a) b an
 // error-free FP32 product with two-sum accumulation, FP64 partials out.
+// PER entries a thread: one up to 16 orbitals, whose 40 instead of 125 registers let
+// three times the blocks share an SM (a batch of 512: 302 -> 174 us).  In the FP64 form,
+// bound by the pipe, it gained nothing.
+template <int PER>
 __global__ void __launch_bounds__(GR_THREADS) k_gram_partial_df(z_t* __restrict__ G, z_t* __restrict__ part,
                                                                 const z_t* __restrict__ A, const z_t* __restrict__ B,
                                                                 const double* __restrict__ w, TRAJ_ARGS, int group,
@@ -966,8 +970,8 @@ __global__ void __launch_bounds__(GR_THREADS) k_gram_partial_df(z_t* __restrict_
   // double-floats, hence R <= 2 chunk / n
   const int R = nn * 2 <= (int)blockDim.x ? min(min(chunk, (int)blockDim.x / nn), 2 * chunk / n) : 1;
   const int e0 = threadIdx.x % nn, ph = threadIdx.x / nn, ii0 = e0 % n, jj0 = e0 / n;
-  zdf_acc acc[GR_PER_THREAD];
-  for (int q = 0; q < GR_PER_THREAD; q++) acc[q] = {0.0f, 0.0f, 0.0f, 0.0f};
+  zdf_acc acc[PER];
+  for (int q = 0; q < PER; q++) acc[q] = {0.0f, 0.0f, 0.0f, 0.0f};
   for (int r0 = blockIdx.x * chunk; r0 < nG; r0 += gridDim.x * chunk) {
     __syncthreads();
     for (int t = threadIdx.x; t < chunk * n; t += blockDim.x) {
@@ -995,7 +999,7 @@ __global__ void __launch_bounds__(GR_THREADS) k_gram_partial_df(z_t* __restrict_
       }
     } else {
 #pragma unroll
-      for (int q = 0; q < GR_PER_THREAD; q++) {
+      for (int q = 0; q < PER; q++) {
         int e = threadIdx.x + q * blockDim.x;
         if (e >= nn) break;
         int ii = e % n, jj = e / n;
@@ -1021,7 +1025,7 @@ __global__ void __launch_bounds__(GR_THREADS) k_gram_partial_df(z_t* __restrict_
     }
   } else {
 #pragma unroll
-    for (int q = 0; q < GR_PER_THREAD; q++) {
+    for (int q = 0; q < PER; q++) {
       int e = threadIdx.x + q * blockDim.x;
       if (e >= nn) break;
       part[(size_t)blockIdx.x * nn + e] = zdf_to_z(acc[q]);
@@ -1036,7 +1040,9 @@ void launch_gram(cgpu_ctx* c, z_t* G, const z_t* A, const z_t* B, int group, int
   size_t sh = 2 * sizeof(z_t) * chunk * nMax;
   if (nMax * nMax > GR_PER_THREAD * GR_THREADS) throw std::string("launch_gram: more than 64 orbitals");
   unsigned* count = c->nb == 1 && nMax * nMax * nBlk <= GR_LAST ? c->gramCount_d : nullptr;
-  auto part = c->ciDf ? k_gram_partial_df : k_gram_partial;
+  auto part = !c->ciDf                        ? k_gram_partial
+              : nMax * nMax <= GR_THREADS ? k_gram_partial_df<1>
+                                          : k_gram_partial_df<GR_PER_THREAD>;
   part<<<bgrid(c, nBlk), GR_THREADS, sh, c->stream>>>(G, c->partial_d, A, B, c->w_d, TRAJ_PASS(c), group, chunk, scale,
                                                       count);
   CODY_LAUNCHED(c);
