@@ -13,9 +13,8 @@ x 6 points on [-nE, nE], sin^2 4-cycle pulses at omega = 0.057 au with
 log-uniform intensity 1e13..1e15 W/cm^2 and uniform CEP; dt = 0.02, Krylov
 order 12; mixed precision mixed_fx6 (the pair-potential, correlation and h2
 contractions on tcgen05 tensor cores with every operand row carried as digit
-slices holding 36 bits of the row maximum -- six base-64 slices on the grid
-contractions, five base-256 slices on the pair contraction -- and exact
-per-level accumulation; FP64 elsewhere; three-term Lanczos recurrence).  The
+slices holding at least 36 bits of the row maximum -- five base-256 slices,
+six on grids of up to 1024 points -- and exact per-level accumulation; FP64 elsewhere; three-term Lanczos recurrence).  The
 faster mixed_fx form (30 bits) is selected with --precision mixed_fx.
 All trajectories advance together: every kernel of the step covers the whole
 batch and the step is one CUDA-graph launch.  The same batch in the plain FP64
@@ -56,11 +55,12 @@ DTYPES = {
     "fp64": "complex128",
     "mixed": "mixed (bf16x3 tcgen05 contractions with fp32 accumulation, fp64 rest)",
     "mixed6": "mixed (bf16x6 tcgen05 contractions with fp32 accumulation, fp64 rest)",
-    "mixed_fx": "mixed (tcgen05 contractions on bf16 digit slices holding 30 bits of each operand row's maximum: "
-                "5 base-64 slices for K = n_grid, 4 base-256 for K = 2 n_pairs; exact per-level accumulation, "
+    "mixed_fx": "mixed (tcgen05 contractions on bf16 digit slices holding at least 30 bits of each operand row's "
+                "maximum: 5 base-256 slices for K = n_grid, 4 or 5 for K = 2 n_pairs; exact per-level accumulation, "
                 "fp64 results; fp64 rest)",
-    "mixed_fx6": "mixed (tcgen05 contractions on bf16 digit slices holding 36 bits of each operand row's maximum: "
-                 "6 base-64 slices for K = n_grid, 5 base-256 for K = 2 n_pairs; exact per-level accumulation, "
+    "mixed_fx6": "mixed (tcgen05 contractions on bf16 digit slices holding at least 36 bits of each operand row's "
+                 "maximum: 5 base-256 slices for K = n_grid (6 up to 1024), 5 or 6 for K = 2 n_pairs; exact per-level "
+                 "accumulation, "
                  "fp64 results; fp64 rest)",
 }
 FAMILIES = ("pair_potentials", "correlation", "h2", "ci_apply", "ci_rdm", "onebody", "lanczos", "rdm_inverse",
@@ -352,13 +352,23 @@ PROFILED_TRAFFIC = {
 
 
 def fx_grid_products(precision, systems):
-    """Slice products per algorithmic product of the fixed-point contractions
-    over the grid: digit width b = 8 / 7 / 6 for K <= 256 / 1024 / longer (the
+    """Slice products per algorithmic product that the accuracy targets of the
+    fixed-point forms need at least, with digits that one chunk over the whole
+    grid sums exactly (what is issued: fx_issued_products): digit width b = 8 / 7 / 6 for K <= 256 / 1024 / longer (the
     two leading level sums stay exact in FP32), L = ceil(bits / b) slices and
     the L (L + 1) / 2 slice products of the levels below L."""
     K = max(s.nG for s in systems)
     b = 8 if K <= 256 else 7 if K <= 1024 else 6
     L = -(-FX_BITS[precision] // b)
+    return L * (L + 1) // 2
+
+
+def fx_issued_products(precision, systems):
+    """Slice products per algorithmic product that the contractions over the grid
+    issue: L (L + 1) / 2 of five base-256 slices, six in mixed_fx6 where the padded
+    grid is at most 1024 long."""
+    K = max(s.nG for s in systems)
+    L = 6 if precision == "mixed_fx6" and -(-K // 64) <= 16 else 5
     return L * (L + 1) // 2
 
 
@@ -653,7 +663,7 @@ def run_batch(args):
         roof.update(bound="tensor", achieved=work / avg_s / 1e12, peak=bf16, unit="TFLOP/s", work_per_launch=work)
         if precision in FX_BITS and dom in ("pair_potentials", "h2"):
             # what the tensor cores execute: every algorithmic product as slice products
-            k = fx_grid_products(precision, systems)
+            k = fx_issued_products(precision, systems)
             roof.update(slice_products_per_product=k, issued_tflops=k * roof["achieved"],
                         issued_frac=k * roof["achieved"] / bf16)
     elif dom == "lanczos":

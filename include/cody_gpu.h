@@ -53,12 +53,14 @@ extern "C" {
 /* As CGPU_PREC_MIXED with three-way split operands (hi + mid + lo, six products). */
 #define CGPU_PREC_MIXED_X6 2
 /* Fixed-point split form: every operand row carried as bf16 digit slices under one power
- * of two per row, holding 30 bits of the row maximum (5 base-64 slices for the contractions
- * over the grid, 4 base-256 slices for the one over orbital pairs); slice products of one
+ * of two per row, in base 256: 5 slices (39 bits of the row maximum) for the contractions
+ * over the grid, 4 or 5 (32, 40) for the one over orbital pairs; slice products of one
  * level summed exactly in their own FP32 tensor-memory accumulator, levels combined in
- * 64-bit integers: the contractions equal the products of the truncated operands. */
+ * 64-bit integers: the contractions equal the products of the truncated operands.  The
+ * FP64 form runs its contractions the same way with 7 slices (55 bits). */
 #define CGPU_PREC_MIXED_FX 3
-/* As CGPU_PREC_MIXED_FX with 36 bits (6 base-64 slices, 5 base-256 slices). */
+/* As CGPU_PREC_MIXED_FX with 5 or 6 slices over the grid (6 up to 1024 points) and 5 or 6
+ * over the pairs. */
 #define CGPU_PREC_MIXED_FX6 4
 
 /* Time-derivative selectors (the TimeDerivative procedure pointers). */
