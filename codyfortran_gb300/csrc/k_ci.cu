@@ -721,15 +721,17 @@ __global__ void k_fold_h2(z_t* __restrict__ h2Lin, float4* __restrict__ h2Df, co
 // others keep the zeros of the set-up.
 // The valid entries i1 < i2, j1 < j2 as pairs p1 = (i1, i2), p2 = (j1, j2) in
 // the triangle order (a shared-memory table of P = nO (nO - 1) / 2 pairs): each
-// block takes FOLD_CHUNK consecutive p1, its threads all p2; entry
+// block takes `chunk` consecutive p1, its threads all p2 (FOLD_CHUNK in a batch; one
+// for a single system, whose eight p1 in turn were a chain of latencies on a few SMs: 8
+// spin orbitals 12.7 -> 5.5 us, 18 25.5 -> 7.1); entry
 // e = ((i1 nO + j1) nO + i2) nO + j2.
 constexpr int FOLD_CHUNK = 8;
 constexpr int FOLD_MAX_NO = 64;
 __global__ void k_fold_h2s(z_t* __restrict__ h2Lin, float4* __restrict__ h2Df, const z_t* __restrict__ H2s,
-                           const int* __restrict__ btOf, TRAJ_ARGS) {
+                           const int* __restrict__ btOf, TRAJ_ARGS, int chunk) {
   const TrajShape& T = shp[blockIdx.z];
   const int nO = T.nO, n = T.nOS, restricted = T.restricted, P = nO * (nO - 1) / 2;
-  const int p1a = blockIdx.x * FOLD_CHUNK;
+  const int p1a = blockIdx.x * chunk;
   if (p1a >= P) return;
   h2Lin = bat(h2Lin, bs);
   h2Df = bat(h2Df, bs);
@@ -742,7 +744,7 @@ __global__ void k_fold_h2s(z_t* __restrict__ h2Lin, float4* __restrict__ h2Df, c
       pb[base + v - u - 1] = (unsigned char)v;
     }
   __syncthreads();
-  for (int p1 = p1a; p1 < min(P, p1a + FOLD_CHUNK); p1++) {
+  for (int p1 = p1a; p1 < min(P, p1a + chunk); p1++) {
     const int i1 = pa[p1], i2 = pb[p1];
     for (int p2 = threadIdx.x; p2 < P; p2 += blockDim.x) {
       const int j1 = pa[p2], j2 = pb[p2];
@@ -1111,8 +1113,9 @@ void launch_fold_h2(cgpu_ctx* c) {
     const bool dfOnly = c->ciDf && c->ciSmem > 0;
     if (c->nO > FOLD_MAX_NO) throw std::string("FillH2Lin: more than 64 spin orbitals is not supported");
     const int P = c->nO * (c->nO - 1) / 2;
-    k_fold_h2s<<<dim3((unsigned)ceil_div(P, FOLD_CHUNK), 1, c->nb), 128, 0, c->stream>>>(
-        dfOnly ? nullptr : c->h2Lin_d, c->ciDf ? c->h2Df_d : nullptr, c->h2s_d, c->btOfOrb_d, TRAJ_PASS(c));
+    const int chunk = c->nb == 1 ? 1 : FOLD_CHUNK;
+    k_fold_h2s<<<dim3((unsigned)ceil_div(P, chunk), 1, c->nb), 128, 0, c->stream>>>(
+        dfOnly ? nullptr : c->h2Lin_d, c->ciDf ? c->h2Df_d : nullptr, c->h2s_d, c->btOfOrb_d, TRAJ_PASS(c), chunk);
   } else {
     k_fold_h2<<<bgrid(c, ew_blocks(c, n4)), 256, 0, c->stream>>>(c->h2Lin_d, c->ciDf ? c->h2Df_d : nullptr, c->h2_d,
                                                                  c->btOfOrb_d, TRAJ_PASS(c));
