@@ -940,9 +940,9 @@ static void fx_potentials(cgpu_ctx* c, const z_t* orbs, bool exact, bool wantW) 
   CODY_LAUNCHED(c);
   fx_run_W(c, exact);
   dim3 gw(m->KgMax / FW_T, m->KpMax / FW_T, c->nb);
-  // fewer tiles than SMs: four times the warps a tile, whose rows are then two in turn instead of
-  // eight (501 points x 10 pairs, 8 tiles: 16.2 -> 8.0 us)
-  const bool few = gw.x * gw.y * gw.z < (unsigned)c->numSms;
+  // fewer than two tiles an SM: four times the warps a tile, whose rows are then two in turn instead
+  // of eight (8 tiles, 501 points x 10 pairs: 16.2 -> 8.0 us; 220 tiles, 2801 x 136: 19.2 -> 12.5)
+  const bool few = gw.x * gw.y * gw.z < 2 * (unsigned)c->numSms;
   auto split = few ? k_fx_split_W<L, L2, 1024> : k_fx_split_W<L, L2, 256>;
   split<<<gw, few ? 1024 : 256, 0, c->stream>>>(wantW ? m->WxA : nullptr, m->WTxB, m->eWr, m->eWc, m->Wd, m->mWr,
                                                  m->mWc, m->KpMax, m->KgMax, TRAJ_PASS(c));
