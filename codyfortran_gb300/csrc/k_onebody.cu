@@ -629,6 +629,35 @@ __global__ void k_dot_partial(z_t* __restrict__ part, const z_t* __restrict__ a,
 }
 
 // dC -= (sum of partials) * C   (dot_product(coeffs, dCoeffs) = sum conj(C) dC)
+// dC -= C <C, dC> by one block (one system's up to PC_ONE coefficients: the two launches
+// of the general form took 4.3 + 4.1 us for 16 coefficients, this one 5.3; for 1296, whose
+// FP64 one SM does alone, 4.3 + 4.0 and 10.2).
+constexpr int PC_ONE = 512;
+__global__ void __launch_bounds__(256) k_project_coeffs_one(z_t* __restrict__ dC, const z_t* __restrict__ C,
+                                                            TRAJ_ARGS) {
+  const TrajShape& S = shp[blockIdx.z];
+  dC = bat(dC, bs);
+  C = bat(C, bs);
+  z_t s = zmk(0.0, 0.0);
+  for (int i = threadIdx.x; i < S.nC; i += 256) {
+    const z_t u = C[i], v = dC[i];
+    s.x += u.x * v.x + u.y * v.y;
+    s.y += u.x * v.y - u.y * v.x;
+  }
+  __shared__ z_t ov;
+  s = block_sum(s);
+  if (threadIdx.x == 0) ov = s;
+  __syncthreads();
+  const z_t o = ov;
+  for (int i = threadIdx.x; i < S.nC; i += 256) {
+    z_t r = dC[i];
+    const z_t c = C[i];
+    r.x -= o.x * c.x - o.y * c.y;
+    r.y -= o.x * c.y + o.y * c.x;
+    dC[i] = r;
+  }
+}
+
 __global__ void k_project_coeffs_apply(z_t* __restrict__ dC, const z_t* __restrict__ C, const z_t* __restrict__ part,
                                        int nBlk, TRAJ_ARGS) {
   const TrajShape& S = shp[blockIdx.z];
@@ -1137,6 +1166,11 @@ void launch_project_orbs(cgpu_ctx* c, z_t* dOrbs, const z_t* orbs) {
 
 void launch_project_coeffs(cgpu_ctx* c, z_t* dC, const z_t* C) {
   ProfScope prof(c, CGPU_KERNEL_PROJECTORS);
+  if (c->nb == 1 && c->nC <= PC_ONE) {
+    k_project_coeffs_one<<<1, 256, 0, c->stream>>>(dC, C, TRAJ_PASS(c));
+    CODY_LAUNCHED(c);
+    return;
+  }
   int nBlk = coeff_blocks(c);
   k_dot_partial<<<bgrid(c, nBlk), 256, 0, c->stream>>>(c->partialC_d, C, dC, TRAJ_PASS(c));
   CODY_LAUNCHED(c);
