@@ -50,7 +50,7 @@
 // kernel's blocks where it can be), FP64 chains.  The FP64 pipe bounds the pair
 // potentials (k_mc_potentials).  501 points x 8 orbitals, K = 12, per field sample:
 // 27.5 ms with g, rho2 and their co-states formed, a launch per vector operation and
-// the stages recomputed for every use; 2.1 ms now.
+// the stages recomputed for every use; 1.9 ms now.
 #include <algorithm>
 #include <cmath>
 #include <vector>

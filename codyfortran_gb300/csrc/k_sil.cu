@@ -23,7 +23,7 @@
 // FP64 pipe is not the bound of this kernel (44 to 100 FMA an entry and
 // iteration): the barriers, the reductions and the chains of dependent FP64
 // instructions are.  One half step of 2801 points x 16 orbitals, K = 16: 1330 us as
-// launches, 460 here; 501 x 4, K = 12: 830 and 170.
+// launches, 460 with two barriers an order, 370 here; 501 x 4, K = 12: 830, 170 and 133.
 //
 // The groups' blocks wait on one another, so the launch is cooperative (at most
 // one block per SM) and every wait is bounded.
@@ -361,7 +361,8 @@ constexpr int SIL_STEP = 0, SIL_KEPT = 1, SIL_SPILLED = 2;
 
 // SIL_T threads a block: 256 for the small pieces (four threads an entry), whose
 // iteration is a chain of latencies; 512 where the basis fits shared memory; 1024
-// where it is read from L2 (10 helium steps 10.1 / 10.6 / 11.9 ms with 256 / 512 /
+// where it is read from L2 (with two barriers an order, before the other steps of the
+// propagation were shortened: 10 helium steps 10.1 / 10.6 / 11.9 ms with 256 / 512 /
 // 1024, 2801 x 16 points 462 / 414 / 488 us, a scan of 24 8.78 / 8.37 / 8.13 ms).
 template <int SIL_T, int MODE = SIL_STEP>
 __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
