@@ -934,7 +934,7 @@ static void fx_potentials(cgpu_ctx* c, const z_t* orbs, bool exact, bool wantW) 
   const size_t need = 2 * sizeof(double) * m->KgMax;
   const int staged = need <= FX_STAGE_MAX;
   if (staged && need > 48 * 1024)
-    CODY_CUDA(cudaFuncSetAttribute(k_fx_split_S<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need));
+    CODY_CUDA(cudaFuncSetAttribute(k_fx_split_S<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FX_STAGE_MAX));
   k_fx_split_S<L><<<dim3(c->nPairs, 1, c->nb), 256, staged ? need : 0, c->stream>>>(
       m->SxA, m->eS, m->mWr, m->mWc, orbs, c->w_d, c->pairL_d, c->pairK_d, m->KgMax, staged, TRAJ_PASS(c));
   CODY_LAUNCHED(c);

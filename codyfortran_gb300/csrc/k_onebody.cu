@@ -1222,8 +1222,8 @@ void launch_orthonormalize(cgpu_ctx* c, z_t* orbs, int col0, int nCols, int rese
   if (resetStatus) batch_zero(c, c->scal_d, sizeof(int));
   const size_t sh = mgs_smem(c->nG, nCols);
   if (sh <= MG_SMEM) {
-    if (sh > 48 * 1024)
-      CODY_CUDA(cudaFuncSetAttribute(k_mgs2_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh));
+    if (sh > 48 * 1024)  // one value for every context: another thread may launch between
+      CODY_CUDA(cudaFuncSetAttribute(k_mgs2_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MG_SMEM));
     k_mgs2_cluster<<<bgrid(c, MG_CTAS), MG_THREADS, sh, c->stream>>>(orbs, c->w_d, TRAJ_PASS(c), col0, nCols,
                                                                      (int*)c->scal_d);
   } else {
