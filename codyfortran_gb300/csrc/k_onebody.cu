@@ -332,7 +332,7 @@ __device__ __forceinline__ bool gram_cols(const TrajShape& S, int group, int& c0
 // order; more of them, and a batch's, by k_gram_final's warp per entry (a batch of 512
 // lost 2 ms a step to the blocks' counters).  4 x 4 entries over 501 points: 10.4 us
 // and another 4.1 in k_gram_final when 16 threads summed a chunk's 32 rows in one
-// chain, 9.2 now.  16 x 16 over 2801 points, where the FP64 pipe bounds the sums: 18.5
+// chain, 8.9 now.  16 x 16 over 2801 points, where the FP64 pipe bounds the sums: 18.5
 // us in 88 chunks, 13.3 in one for each SM.
 // ---------------------------------------------------------------------------
 constexpr int GR_CHUNK = 32, GR_CHUNK_MIN = 8;
@@ -946,11 +946,14 @@ unsigned vec_blocks(const cgpu_ctx* c, size_t n) {
   return (unsigned)std::max<size_t>(1, std::min(b, cap));
 }
 
-// Rows of a block: at most 32 KB of tiles; a single system's in the FP64 form, whose
-// pipe is the bound, cut to a chunk per SM.
+// Rows of a block: at most 32 KB of tiles; a single system's of more than 8 orbitals in
+// the FP64 form, whose pipe is the bound there, cut to a chunk per SM (16 orbitals of
+// 2801 points 18.6 -> 13.1 us).  Fewer orbitals gain nothing from more blocks than their
+// counter costs: 4 of 501 points 8.9 us in 16 blocks, 9.6 in 63; 4 of 21 points 5.3 us in
+// one, 7.6 in three.
 int gram_chunk(const cgpu_ctx* c, int n) {
   int chunk = std::max(1, std::min(GR_CHUNK, 1024 / std::max(n, 1)));
-  if (c->nb == 1 && !c->ciDf)
+  if (c->nb == 1 && !c->ciDf && n > 8)
     chunk = std::min(chunk, std::max(GR_CHUNK_MIN, (c->nG + c->numSms - 1) / c->numSms));
   return chunk;
 }
