@@ -286,6 +286,13 @@ struct CiWork {
   int traj, t0, t1;
 };
 
+// Page-locked host words that kernels write: the error of a bounded wait (0: none), and what
+// one launch of an adaptive SIL leaves (k_sil.cu).
+struct SilFlags {
+  int err, warnings, restarts;
+  double t, rem, dtSub;
+};
+
 // ---------------------------------------------------------------------------
 // The context: nb systems, their device-resident operators, tables and work
 // buffers, and one CUDA stream.  Not reentrant (one host thread at a time),
@@ -376,9 +383,8 @@ struct cgpu_ctx {
   void* silBlk_d = nullptr;
   z_t* silPart_d = nullptr;
   unsigned* silBar_d = nullptr;
-  // page-locked host words that kernels write: [0] error of a bounded wait, [1] warnings of the last adaptive SIL
-  volatile int* flags_h = nullptr;
-  int* flags_d = nullptr;
+  volatile SilFlags* flags_h = nullptr;  // and its device address
+  SilFlags* flags_d = nullptr;
   // TDCI static data
   z_t* tdciOrbs_d = nullptr;
   // stream / graph
@@ -574,7 +580,8 @@ void launch_lz_set(cgpu_ctx* c, int idx, double v);
 // exponential of the launch-per-pass form
 void sil_init(cgpu_ctx* c);
 void sil_free(cgpu_ctx* c);
-void launch_sil(cgpu_ctx* c, z_t* state, double t, double dt, int K, double tol, int maxRestarts);
+void launch_sil(cgpu_ctx* c, z_t* state, double t, double dt, int K, double tol, int maxRestarts, double dtSub,
+                int restarts);
 void launch_lz_expsub(cgpu_ctx* c, int j, double dt);
 // One fixed-order pass of a single system and its reverse, for the pulse
 // gradient: what the pass leaves behind (V: K state vectors, last: one, the

@@ -606,9 +606,9 @@ void build_ctx(cgpu_ctx* c, const cgpu_desc* descs, int nSys) {
   sil_init(c);
   {
     void* h = nullptr;
-    CODY_CUDA(cudaHostAlloc(&h, sizeof(int) * 2, cudaHostAllocMapped));
-    c->flags_h = (volatile int*)h;
-    c->flags_h[0] = c->flags_h[1] = 0;
+    CODY_CUDA(cudaHostAlloc(&h, sizeof(SilFlags), cudaHostAllocMapped));
+    std::memset(h, 0, sizeof(SilFlags));
+    c->flags_h = (volatile SilFlags*)h;
     CODY_CUDA(cudaHostGetDevicePointer((void**)&c->flags_d, h, 0));
   }
   CODY_CUDA(cudaMallocHost(&c->lz_h, sizeof(double) * 512));
@@ -820,9 +820,9 @@ int lanczos_pass(cgpu_ctx* c, int which, double tBase, double dt, int maxDim, do
 }
 
 // SIL Integrate (src/IntegratorList/Sil/S_IntegratorList_Sil.f90:114-177) on a device state.
-// Returns the passes that did not converge (wantWarnings; else it may return before they are known).
+// Returns the sub-steps that did not converge.
 int sil_device(cgpu_ctx* c, int which, z_t* state, double t0, double t1, int krylovDim, double tol, int maxRestarts,
-               const double* metric_d, bool wantWarnings = false) {
+               const double* metric_d) {
   const double zeroThreshold = 1.0e-14;
   if (std::fabs(t1 - t0) <= zeroThreshold) return 0;
   int maxDim = std::max(1, std::min(krylovDim, c->minS));
@@ -831,11 +831,20 @@ int sil_device(cgpu_ctx* c, int which, z_t* state, double t0, double t1, int kry
   int warnings = 0;
   if (tol > 0.0 && c->nb > 1) throw std::string("SIL: adaptive (tolerance > 0) steps need a single system");
   if (which == CGPU_TD_ORBS_LIN && c->silGroup > 0 && c->silFits) {
-    launch_sil(c, state, t0, t1 - t0, maxDim, tol, maxRestarts);
-    if (!(tol > 0.0)) return 1;
-    if (!wantWarnings) return 0;
-    sync(c);
-    return c->flags_h[1];
+    double t = t0, rem = t1 - t0, dtSub = rem;
+    int restarts = 0;
+    for (;;) {
+      launch_sil(c, state, t, rem, maxDim, tol, maxRestarts, dtSub, restarts);
+      if (!(tol > 0.0)) return 1;
+      sync(c);
+      const volatile SilFlags& f = *c->flags_h;
+      warnings += f.warnings;
+      t = f.t;
+      rem = f.rem;
+      dtSub = f.dtSub;
+      restarts = f.restarts;
+      if (!(std::fabs(rem) > zeroThreshold)) return warnings;
+    }
   }
   if (!(tol > 0.0)) {
     // fixed order: one pass, no acceptance test; the basis holds the start
@@ -1527,7 +1536,7 @@ int cgpu_integrate_sil(cgpu_ctx* c, int which, cgpu_complex* state, double t0, d
     CODY_CUDA(cudaMemcpyAsync(c->metricUser_d, metric, sizeof(double) * c->nS, cudaMemcpyHostToDevice, c->stream));
     m = c->metricUser_d;
   }
-  int w = sil_device(c, which, c->state_d, t0, t1, krylov_dim, tolerance, max_restarts, m, warnings != nullptr);
+  int w = sil_device(c, which, c->state_d, t0, t1, krylov_dim, tolerance, max_restarts, m);
   if (warnings) *warnings = w;
   down(c, state, c->state_d, c->nS);
   sync(c);

@@ -17,7 +17,9 @@
 // fit) its basis vectors stay in shared memory.  Every block sums the same partials in
 // the same order and evaluates exp(-i dt T) e1 itself, so all of them take the same
 // decisions: second pass, breakdown, convergence, halving of the step.  An adaptive
-// integration therefore runs to its end without the host.
+// integration runs without the host for SIL_PASSES Krylov passes; what is left then (a
+// tolerance that is never met, a long interval) is handed back, and the host launches the
+// next part, so that no launch holds the GPU for longer than a fraction of a second.
 //
 // FP64 throughout, also for the mixed forms: up to one group block per SM the
 // FP64 pipe is not the bound of this kernel (44 to 100 FMA an entry and
@@ -39,6 +41,7 @@ constexpr int SIL_PART = SIL_K + 8;            // partial sums of a block (two s
 constexpr int SIL_MIN = 32;                    // smallest piece worth a block of its own
 constexpr size_t SIL_SMEM = 200 * 1024;
 constexpr long long SIL_WAIT = 4000000000LL;   // cycles after which a barrier gives up
+constexpr int SIL_PASSES = 64;                 // Krylov passes of one launch (about 1 ms each at most)
 constexpr double SIL_ZERO = 1.0e-14, SIL_ETA2 = 1.0e-2;  // as k_lanczos.cu
 
 // One block's place: its trajectory, its rank in the trajectory's group, the group's size.
@@ -346,8 +349,9 @@ struct SilArgs {
   double tOff, dt;
   int K, window;
   double tol;
-  int maxRestarts;
-  int* flags;      // host memory: [0] error, [1] warnings of trajectory 0
+  double dtSub;    // the step to try first, and the halvings that led to it
+  int restarts, maxRestarts;
+  SilFlags* flags;  // host memory; what an adaptive integration (trajectory 0) leaves
   int cap, smemV;  // entries of the largest piece; basis vectors in shared memory
   int pt;          // threads per entry (4 where the pieces leave most of the block idle, else 1)
   // for the pulse gradient: a given field value, and what its reverse pass reads
@@ -402,7 +406,7 @@ __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
   auto vec = [&](int k, int e) -> z_t& { return A.smemV ? V[(size_t)k * cap + e] : basis[A.ldv * k + vidx(S, l0 + e)]; };
   auto barrier = [&]() {
     target += B.n;
-    return group_barrier(bar, target, B.n, A.flags);
+    return group_barrier(bar, target, B.n, &A.flags->err);
   };
   auto mine = [&]() { return part0 + (size_t)B.rank * PS + set * SIL_PART; };
   // after a barrier: sums over the group of the partial slots [0, n), one or two slots a
@@ -524,14 +528,14 @@ __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
     }
   };
 
-  double tCur = A.tOff, rem = A.dt;
-  int warnings = 0, it = 0;
+  double tCur = A.tOff, rem = A.dt, dtS = A.dtSub;
+  int warnings = 0, it = 0, restarts = A.restarts, pass = 0;
   bool ok = true;
-  while (ok && fabs(rem) > SIL_ZERO) {
-    double dtS = rem, nrm = 0.0;
-    int restarts = 0;
-    bool conv = false;
-    for (;;) {
+  while (ok && fabs(rem) > SIL_ZERO && pass < SIL_PASSES) {
+    double nrm = 0.0;
+    bool conv = false, done = false;
+    while (pass < SIL_PASSES) {
+      pass++;
       __syncthreads();
       // w_1 and its halo; the field takes a few microseconds of FP64 on one lane beside it
       if (tid == SIL_T - 1)
@@ -665,7 +669,8 @@ __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
           }
         }
       }
-      if (!ok || mDim == 0) break;
+      done = mDim == 0;
+      if (!ok || done) break;
       if (conv || !(A.tol > 0.0) || fabs(dtS) <= SIL_ZERO || restarts >= A.maxRestarts) {
         for (int e = tid; e < cnt; e += SIL_T) {
           z_t acc = zmk(0.0, 0.0);
@@ -681,20 +686,29 @@ __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
             if (tid == 0) *A.keep.norm = nrm;
           }
         }
+        done = true;
         break;
       }
       dtS = 0.5 * dtS;
       restarts++;
     }
-    if (!ok) break;
+    if (!ok || !done) break;
     if (!conv) warnings++;
     if (!(A.tol > 0.0)) break;  // fixed order: one pass over the whole step
     tCur += dtS;
     rem -= dtS;
+    dtS = rem;
+    restarts = 0;
     if (fabs(rem) > SIL_ZERO) ok = barrier();  // the neighbours' pieces of the new start
   }
   if (tid == 0) {
-    if (B.traj == 0 && B.rank == 0) A.flags[1] = A.tol > 0.0 ? warnings : 1;
+    if (B.traj == 0 && B.rank == 0 && A.tol > 0.0) {
+      A.flags->warnings = warnings;
+      A.flags->t = tCur;
+      A.flags->rem = rem;
+      A.flags->dtSub = dtS;
+      A.flags->restarts = restarts;
+    }
     if (B.n > 1 && atomicAdd(bar + 1, 1u) == (unsigned)B.n - 1) {
       bar[0] = 0u;
       bar[1] = 0u;
@@ -718,7 +732,7 @@ struct SilVjpArgs {
   z_t* part;
   unsigned* bar;
   int cap, nBlk;
-  int* flags;
+  SilFlags* flags;
 };
 
 // The reverse of one kept pass: sbar = (d out / d start)^H obar, grad += the field
@@ -751,7 +765,7 @@ __global__ void __launch_bounds__(256, 1) k_sil_vjp(const SilVjpArgs A, TRAJ_ARG
   const int per = (nS + A.nBlk - 1) / A.nBlk, l0 = min(nS, rank * per), cnt = min(nS, l0 + per) - l0;
   auto barrier = [&]() {
     target += A.nBlk;
-    return group_barrier(A.bar, target, A.nBlk, A.flags);
+    return group_barrier(A.bar, target, A.nBlk, &A.flags->err);
   };
   auto gather = [&](int s0, int n) {
     for (int k = wid; k < n; k += W) {
@@ -935,7 +949,7 @@ void sil_init(cgpu_ctx* c) {
 }
 
 void sil_check(cgpu_ctx* c) {
-  if (c->flags_h && c->flags_h[0]) throw std::string("SIL: a bounded wait between blocks expired");
+  if (c->flags_h && c->flags_h->err) throw std::string("SIL: a bounded wait between blocks expired");
 }
 
 void sil_free(cgpu_ctx* c) {
@@ -961,7 +975,7 @@ static SilArgs sil_args(cgpu_ctx* c, const z_t* start, z_t* state, double dt, in
   a.part = c->silPart_d;
   a.bar = c->silBar_d;
   a.tBase = c->zero_d;
-  a.dt = dt;
+  a.dt = a.dtSub = dt;
   a.K = K;
   a.window = c->krylovWindow;
   a.flags = c->flags_d;
@@ -982,14 +996,19 @@ static void sil_launch(cgpu_ctx* c, SilArgs& a, int mode) {
   CODY_LAUNCHED(c);
 }
 
-// SIL on OrbsLin from t over dt on a state (all trajectories), in place.
-void launch_sil(cgpu_ctx* c, z_t* state, double t, double dt, int K, double tol, int maxRestarts) {
+// SIL on OrbsLin from t over dt on a state (all trajectories), in place.  With a tolerance
+// it may leave some of dt: flags_h holds, after a synchronisation, the time reached, what is
+// left of dt, and the step and the halvings to go on with (dtSub, restarts).
+void launch_sil(cgpu_ctx* c, z_t* state, double t, double dt, int K, double tol, int maxRestarts, double dtSub,
+                int restarts) {
   ProfScope prof(c, CGPU_KERNEL_LANCZOS);
   SilArgs a = sil_args(c, state, state, dt, K);
   a.m = c->metric_d;
   a.tBase = (c->inCapture || c->useStepTime) ? c->stepT_d : c->zero_d;
   a.tOff = c->inCapture ? t - c->captureT0 : t;
   a.tol = tol;
+  a.dtSub = dtSub;
+  a.restarts = restarts;
   a.maxRestarts = maxRestarts;
   sil_launch(c, a, SIL_STEP);
 }

@@ -1,0 +1,72 @@
+"""The decisions of an adaptive SIL on the device: the count of sub-steps that did not
+reach the tolerance, against the oracle's, and the bound on the work of one launch.
+
+The tolerances lie far from the error estimates they are compared with (1e-200 is below
+every estimate, 1e-7 is met or missed by factors), so rounding decides nothing.  States:
+1e-12 relative, the FP64 form's parity bound, for each of the sub-steps.
+"""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from oracle import Oracle
+from oracle import lib as oracle_lib
+from codyfortran_gb300 import init as I
+from codyfortran_gb300 import spec as S
+
+pytestmark = pytest.mark.gpu
+
+
+def _system(n_el=10, m=2):
+    sp = S.helium_fedvr(n_el, 6, m, laser=S.sin2_pulse(0.05, omega=0.2, n_cycles=2.0))
+    sp.xmin, sp.xmax = -0.5 * n_el, 0.5 * n_el
+    o = Oracle(sp)
+    rng = np.random.default_rng(n_el)
+    c = rng.normal(size=o.nC) + 1j * rng.normal(size=o.nC)
+    return sp, o, I.pack_state(c / np.linalg.norm(c), I.seeded_gaussian_orbitals(sp, o.x, o.w, 5))
+
+
+def _engine_sil(e, state, dt, K, tol, restarts):
+    s, w = state.copy(), C.c_int(-1)
+    e._check(e.lib.cgpu_integrate_sil(e.h, 1, s.ctypes.data_as(C.c_void_p), C.c_double(2.0), C.c_double(2.0 + dt), K,
+                                      C.c_double(tol), restarts, None, C.byref(w)))
+    return s, w.value
+
+
+def _oracle_sil(o, state, dt, K, tol, restarts):
+    s = state.copy()
+    return s, oracle_lib().orc_integrate_sil(o.h, 1, s.ctypes.data_as(C.c_void_p), C.c_double(2.0), C.c_double(2.0 + dt),
+                                             K, C.c_double(tol), restarts, None)
+
+
+def _sub_steps(dt, restarts):
+    """Sub-steps of an integration that never converges."""
+    n, rem = 0, dt
+    while abs(rem) > 1e-14:
+        d = rem
+        for _ in range(restarts):
+            if abs(d) <= 1e-14:
+                break
+            d *= 0.5
+        rem -= d
+        n += 1
+    return n
+
+
+def test_a_launch_is_bounded():
+    """A tolerance that is never met: hundreds of Krylov passes, of which a launch takes 64."""
+    from codyfortran_gb300.engine import Engine
+    sp, o, st = _system()
+    e = Engine(sp, max_krylov=6)
+    dt, restarts = 0.01, 3
+    n = _sub_steps(dt, restarts)
+    e.launch_count(reset=True)
+    a, wa = _engine_sil(e, st, dt, 6, 1e-200, restarts)
+    launches = e.launch_count()
+    b, wb = _oracle_sil(o, st, dt, 6, 1e-200, restarts)
+    e.close()
+    print(n, "sub-steps,", launches, "launches", wa, wb, np.linalg.norm(a - b) / np.linalg.norm(b))
+    assert wa == n
+    assert launches >= n * (restarts + 1) // 64
+    assert np.linalg.norm(a - b) < n * 1e-12 * np.linalg.norm(b)
