@@ -289,7 +289,7 @@ struct CiWork {
 // Page-locked host words that kernels write: the error of a bounded wait (0: none), and what
 // one launch of an adaptive SIL leaves (k_sil.cu).
 struct SilFlags {
-  int err, warnings, restarts;
+  int err, warnings, restarts, notFinite;
   double t, rem, dtSub;
 };
 

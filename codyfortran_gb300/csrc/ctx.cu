@@ -843,6 +843,21 @@ int sil_device(cgpu_ctx* c, int which, z_t* state, double t0, double t1, int kry
       rem = f.rem;
       dtSub = f.dtSub;
       restarts = f.restarts;
+      if (f.notFinite) {
+        // the state is NaN now and stays so: count the sub-steps that are left, none of which
+        // converges (of 2^restarts ln(rem / 1e-14) at most the first million)
+        while (std::fabs(rem) > zeroThreshold && warnings < 1000000) {
+          while (std::fabs(dtSub) > zeroThreshold && restarts < maxRestarts) {
+            dtSub *= 0.5;
+            restarts++;
+          }
+          warnings++;
+          rem -= dtSub;
+          dtSub = rem;
+          restarts = 0;
+        }
+        return warnings;
+      }
       if (!(std::fabs(rem) > zeroThreshold)) return warnings;
     }
   }

@@ -529,11 +529,11 @@ __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
   };
 
   double tCur = A.tOff, rem = A.dt, dtS = A.dtSub;
-  int warnings = 0, it = 0, restarts = A.restarts, pass = 0;
+  int warnings = 0, it = 0, restarts = A.restarts, pass = 0, notFinite = 0;
   bool ok = true;
   while (ok && fabs(rem) > SIL_ZERO && pass < SIL_PASSES) {
     double nrm = 0.0;
-    bool conv = false, done = false;
+    bool conv = false, done = false, bad = false;
     while (pass < SIL_PASSES) {
       pass++;
       __syncthreads();
@@ -648,7 +648,8 @@ __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
           __syncthreads();
           n1 = shN1;
         }
-        const double be = sqrt(fmax(n1, 0.0));
+        // a rounding below zero is zero; NaN (an infinity or a NaN in the state) stays NaN: no breakdown
+        const double be = n1 < 0.0 ? 0.0 : sqrt(n1);
         const bool broke = be <= SIL_ZERO && !KEEP;  // the kept pass runs over all orders
         const bool last = broke || j == A.K;
         if (A.tol > 0.0 || last) {
@@ -662,7 +663,10 @@ __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
           }
           __syncthreads();
           conv = errEst <= A.tol;
-          if ((A.tol > 0.0 && conv) || last) {
+          // not finite: no step converges from here, however short (the kept pass and the fixed
+          // orders run on)
+          bad = A.tol > 0.0 && !(fabs(nrm) + fabs(alpha[j - 1]) + be < INFINITY);
+          if (bad || (A.tol > 0.0 && conv) || last) {
             mDim = j;
             it++;
             break;
@@ -671,7 +675,7 @@ __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
       }
       done = mDim == 0;
       if (!ok || done) break;
-      if (conv || !(A.tol > 0.0) || fabs(dtS) <= SIL_ZERO || restarts >= A.maxRestarts) {
+      if (conv || bad || !(A.tol > 0.0) || fabs(dtS) <= SIL_ZERO || restarts >= A.maxRestarts) {
         for (int e = tid; e < cnt; e += SIL_T) {
           z_t acc = zmk(0.0, 0.0);
           for (int k = 0; k < mDim; k++) zfma(acc, vec(k, e), phi[k]);
@@ -693,7 +697,11 @@ __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
       restarts++;
     }
     if (!ok || !done) break;
-    if (!conv) warnings++;
+    if (!conv && !bad) warnings++;
+    if (bad) {
+      notFinite = 1;
+      break;
+    }
     if (!(A.tol > 0.0)) break;  // fixed order: one pass over the whole step
     tCur += dtS;
     rem -= dtS;
@@ -708,6 +716,7 @@ __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
       A.flags->rem = rem;
       A.flags->dtSub = dtS;
       A.flags->restarts = restarts;
+      A.flags->notFinite = notFinite;
     }
     if (B.n > 1 && atomicAdd(bar + 1, 1u) == (unsigned)B.n - 1) {
       bar[0] = 0u;

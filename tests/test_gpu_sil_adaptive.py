@@ -70,3 +70,35 @@ def test_a_launch_is_bounded():
     assert wa == n
     assert launches >= n * (restarts + 1) // 64
     assert np.linalg.norm(a - b) < n * 1e-12 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("restarts", [0, 2])
+def test_a_state_that_is_not_finite_does_not_converge(bad, restarts):
+    from codyfortran_gb300.engine import Engine
+    sp, o, st = _system()
+    e = Engine(sp, max_krylov=6)
+    st[o.nC + 7] = bad
+    a, w = _engine_sil(e, st, 0.01, 6, 1e-7, restarts)
+    assert w == _sub_steps(0.01, restarts)
+    assert np.isnan(a).all()
+    # and the context is usable afterwards
+    sp, o, st = _system()
+    a, w = _engine_sil(e, st, 0.01, 6, 1e-7, 4)
+    b, wb = _oracle_sil(o, st, 0.01, 6, 1e-7, 4)
+    e.close()
+    assert w == wb
+    assert np.linalg.norm(a - b) < 1e-12 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("K,tol,restarts,dt", [(2, 1e-7, 0, 0.05), (3, 1e-7, 2, 0.2), (6, 1e-7, 6, 0.05), (6, 1e-3, 0, 0.001)])
+def test_warnings_are_the_oracles(K, tol, restarts, dt):
+    from codyfortran_gb300.engine import Engine
+    sp, o, st = _system()
+    e = Engine(sp, max_krylov=6)
+    a, wa = _engine_sil(e, st, dt, K, tol, restarts)
+    b, wb = _oracle_sil(o, st, dt, K, tol, restarts)
+    e.close()
+    print(wa, wb)
+    assert wa == wb
+    assert np.linalg.norm(a - b) < (1 + wb) * 1e-12 * np.linalg.norm(b)
