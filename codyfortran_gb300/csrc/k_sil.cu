@@ -122,6 +122,9 @@ __device__ __forceinline__ double warp_sum4(double v0, double v1, double v2, dou
 // jb[k] = 2 J_k of the series of exp(-i dt/n T); PARTS (the pulse gradient): n > 1
 // where |dt| R is above LZ_PART, so that jb holds every term.
 constexpr double LZ_PART = 700.0;
+// Below it J_0 is 1 and the other terms are nothing.  The recurrence's 2k/z would overflow: one
+// Krylov vector (m = 1: R is the 1e-300 added to a spectrum of no width) with |dt| >= 1.
+constexpr double LZ_TINY = 1e-30;
 template <bool PARTS>
 __device__ void lz_series_warp(const double* alpha, const double* beta, int m, double dt, double* jb, double& c,
                                double& R, int& K, int& n) {
@@ -141,7 +144,7 @@ __device__ void lz_series_warp(const double* alpha, const double* beta, int m, d
   if (PARTS) n = (int)fmin(fmax(ceil(fabs(dt) * R / LZ_PART), 1.0), (double)SIL_KEEP_PARTS);
   const double z = PARTS ? fabs(dt) * R / n : fabs(dt) * R;
   K = 1;
-  if (z >= 1e-300) {
+  if (z >= LZ_TINY) {
     // log2 of (z/2)^n / n! below -64
     const float l2 = log2f((float)fmin(z, 1e30) * 0.5f);
     float lg = 0.0f;
@@ -151,7 +154,7 @@ __device__ void lz_series_warp(const double* alpha, const double* beta, int m, d
     }
   }
   __syncwarp();
-  if (z < 1e-300) {
+  if (z < LZ_TINY) {
     if (lane == 0) {
       jb[0] = 1.0;
       jb[1] = 0.0;

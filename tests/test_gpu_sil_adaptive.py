@@ -102,3 +102,20 @@ def test_warnings_are_the_oracles(K, tol, restarts, dt):
     print(wa, wb)
     assert wa == wb
     assert np.linalg.norm(a - b) < (1 + wb) * 1e-12 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("dt", [0.1, 1.0, 2.0, -3.0])
+@pytest.mark.parametrize("tol", [0.0, 1e-9])
+def test_one_krylov_vector(dt, tol):
+    """A spectrum of no width, whatever the step: the Krylov order 1, and a state of
+    coefficients alone (H v = 0, a breakdown at once)."""
+    from codyfortran_gb300.engine import Engine
+    sp, o, st = _system()
+    e = Engine(sp, max_krylov=6)
+    a, _ = _engine_sil(e, st, dt, 1, tol, 0)
+    b, _ = _oracle_sil(o, st, dt, 1, tol, 0)
+    assert np.linalg.norm(a - b) < 1e-12 * np.linalg.norm(b)
+    st[o.nC:] = 0.0
+    a, w = _engine_sil(e, st, dt, 6, tol, 0)
+    e.close()
+    assert np.linalg.norm(a - st) < 1e-12 * np.linalg.norm(st) and (tol == 0.0 or w == 0)
