@@ -152,7 +152,7 @@ void autotune_run(cgpu_ctx* c, const char* cachePath, int force, std::string& re
     // the operands of the contractions: one NonLin derivative of the resident states
     if (c->method != CGPU_METHOD_TDCI) {
       td_device_public(c, CGPU_TD_NONLIN, c->dstate_d, c->state_d, 0.0);
-      CODY_CUDA(cudaStreamSynchronize(c->stream));
+      ctx_sync(c);
     }
     int cur[9];
     if (fx_tiles_get(c, cur)) {

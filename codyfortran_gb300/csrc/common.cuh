@@ -549,6 +549,7 @@ double fx_time_contraction(cgpu_ctx* c, int g, int reps);
 // (OrbsLin, krylov vectors) on a scratch copy of the resident states; drops the
 // captured step graph (tile and block choices are baked into it).
 double time_sil_lanczos(cgpu_ctx* c, int krylov);
+void ctx_sync(cgpu_ctx* c);  // waits for the context's stream; throws if a kernel's bounded wait expired
 void drop_step_graph(cgpu_ctx* c);
 // ctx.cu: the time derivative `which` of every trajectory's state `in` into `out`.
 void td_device_public(cgpu_ctx* c, int which, z_t* out, const z_t* in, double t);

@@ -776,7 +776,7 @@ void euler_device(cgpu_ctx* c, int which, int imag, z_t* state, double t0, doubl
   launch_axpby(c, state, c->dstate_d, zmk(t1 - t0, 0.0), zmk(1.0, 0.0), VSEL_STATE);
 }
 
-void sync(cgpu_ctx* c);
+void sync(cgpu_ctx* c) { ctx_sync(c); }
 
 // One PerformLanczosStep from start (device) into out (may be start itself).
 // Returns converged (adaptive) or -1 (not checked).
@@ -798,7 +798,7 @@ int lanczos_pass(cgpu_ctx* c, int which, double tBase, double dt, int maxDim, do
     if (adaptive) {
       launch_lanczos_tail(c, j, dt, 1);
       CODY_CUDA(cudaMemcpyAsync(c->lz_h, c->lz_d, sizeof(double) * 400, cudaMemcpyDeviceToHost, c->stream));
-      CODY_CUDA(cudaStreamSynchronize(c->stream));
+      sync(c);
       double err = c->lz_h[CODY_LZ_ERR];
       bool breakdown = c->lz_h[CODY_LZ_BREAKJ] == (double)j;
       bool conv = err <= tol;
@@ -915,7 +915,7 @@ void capture_step_graph(cgpu_ctx* c, double t0, double dt, int krylov, int useMe
   }
   batch_copy(c, c->warm_d, c->state_d, sizeof(z_t) * c->nS);
   split2_device(c, c->warm_d, t0, t0 + dt, krylov, 0.0, 0, useMetric);
-  CODY_CUDA(cudaStreamSynchronize(c->stream));
+  sync(c);
   // profiling events of the selected kernel family become event-record nodes of the graph
   c->profUsed = 0;
   long before = c->launches;
@@ -950,6 +950,14 @@ void capture_step_graph(cgpu_ctx* c, double t0, double dt, int krylov, int useMe
 
 }  // namespace
 
+// Every wait for results ends here: a kernel whose bounded wait expired has left its output
+// incomplete and says so in host memory.
+void ctx_sync(cgpu_ctx* c) {
+  CODY_CUDA(cudaStreamSynchronize(c->stream));
+  sil_check(c);
+  if (c->mixed && mixed_error(c)) throw std::string("tensor-core GEMM: a bounded mbarrier wait expired");
+}
+
 void td_device_public(cgpu_ctx* c, int which, z_t* out, const z_t* in, double t) {
   td_device(c, which, out, in, t, zmk(0.0, 1.0));
 }
@@ -968,7 +976,7 @@ double time_sil_lanczos(cgpu_ctx* c, int krylov) {
   c->profTarget = CGPU_KERNEL_LANCZOS;
   c->profUsed = 0;
   sil_device(c, CGPU_TD_ORBS_LIN, c->warm_d, 0.0, 0.005, krylov, 0.0, 0, c->metricW_d);
-  CODY_CUDA(cudaStreamSynchronize(c->stream));
+  sync(c);
   double tot = 0.0;
   for (size_t i = 0; i + 1 < c->profUsed; i += 2) {
     float ms = 0.f;
@@ -1018,7 +1026,7 @@ double energy_device(cgpu_ctx* c, const z_t* state, double t) {
   energy_launch(c, state, t);
   double e = 0.0;
   CODY_CUDA(cudaMemcpyAsync(&e, c->scal_d + CODY_SCAL_ENERGY, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-  CODY_CUDA(cudaStreamSynchronize(c->stream));
+  sync(c);
   return e;
 }
 
@@ -1073,7 +1081,6 @@ void read_file(const std::string& path, void* p, size_t bytes) {
 
 void down_state(cgpu_ctx* c, int b, cgpu_complex* dst, const z_t* src0);
 void up_state(cgpu_ctx* c, int b, z_t* dst0, const cgpu_complex* src);
-void sync(cgpu_ctx* c);
 
 // Trajectory b's resident state (and, when withRdm2, its rdm2 as left by
 // launch_ci_rdm) into the files under pre.
@@ -1145,12 +1152,6 @@ std::string traj_prefix(const char* dir, int b, bool create) {
   if (create && mkdir(path.c_str(), 0755) != 0 && errno != EEXIST)
     throw std::string("batch_save_restart: cannot create ") + path;
   return path + "/";
-}
-
-void sync(cgpu_ctx* c) {
-  CODY_CUDA(cudaStreamSynchronize(c->stream));
-  sil_check(c);
-  if (c->mixed && mixed_error(c)) throw std::string("tensor-core GEMM: a bounded mbarrier wait expired");
 }
 
 int fail(cgpu_ctx* c, const std::string& msg, int code) {
@@ -1620,6 +1621,7 @@ int cgpu_propagate_resident_timed(cgpu_ctx* c, double t0, double dt, int n_steps
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (rc != CGPU_OK) return rc;
+  sync(c);
   if (elapsed_ms) *elapsed_ms = ms;
   CODY_API_END(c)
 }

@@ -299,7 +299,7 @@ void adjoint_tdci(cgpu_ctx* c, const z_t* C0_h, const double* E_h, int nT, doubl
     CODY_CUDA(cudaMemcpyAsync(o, out, sizeof(o), cudaMemcpyDeviceToHost, c->stream));
     if (CN_h) CODY_CUDA(cudaMemcpyAsync(CN_h, CN, sizeof(z_t) * nC, cudaMemcpyDeviceToHost, c->stream));
     if (grad_h) CODY_CUDA(cudaMemcpyAsync(grad_h, grad, sizeof(double) * nT, cudaMemcpyDeviceToHost, c->stream));
-    CODY_CUDA(cudaStreamSynchronize(c->stream));
+    ctx_sync(c);
     *J = o[0];
     if (aOut) {
       aOut[0] = o[1];
@@ -311,7 +311,7 @@ void adjoint_tdci(cgpu_ctx* c, const z_t* C0_h, const double* E_h, int nT, doubl
     launch_fill_h2(c, c->tdciOrbs_d);
     launch_fold_h1(c);
     launch_fold_h2(c);
-    CODY_CUDA(cudaStreamSynchronize(c->stream));
+    ctx_sync(c);
   } catch (...) {
     cudaFree(buf);
     throw;

@@ -816,11 +816,6 @@ void step_vjp(cgpu_ctx* c, McAdjoint& A, const z_t* s, z_t* lam, int n) {
   launch_sil_vjp(c, A.lam, lam, Ea, 0.5 * dt, A.lzA, grad_at(A, na));
 }
 
-void mc_sync(cgpu_ctx* c) {
-  CODY_CUDA(cudaStreamSynchronize(c->stream));
-  sil_check(c);
-}
-
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -937,7 +932,7 @@ void mc_adjoint_forward(cgpu_ctx* c, const z_t* state0_h, const z_t* ref_h, cons
   CODY_CUDA(cudaMemcpyAsync(jo, A->J, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   CODY_CUDA(cudaMemcpyAsync(&ov, A->Ov, sizeof(z_t), cudaMemcpyDeviceToHost, c->stream));
   if (final_h) CODY_CUDA(cudaMemcpyAsync(final_h, A->cur, sizeof(z_t) * nS, cudaMemcpyDeviceToHost, c->stream));
-  mc_sync(c);
+  ctx_sync(c);
   if (J) *J = jo[0];
   if (overlap) {
     overlap[0] = ov.x;
@@ -969,5 +964,5 @@ void mc_adjoint_backward(cgpu_ctx* c, double* grad_h) {
     for (int n = n1 - 1; n >= n0; n--) step_vjp(c, *A, A->seg + (size_t)nS * (n - n0), A->co, n);
   }
   CODY_CUDA(cudaMemcpyAsync(grad_h, A->grad, sizeof(double) * nT, cudaMemcpyDeviceToHost, c->stream));
-  mc_sync(c);
+  ctx_sync(c);
 }

@@ -871,7 +871,7 @@ void fx_tiles_set(cgpu_ctx* c, const int* t) {
     if (sp[g] < fx_min_splits(kTiles) || sp[g] > cap || (sp[g] > 1 && sp[g] > kTiles / 2))
       throw std::string("tiles: K split outside the range of the level sums or the partial buffers");
   }
-  CODY_CUDA(cudaStreamSynchronize(c->stream));
+  ctx_sync(c);
   FxGemm* gm[3] = {&m->gW, &m->gZ, &m->gH};
   for (int g = 0; g < 3; g++) {
     FxGemm& G = *gm[g];
