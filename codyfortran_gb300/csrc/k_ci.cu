@@ -30,6 +30,8 @@ constexpr int CI_RDM_THREADS = 512;
 // threads of an H.C block (one configuration per warp): with 55 registers per
 // thread two 512-thread blocks fit an SM, 32 warps sharing two staged CI vectors
 constexpr int CI_APPLY_THREADS = 512;
+// largest CI vector kept in shared memory: leaves room for three blocks per SM
+constexpr size_t CI_SMEM = 72 * 1024;
 // threads of the FP64 forms' blocks (the codes, H.C)
 constexpr int CI_FP64_THREADS = 256;
 
@@ -1021,7 +1023,7 @@ void ci_build_work(cgpu_ctx* c) {
   while (c->ciPairLanes < 32 && nPairTot * c->ciPairLanes < 512L * c->numSms &&
          16 * c->ciPairLanes <= pTot / std::max(1L, nPairTot))
     c->ciPairLanes *= 2;
-  const bool df = c->ciDf && sizeof(z_t) * (size_t)c->nC <= 72 * 1024;
+  const bool df = c->ciDf && sizeof(z_t) * (size_t)c->nC <= CI_SMEM;
   const long aWarps = (df ? CI_APPLY_THREADS : CI_FP64_THREADS) / 32;
   cut(aw, std::max({64L, aTot / (8 * 152), aWarps * aTot / std::max(1L, nConfTot)}), 1 << 20,
       apply);
@@ -1039,16 +1041,12 @@ void ci_build_work(cgpu_ctx* c) {
   put(c->rdmWork_d, rdm);
   put(c->pairWork_d, pairs);
   // the CI vector of one trajectory in shared memory when it fits
-  size_t need = sizeof(z_t) * (size_t)c->nC;
-  c->ciSmem = need <= 72 * 1024 ? (int)need : 0;  // leaves room for three blocks per SM
-  if (c->ciSmem > 48 * 1024) {
-    CODY_CUDA(cudaFuncSetAttribute(k_ci_apply, cudaFuncAttributeMaxDynamicSharedMemorySize, c->ciSmem));
-    CODY_CUDA(cudaFuncSetAttribute(k_ci_apply_df, cudaFuncAttributeMaxDynamicSharedMemorySize, c->ciSmem));
-    CODY_CUDA(cudaFuncSetAttribute(k_ci_rdm_codes_df, cudaFuncAttributeMaxDynamicSharedMemorySize, c->ciSmem));
-    CODY_CUDA(cudaFuncSetAttribute(k_ci_rdm_pairs_df, cudaFuncAttributeMaxDynamicSharedMemorySize, c->ciSmem));
-    CODY_CUDA(cudaFuncSetAttribute(k_ci_rdm_codes, cudaFuncAttributeMaxDynamicSharedMemorySize, c->ciSmem));
-    CODY_CUDA(cudaFuncSetAttribute(k_ci_rdm_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, c->ciSmem));
-  }
+  const size_t need = sizeof(z_t) * (size_t)c->nC;
+  c->ciSmem = need <= CI_SMEM ? (int)need : 0;
+  if (c->ciSmem > 48 * 1024)  // one value for every context: another one's set-up must not lower it
+    for (const void* k : {(const void*)k_ci_apply, (const void*)k_ci_apply_df, (const void*)k_ci_rdm_codes_df,
+                          (const void*)k_ci_rdm_pairs_df, (const void*)k_ci_rdm_codes, (const void*)k_ci_rdm_pairs})
+      CODY_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CI_SMEM));
 }
 
 void launch_ci_apply(cgpu_ctx* c, const z_t* C, z_t* dC, int useH1, int useH2) {
