@@ -1,9 +1,9 @@
 """The decisions of an adaptive SIL on the device: the count of sub-steps that did not
 reach the tolerance, against the oracle's, and the bound on the work of one launch.
 
-The tolerances lie far from the error estimates they are compared with (1e-200 is below
-every estimate, 1e-7 is met or missed by factors), so rounding decides nothing.  States:
-1e-12 relative, the FP64 form's parity bound, for each of the sub-steps.
+The tolerances (1e-9 at the smallest) lie far above the estimates' rounding, and an
+estimate a tenth off decides at most one sub-step of a hundred otherwise.  States: 1e-12
+relative, the FP64 form's parity bound, for each of the sub-steps.
 """
 import ctypes as C
 
@@ -55,21 +55,20 @@ def _sub_steps(dt, restarts):
 
 
 def test_a_launch_is_bounded():
-    """A tolerance that is never met: hundreds of Krylov passes, of which a launch takes 64."""
+    """A tolerance that most sub-steps miss: hundreds of Krylov passes, of which a launch takes 64."""
     from codyfortran_gb300.engine import Engine
     sp, o, st = _system()
     e = Engine(sp, max_krylov=6)
-    dt, restarts = 0.01, 3
-    n = _sub_steps(dt, restarts)
+    restarts = 3
     e.launch_count(reset=True)
-    a, wa = _engine_sil(e, st, dt, 6, 1e-200, restarts)
+    a, wa = _engine_sil(e, st, 0.2, 2, 1e-9, restarts)
     launches = e.launch_count()
-    b, wb = _oracle_sil(o, st, dt, 6, 1e-200, restarts)
+    b, wb = _oracle_sil(o, st, 0.2, 2, 1e-9, restarts)
     e.close()
-    print(n, "sub-steps,", launches, "launches", wa, wb, np.linalg.norm(a - b) / np.linalg.norm(b))
-    assert wa == n
-    assert launches >= n * (restarts + 1) // 64
-    assert np.linalg.norm(a - b) < n * 1e-12 * np.linalg.norm(b)
+    print(wa, wb, "warnings,", launches, "launches", np.linalg.norm(a - b) / np.linalg.norm(b))
+    assert wa == wb > 100
+    assert launches >= wb * (restarts + 1) // 64
+    assert np.linalg.norm(a - b) < _sub_steps(0.2, restarts) * 1e-12 * np.linalg.norm(b)
 
 
 @pytest.mark.parametrize("bad", [np.nan, np.inf])
