@@ -10,8 +10,9 @@
 //     own (GEMM plus its K-split reduction), every instantiated tile
 //     configuration of its slice count at every K split the partial buffers
 //     hold and the digits' exact range allows;
-//   * the Lanczos family of one fixed-order SIL half step at half, one and two
-//     times the heuristic's blocks per trajectory (as far as the partials hold).
+//   * the Lanczos family of one fixed-order SIL half step, in its form of a launch a
+//     pass (the only one that the block count is for), at half, one and two times the
+//     heuristic's blocks per trajectory (as far as the partials hold).
 // The fixed-point contractions are exact sums of digit products, so the tile
 // choice does not change their results; a K split adds one FP64 rounding per
 // partial, and the Lanczos block count changes the order of the FP64 partial
@@ -19,10 +20,11 @@
 //
 // Winners are kept in a JSON-lines cache, one object per shape key:
 //   {"key": "...", "W": [bn, compact, splits], "Z": [...], "H2": [...], "lz_blocks": n}
-// The key holds the precision, the device name and SM count, the Krylov
-// order and window, the number of trajectories and a 64-bit FNV-1a hash of
-// every trajectory's sizes, so a cache entry is reused only for the same
-// batch shapes on the same kind of GPU.
+// The key holds the precision, the digit slices and the version of the GEMM that was
+// timed, the device name and SM count, the Krylov order and window, the number of
+// trajectories and a 64-bit FNV-1a hash of every trajectory's sizes, so a cache entry is
+// reused only for the same kernels on the same batch shapes and kind of GPU.  An entry
+// that this context cannot apply counts as absent.
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
@@ -30,6 +32,7 @@
 #include <sstream>
 
 #include "common.cuh"
+#include "tc.cuh"
 
 namespace {
 
@@ -52,8 +55,10 @@ std::string tune_key(const cgpu_ctx* c) {
   std::memset(&prop, 0, sizeof(prop));
   if (cudaGetDevice(&dev) == cudaSuccess) cudaGetDeviceProperties(&prop, dev);
   char buf[512];
-  std::snprintf(buf, sizeof(buf), "prec=%d;dev=%s;sms=%d;krylov=%d;window=%d;nb=%d;shape=%016llx", c->precision,
-                prop.name, c->numSms, c->maxKrylov, c->krylovWindow, c->nb, (unsigned long long)h);
+  int L, L2;
+  fx_slice_plan(c, &L, &L2);
+  std::snprintf(buf, sizeof(buf), "prec=%d;fx=%d,%d,v%d;dev=%s;sms=%d;krylov=%d;window=%d;nb=%d;shape=%016llx",
+                c->precision, L, L2, FX_VERSION, prop.name, c->numSms, c->maxKrylov, c->krylovWindow, c->nb, (unsigned long long)h);
   return buf;
 }
 
@@ -122,16 +127,24 @@ void tiles_get(const cgpu_ctx* c, int* t) {
   t[9] = c->lzBlocks;
 }
 
-void tiles_set(cgpu_ctx* c, const int* t) {
-  if (t[9] < 1 || t[9] > c->lzBlocksCap) throw std::string("tiles: Lanczos blocks per trajectory out of range");
+static bool gemm_tiles_differ(const cgpu_ctx* c, const int* t) {
   int cur[10];
   tiles_get(c, cur);
-  bool gemm = false;
-  for (int i = 0; i < 9; i++) gemm |= cur[i] != t[i];
-  if (gemm) {
-    if (!fx_tiles_get(c, cur)) throw std::string("tiles: GEMM tiles exist only in the fixed-point forms");
-    fx_tiles_set(c, t);
-  }
+  return std::memcmp(cur, t, 9 * sizeof(int)) != 0;
+}
+
+// Why tiles_set would throw, or null.
+static const char* tiles_refused(const cgpu_ctx* c, const int* t) {
+  if (t[9] < 1 || t[9] > c->lzBlocksCap) return "tiles: Lanczos blocks per trajectory out of range";
+  if (!gemm_tiles_differ(c, t)) return nullptr;
+  int cur[9];
+  if (!fx_tiles_get(c, cur)) return "tiles: GEMM tiles exist only in the fixed-point forms";
+  return fx_tiles_refused(c, t);
+}
+
+void tiles_set(cgpu_ctx* c, const int* t) {
+  if (const char* why = tiles_refused(c, t)) throw std::string(why);
+  if (gemm_tiles_differ(c, t)) fx_tiles_set(c, t);
   c->lzBlocks = t[9];
   drop_step_graph(c);
 }
@@ -143,7 +156,7 @@ void autotune_run(cgpu_ctx* c, const char* cachePath, int force, std::string& re
   int t[10];
   std::ostringstream js;
   js.precision(5);
-  if (!force && cachePath && cache_read(cachePath, key, t)) {
+  if (!force && cachePath && cache_read(cachePath, key, t) && !tiles_refused(c, t)) {
     tiles_set(c, t);
     js << "{\"source\": \"cache\", \"key\": \"" << key << "\"";
   } else {

@@ -542,7 +542,9 @@ void launch_fx_h2(cgpu_ctx* c);  // FillH2 with the FP64 form's slices (fxOn)
 // fx_time_contraction times GEMM g (with its K-split reduction) on the
 // operands in the arena, ms per launch.
 bool fx_tiles_get(const cgpu_ctx* c, int* t);
+const char* fx_tiles_refused(const cgpu_ctx* c, const int* t);  // why fx_tiles_set would throw, or null
 void fx_tiles_set(cgpu_ctx* c, const int* t);
+void fx_slice_plan(const cgpu_ctx* c, int* L, int* L2);  // digit slices over the grid and the pairs (0: none)
 void fx_tile_candidates(const cgpu_ctx* c, int g, std::vector<std::array<int, 3>>& out);
 double fx_time_contraction(cgpu_ctx* c, int g, int reps);
 // ctx.cu: device ms of the Lanczos family over one fixed-order SIL half step

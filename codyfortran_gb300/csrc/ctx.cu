@@ -971,6 +971,12 @@ void drop_step_graph(cgpu_ctx* c) {
 }
 
 double time_sil_lanczos(cgpu_ctx* c, int krylov) {
+  struct PerPass {  // the launch-per-pass form, whichever serves the context's steps
+    cgpu_ctx* c;
+    bool prev;
+    explicit PerPass(cgpu_ctx* cc) : c(cc), prev(cc->silFits) { c->silFits = false; }
+    ~PerPass() { c->silFits = prev; }
+  } perPass(c);
   drop_step_graph(c);
   batch_copy(c, c->warm_d, c->state_d, sizeof(z_t) * c->nS);
   c->profTarget = CGPU_KERNEL_LANCZOS;

@@ -836,6 +836,11 @@ static void fx_run_H2(cgpu_ctx* c, bool exact) {
 // The FP64 form has one tile width and is not tuned.
 static bool fx_tunable(const cgpu_ctx* c) { return c->mixed && c->mixed->L && c->precision != CGPU_PREC_FP64; }
 
+void fx_slice_plan(const cgpu_ctx* c, int* L, int* L2) {
+  *L = c->mixed ? c->mixed->L : 0;
+  *L2 = c->mixed ? c->mixed->L2 : 0;
+}
+
 bool fx_tiles_get(const cgpu_ctx* c, int* t) {
   if (!fx_tunable(c)) return false;
   const MixedBufs* m = c->mixed;
@@ -856,31 +861,39 @@ static void fx_gemm_plan(const cgpu_ctx* c, int g, int& kTiles, int& cap, int& N
   else { kTiles = m->KgMax / 64; cap = m->sCapH; N = 2 * c->nPairs; }
 }
 
-void fx_tiles_set(cgpu_ctx* c, const int* t) {
-  MixedBufs* m = c->mixed;
-  if (!fx_tunable(c)) throw std::string("tiles: not a fixed-point context");
-  int sp[3];
+const char* fx_tiles_refused(const cgpu_ctx* c, const int* t) {
+  const MixedBufs* m = c->mixed;
+  if (!fx_tunable(c)) return "tiles: not a fixed-point context";
   for (int g = 0; g < 3; g++) {
     int kTiles, cap, N;
     fx_gemm_plan(c, g, kTiles, cap, N);
     if (!fx_tile_supported(t[3 * g], g == TC_GEMM_Z ? m->L2 : m->L, t[3 * g + 1] != 0))
-      throw std::string("tiles: no fixed-point GEMM configuration for that tile");
-    if (t[3 * g + 2] < 1 || t[3 * g + 2] > kTiles) throw std::string("tiles: K split count outside 1..K blocks");
-    sp[g] = fx_normalize_splits(kTiles, t[3 * g + 2]);
+      return "tiles: no fixed-point GEMM configuration for that tile";
+    if (t[3 * g + 2] < 1 || t[3 * g + 2] > kTiles) return "tiles: K split count outside 1..K blocks";
+    const int s = fx_normalize_splits(kTiles, t[3 * g + 2]);
     // every split keeps at least two K blocks, as the set-up heuristic does
-    if (sp[g] < fx_min_splits(kTiles) || sp[g] > cap || (sp[g] > 1 && sp[g] > kTiles / 2))
-      throw std::string("tiles: K split outside the range of the level sums or the partial buffers");
+    if (s < fx_min_splits(kTiles) || s > cap || (s > 1 && s > kTiles / 2))
+      return "tiles: K split outside the range of the level sums or the partial buffers";
   }
+  return nullptr;
+}
+
+void fx_tiles_set(cgpu_ctx* c, const int* t) {
+  if (const char* why = fx_tiles_refused(c, t)) throw std::string(why);
+  MixedBufs* m = c->mixed;
   ctx_sync(c);
   FxGemm* gm[3] = {&m->gW, &m->gZ, &m->gH};
   for (int g = 0; g < 3; g++) {
     FxGemm& G = *gm[g];
     if (G.tiles) CODY_CUDA(cudaFree(G.tiles));
     G.tiles = nullptr;
-    G.tiles = fx_build_tiles(c, g, t[3 * g], sp[g], &G.nTiles);
+    int kTiles, cap, N;
+    fx_gemm_plan(c, g, kTiles, cap, N);
+    const int s = fx_normalize_splits(kTiles, t[3 * g + 2]);
+    G.tiles = fx_build_tiles(c, g, t[3 * g], s, &G.nTiles);
     G.bn = t[3 * g];
     G.compact = t[3 * g + 1] != 0;
-    G.s = sp[g];
+    G.s = s;
   }
 }
 

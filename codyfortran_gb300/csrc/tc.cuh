@@ -57,6 +57,9 @@ CUtensorMap tc_make_map_planes(const __nv_bfloat16* base, int rowsMax, int pitch
 int fx_tile_n(int N, int L, bool compact);
 // Whether a compact configuration exists for L slices.
 bool fx_compact_ok(int L);
+// Version of the fixed-point GEMM that timings of its tiles belong to: raised when its
+// configurations or what they cost change.
+constexpr int FX_VERSION = 2;
 // The instantiated (N tile width, compact) configurations for L slices.
 void fx_tile_configs(int L, std::vector<std::pair<int, bool>>& out);
 bool fx_tile_supported(int bn, int L, bool compact);

@@ -382,14 +382,17 @@ int cgpu_batch_shared_interactions(const cgpu_batch* batch);
  * tiles[0..8] = for the fixed-point contractions W = V S, Z = W R'' and
  * h2 = S^T W in turn: N-tile width, compact flag (two CTAs per SM), K splits
  * (zero outside CGPU_PREC_MIXED_FX / _FX6); tiles[9] = blocks per trajectory
- * of the Lanczos reductions.  The set-up heuristics choose the initial table.
+ * of the Lanczos reductions of the steps that take a launch a pass (batches of more
+ * trajectories than SMs; Krylov steps of other derivatives than the one-body
+ * part).  The set-up heuristics choose the initial table.
  * cgpu_autotune times the candidates on the resident states (upload them
  * first) with CUDA events on the context's stream and applies the fastest:
  * every instantiated tile configuration and feasible K split of each
  * contraction, and half / one / two times the heuristic's Lanczos blocks.
  * cache_path (may be NULL) is a JSON-lines file of winners keyed by the
- * precision, device, Krylov order and window and the trajectories' sizes:
- * CGPU_TUNE_CACHED applies the cached entry of this shape if there is one and
+ * precision, digit slices, kernel version, device, Krylov order and window and
+ * the trajectories' sizes:
+ * CGPU_TUNE_CACHED applies the cached entry of this shape if there is one that fits and
  * otherwise tunes and adds it; CGPU_TUNE_FORCE always tunes and replaces it.
  * report (may be NULL) receives a JSON object with the source ("tuned" or
  * "cache"), the key, the timed candidates [tile..., ms] and the chosen table.
