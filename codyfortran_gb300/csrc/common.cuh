@@ -310,6 +310,7 @@ struct cgpu_ctx {
   TrajShape* shape_d = nullptr;
   // sizes (maxima over the systems; uniform: nBt, restricted, method, precision, hasInteraction)
   int nG = 0, nBt = 0, nO = 0, nOS = 0, nC = 0, nS = 0, nGO = 0, restricted = 0, method = 0, precision = 0;
+  int precisionAsked = 0;  // the descriptor's: CGPU_PREC_FP64_PIPE is precision FP64 without digit slices
   int band = 0, nBtK = 1, nPairs = 0;
   int minS = 0;                   // smallest state size (bounds the Krylov order)
   // CI work lists (blocks balanced by the number of terms; see ci_build_work)
@@ -524,6 +525,7 @@ size_t zgemm_partial_need(const cgpu_ctx* c);
 // k_mixed.cu
 size_t mixed_layout(cgpu_ctx* c, char* base, size_t off);  // sizes (base == nullptr) or places the buffers
 size_t mixed_outside_bytes(const cgpu_ctx* c);  // device bytes beside the arena (shared interaction slices)
+bool mixed_alloc_outside(cgpu_ctx* c);          // allocates them (false: no memory)
 void mixed_init(cgpu_ctx* c);
 void mixed_free(cgpu_ctx* c);
 int mixed_error(cgpu_ctx* c);

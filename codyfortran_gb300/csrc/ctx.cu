@@ -222,7 +222,7 @@ __global__ void k_gather_states(z_t* __restrict__ dst, const z_t* __restrict__ s
 void build_system(cgpu_ctx* c, SysHost& s, const cgpu_desc* d) {
   if (d->n_body_types != c->nBt) throw std::string("batch: every system needs the same number of body types");
   if ((d->restricted ? 1 : 0) != c->restricted) throw std::string("batch: mixed restricted / unrestricted systems");
-  if (d->method != c->method || d->precision != c->precision)
+  if (d->method != c->method || d->precision != c->precisionAsked)
     throw std::string("batch: every system needs the same method and precision");
   if ((d->has_interaction ? 1 : 0) != c->hasInteraction) throw std::string("batch: mixed interaction settings");
   s.regEps = d->regularization > 0 ? d->regularization : 1e-10;
@@ -440,12 +440,13 @@ void detect_shared_interaction(cgpu_ctx* c) {
 void build_ctx(cgpu_ctx* c, const cgpu_desc* descs, int nSys) {
   const cgpu_desc* d0 = &descs[0];
   if (d0->n_body_types < 1 || d0->n_body_types > CODY_MAX_BT) throw std::string("method.mb.nBodyTypes out of range");
-  if (d0->precision < CGPU_PREC_FP64 || d0->precision > CGPU_PREC_MIXED_FX6) throw std::string("unknown precision");
+  if (d0->precision < CGPU_PREC_FP64 || d0->precision > CGPU_PREC_FP64_PIPE) throw std::string("unknown precision");
   c->nb = nSys;
   c->nBt = d0->n_body_types;
   c->restricted = d0->restricted ? 1 : 0;
   c->method = d0->method;
-  c->precision = d0->precision;
+  c->precisionAsked = d0->precision;
+  c->precision = d0->precision == CGPU_PREC_FP64_PIPE ? CGPU_PREC_FP64 : d0->precision;
   c->ciDf = (c->precision == CGPU_PREC_MIXED_FX || c->precision == CGPU_PREC_MIXED_FX6) ? 1 : 0;
   c->hasInteraction = d0->has_interaction ? 1 : 0;
   CODY_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
@@ -508,22 +509,36 @@ void build_ctx(cgpu_ctx* c, const cgpu_desc* descs, int nSys) {
   };
   // The contractions run as digit slices in both fixed-point forms.  In the FP64
   // form they do too (28 slice products on the tensor cores against the FP64
-  // pipe, 12 to 40 times slower on every shape measured), unless only the
-  // FP64-pipe kernels' smaller footprint fits the device.
+  // pipe, 12 to 40 times slower on every shape measured), unless the caller asks for
+  // the FP64 pipe or the slices' larger footprint takes more than three quarters of
+  // the device (the rest is for what is allocated on first use).  That is a matter of
+  // the sizes, not of what else the device holds; only a context that would fail for
+  // want of memory takes the FP64-pipe kernels because of it, as
+  // cgpu_contraction_slices tells.
   const bool fxForm = d0->precision == CGPU_PREC_MIXED_FX || d0->precision == CGPU_PREC_MIXED_FX6;
-  const bool fp64 = d0->precision == CGPU_PREC_FP64 && c->hasInteraction && c->method != CGPU_METHOD_TDCI;
-  size_up(fxForm || fp64);
-  if (!fxForm && fp64) {
+  bool slices = d0->precision == CGPU_PREC_FP64 && c->hasInteraction && c->method != CGPU_METHOD_TDCI;
+  size_up(fxForm || slices);
+  if (slices) {
     size_t freeB = 0, totB = 0;
     CODY_CUDA(cudaMemGetInfo(&freeB, &totB));
-    if (total + ((size_t)512 << 20) > freeB) {
+    slices = total <= totB / 4 * 3;
+    // arena, and what lies beside it
+    if (slices && (cudaMalloc(&c->arena, c->bs * (size_t)nSys) != cudaSuccess || !mixed_alloc_outside(c))) {
+      cudaGetLastError();
+      if (c->arena) cudaFree(c->arena);
+      c->arena = nullptr;
+      slices = false;
+    }
+    if (!slices) {
       mixed_free(c);
       size_up(0);
     }
   }
-  // arena
   total = c->bs * (size_t)nSys;
-  CODY_CUDA(cudaMalloc(&c->arena, total));
+  if (!c->arena) {
+    CODY_CUDA(cudaMalloc(&c->arena, total));
+    if (!mixed_alloc_outside(c)) throw std::string("cuda: out of memory for the shared interaction slices");
+  }
   CODY_CUDA(cudaMemset(c->arena, 0, total));
   CODY_CUDA(cudaDeviceSynchronize());
   layout(c, c->arena);
@@ -1359,6 +1374,12 @@ int cgpu_configlist_tables(cgpu_ctx* c, int bt, int kind, int* n_conf, int* max_
   CODY_API_END(c)
 }
 
+int cgpu_contraction_slices(const cgpu_ctx* c) {
+  int L = 0, L2 = 0;
+  if (c) fx_slice_plan(c, &L, &L2);
+  return L;
+}
+
 int cgpu_synchronize(cgpu_ctx* c) {
   CODY_API_BEGIN(c)
   sync(c);
@@ -1947,6 +1968,8 @@ int cgpu_batch_observables(cgpu_batch* b, const double* t, double* out) {
 long cgpu_batch_kernels_per_step(const cgpu_batch* b) { return (b && b->c) ? b->c->graphKernels : 0; }
 
 long cgpu_batch_launch_count(cgpu_batch* b, int reset) { return (b && b->c) ? cgpu_launch_count(b->c, reset) : -1; }
+
+int cgpu_batch_contraction_slices(const cgpu_batch* b) { return b ? cgpu_contraction_slices(b->c) : 0; }
 
 int cgpu_batch_shared_interactions(const cgpu_batch* b) {
   if (!b || !b->c || b->c->precision == CGPU_PREC_FP64) return 0;  // counts the mixed fixed-point forms' matrices

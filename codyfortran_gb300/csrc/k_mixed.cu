@@ -705,6 +705,15 @@ size_t mixed_outside_bytes(const cgpu_ctx* c) {
   return c->fxRoots.size() * (size_t)c->nG * (FX_L64 * kgBig * sizeof(__nv_bfloat16) + sizeof(int));
 }
 
+bool mixed_alloc_outside(cgpu_ctx* c) {
+  MixedBufs* m = c->mixed;
+  if (!m || mixed_outside_bytes(c) == 0) return true;
+  const size_t rows = (size_t)c->nG * c->fxRoots.size();
+  m->KgBig = (c->nG + 63) / 64 * 64;
+  return cudaMalloc(&m->Vsh, sizeof(__nv_bfloat16) * rows * FX_L64 * m->KgBig) == cudaSuccess &&
+         cudaMalloc(&m->eVsh, sizeof(int) * rows) == cudaSuccess;
+}
+
 void mixed_free(cgpu_ctx* c) {
   if (c->mixed) {
     MixedBufs* m = c->mixed;
@@ -735,10 +744,7 @@ void mixed_init(cgpu_ctx* c) {
     if (c->fxShared) {
       // each root trajectory's interaction matrix, sliced once for the batch
       const int nR = (int)c->fxRoots.size();
-      m->KgBig = (c->nG + 63) / 64 * 64;
       const size_t plane = (size_t)c->nG * FX_L64 * m->KgBig;  // elements per root
-      CODY_CUDA(cudaMalloc(&m->Vsh, sizeof(__nv_bfloat16) * plane * nR));
-      CODY_CUDA(cudaMalloc(&m->eVsh, sizeof(int) * (size_t)c->nG * nR));
       CODY_CUDA(cudaMemsetAsync(m->Vsh, 0, sizeof(__nv_bfloat16) * plane * nR, c->stream));
       for (int r = 0; r < nR; r++) {
         const int root = c->fxRoots[r], nGb = c->sys[root].nG;

@@ -42,7 +42,7 @@ EXPORTED = [
     "cgpu_autotune", "cgpu_get_tiles", "cgpu_set_tiles", "cgpu_batch_autotune", "cgpu_batch_get_tiles",
     "cgpu_batch_set_tiles", "cgpu_sys_kinetic_multiply", "cgpu_sys_potential_fill", "cgpu_sys_potential_multiply",
     "cgpu_sys_interaction_src", "cgpu_sys_interaction_potential", "cgpu_sys_interaction_multiply",
-    "cgpu_mc_adjoint_forward", "cgpu_mc_adjoint_backward",
+    "cgpu_mc_adjoint_forward", "cgpu_mc_adjoint_backward", "cgpu_contraction_slices", "cgpu_batch_contraction_slices",
 ]
 
 TUNE_CACHED, TUNE_FORCE = 0, 1
@@ -99,8 +99,9 @@ def load_library(path: str = LIB_PATH):
     lib.cgpu_batch_kernels_per_step.argtypes = [C.c_void_p]
     lib.cgpu_batch_launch_count.restype = C.c_long
     lib.cgpu_batch_launch_count.argtypes = [C.c_void_p, C.c_int]
-    lib.cgpu_batch_shared_interactions.restype = C.c_int
-    lib.cgpu_batch_shared_interactions.argtypes = [C.c_void_p]
+    for f in (lib.cgpu_batch_shared_interactions, lib.cgpu_contraction_slices, lib.cgpu_batch_contraction_slices):
+        f.restype = C.c_int
+        f.argtypes = [C.c_void_p]
     lib.cgpu_host_alloc.argtypes = [C.c_size_t, C.POINTER(C.c_void_p)]
     lib.cgpu_host_free.argtypes = [C.c_void_p]
     lib.cgpu_save_restart.argtypes = [C.c_void_p, C.c_char_p, C.c_int]
@@ -230,7 +231,8 @@ def make_desc(spec: SystemSpec, precision: str = "fp64", max_krylov: int = 32, k
         d.n_field_samples = len(keep)
         d.field_dt, d.field_t0 = L.sample_dt, L.sample_t0
     d.method = 1 if spec.method == "tdci" else 0
-    d.precision = {"fp64": 0, "mixed": 1, "mixed6": 2, "mixed_fx": 3, "mixed_fx6": 4}[precision]
+    d.precision = {"fp64": 0, "mixed": 1, "mixed6": 2, "mixed_fx": 3, "mixed_fx6": 4,
+                   "fp64_pipe": 5}[precision]
     d.max_krylov = max_krylov
     d.krylov_window = int(krylov_window)
     return d, keep
@@ -269,6 +271,10 @@ class Engine(_Tunable):
     def _check(self, rc):
         if rc != 0:
             raise CodyError(self.lib.cgpu_last_error(self.h).decode())
+
+    def contraction_slices(self):
+        """Digit slices of the contractions over the grid, 0 where they do not run in slices."""
+        return self.lib.cgpu_contraction_slices(self.h)
 
     def launch_count(self, reset=False):
         return self.lib.cgpu_launch_count(self.h, int(reset))
@@ -685,6 +691,10 @@ class Batch(_Tunable):
     def shared_interactions(self):
         """Number of interaction matrices shared by the batch (fixed-point form), 0 if none."""
         return self.lib.cgpu_batch_shared_interactions(self.h)
+
+    def contraction_slices(self):
+        """Digit slices of the contractions over the grid, 0 where they do not run in slices."""
+        return self.lib.cgpu_batch_contraction_slices(self.h)
 
     def kernels_per_step(self):
         return self.lib.cgpu_batch_kernels_per_step(self.h)

@@ -19,7 +19,8 @@ module M_CodyGpu
   integer(c_int), parameter :: CGPU_INT_TOEPLITZ = 0, CGPU_INT_DENSE = 1
   integer(c_int), parameter :: CGPU_LASER_NONE = 0, CGPU_LASER_SIN2 = 1, CGPU_LASER_SAMPLED = 2
   integer(c_int), parameter :: CGPU_METHOD_MCTDHX = 0, CGPU_METHOD_TDCI = 1
-  integer(c_int), parameter :: CGPU_PREC_FP64 = 0, CGPU_PREC_MIXED_FX = 3, CGPU_PREC_MIXED_FX6 = 4
+  integer(c_int), parameter :: CGPU_PREC_FP64 = 0, CGPU_PREC_MIXED_FX = 3, CGPU_PREC_MIXED_FX6 = 4, &
+       CGPU_PREC_FP64_PIPE = 5
   integer(c_int), parameter :: CGPU_TD_FULL = 0, CGPU_TD_ORBS_LIN = 1, CGPU_TD_NONLIN = 2, CGPU_TD_TDCI = 3
   integer(c_int), parameter :: CGPU_TUNE_CACHED = 0, CGPU_TUNE_FORCE = 1
 

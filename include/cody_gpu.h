@@ -62,6 +62,8 @@ extern "C" {
 /* As CGPU_PREC_MIXED_FX with 5 or 6 slices over the grid (6 up to 1024 points) and 5 or 6
  * over the pairs. */
 #define CGPU_PREC_MIXED_FX6 4
+/* As CGPU_PREC_FP64 with every contraction on the FP64 pipe (12 to 40 times slower there). */
+#define CGPU_PREC_FP64_PIPE 5
 
 /* Time-derivative selectors (the TimeDerivative procedure pointers). */
 #define CGPU_TD_FULL 0   /* Method_TimeDerivative (Mctdhx :101-149)                        */
@@ -142,6 +144,11 @@ int cgpu_grid(const cgpu_ctx* ctx, double* x, double* w);
 int cgpu_configlist_tables(cgpu_ctx* ctx, int bt, int kind, int* n_conf, int* max_conn, int64_t* codes,
                            int* n_connected, int* excited_c, int* orb_code, double* factor);
 int cgpu_synchronize(cgpu_ctx* ctx);
+/* Digit slices that carry an operand of the contractions over the grid; 0 where they do
+ * not run in slices (CGPU_PREC_FP64_PIPE, _MIXED, _MIXED_X6, TDCI in FP64, no interaction,
+ * and contexts whose slices would take more than three quarters of the device's memory or
+ * did not find theirs free). */
+int cgpu_contraction_slices(const cgpu_ctx* ctx);
 /* Number of CUDA kernels this context launched since the last reset. */
 long cgpu_launch_count(cgpu_ctx* ctx, int reset);
 
@@ -376,6 +383,7 @@ long cgpu_batch_launch_count(cgpu_batch* batch, int reset);
 /* Fixed-point form: the number of shared interaction matrices (root grids in which every
  * trajectory's grid is a contiguous piece), 0 when each trajectory keeps its own. */
 int cgpu_batch_shared_interactions(const cgpu_batch* batch);
+int cgpu_batch_contraction_slices(const cgpu_batch* batch);
 
 /* ---- tile autotuner ------------------------------------------------------ */
 /* No counterpart in the reference.  The tile table of a context or batch:
