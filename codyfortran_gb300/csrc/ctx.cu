@@ -1972,7 +1972,7 @@ long cgpu_batch_launch_count(cgpu_batch* b, int reset) { return (b && b->c) ? cg
 int cgpu_batch_contraction_slices(const cgpu_batch* b) { return b ? cgpu_contraction_slices(b->c) : 0; }
 
 int cgpu_batch_shared_interactions(const cgpu_batch* b) {
-  if (!b || !b->c || b->c->precision == CGPU_PREC_FP64) return 0;  // counts the mixed fixed-point forms' matrices
+  if (!b || !b->c) return 0;
   return b->c->fxShared ? (int)b->c->fxRoots.size() : 0;
 }
 

@@ -689,7 +689,7 @@ class Batch(_Tunable):
         return e
 
     def shared_interactions(self):
-        """Number of interaction matrices shared by the batch (fixed-point form), 0 if none."""
+        """Number of interaction matrices shared by the batch (contractions in digit slices), 0 if none."""
         return self.lib.cgpu_batch_shared_interactions(self.h)
 
     def contraction_slices(self):

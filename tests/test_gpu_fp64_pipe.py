@@ -84,3 +84,18 @@ def test_the_choice_is_the_callers():
         b.close()
     for x, y in zip(*out):
         assert _rel(x, y) < 1e-11
+
+
+@pytest.mark.parametrize("precision,shared", [("fp64", True), ("mixed_fx", True), ("fp64_pipe", False)])
+def test_shared_interactions_are_reported(precision, shared):
+    """FEDVR grids of one element size and count parity: pieces of the longest one."""
+    from codyfortran_gb300.engine import Batch
+    specs = []
+    for n in (12, 20, 16):
+        q = _spec("helium")
+        q.n_elements, q.xmin, q.xmax = n, -1.0 * n, 1.0 * n
+        specs.append(q)
+    b = Batch(specs, precision, max_krylov=4)
+    n = b.shared_interactions()
+    b.close()
+    assert n == (1 if shared else 0)
