@@ -409,9 +409,9 @@ struct cgpu_ctx {
   std::string lastError;
   long launches = 0;  // kernels launched by this context (since the last reset)
   MixedBufs* mixed = nullptr;
-  // the contractions as digit slices on the tensor cores: mixed_fx / mixed_fx6, and the FP64 form unless its
-  // digit planes (14 bytes per interaction matrix entry) leave no room for the context (choose_fixed_point)
-  int fxOn = 0;
+  // the contractions as digit slices on the tensor cores (fxOn): mixed_fx / mixed_fx6, and the FP64 form with
+  // fx64 slices (build_ctx, fx_slices_fp64).  fx64 also serves FillH2 of the mixed forms; 0: the FP64 pipe.
+  int fxOn = 0, fx64 = 0;
   z_t* sysTmp_d = nullptr;  // three nG-point vectors of the Sys* entry points (first use)
   McAdjoint* mcAdj = nullptr;  // MCTDHF pulse gradient: checkpoints and work buffers (first use)
   // profiling: CUDA events around every launch of one kernel family

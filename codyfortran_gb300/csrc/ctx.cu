@@ -347,7 +347,7 @@ size_t layout(cgpu_ctx* c, char* base) {
   Z(c->h1_d, nO2);
   Z(c->rdm2_d, nO4);
   Z(c->h2_d, nO4);
-  if (!c->fxOn) {
+  if (!c->fx64) {
     Z(c->S_d, nG * P);
     Z(c->W_d, nG * P);
     Z(c->Sfull_d, nG * Q);
@@ -437,6 +437,34 @@ void detect_shared_interaction(cgpu_ctx* c) {
   c->fxKgMax = kgMax;
 }
 
+// Digit slices that carry the operands of the FP64 form's contractions with an error no
+// larger than FP64 sums have, 0 where there are no kernels with so many.
+//
+// A slice product is exact; what is lost is each operand's rounding, 2^-8L of its row's
+// maximum, and the levels below the L-th, about as much.  With the interaction between
+// V(0) and V(longest distance), R = V(0) / V(longest), a potential (V |S|)(x) is at least
+// V(longest) sum |S|, so those losses stay below about 2^-8L R sqrt(points) of it, whatever
+// the source; the same bound holds for h2 = S^T W, as |W| and its own rounding are bounded
+// by V |S| too.  FP64 sums lose 2^-53 times a factor of the same kind.  Worst point of W
+// relative to V |S| (seven sources from one point to the whole box; FP64 summed in order, 7,
+// 8, 9 slices):
+//   2801 points, R = 800 = 2^9.6       5e-15  1e-12  5e-15  9e-17
+//   2801 points, R = 8000 = 2^13       5e-15  9e-12  4e-14  2e-16
+//   2801 points, R = 80000 = 2^16.3    4e-15  8e-11  3e-13  2e-15
+// so eight up to R = 2^10, nine up to 2^16.
+int fx_slices_fp64(const cgpu_ctx* c) {
+  double R = 1.0;
+  for (const SysHost& s : c->sys) {
+    if (!(s.intS2 >= 0.0) || !(s.intDamp >= 0.0)) return 0;  // decreasing with the distance otherwise
+    const double d = s.nG < 2 ? 0.0 : s.intToeplitz ? (s.nG - 1) * (s.x[1] - s.x[0]) : s.x.back() - s.x.front();
+    const double v0 = std::fabs(soft_kernel(s.intS, s.intS1, s.intS2, s.intDamp, 0.0));
+    const double v1 = std::fabs(soft_kernel(s.intS, s.intS1, s.intS2, s.intDamp, d));
+    if (s.intS != 0.0) R = std::max(R, v0 / v1);
+    if (!(R <= 65536.0)) return 0;
+  }
+  return R <= 1024.0 ? 8 : 9;
+}
+
 void build_ctx(cgpu_ctx* c, const cgpu_desc* descs, int nSys) {
   const cgpu_desc* d0 = &descs[0];
   if (d0->n_body_types < 1 || d0->n_body_types > CODY_MAX_BT) throw std::string("method.mb.nBodyTypes out of range");
@@ -497,8 +525,9 @@ void build_ctx(cgpu_ctx* c, const cgpu_desc* descs, int nSys) {
     c->lzBlocksCap = (int)std::max<size_t>(1, std::min(need, (size_t)2 * c->lzBlocks));
   }
   size_t total = 0;
-  auto size_up = [&](int fx) {
+  auto size_up = [&](int fx, int fx64) {
     c->fxOn = fx;
+    c->fx64 = fx64;
     detect_shared_interaction(c);
     c->lzBlocks = c->lzBlocksCap;
     c->partialCap = std::max({lanczos_partial_need(c), gram_partial_need(c, c->nOS), zgemm_partial_need(c),
@@ -508,16 +537,18 @@ void build_ctx(cgpu_ctx* c, const cgpu_desc* descs, int nSys) {
     total = c->bs * (size_t)nSys + mixed_outside_bytes(c);
   };
   // The contractions run as digit slices in both fixed-point forms.  In the FP64
-  // form they do too (28 slice products on the tensor cores against the FP64
-  // pipe, 12 to 40 times slower on every shape measured), unless the caller asks for
-  // the FP64 pipe or the slices' larger footprint takes more than three quarters of
+  // form they do too (36 or 45 slice products on the tensor cores against the FP64
+  // pipe, several times slower on every shape measured), unless the caller asks for
+  // the FP64 pipe, the interaction's range needs more slices than there are kernels
+  // for (fx_slices_fp64) or the slices' larger footprint takes more than three quarters of
   // the device (the rest is for what is allocated on first use).  That is a matter of
   // the sizes, not of what else the device holds; only a context that would fail for
   // want of memory takes the FP64-pipe kernels because of it, as
   // cgpu_contraction_slices tells.
   const bool fxForm = d0->precision == CGPU_PREC_MIXED_FX || d0->precision == CGPU_PREC_MIXED_FX6;
-  bool slices = d0->precision == CGPU_PREC_FP64 && c->hasInteraction && c->method != CGPU_METHOD_TDCI;
-  size_up(fxForm || slices);
+  const int fx64 = c->hasInteraction ? fx_slices_fp64(c) : 0;
+  bool slices = d0->precision == CGPU_PREC_FP64 && fx64 > 0 && c->method != CGPU_METHOD_TDCI;
+  size_up(fxForm || slices, fxForm || slices ? fx64 : 0);
   if (slices) {
     size_t freeB = 0, totB = 0;
     CODY_CUDA(cudaMemGetInfo(&freeB, &totB));
@@ -531,7 +562,7 @@ void build_ctx(cgpu_ctx* c, const cgpu_desc* descs, int nSys) {
     }
     if (!slices) {
       mixed_free(c);
-      size_up(0);
+      size_up(0, 0);
     }
   }
   total = c->bs * (size_t)nSys;

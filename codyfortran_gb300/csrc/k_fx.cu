@@ -87,7 +87,8 @@ using namespace tcdev;
 
 constexpr int FX_SMEM_MAX = 232448;
 
-constexpr int FX_CHUNK = 4;  // 64-wide K blocks per accumulation in tensor memory (K = 256)
+// 64-wide K blocks per accumulation in tensor memory: K = 256, in the FP64 form 128
+__host__ __device__ constexpr int fx_chunk(int L) { return L > 6 ? 2 : 4; }
 
 template <int BN, int L, int NA_, int NB_>
 struct FxCfg {
@@ -109,10 +110,11 @@ struct FxCfg {
 
 // The level sums of one output over its chunks as integers: T = sum_l D_l
 // 256^(L-1-l).  L <= 5 fits 64 bits (|D_0| <= 2^22 a chunk: below 2^63 for 512
-// chunks, which fx_min_splits keeps); longer ones are held as hi 2^24 + lo.
+// chunks, which fx_min_splits keeps); longer ones are held as hi 256^(L - LH) + lo
+// (L = 9: lo of five levels of at most 9 2^21 a chunk is below 2^56 a chunk, 2^63 for 128).
 template <int L>
 struct FxAcc {
-  static constexpr int LH = L <= 5 ? L : L - 3;  // levels in hi
+  static constexpr int LH = L <= 5 ? L : L == 6 ? 3 : 4;  // levels in hi
   long long hi, lo;
   __device__ __forceinline__ void clear() { hi = lo = 0; }
   // levels [l0, l0 + n) of column j
@@ -164,8 +166,9 @@ __device__ __forceinline__ double ll_scaled(long long T, int e) {
 
 template <int L>
 __device__ __forceinline__ double FxAcc<L>::value(int e) const {
-  // hi and lo are exact as doubles (hi < 2^53 for 128 chunks), so the fma is the one rounding
-  if constexpr (L > 5) return d_scaled(fma((double)hi, 16777216.0, (double)lo), e);
+  // hi is exact as a double (below 2^46 a chunk), lo too unless its top levels add up to a
+  // million times the last one, so the fma is the one rounding that counts
+  if constexpr (L > 5) return d_scaled(fma((double)hi, (double)(1ll << (8 * (L - LH))), (double)lo), e);
   else return ll_scaled(hi, e);
 }
 
@@ -199,7 +202,7 @@ __global__ void __launch_bounds__(32 * (EW + 2), NA_ > 0 ? 2 : 1)
               unsigned* __restrict__ maxCol, TRAJ_ARGS, int gemmId, int segPitchA, int aShared, int kPer,
               const FxTile* __restrict__ tiles, int nTiles, int* __restrict__ err) {
   using C = FxCfg<BN, L, NA_, NB_>;
-  constexpr int NA = C::NA, NB = C::NB, CB = 8;
+  constexpr int NA = C::NA, NB = C::NB, CB = 8, CH = fx_chunk(L);
   static_assert(EW % 4 == 0 && BN % CB == 0, "epilogue warps / column batch");
   constexpr int NBAT = (BN / CB + EW / 4 - 1) / (EW / 4);  // column batches of one epilogue warp
   constexpr uint32_t HALF = C::TMEM_COLS / 2;
@@ -316,7 +319,7 @@ __global__ void __launch_bounds__(32 * (EW + 2), NA_ > 0 ? 2 : 1)
           id1[i] = cols > n0 ? base | ((uint32_t)((cols - n0) >> 3) << 17) : 0u;
         }
         for (int kb = 0; kb < nk && ok; kb++) {
-          const bool first = kb % FX_CHUNK == 0;
+          const bool first = kb % CH == 0;
           if (first) {  // a new phase: its half (or both) drained by the epilogue
             if ((ph > 1 && !mbar_wait(&accEmpty[ph & 1], ((ph >> 1) - 1) & 1, &abortFlag)) ||
                 (ph > 0 && !(narrow && prevNarrow) &&
@@ -373,7 +376,7 @@ __global__ void __launch_bounds__(32 * (EW + 2), NA_ > 0 ? 2 : 1)
           }
           if (!ok) break;
           umma_commit(&bEmpty[sb]);
-          if (kb % FX_CHUNK == FX_CHUNK - 1 || kb == nk - 1) {
+          if (kb % CH == CH - 1 || kb == nk - 1) {
             umma_commit(&accFull[ph & 1]);
             ph++;
           }
@@ -406,7 +409,7 @@ __global__ void __launch_bounds__(32 * (EW + 2), NA_ > 0 ? 2 : 1)
 #pragma unroll
         for (int j = 0; j < CB; j++) T[bt][j].clear();
       bool waited = true;
-      for (int k0 = 0; k0 < nk; k0 += FX_CHUNK) {
+      for (int k0 = 0; k0 < nk; k0 += CH) {
         waited = mbar_wait(&accFull[ph & 1], (ph >> 1) & 1, &abortFlag);
         if (__any_sync(0xffffffffu, !waited)) {
           waited = false;
@@ -418,20 +421,17 @@ __global__ void __launch_bounds__(32 * (EW + 2), NA_ > 0 ? 2 : 1)
         for (int bt = 0; bt < NBAT; bt++) {
           const int c = (cg + bt * (EW / 4)) * CB;
           if (c < tl.nT) {
-            // the levels of hi, then those of lo (registers for one group at a time)
-            constexpr int LH = FxAcc<L>::LH;
-            uint32_t d[LH][CB];
+            // registers for one group of levels at a time
+            constexpr int G = L <= 5 ? L : L == 6 ? 3 : 4;
 #pragma unroll
-            for (int l = 0; l < LH; l++) TMEM_LD_X8(tcol + (uint32_t)(l * tl.nT + c), d[l]);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            for (int l0 = 0; l0 < L; l0 += G) {
+              uint32_t d[G][CB];
 #pragma unroll
-            for (int j = 0; j < CB; j++) T[bt][j].add(d, j, 0, LH);
-            if constexpr (L > LH) {
-#pragma unroll
-              for (int l = LH; l < L; l++) TMEM_LD_X8(tcol + (uint32_t)(l * tl.nT + c), d[l - LH]);
+              for (int l = 0; l < G; l++)
+                if (l0 + l < L) TMEM_LD_X8(tcol + (uint32_t)((l0 + l) * tl.nT + c), d[l]);
               asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-              for (int j = 0; j < CB; j++) T[bt][j].add(d, j, LH, L - LH);
+              for (int j = 0; j < CB; j++) T[bt][j].add(d, j, l0, L - l0);
             }
           }
         }
@@ -530,8 +530,8 @@ struct FxTileCfg {
 };
 static const FxTileCfg kFxTiles[] = {{32, 4, false}, {64, 4, false}, {96, 4, false},
                                      {32, 5, false}, {64, 5, false}, {80, 5, false}, {96, 5, false},
-                                     {32, 6, false}, {64, 6, false}, {64, 7, false}, {32, 4, true},  {64, 4, true},  {32, 5, true},
-                                     {48, 5, true}};
+                                     {32, 6, false}, {64, 6, false}, {64, 8, false}, {48, 9, false}, {32, 4, true}, {64, 4, true},
+                                     {32, 5, true},  {48, 5, true}};
 
 static int fx_max_bn(int L, bool compact) {
   int m = 0;
@@ -554,8 +554,12 @@ bool fx_tile_supported(int bn, int L, bool compact) {
   return false;
 }
 
-// 512 chunks (K = 131072) keep the integer level sums inside 64 bits.
-int fx_min_splits(int kTiles) { return std::max(1, (kTiles + 512 * FX_CHUNK - 1) / (512 * FX_CHUNK)); }
+// 512 chunks (K = 131072), in the FP64 form 128 (K = 16384), keep the integer level sums
+// inside 64 bits.
+int fx_min_splits(int kTiles, int L) {
+  const int most = (L > 6 ? 128 : 512) * fx_chunk(L);
+  return std::max(1, (kTiles + most - 1) / most);
+}
 
 int fx_normalize_splits(int kTiles, int s) {
   s = std::max(1, std::min(s, kTiles));
@@ -583,7 +587,7 @@ int fx_tile_n(int N, int L, bool compact) {
 int fx_split_count(int M, int N, int BN, int L, int kTiles, int nb, bool reduceExtra) {
   const int nt = (N + BN - 1) / BN, nT = ((N + nt - 1) / nt + 15) / 16 * 16;
   const long tiles = (long)((M + TC_BM - 1) / TC_BM) * nt * nb;
-  const int lo = fx_min_splits(kTiles);
+  const int lo = fx_min_splits(kTiles, L);
   if (tiles >= 152) return fx_normalize_splits(kTiles, lo);
   int best = lo;
   double bestCost = 1e300;
@@ -647,7 +651,7 @@ void fx_gemm(cgpu_ctx* c, int L, bool compact, int gemmId, const CUtensorMap& ta
     throw std::string("fx_gemm: segment pitch must be a multiple of 64");
   if (nSplit > 1 && (maxRow || maxCol)) throw std::string("fx_gemm: output maxima need an unsplit K");
   const int kTiles = segPitch / TC_BK, kPer = (kTiles + nSplit - 1) / nSplit;  // K blocks per split
-  if (nSplit < fx_min_splits(kTiles)) throw std::string("fx_gemm: K split beyond the range of the level sums");
+  if (nSplit < fx_min_splits(kTiles, L)) throw std::string("fx_gemm: K split beyond the range of the level sums");
   const FxTile* tl = (const FxTile*)tiles;
 #define FX_CASE(BN_, L_, NA_, NB_, CMP_)                                                                        \
   if (bn == BN_ && L == L_ && compact == CMP_) {                                                                \
@@ -657,7 +661,8 @@ void fx_gemm(cgpu_ctx* c, int L, bool compact, int gemmId, const CUtensorMap& ta
   }
   FX_CASE(32, 4, 0, 2, false) FX_CASE(64, 4, 0, 2, false) FX_CASE(96, 4, 0, 2, false)
   FX_CASE(32, 5, 0, 2, false) FX_CASE(64, 5, 0, 2, false) FX_CASE(80, 5, 0, 2, false) FX_CASE(96, 5, 0, 2, false)
-  FX_CASE(32, 6, 0, 2, false) FX_CASE(64, 6, 0, 2, false) FX_CASE(64, 7, 0, 2, false)
+  FX_CASE(32, 6, 0, 2, false) FX_CASE(64, 6, 0, 2, false) FX_CASE(64, 8, 0, 2, false)
+  FX_CASE(48, 9, 0, 2, false)
   FX_CASE(32, 4, 4, 1, true) FX_CASE(64, 4, 4, 1, true)
   FX_CASE(32, 5, 5, 1, true) FX_CASE(48, 5, 5, 1, true)
 #undef FX_CASE

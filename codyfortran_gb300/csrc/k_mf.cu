@@ -577,7 +577,7 @@ void zgemm(cgpu_ctx* c, int mode, const z_t* A, const z_t* B, z_t* C, double sca
 }  // namespace
 
 size_t zgemm_partial_need(const cgpu_ctx* c) {
-  if (c->fxOn) return 0;
+  if (c->fx64) return 0;
   int Q = c->nOS * c->nOS;
   size_t need = 0;
   // ZG_H2 always goes through the partial buffer (scale 1/2); ZG_Z only when split
@@ -681,7 +681,7 @@ void launch_fill_h2(cgpu_ctx* c, const z_t* orbs) {
     batch_zero(c, c->h2_d, sizeof(z_t) * (size_t)c->nO * c->nO * c->nO * c->nO);
     return;
   }
-  if (c->fxOn) return launch_fill_h2_fx(c, orbs);
+  if (c->fx64) return launch_fill_h2_fx(c, orbs);
   launch_pair_potentials(c, orbs);
   expand_pairs(c, orbs, 1);
   h2_from_pairs(c);

@@ -26,13 +26,13 @@
 #include <cuda_bf16.h>
 
 #include <array>
+#include <type_traits>
 
 #include <algorithm>
 
 #include "common.cuh"
 #include "tc.cuh"
 
-constexpr int FX_L64 = 7;  // slices of the FP64 form (55 bits of each row's maximum)
 
 // One fixed-point GEMM: N-tile width, two-CTAs-per-SM configuration, K splits, its tile list.
 struct FxGemm {
@@ -53,13 +53,14 @@ struct MixedBufs {
   double* Zd = nullptr;     // (nG, Q) complex
   CUtensorMap mV, mS, mSasB, mW, mWT, mR;  // TMA maps (A operands box 128 rows, B operands box BN rows)
   // fixed-point forms (L > 0): digit slices of GEMM1 / GEMM3 and of GEMM2 (L2); V
-  // carries FX_L64 slices of which a GEMM reads the first L
+  // carries LV slices of which a GEMM reads the first L
   int L = 0, L2 = 0;
-  FxGemm gW, gZ, gH, gWx, gHx;      // the form's three GEMMs; W and h2 at FX_L64 slices for FillH2
+  int L64 = 0, LV = 0;              // slices of the FP64 form (cgpu_ctx::fx64; 0: FP64 pipe), of V and S: the most of both
+  FxGemm gW, gZ, gH, gWx, gHx;      // the form's three GEMMs; W and h2 at L64 slices for FillH2
   int sCapW = 1, sCapZ = 1, sCapH = 1;  // K splits the FP64 partial buffers hold (the tuner stays within them)
-  FxMaps bS, bWT, bR, bSx, bWTx;    // B operands (x: at FX_L64 slices)
-  CUtensorMap mSxasB;               // S rows as the A operand at FX_L64 slices
-  // one interaction matrix per root grid (cgpu_ctx::fxShared): slices [root][c->nG][FX_L64 KgBig]
+  FxMaps bS, bWT, bR, bSx, bWTx;    // B operands (x: at L64 slices)
+  CUtensorMap mSxasB;               // S rows as the A operand at L64 slices
+  // one interaction matrix per root grid (cgpu_ctx::fxShared): slices [root][c->nG][LV KgBig]
   // and row exponents [root][c->nG], outside the per-trajectory arena
   int KgBig = 0;
   __nv_bfloat16* Vsh = nullptr;
@@ -311,9 +312,9 @@ __global__ void k_reduce_H2(z_t* __restrict__ H2s, const PT* __restrict__ P3, in
 // mixed forms' targets are 30 and 36 bits of the row maxima; at a contraction
 // length of at most 1024 they held 35 and 42 with the 7-bit digits they used to
 // have there (up to 256: 32 and 40), which five or six 8-bit slices keep.
-void fx_slices(int precision, int kTiles, int pTiles, int* L, int* L2) {
+void fx_slices(int precision, int fx64, int kTiles, int pTiles, int* L, int* L2) {
   if (precision == CGPU_PREC_FP64) {
-    *L = *L2 = FX_L64;
+    *L = *L2 = fx64;
   } else {
     const int x6 = precision == CGPU_PREC_MIXED_FX6 ? 1 : 0;
     *L = x6 && kTiles <= 16 ? 6 : 5;
@@ -321,7 +322,7 @@ void fx_slices(int precision, int kTiles, int pTiles, int* L, int* L2) {
   }
 }
 
-// Signed base-256 digits of x relative to 2^e (|x| < 2^(e-1), or < 2^e for L < 7): X = round(x 2^(8L-e))
+// Signed base-256 digits of x relative to 2^e (|x| < 2^(e-1), or < 2^e for L <= 6): X = round(x 2^(8L-e))
 // = sum_i d_i 2^(8(L-1-i)), d_i in [-128, 128) for i > 0, |d_0| <= 128.
 // Integer operations only.  With H = 128 sum_{k<L-1} 256^k, the digits of Y = X + H
 // below the top one are the plain base-256 digits d_i + 128, so every digit is an
@@ -331,22 +332,23 @@ template <int L>
 __device__ __forceinline__ void fx_digits(double x, int e, int (&d)[L]) {
   const unsigned long long u = (unsigned long long)__double_as_longlong(x);
   const int ex = (int)((u >> 52) & 0x7FF);
-  long long X = 0;
+  using Int = std::conditional_t<(L > 7), __int128, long long>;  // |Y| <= 2^(8L - 1) + H
+  Int X = 0;
   if (ex != 0) {
     const unsigned long long mant = (u & 0xFFFFFFFFFFFFFull) | (1ull << 52);
     const int sh = 1075 - ex - 8 * L + e;  // >= 54 - 8L because |x| < 2^(e-1) (53 - 8L: < 2^e)
-    if (8 * L > 53 && sh <= 0) X = (long long)(mant << -sh);
-    else if (sh < 63) X = (long long)((mant + (1ull << (sh - 1))) >> sh);
+    if (8 * L > 53 && sh <= 0) X = (Int)mant << -sh;
+    else if (sh < 63) X = (Int)((mant + (1ull << (sh - 1))) >> sh);
     if (u >> 63) X = -X;
   }
-  constexpr long long H = [] {
-    long long h = 0;
+  constexpr Int H = [] {
+    Int h = 0;
     for (int i = 1; i < L; i++) h = (h << 8) | 128;
     return h;
   }();
-  const long long Y = X + H;
+  const Int Y = X + H;
 #pragma unroll
-  for (int i = 1; i < L; i++) d[i] = (int)((unsigned long long)Y >> (8 * (L - 1 - i)) & 255) - 128;
+  for (int i = 1; i < L; i++) d[i] = (int)(Y >> (8 * (L - 1 - i)) & 255) - 128;
   d[0] = (int)(Y >> (8 * (L - 1)));
 }
 
@@ -409,6 +411,7 @@ __device__ void fx_row(__nv_bfloat16* rowBase, int* expOut, int K, int Kpad, int
 
 constexpr size_t FX_STAGE_MAX = 200 * 1024;  // shared memory for staged rows; longer rows are formed twice
 
+template <int L>
 __global__ void __launch_bounds__(256) k_fx_split_V(__nv_bfloat16* __restrict__ out, int* __restrict__ eV,
                                                      const double* __restrict__ V, int pitch, TRAJ_ARGS) {
   const TrajShape& T = shp[blockIdx.z];
@@ -418,7 +421,7 @@ __global__ void __launch_bounds__(256) k_fx_split_V(__nv_bfloat16* __restrict__ 
   eV = bat(eV, bs);
   V = bat(V, bs);
   const double* row = V + (size_t)g * nG;
-  fx_row<FX_L64>(out + (size_t)g * FX_L64 * pitch, eV + g, nG, (nG + 63) / 64 * 64, pitch, 0, false,
+  fx_row<L>(out + (size_t)g * L * pitch, eV + g, nG, (nG + 63) / 64 * 64, pitch, 0, false,
                  [&](int k) { return row[k]; });
 }
 
@@ -426,7 +429,7 @@ __global__ void __launch_bounds__(256) k_fx_split_V(__nv_bfloat16* __restrict__ 
 // over the grid (p = (l, k)), one block per pair, both rows staged in shared
 // memory, each with the exponent of its own maximum.  In the mixed forms the
 // complex product and the weight are double-float (FP32 pipe; ~2^-44 relative,
-// below the digits' 2^-31 / 2^-39 of the row maximum); with FX_L64 slices they
+// below the digits' 2^-31 / 2^-39 of the row maximum); in the FP64 form they
 // are FP64, rounded as FillInteractionSrc rounds them.  Block 0 of a trajectory
 // also clears the W exponent maxima for GEMM1.
 template <int L>
@@ -455,7 +458,7 @@ __global__ void __launch_bounds__(256) k_fx_split_S(__nv_bfloat16* __restrict__ 
   const z_t* bo = orbs + (size_t)nG * pk[p];
   auto value = [&](int g) -> z_t {
     const z_t av = a[g], bv = bo[g];
-    if (L == FX_L64) return zscale(zcmul(av, bv), w[g]);
+    if (L > 6) return zscale(zcmul(av, bv), w[g]);
     const float2 ar = df_split(av.x), ai = df_split(av.y), br = df_split(bv.x), bi = df_split(bv.y);
     const float2 wg = df_split(w[g]);
     // conj(a) b = (ar br + ai bi) + i (ar bi - ai br)
@@ -510,7 +513,7 @@ __global__ void k_fx_split_R(__nv_bfloat16* __restrict__ out, int* __restrict__ 
   pl = bat(pl, bs);
   pk = bat(pk, bs);
   const int q = row >> 1, s = row & 1;
-  fx_row<L>(out + (size_t)row * L * pitch, eR + row, 2 * nP, T.Kp, pitch, 1, L < FX_L64, [&](int k) {
+  fx_row<L>(out + (size_t)row * L * pitch, eR + row, 2 * nP, T.Kp, pitch, 1, L <= 6, [&](int k) {
     const int p = k >> 1, t = k & 1;
     const int l = pl[p], kk = pk[p];
     const z_t R1 = Rp[(size_t)(l * n + kk) * Q + q];
@@ -578,7 +581,7 @@ __global__ void __launch_bounds__(THREADS) k_fx_split_W(__nv_bfloat16* __restric
     for (int r = warp; r < FW_T; r += THREADS / 32) {
       const int g = c0 + r - sh;
       if (g < 0 || g >= nG) continue;
-      const int e = fx_exp(mWr[g], L2 < FX_L64);
+      const int e = fx_exp(mWr[g], L2 <= 6);
       if (n0 == 0 && lane == 0) eWr[g] = e;
       fx_store2<L2>(WxA + (size_t)g * L2 * pitchP, pitchP, n0 + 2 * lane, tile[r][2 * lane], tile[r][2 * lane + 1], e);
     }
@@ -613,8 +616,10 @@ size_t mixed_layout(cgpu_ctx* c, char* base, size_t off) {
   if (c->fxOn) {
     m->KgMax = c->fxKgMax;  // includes the K-tile offsets of a shared interaction matrix
     const int kg = m->KgMax / 64, kp = m->KpMax / 64;
-    fx_slices(c->precision, kg, kp, &m->L, &m->L2);
-    const int L = m->L, L2 = m->L2;
+    fx_slices(c->precision, c->fx64, kg, kp, &m->L, &m->L2);
+    m->L64 = c->fx64;
+    m->LV = std::max(m->L, m->L64);
+    const int L = m->L, L2 = m->L2, L64 = m->L64, LV = m->LV;
     auto plan = [&](FxGemm& g, int Lg, int M, int N, int kTiles, bool compact, bool extra) {
       g.compact = compact;
       g.bn = fx_tile_n(N, Lg, compact);
@@ -623,19 +628,21 @@ size_t mixed_layout(cgpu_ctx* c, char* base, size_t off) {
     plan(m->gW, L, nG, 2 * nP, kg, false, true);
     plan(m->gZ, L2, nG, 2 * Q, kp, c->nb > 1 && fx_compact_ok(L2), true);
     plan(m->gH, L, 2 * nP, 2 * nP, kg, false, false);
-    plan(m->gWx, FX_L64, nG, 2 * nP, kg, false, true);
-    plan(m->gHx, FX_L64, 2 * nP, 2 * nP, kg, false, false);
+    if (L64) {
+      plan(m->gWx, L64, nG, 2 * nP, kg, false, true);
+      plan(m->gHx, L64, 2 * nP, 2 * nP, kg, false, false);
+    }
     // partial buffers: a single system of a tunable form holds twice the
     // heuristic's K splits (room for the tile tuner), else exactly the heuristic's
-    const int grow = c->nb == 1 && L != FX_L64 ? 2 : 1;
+    const int grow = c->nb == 1 && L != L64 ? 2 : 1;
     m->sCapW = std::max(std::min(m->gW.s * grow, kg), m->gWx.s);
     m->sCapZ = std::min(m->gZ.s * grow, kp);
     m->sCapH = std::max(std::min(m->gH.s * grow, kg), m->gHx.s);
     const size_t perTrajV = c->fxShared ? 0 : 1;
-    size_t oV = take(off, perTrajV * sizeof(bf) * (size_t)nG * FX_L64 * m->KgMax);
-    size_t oS = take(off, sizeof(bf) * (size_t)2 * nP * FX_L64 * m->KgMax);
+    size_t oV = take(off, perTrajV * sizeof(bf) * (size_t)nG * LV * m->KgMax);
+    size_t oS = take(off, sizeof(bf) * (size_t)2 * nP * LV * m->KgMax);
     size_t oW = take(off, sizeof(bf) * (size_t)nG * L2 * m->KpMax);
-    size_t oWT = take(off, sizeof(bf) * (size_t)2 * nP * FX_L64 * m->KgMax);
+    size_t oWT = take(off, sizeof(bf) * (size_t)2 * nP * LV * m->KgMax);
     size_t oR = take(off, sizeof(bf) * (size_t)2 * Q * L2 * m->KpMax);
     size_t oWd = take(off, sizeof(double) * (size_t)m->sCapW * nG * 2 * nP);
     size_t oZp = take(off, m->sCapZ > 1 ? sizeof(double) * (size_t)m->sCapZ * nG * 2 * Q : 0);
@@ -700,9 +707,9 @@ size_t mixed_layout(cgpu_ctx* c, char* base, size_t off) {
 }
 
 size_t mixed_outside_bytes(const cgpu_ctx* c) {
-  if (!c->fxOn || !c->fxShared) return 0;
+  if (!c->fxOn || !c->fxShared || !c->mixed) return 0;
   const size_t kgBig = (c->nG + 63) / 64 * 64;
-  return c->fxRoots.size() * (size_t)c->nG * (FX_L64 * kgBig * sizeof(__nv_bfloat16) + sizeof(int));
+  return c->fxRoots.size() * (size_t)c->nG * (c->mixed->LV * kgBig * sizeof(__nv_bfloat16) + sizeof(int));
 }
 
 bool mixed_alloc_outside(cgpu_ctx* c) {
@@ -710,7 +717,7 @@ bool mixed_alloc_outside(cgpu_ctx* c) {
   if (!m || mixed_outside_bytes(c) == 0) return true;
   const size_t rows = (size_t)c->nG * c->fxRoots.size();
   m->KgBig = (c->nG + 63) / 64 * 64;
-  return cudaMalloc(&m->Vsh, sizeof(__nv_bfloat16) * rows * FX_L64 * m->KgBig) == cudaSuccess &&
+  return cudaMalloc(&m->Vsh, sizeof(__nv_bfloat16) * rows * m->LV * m->KgBig) == cudaSuccess &&
          cudaMalloc(&m->eVsh, sizeof(int) * rows) == cudaSuccess;
 }
 
@@ -740,38 +747,41 @@ void mixed_init(cgpu_ctx* c) {
   }
   const int P2 = 2 * c->nPairs, Q2 = 2 * c->nOS * c->nOS;
   if (m->L) {
-    const int L = m->L, pV = FX_L64 * m->KgMax, pG = L * m->KgMax, pP = m->L2 * m->KpMax;
+    const int L = m->L, L64 = m->L64, LV = m->LV, pV = LV * m->KgMax, pG = L * m->KgMax, pP = m->L2 * m->KpMax;
+    auto splitV = LV == 9 ? k_fx_split_V<9> : LV == 8 ? k_fx_split_V<8> : LV == 6 ? k_fx_split_V<6> : k_fx_split_V<5>;
     if (c->fxShared) {
       // each root trajectory's interaction matrix, sliced once for the batch
       const int nR = (int)c->fxRoots.size();
-      const size_t plane = (size_t)c->nG * FX_L64 * m->KgBig;  // elements per root
+      const size_t plane = (size_t)c->nG * LV * m->KgBig;  // elements per root
       CODY_CUDA(cudaMemsetAsync(m->Vsh, 0, sizeof(__nv_bfloat16) * plane * nR, c->stream));
       for (int r = 0; r < nR; r++) {
         const int root = c->fxRoots[r], nGb = c->sys[root].nG;
         const double* Vb = (const double*)((const char*)c->Vint_d + (size_t)root * c->bs);
-        k_fx_split_V<<<dim3(nGb, 1, 1), 256, 0, c->stream>>>(m->Vsh + plane * r, m->eVsh + (size_t)c->nG * r, Vb,
+        splitV<<<dim3(nGb, 1, 1), 256, 0, c->stream>>>(m->Vsh + plane * r, m->eVsh + (size_t)c->nG * r, Vb,
                                                              m->KgBig, c->shape_d + root, 0);
         CODY_LAUNCHED(c);
       }
-      m->mVsh = tc_make_map_planes(m->Vsh, c->nG, FX_L64 * m->KgBig, 128, nR, sizeof(__nv_bfloat16) * plane);
+      m->mVsh = tc_make_map_planes(m->Vsh, c->nG, LV * m->KgBig, 128, nR, sizeof(__nv_bfloat16) * plane);
     } else {
-      k_fx_split_V<<<dim3(c->nG, 1, c->nb), 256, 0, c->stream>>>(m->VxB, m->eV, c->Vint_d, m->KgMax, TRAJ_PASS(c));
+      splitV<<<dim3(c->nG, 1, c->nb), 256, 0, c->stream>>>(m->VxB, m->eV, c->Vint_d, m->KgMax, TRAJ_PASS(c));
       CODY_LAUNCHED(c);
       m->mV = tc_make_map(c, m->VxB, c->nG, pV, 128);
     }
     m->mSasB = tc_make_map(c, m->SxA, P2, pG, 128);
-    m->mSxasB = tc_make_map(c, m->SxA, P2, pV, 128);
     m->mW = tc_make_map(c, m->WxA, c->nG, pP, 128);
     m->bS = fx_make_maps(c, m->SxA, P2, m->KgMax, L);
-    m->bSx = fx_make_maps(c, m->SxA, P2, m->KgMax, FX_L64);
     m->bWT = fx_make_maps(c, m->WTxB, P2, m->KgMax, L);
-    m->bWTx = fx_make_maps(c, m->WTxB, P2, m->KgMax, FX_L64);
     m->bR = fx_make_maps(c, m->RxB, Q2, m->KpMax, m->L2);
     auto tiles = [&](FxGemm& g, int id) { g.tiles = fx_build_tiles(c, id, g.bn, g.s, &g.nTiles); };
     tiles(m->gW, TC_GEMM_W);
     tiles(m->gZ, TC_GEMM_Z);
     tiles(m->gH, TC_GEMM_H2);
-    if (L != FX_L64) {  // the FP64 form's FillH2 uses its own gW, gH
+    if (L64) {
+      m->mSxasB = tc_make_map(c, m->SxA, P2, L64 * m->KgMax, 128);
+      m->bSx = fx_make_maps(c, m->SxA, P2, m->KgMax, L64);
+      m->bWTx = fx_make_maps(c, m->WTxB, P2, m->KgMax, L64);
+    }
+    if (L64 && L != L64) {  // the FP64 form's FillH2 uses its own gW, gH
       tiles(m->gWx, TC_GEMM_W);
       tiles(m->gHx, TC_GEMM_H2);
     }
@@ -796,14 +806,14 @@ int mixed_error(cgpu_ctx* c) { return c->mixed && c->mixed->err_h ? *c->mixed->e
 
 // The three fixed-point contractions with their K-split reductions, on the
 // operands the digit splits left in the arena (one call = one launch of the
-// GEMM, plus the reduction when K is split).  exact: FX_L64 slices (FillH2).
+// GEMM, plus the reduction when K is split).  exact: L64 slices (FillH2).
 // W = V S (pair potentials; row / column exponent maxima for the W split).
 static void fx_run_W(cgpu_ctx* c, bool exact) {
   MixedBufs* m = c->mixed;
   const int nG = c->nG, nP = c->nPairs;
-  const FxGemm& g = exact && m->L != FX_L64 ? m->gWx : m->gW;
+  const FxGemm& g = exact && m->L != m->L64 ? m->gWx : m->gW;
   const bool one = g.s == 1;
-  fx_gemm(c, exact ? FX_L64 : m->L, g.compact, TC_GEMM_W, c->fxShared ? m->mVsh : m->mV, exact ? m->bSx : m->bS, g.bn,
+  fx_gemm(c, exact ? m->L64 : m->L, g.compact, TC_GEMM_W, c->fxShared ? m->mVsh : m->mV, exact ? m->bSx : m->bS, g.bn,
           m->Wd, c->fxShared ? m->eVsh : m->eV, m->eS, one ? m->mWr : nullptr, one ? m->mWc : nullptr,
           c->fxShared ? m->KgBig : m->KgMax, m->KgMax, c->fxShared, g.s, g.tiles, g.nTiles, m->err);
   if (!one) {
@@ -830,8 +840,8 @@ static void fx_run_Z(cgpu_ctx* c) {
 static void fx_run_H2(cgpu_ctx* c, bool exact) {
   MixedBufs* m = c->mixed;
   const int Q = c->nOS * c->nOS;
-  const FxGemm& g = exact && m->L != FX_L64 ? m->gHx : m->gH;
-  fx_gemm(c, exact ? FX_L64 : m->L, g.compact, TC_GEMM_H2, exact ? m->mSxasB : m->mSasB, exact ? m->bWTx : m->bWT, g.bn,
+  const FxGemm& g = exact && m->L != m->L64 ? m->gHx : m->gH;
+  fx_gemm(c, exact ? m->L64 : m->L, g.compact, TC_GEMM_H2, exact ? m->mSxasB : m->mSasB, exact ? m->bWTx : m->bWT, g.bn,
           m->Gd, m->eS, m->eWc, nullptr, nullptr, m->KgMax, m->KgMax, 0, g.s, g.tiles, g.nTiles, m->err);
   k_reduce_H2<<<bgrid(c, ew_blocks(c, (size_t)Q * Q)), 256, 0, c->stream>>>(c->h2s_d, m->Gd, g.s, c->pidx_d,
                                                                       TRAJ_PASS(c));
@@ -878,7 +888,7 @@ const char* fx_tiles_refused(const cgpu_ctx* c, const int* t) {
     if (t[3 * g + 2] < 1 || t[3 * g + 2] > kTiles) return "tiles: K split count outside 1..K blocks";
     const int s = fx_normalize_splits(kTiles, t[3 * g + 2]);
     // every split keeps at least two K blocks, as the set-up heuristic does
-    if (s < fx_min_splits(kTiles) || s > cap || (s > 1 && s > kTiles / 2))
+    if (s < fx_min_splits(kTiles, g == TC_GEMM_Z ? m->L2 : m->L) || s > cap || (s > 1 && s > kTiles / 2))
       return "tiles: K split outside the range of the level sums or the partial buffers";
   }
   return nullptr;
@@ -913,7 +923,7 @@ void fx_tile_candidates(const cgpu_ctx* c, int g, std::vector<std::array<int, 3>
   std::vector<int> splits;
   for (int s : {1, 2, 3, 4, cap}) {
     int v = fx_normalize_splits(kTiles, s);
-    if (v >= fx_min_splits(kTiles) && v <= cap && (v == 1 || v <= kTiles / 2) &&
+    if (v >= fx_min_splits(kTiles, g == TC_GEMM_Z ? c->mixed->L2 : c->mixed->L) && v <= cap && (v == 1 || v <= kTiles / 2) &&
         std::find(splits.begin(), splits.end(), v) == splits.end())
       splits.push_back(v);
   }
@@ -972,7 +982,8 @@ static void fx_potentials(cgpu_ctx* c, const z_t* orbs, bool exact, bool wantW) 
 template <class F>
 static void fx_plan(const cgpu_ctx* c, F f) {
   const int L = c->mixed->L, L2 = c->mixed->L2;
-  if (L == FX_L64) return f(std::integral_constant<int, FX_L64>(), std::integral_constant<int, FX_L64>());
+  if (L == 8) return f(std::integral_constant<int, 8>(), std::integral_constant<int, 8>());
+  if (L == 9) return f(std::integral_constant<int, 9>(), std::integral_constant<int, 9>());
   if (L == 5 && L2 == 4) return f(std::integral_constant<int, 5>(), std::integral_constant<int, 4>());
   if (L == 5 && L2 == 5) return f(std::integral_constant<int, 5>(), std::integral_constant<int, 5>());
   if (L == 5 && L2 == 6) return f(std::integral_constant<int, 5>(), std::integral_constant<int, 6>());
@@ -1053,7 +1064,8 @@ static void correlation_fx(cgpu_ctx* c, z_t* dOrbs, const z_t* orbs, int wantH2)
 }
 
 void launch_fill_h2_fx(cgpu_ctx* c, const z_t* orbs) {
-  fx_potentials<FX_L64, FX_L64>(c, orbs, true, false);
+  if (c->fx64 == 9) fx_potentials<9, 9>(c, orbs, true, false);
+  else fx_potentials<8, 8>(c, orbs, true, false);
   ProfScope prof(c, CGPU_KERNEL_H2);
   fx_run_H2(c, true);
   launch_h2_layout(c);

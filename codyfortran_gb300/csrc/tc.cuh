@@ -59,12 +59,12 @@ int fx_tile_n(int N, int L, bool compact);
 bool fx_compact_ok(int L);
 // Version of the fixed-point GEMM that timings of its tiles belong to: raised when its
 // configurations or what they cost change.
-constexpr int FX_VERSION = 2;
+constexpr int FX_VERSION = 3;
 // The instantiated (N tile width, compact) configurations for L slices.
 void fx_tile_configs(int L, std::vector<std::pair<int, bool>>& out);
 bool fx_tile_supported(int bn, int L, bool compact);
 // Fewest K splits that keep the level sums of every split inside their integers.
-int fx_min_splits(int kTiles);
+int fx_min_splits(int kTiles, int L);
 // The split count fx_gemm runs for a request of s splits (balanced K blocks per split).
 int fx_normalize_splits(int kTiles, int s);
 // K splits of the fixed-point GEMM for kTiles 64-wide K blocks (reduceExtra:
