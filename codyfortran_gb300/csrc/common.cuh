@@ -392,7 +392,7 @@ struct cgpu_ctx {
   cudaStream_t stream = nullptr;
   // the branches of the equation of motion beside `stream` (ctx.cu: td_device)
   cudaStream_t side[2] = {nullptr, nullptr};
-  cudaEvent_t branchEv[5] = {};
+  cudaEvent_t branchEv[6] = {};
   cudaGraphExec_t stepGraph = nullptr;
   double graphDt = 0;
   int graphKrylov = 0, graphMetric = -1, graphKernels = 0, graphProf = 0;
@@ -619,7 +619,7 @@ size_t lanczos_partial_need(const cgpu_ctx* c);
   } while (0)
 
 // The branches' events, and launches on another stream than the context's.
-enum { BR_START, BR_DENSITY, BR_ONEBODY, BR_POTENTIALS, BR_COEFFS };
+enum { BR_START, BR_SOURCES, BR_DENSITY, BR_ONEBODY, BR_POTENTIALS, BR_COEFFS };
 inline void branch_record(cgpu_ctx* c, int e) { CODY_CUDA(cudaEventRecord(c->branchEv[e], c->stream)); }
 inline void branch_wait(cgpu_ctx* c, int e) { CODY_CUDA(cudaStreamWaitEvent(c->stream, c->branchEv[e], 0)); }
 struct BranchStream {

@@ -760,6 +760,7 @@ void td_device(cgpu_ctx* c, int which, z_t* out, const z_t* in, double t, z_t po
       wait(BR_START);
       launch_ci_rdm(c, C, 1, 1);
       launch_rdm_inverse(c);
+      wait(BR_SOURCES);
       launch_fx_split_R(c);
       record(BR_DENSITY);
     }

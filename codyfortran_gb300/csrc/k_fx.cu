@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(32 * (EW + 2), NA_ > 0 ? 2 : 1)
     k_fx_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ FxMaps tB, double* __restrict__ out,
               const int* __restrict__ expA, const int* __restrict__ expB, unsigned* __restrict__ maxRow,
               unsigned* __restrict__ maxCol, TRAJ_ARGS, int gemmId, int segPitchA, int aShared, int kPer,
-              const FxTile* __restrict__ tiles, int nTiles, int* __restrict__ err) {
+              const FxTile* __restrict__ tiles, int nTiles, int* __restrict__ err, const int* __restrict__ colScale) {
   using C = FxCfg<BN, L, NA_, NB_>;
   constexpr int NA = C::NA, NB = C::NB, CB = 8, CH = fx_chunk(L);
   static_assert(EW % 4 == 0 && BN % CB == 0, "epilogue warps / column batch");
@@ -464,12 +464,14 @@ __global__ void __launch_bounds__(32 * (EW + 2), NA_ > 0 ? 2 : 1)
               v[j] = T[bt][j].value(e);
               if (e > FX_EXP_NAN / 2) v[j] = __longlong_as_double(0x7FF8000000000000LL);
               ex = (unsigned)(__double2hiint(v[j]) >> 20) & 0x7FFu;
+              // the FP64 form: the row's maximum over the scaled columns (fx_scale_key)
+              if (L > 6 && colScale) rowMaxEx = max(rowMaxEx, fx_scale_key(ex, -batn(colScale, bs, tl.traj)[col]));
+              else rowMaxEx = max(rowMaxEx, ex);
             }
             if (maxCol) {
               unsigned m = __reduce_max_sync(0xffffffffu, ex);
               if (lane == 0 && m) atomicMax(batn(maxCol, bs, tl.traj) + col, m);
             }
-            rowMaxEx = max(rowMaxEx, ex);
           }
           if (rowOk) {
             double* dst = Oz + (size_t)row * N + tl.n0 + c;
@@ -502,7 +504,7 @@ __global__ void __launch_bounds__(32 * (EW + 2), NA_ > 0 ? 2 : 1)
 template <int BN, int L, int NA_, int NB_>
 void launch_fx_t(cgpu_ctx* c, const CUtensorMap& ta, const FxMaps& tb, double* out, const int* expA,
                  const int* expB, unsigned* maxRow, unsigned* maxCol, int gemmId, int segPitchA, int aShared, int kPer,
-                 const FxTile* tiles, int nTiles, int ctasPerSm, int* err) {
+                 const FxTile* tiles, int nTiles, int ctasPerSm, int* err, const int* colScale) {
   using C = FxCfg<BN, L, NA_, NB_>;
   // eight epilogue warps (two per tensor-memory lane quarter); sixteen for L >
   // 5, whose two 64-bit sums per output would not fit the registers of eight
@@ -516,7 +518,7 @@ void launch_fx_t(cgpu_ctx* c, const CUtensorMap& ta, const FxMaps& tb, double* o
   if (nTiles <= 0) return;
   const int grid = std::min(nTiles, c->numSms * ctasPerSm);
   kern<<<grid, 32 * (EW + 2), C::SMEM, c->stream>>>(ta, tb, out, expA, expB, maxRow, maxCol, TRAJ_PASS(c), gemmId,
-                                                    segPitchA, aShared, kPer, tiles, nTiles, err);
+                                                    segPitchA, aShared, kPer, tiles, nTiles, err, colScale);
   CODY_LAUNCHED(c);
 }
 
@@ -646,7 +648,7 @@ void* fx_build_tiles(cgpu_ctx* c, int gemmId, int bn, int nSplit, int* nTiles) {
 
 void fx_gemm(cgpu_ctx* c, int L, bool compact, int gemmId, const CUtensorMap& ta, const FxMaps& tb, int bn,
              double* out, const int* expA, const int* expB, unsigned* maxRow, unsigned* maxCol, int segPitchA,
-             int segPitch, int aShared, int nSplit, const void* tiles, int nTiles, int* err) {
+             int segPitch, int aShared, int nSplit, const void* tiles, int nTiles, int* err, const int* colScale) {
   if (segPitch % TC_BK != 0 || segPitchA % TC_BK != 0)
     throw std::string("fx_gemm: segment pitch must be a multiple of 64");
   if (nSplit > 1 && (maxRow || maxCol)) throw std::string("fx_gemm: output maxima need an unsplit K");
@@ -656,7 +658,7 @@ void fx_gemm(cgpu_ctx* c, int L, bool compact, int gemmId, const CUtensorMap& ta
 #define FX_CASE(BN_, L_, NA_, NB_, CMP_)                                                                        \
   if (bn == BN_ && L == L_ && compact == CMP_) {                                                                \
     launch_fx_t<BN_, L_, NA_, NB_>(c, ta, tb, out, expA, expB, maxRow, maxCol, gemmId, segPitchA, aShared,     \
-                                   kPer, tl, nTiles, CMP_ ? 2 : 1, err);                              \
+                                   kPer, tl, nTiles, CMP_ ? 2 : 1, err, colScale);                    \
     return;                                                                                                     \
   }
   FX_CASE(32, 4, 0, 2, false) FX_CASE(64, 4, 0, 2, false) FX_CASE(96, 4, 0, 2, false)

@@ -66,7 +66,7 @@ struct MixedBufs {
   __nv_bfloat16* Vsh = nullptr;
   int* eVsh = nullptr;
   CUtensorMap mVsh;
-  int *eV = nullptr, *eS = nullptr, *eWr = nullptr, *eWc = nullptr, *eR = nullptr;  // row exponents
+  int *eV = nullptr, *eS = nullptr, *sS = nullptr, *eWr = nullptr, *eWc = nullptr, *eR = nullptr;  // row exponents (sS: see fx_scale_key)
   unsigned *mWr = nullptr, *mWc = nullptr;  // largest biased exponent of |W| per row g / column n
   double *Wd = nullptr, *Zp = nullptr, *Gd = nullptr;  // FP64 results [split][M][N]
 };
@@ -368,14 +368,36 @@ __device__ __forceinline__ int fx_exp(unsigned m, bool wide = false) {
   return m == 0 ? 0 : m == 2047u ? FX_EXP_NAN : (int)m - (wide ? 1022 : 1021);
 }
 
-// Columns k, k + 1 (k even) of a row's L digit planes, zeros where not valid.
+// Columns k, k + 1 (k even) of a row's L digit planes, relative to 2^e0 and 2^e1.
 template <int L>
-__device__ __forceinline__ void fx_store2(__nv_bfloat16* rowBase, size_t pitch, int k, double v0, double v1, int e) {
+__device__ __forceinline__ void fx_store2(__nv_bfloat16* rowBase, size_t pitch, int k, double v0, double v1, int e0,
+                                          int e1) {
   int d0[L], d1[L];
-  fx_digits<L>(v0, e, d0);
-  fx_digits<L>(v1, e, d1);
+  fx_digits<L>(v0, e0, d0);
+  fx_digits<L>(v1, e1, d1);
 #pragma unroll
   for (int l = 0; l < L; l++) *reinterpret_cast<unsigned*>(rowBase + (size_t)l * pitch + k) = fx_bf16x2(d0[l], d1[l]);
+}
+
+// Sums of two values over the block, to its first warp.
+__device__ z_t fx_block_sum(double a, double b) {
+  __shared__ double red[2][32];
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, o);
+    b += __shfl_xor_sync(0xffffffffu, b, o);
+  }
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  if (lane == 0) {
+    red[0][threadIdx.x >> 5] = a;
+    red[1][threadIdx.x >> 5] = b;
+  }
+  __syncthreads();
+  a = b = 0.0;
+  for (int w = 0; w < nw; w++) {
+    a += red[0][w];
+    b += red[1][w];
+  }
+  return zmk(a, b);
 }
 
 __device__ unsigned fx_block_max(unsigned m) {
@@ -391,22 +413,35 @@ __device__ unsigned fx_block_max(unsigned m) {
   return r;
 }
 
+// Scales of the pair contraction Z = W R'' in the FP64 form.  Its K index runs over the
+// pairs, and a pair of orbitals that hardly overlap has a potential many orders below the
+// others' with perhaps a large coefficient: rounded to their row's maximum, W's entry and R''s
+// would lose what an FP64 sum keeps.  So W's column of pair p is taken times 2^-s_p and R''s
+// row times 2^s_p, with sum_y |S_p| < 2^s_p: then the entries of a row of W lie within V's range
+// of one another or below their own rounding error.  The scales enter as exponents
+// alone (fx_scale_key).
+
 // One block per row of K values: the exponent of its maximum, then the L digit
 // planes, zero in [K, Kpad).  The values are staged in dynamic shared memory
-// when `staged`, else formed twice (rows longer than shared memory).
+// when `staged`, else formed twice (rows longer than shared memory).  scale (null: none):
+// value k counts as value times 2^scale[k].
 template <int L, class F>
-__device__ void fx_row(__nv_bfloat16* rowBase, int* expOut, int K, int Kpad, int pitch, int staged, bool wide, F value) {
+__device__ void fx_row(__nv_bfloat16* rowBase, int* expOut, int K, int Kpad, int pitch, int staged, bool wide,
+                       const int* scale, F value) {
   extern __shared__ double fxbuf[];
   unsigned m = 0;
   for (int k = threadIdx.x; k < K; k += blockDim.x) {
     const double v = value(k);
     if (staged) fxbuf[k] = v;
-    m = max(m, fx_biased_exp(v));
+    m = max(m, scale ? fx_scale_key(fx_biased_exp(v), scale[k]) : fx_biased_exp(v));
   }
-  const int e = fx_exp(fx_block_max(m), wide);
+  const unsigned M = fx_block_max(m);
+  const int e = scale ? fx_key_exp(M) : fx_exp(M, wide);
   if (threadIdx.x == 0) *expOut = e;
   auto at = [&](int k) { return k < K ? (staged ? fxbuf[k] : value(k)) : 0.0; };
-  for (int k = 2 * threadIdx.x; k < Kpad; k += 2 * blockDim.x) fx_store2<L>(rowBase, pitch, k, at(k), at(k + 1), e);
+  auto ex = [&](int k) { return scale && k < K ? e - scale[k] : e; };
+  for (int k = 2 * threadIdx.x; k < Kpad; k += 2 * blockDim.x)
+    fx_store2<L>(rowBase, pitch, k, at(k), at(k + 1), ex(k), ex(k + 1));
 }
 
 constexpr size_t FX_STAGE_MAX = 200 * 1024;  // shared memory for staged rows; longer rows are formed twice
@@ -422,7 +457,7 @@ __global__ void __launch_bounds__(256) k_fx_split_V(__nv_bfloat16* __restrict__ 
   V = bat(V, bs);
   const double* row = V + (size_t)g * nG;
   fx_row<L>(out + (size_t)g * L * pitch, eV + g, nG, (nG + 63) / 64 * 64, pitch, 0, false,
-                 [&](int k) { return row[k]; });
+            nullptr, [&](int k) { return row[k]; });
 }
 
 // Rows 2p (real part) and 2p + 1 (imaginary part) of S = conj(phi_l) phi_k w
@@ -437,10 +472,11 @@ __global__ void __launch_bounds__(256) k_fx_split_S(__nv_bfloat16* __restrict__ 
                                                      unsigned* __restrict__ mWr, unsigned* __restrict__ mWc,
                                                      const z_t* __restrict__ orbs, const double* __restrict__ w,
                                                      const int* __restrict__ pl, const int* __restrict__ pk, int pitch,
-                                                     int staged, TRAJ_ARGS) {
+                                                     int* __restrict__ sS, int staged, TRAJ_ARGS) {
   const TrajShape& T = shp[blockIdx.z];
   const int p = blockIdx.x, nG = T.nG, nP = T.nPairs;
   if (p >= nP) return;
+  sS = bat(sS, bs);
   out = bat(out, bs);
   eS = bat(eS, bs);
   orbs = bat(orbs, bs);
@@ -470,6 +506,7 @@ __global__ void __launch_bounds__(256) k_fx_split_S(__nv_bfloat16* __restrict__ 
     return zmk(df_to_d(make_float2(s0, c0)), df_to_d(make_float2(s1, c1)));
   };
   unsigned mr = 0, mi = 0;
+  double sr = 0.0, si = 0.0;  // sums of the sizes (FP64 form)
   for (int g = threadIdx.x; g < nG; g += blockDim.x) {
     const z_t v = value(g);
     if (staged) {
@@ -478,6 +515,17 @@ __global__ void __launch_bounds__(256) k_fx_split_S(__nv_bfloat16* __restrict__ 
     }
     mr = max(mr, fx_biased_exp(v.x));
     mi = max(mi, fx_biased_exp(v.y));
+    if (L > 6) {
+      sr += fabs(v.x);
+      si += fabs(v.y);
+    }
+  }
+  if (L > 6) {
+    const z_t sum = fx_block_sum(sr, si);
+    if (threadIdx.x < 2) {
+      const unsigned ex = fx_biased_exp(threadIdx.x ? sum.y : sum.x);
+      sS[2 * p + threadIdx.x] = ex ? (int)ex - 1022 : FX_NO_SOURCE;
+    }
   }
   const int er = fx_exp(fx_block_max(mr));
   const int ei = fx_exp(fx_block_max(mi));
@@ -494,26 +542,28 @@ __global__ void __launch_bounds__(256) k_fx_split_S(__nv_bfloat16* __restrict__ 
   };
   for (int k = 2 * threadIdx.x; k < Kpad; k += 2 * blockDim.x) {
     const z_t v0 = at(k - shift), v1 = at(k + 1 - shift);
-    fx_store2<L>(rowR, pitch, k, v0.x, v1.x, er);
-    fx_store2<L>(rowI, pitch, k, v0.y, v1.y, ei);
+    fx_store2<L>(rowR, pitch, k, v0.x, v1.x, er, er);
+    fx_store2<L>(rowI, pitch, k, v0.y, v1.y, ei, ei);
   }
 }
 
 // Row n = 2q + s of R'' (K = 2p + t), as k_split_R.
 template <int L>
 __global__ void k_fx_split_R(__nv_bfloat16* __restrict__ out, int* __restrict__ eR, const z_t* __restrict__ Rp,
-                             const int* __restrict__ pl, const int* __restrict__ pk, int pitch, TRAJ_ARGS) {
+                             const int* __restrict__ pl, const int* __restrict__ pk, int pitch,
+                             const int* __restrict__ sS, TRAJ_ARGS) {
   const TrajShape& T = shp[blockIdx.z];
   const int n = T.nOS, nP = T.nPairs, Q = n * n;
   const int row = blockIdx.x;
   if (row >= 2 * Q) return;
   out = bat(out, bs);
   eR = bat(eR, bs);
+  sS = bat(sS, bs);
   Rp = bat(Rp, bs);
   pl = bat(pl, bs);
   pk = bat(pk, bs);
   const int q = row >> 1, s = row & 1;
-  fx_row<L>(out + (size_t)row * L * pitch, eR + row, 2 * nP, T.Kp, pitch, 1, L <= 6, [&](int k) {
+  fx_row<L>(out + (size_t)row * L * pitch, eR + row, 2 * nP, T.Kp, pitch, 1, L <= 6, L > 6 ? sS : nullptr, [&](int k) {
     const int p = k >> 1, t = k & 1;
     const int l = pl[p], kk = pk[p];
     const z_t R1 = Rp[(size_t)(l * n + kk) * Q + q];
@@ -529,12 +579,13 @@ __global__ void k_fx_split_R(__nv_bfloat16* __restrict__ out, int* __restrict__ 
 // it is raised: almost every entry is below it, and an atomic each would queue
 // the whole matrix on 2P + nG words.
 __global__ void k_fx_reduce_W(double* __restrict__ Wd, unsigned* __restrict__ mWr, unsigned* __restrict__ mWc,
-                              int nSplit, TRAJ_ARGS) {
+                              const int* __restrict__ sS, int nSplit, TRAJ_ARGS) {
   const TrajShape& T = shp[blockIdx.z];
   const int nG = T.nG, N = 2 * T.nPairs;
   Wd = bat(Wd, bs);
   mWr = bat(mWr, bs);
   mWc = bat(mWc, bs);
+  sS = bat(sS, bs);  // null: no scales
   const size_t tot = (size_t)nG * N;
   GRID_STRIDE(e, tot) {
     double v = 0.0;
@@ -542,7 +593,8 @@ __global__ void k_fx_reduce_W(double* __restrict__ Wd, unsigned* __restrict__ mW
     Wd[e] = v;
     const unsigned ex = fx_biased_exp(v);
     unsigned *r = mWr + e / N, *q = mWc + e % N;
-    if (ex > *(volatile unsigned*)r) atomicMax(r, ex);
+    const unsigned key = sS ? fx_scale_key(ex, -sS[e % N]) : ex;
+    if (key > *(volatile unsigned*)r) atomicMax(r, key);
     if (ex > *(volatile unsigned*)q) atomicMax(q, ex);
   }
 }
@@ -557,8 +609,8 @@ template <int L, int L2, int THREADS>
 __global__ void __launch_bounds__(THREADS) k_fx_split_W(__nv_bfloat16* __restrict__ WxA, __nv_bfloat16* __restrict__ WTxB,
                                                      int* __restrict__ eWr, int* __restrict__ eWc,
                                                      const double* __restrict__ Wd, const unsigned* __restrict__ mWr,
-                                                     const unsigned* __restrict__ mWc, int pitchP, int pitchG,
-                                                     TRAJ_ARGS) {
+                                                     const unsigned* __restrict__ mWc, const int* __restrict__ sS,
+                                                     int pitchP, int pitchG, TRAJ_ARGS) {
   __shared__ double tile[FW_T][FW_T + 1];
   const TrajShape& T = shp[blockIdx.z];
   const int nG = T.nG, N2P = 2 * T.nPairs, KpP = T.Kp, KpG = T.Kg, sh = T.gShift;
@@ -571,26 +623,32 @@ __global__ void __launch_bounds__(THREADS) k_fx_split_W(__nv_bfloat16* __restric
   Wd = bat(Wd, bs);
   mWr = bat(mWr, bs);
   mWc = bat(mWc, bs);
+  sS = bat(sS, bs);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int i = threadIdx.x; i < FW_T * FW_T; i += THREADS) {
     const int r = i / FW_T, c = i % FW_T, g = c0 + r - sh, n = n0 + c;
     tile[r][c] = (g >= 0 && g < nG && n < N2P) ? Wd[(size_t)g * N2P + n] : 0.0;
   }
   __syncthreads();
-  if (WxA)
+  if (WxA) {
+    const int n = n0 + 2 * lane;
+    const bool scaled = L2 > 6 && n < N2P;
+    const int s0 = scaled ? sS[n] : 0, s1 = scaled ? sS[n + 1] : 0;
     for (int r = warp; r < FW_T; r += THREADS / 32) {
       const int g = c0 + r - sh;
       if (g < 0 || g >= nG) continue;
-      const int e = fx_exp(mWr[g], L2 <= 6);
+      const int e = L2 > 6 ? fx_key_exp(mWr[g]) : fx_exp(mWr[g], true);
       if (n0 == 0 && lane == 0) eWr[g] = e;
-      fx_store2<L2>(WxA + (size_t)g * L2 * pitchP, pitchP, n0 + 2 * lane, tile[r][2 * lane], tile[r][2 * lane + 1], e);
+      fx_store2<L2>(WxA + (size_t)g * L2 * pitchP, pitchP, n, tile[r][2 * lane], tile[r][2 * lane + 1], e + s0, e + s1);
     }
+  }
   for (int r = warp; r < FW_T; r += THREADS / 32) {
     const int n = n0 + r;
     if (n >= N2P) break;
     const int e = fx_exp(mWc[n]);
     if (c0 == 0 && lane == 0) eWc[n] = e;
-    fx_store2<L>(WTxB + (size_t)n * L * pitchG, pitchG, c0 + 2 * lane, tile[2 * lane][r], tile[2 * lane + 1][r], e);
+    fx_store2<L>(WTxB + (size_t)n * L * pitchG, pitchG, c0 + 2 * lane, tile[2 * lane][r], tile[2 * lane + 1][r], e,
+                 e);
   }
 }
 
@@ -650,6 +708,7 @@ size_t mixed_layout(cgpu_ctx* c, char* base, size_t off) {
     size_t oZ = take(off, sizeof(double) * (size_t)2 * nG * Q);
     size_t oeV = take(off, perTrajV * sizeof(int) * (size_t)nG);
     size_t oeS = take(off, sizeof(int) * (size_t)2 * nP);
+    size_t osS = take(off, sizeof(int) * (size_t)2 * nP);
     size_t oeWr = take(off, sizeof(int) * (size_t)nG);
     size_t oeWc = take(off, sizeof(int) * (size_t)2 * nP);
     size_t oeR = take(off, sizeof(int) * (size_t)2 * Q);
@@ -667,6 +726,7 @@ size_t mixed_layout(cgpu_ctx* c, char* base, size_t off) {
       m->Zd = (double*)(base + oZ);
       m->eV = perTrajV ? (int*)(base + oeV) : nullptr;
       m->eS = (int*)(base + oeS);
+      m->sS = (int*)(base + osS);
       m->eWr = (int*)(base + oeWr);
       m->eWc = (int*)(base + oeWc);
       m->eR = (int*)(base + oeR);
@@ -813,11 +873,12 @@ static void fx_run_W(cgpu_ctx* c, bool exact) {
   const int nG = c->nG, nP = c->nPairs;
   const FxGemm& g = exact && m->L != m->L64 ? m->gWx : m->gW;
   const bool one = g.s == 1;
+  const int* scale = exact || m->L == m->L64 ? m->sS : nullptr;  // the FP64 form's slices
   fx_gemm(c, exact ? m->L64 : m->L, g.compact, TC_GEMM_W, c->fxShared ? m->mVsh : m->mV, exact ? m->bSx : m->bS, g.bn,
           m->Wd, c->fxShared ? m->eVsh : m->eV, m->eS, one ? m->mWr : nullptr, one ? m->mWc : nullptr,
-          c->fxShared ? m->KgBig : m->KgMax, m->KgMax, c->fxShared, g.s, g.tiles, g.nTiles, m->err);
+          c->fxShared ? m->KgBig : m->KgMax, m->KgMax, c->fxShared, g.s, g.tiles, g.nTiles, m->err, scale);
   if (!one) {
-    k_fx_reduce_W<<<bgrid(c, ew_blocks(c, (size_t)nG * 2 * nP)), 256, 0, c->stream>>>(m->Wd, m->mWr, m->mWc, g.s,
+    k_fx_reduce_W<<<bgrid(c, ew_blocks(c, (size_t)nG * 2 * nP)), 256, 0, c->stream>>>(m->Wd, m->mWr, m->mWc, scale, g.s,
                                                                                    TRAJ_PASS(c));
     CODY_LAUNCHED(c);
   }
@@ -965,8 +1026,9 @@ static void fx_potentials(cgpu_ctx* c, const z_t* orbs, bool exact, bool wantW) 
   if (staged && need > 48 * 1024)
     CODY_CUDA(cudaFuncSetAttribute(k_fx_split_S<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FX_STAGE_MAX));
   k_fx_split_S<L><<<dim3(c->nPairs, 1, c->nb), 256, staged ? need : 0, c->stream>>>(
-      m->SxA, m->eS, m->mWr, m->mWc, orbs, c->w_d, c->pairL_d, c->pairK_d, m->KgMax, staged, TRAJ_PASS(c));
+      m->SxA, m->eS, m->mWr, m->mWc, orbs, c->w_d, c->pairL_d, c->pairK_d, m->KgMax, m->sS, staged, TRAJ_PASS(c));
   CODY_LAUNCHED(c);
+  branch_record(c, BR_SOURCES);
   fx_run_W(c, exact);
   dim3 gw(m->KgMax / FW_T, m->KpMax / FW_T, c->nb);
   // fewer than two tiles an SM: four times the warps a tile, whose rows are then two in turn instead
@@ -974,7 +1036,7 @@ static void fx_potentials(cgpu_ctx* c, const z_t* orbs, bool exact, bool wantW) 
   const bool few = gw.x * gw.y * gw.z < 2 * (unsigned)c->numSms;
   auto split = few ? k_fx_split_W<L, L2, 1024> : k_fx_split_W<L, L2, 256>;
   split<<<gw, few ? 1024 : 256, 0, c->stream>>>(wantW ? m->WxA : nullptr, m->WTxB, m->eWr, m->eWc, m->Wd, m->mWr,
-                                                 m->mWc, m->KpMax, m->KgMax, TRAJ_PASS(c));
+                                                 m->mWc, m->sS, m->KpMax, m->KgMax, TRAJ_PASS(c));
   CODY_LAUNCHED(c);
 }
 
@@ -994,7 +1056,7 @@ static void fx_plan(const cgpu_ctx* c, F f) {
 
 // The pieces of the correlation in the fixed-point forms, for callers that place
 // them on several streams: the pair potentials; the digits of rho^-1 rho2 (after
-// launch_rdm_inverse); Z from both, dOrbs += its contraction with the orbitals; h2
+// launch_rdm_inverse and, in the FP64 form, BR_SOURCES: the pair sources' scales); Z from both, dOrbs += its contraction with the orbitals; h2
 // from the potentials.
 bool fx_ready(const cgpu_ctx* c) { return c->fxOn && c->mixed && c->mixed->L > 0 && c->hasInteraction; }
 
@@ -1007,7 +1069,7 @@ void launch_fx_split_R(cgpu_ctx* c) {
   MixedBufs* m = c->mixed;
   fx_plan(c, [&](auto, auto L2) {
     k_fx_split_R<L2()><<<dim3(2 * c->nOS * c->nOS, 1, c->nb), 64, sizeof(double) * m->KpMax, c->stream>>>(
-        m->RxB, m->eR, c->Rp_d, c->pairL_d, c->pairK_d, m->KpMax, TRAJ_PASS(c));
+        m->RxB, m->eR, c->Rp_d, c->pairL_d, c->pairK_d, m->KpMax, m->sS, TRAJ_PASS(c));
   });
   CODY_LAUNCHED(c);
 }
@@ -1040,6 +1102,7 @@ static void correlation_fx(cgpu_ctx* c, z_t* dOrbs, const z_t* orbs, int wantH2)
       BranchStream on(c, c->side[0]);
       branch_wait(c, BR_START);
       launch_rdm_inverse(c);
+      branch_wait(c, BR_SOURCES);
       launch_fx_split_R(c);
       branch_record(c, BR_DENSITY);
     }

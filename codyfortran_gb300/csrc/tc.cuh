@@ -26,6 +26,19 @@ void tc_gemm(cgpu_ctx* c, int gemmId, const CUtensorMap& ta, const CUtensorMap& 
 
 // Row exponent of an operand row that holds an infinity or a NaN.
 constexpr int FX_EXP_NAN = 1 << 20;
+// A row's maximum over columns with scales of their own (the pair contraction of the FP64
+// form, k_mixed.cu): of ex + scale + FX_KEY over the biased exponents ex (0: all zero).
+constexpr int FX_KEY = 4096;             // |ex + scale| < 4096 but for FX_NO_SOURCE, which drowns
+constexpr int FX_NO_SOURCE = -4000;      // scale of a pair without a source (W = 0)
+constexpr unsigned FX_KEY_NAN = 1u << 20;
+__device__ __forceinline__ unsigned fx_scale_key(unsigned ex, int scale) {
+  return ex == 0 ? 0u : ex == 2047u ? FX_KEY_NAN : (unsigned)max(1, (int)ex + scale + FX_KEY);
+}
+// smallest e with |x 2^scale| < 2^(e-1) for the largest key of a row
+__device__ __forceinline__ int fx_key_exp(unsigned m) {
+  return m == 0 ? 0 : m >= FX_KEY_NAN ? FX_EXP_NAN : (int)m - FX_KEY - 1021;
+}
+
 // The TMA maps of a fixed-point B operand, one per tile width 16, 32, ...
 constexpr int FX_MAPS = 6;
 struct FxMaps {
@@ -39,14 +52,16 @@ CUtensorMap tc_encode_map(const __nv_bfloat16* base, int rank, const unsigned lo
 // A map with 128-row boxes) for operands carried as L base-256 digit slices (K segments of
 // segPitchA / segPitch elements) with row exponents expA / expB; maxRow /
 // maxCol (unsplit K only) receive the largest biased exponent of |C| per row /
-// column.  compact: the two-CTAs-per-SM configuration (small K).  aShared: A
-// is one matrix shared by the trajectories, read at each trajectory's vRow.
+// column (colScale: a row's over the columns times 2^-colScale, as fx_scale_key).
+// compact: the two-CTAs-per-SM configuration (small K).  aShared: A is one matrix
+// shared by the trajectories, read at each trajectory's vRow.
 // nSplit: K splits of the longest contraction (segPitch / 64 K blocks, kPer
 // blocks per split); a trajectory of fewer K blocks takes only the splits its
 // own K needs, balanced, and its remaining partials are written as zeros.
 void fx_gemm(cgpu_ctx* c, int L, bool compact, int gemmId, const CUtensorMap& ta, const FxMaps& tb, int bn,
              double* out, const int* expA, const int* expB, unsigned* maxRow, unsigned* maxCol, int segPitchA,
-             int segPitch, int aShared, int nSplit, const void* tiles, int nTiles, int* err);
+             int segPitch, int aShared, int nSplit, const void* tiles, int nTiles, int* err,
+             const int* colScale = nullptr);
 // Device list of the fixed-point GEMM's tiles (trajectory, row, column, K split) of the
 // context for an N tile of bn columns: only tiles inside a trajectory's output.
 void* fx_build_tiles(cgpu_ctx* c, int gemmId, int bn, int nSplit, int* nTiles);

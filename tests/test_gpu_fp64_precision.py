@@ -73,3 +73,37 @@ def test_integrals_entry_by_entry(n_el, box, soft, n, slices, kind):
         print(f"{name} {nG} points, softening {soft}, {kind}: {worst:.1f} units")
         assert worst <= (12.0 if slices else 2.0 * nG), name
         assert np.all(err[~ok] <= 1e-250)
+
+
+@pytest.mark.parametrize("kind", ["compact", "apart"])
+@pytest.mark.parametrize("weight", [1.0, 1e-12, 1e-30])
+@pytest.mark.parametrize("n_el,box,soft,n", [(4, 4.0, 1.0, 2), (51, 100.0, 1.0, 3), (100, 100.0, 1.0, 4), (100, 100.0, 0.01, 3)])
+def test_mean_field_entry_by_entry(n_el, box, soft, n, weight, kind):
+    """dphi_j(x) in units of the sum of the sizes of its terms.  The coefficients of the pairs
+    of orbitals on one side are small, so that with the sides far apart the sum lies in pairs
+    whose potentials are 1e-17 of the others'.  V and S six roundings, W one, rho2's spin blocks three, rho^-1 of a
+    multiple of the identity four, R'' two, the product one, the sum over the orbitals n + 1: 24.
+    """
+    from codyfortran_gb300.engine import Engine
+    sp = _spec(n_el, box, soft, n)
+    e = Engine(sp)
+    rng = np.random.default_rng(n_el)
+    F = _orbitals(kind, e.x, e.w, n, rng)
+    P, W, A = _exact(sp, e.x, e.w, F)
+    r2 = rng.normal(size=(2 * n,) * 4) + 1j * rng.normal(size=(2 * n,) * 4)
+    o = np.arange(2 * n) % n
+    r2 = np.asfortranarray(r2 * np.where((o[None, :, None, None] - o[None, None, None, :]) % 2 == 0, weight, 1.0))
+    d, _ = e.apply_correlation_op(F, np.eye(2 * n, dtype=complex), r2, 0.0)
+    e.close()
+    spins = (slice(0, n), slice(n, 2 * n))
+    R = sum(r2[a, b, a, b].astype(np.clongdouble) for a in spins for b in spins)
+    R = R * (np.longdouble(2) / (np.longdouble(4) + np.longdouble(1e-10)))  # rho1 = 2, regularised
+
+    def field(W, R, F):
+        Z = W @ R.transpose(3, 1, 0, 2).reshape(n * n, n * n)  # (l2 k2) -> (k1 j)
+        return np.einsum("xk,xkj->xj", F, Z.reshape(-1, n, n))
+    want, size = field(W, R, F.astype(np.clongdouble)), field(A, np.abs(R).astype(float), np.abs(F))
+    ok = size > 1e-250
+    worst = float(np.max(np.abs(d - want).astype(float)[ok] / size[ok])) / UNIT
+    print(f"{n_el} elements, softening {soft}, weight {weight}, {kind}: {worst:.1f} units")
+    assert worst <= 24.0
