@@ -288,9 +288,13 @@ struct CiWork {
 
 // Page-locked host words that kernels write: the error of a bounded wait (0: none), and what
 // one launch of an adaptive SIL leaves (k_sil.cu).
-struct SilFlags {
-  int err, warnings, restarts, notFinite;
+struct SilLeft {
+  int warnings, restarts, notFinite;
   double t, rem, dtSub;
+};
+struct SilFlags {
+  int err;
+  SilLeft left[2];  // of the last launch that was given this place
 };
 
 // ---------------------------------------------------------------------------
@@ -586,7 +590,7 @@ void launch_lz_set(cgpu_ctx* c, int idx, double v);
 void sil_init(cgpu_ctx* c);
 void sil_free(cgpu_ctx* c);
 void launch_sil(cgpu_ctx* c, z_t* state, double t, double dt, int K, double tol, int maxRestarts, double dtSub,
-                int restarts);
+                int restarts, int place);
 void launch_lz_expsub(cgpu_ctx* c, int j, double dt);
 // One fixed-order pass of a single system and its reverse, for the pulse
 // gradient: what the pass leaves behind (V: K state vectors, last: one, the

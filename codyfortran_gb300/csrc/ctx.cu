@@ -867,9 +867,11 @@ int lanczos_pass(cgpu_ctx* c, int which, double tBase, double dt, int maxDim, do
 }
 
 // SIL Integrate (src/IntegratorList/Sil/S_IntegratorList_Sil.f90:114-177) on a device state.
-// Returns the sub-steps that did not converge.
+// Returns the sub-steps that did not converge.  place >= 0 (one-launch form with a tolerance):
+// the first launch alone, without waiting; sil_unfinished(place) tells, after a
+// synchronisation, whether it left anything, and then the state is not the result.
 int sil_device(cgpu_ctx* c, int which, z_t* state, double t0, double t1, int krylovDim, double tol, int maxRestarts,
-               const double* metric_d) {
+               const double* metric_d, int place = -1) {
   const double zeroThreshold = 1.0e-14;
   if (std::fabs(t1 - t0) <= zeroThreshold) return 0;
   int maxDim = std::max(1, std::min(krylovDim, c->minS));
@@ -881,10 +883,11 @@ int sil_device(cgpu_ctx* c, int which, z_t* state, double t0, double t1, int kry
     double t = t0, rem = t1 - t0, dtSub = rem;
     int restarts = 0;
     for (;;) {
-      launch_sil(c, state, t, rem, maxDim, tol, maxRestarts, dtSub, restarts);
+      launch_sil(c, state, t, rem, maxDim, tol, maxRestarts, dtSub, restarts, std::max(place, 0));
       if (!(tol > 0.0)) return 1;
+      if (place >= 0) return 0;
       sync(c);
-      const volatile SilFlags& f = *c->flags_h;
+      const volatile SilLeft& f = c->flags_h->left[0];
       warnings += f.warnings;
       t = f.t;
       rem = f.rem;
@@ -939,14 +942,22 @@ int sil_device(cgpu_ctx* c, int which, z_t* state, double t0, double t1, int kry
   return warnings;
 }
 
+bool sil_unfinished(const cgpu_ctx* c, int place) {
+  const volatile SilLeft& f = c->flags_h->left[place];
+  return std::fabs(f.rem) > 1.0e-14 && !f.notFinite;
+}
+
+// later: the SIL steps do not wait for what they leave (places 0 and 1)
 void split2_device(cgpu_ctx* c, z_t* state, double t0, double t1, int krylov, double tol, int maxRestarts,
-                   int useMetric) {
+                   int useMetric, bool later = false) {
   double dt = t1 - t0, time1 = t0, time2 = time1 + 0.5 * dt;
   const double* m = useMetric ? c->metricW_d : c->metricOne_d;
-  if (krylov > 0) sil_device(c, CGPU_TD_ORBS_LIN, state, time1, time1 + 0.5 * dt, krylov, tol, maxRestarts, m);
+  if (krylov > 0) sil_device(c, CGPU_TD_ORBS_LIN, state, time1, time1 + 0.5 * dt, krylov, tol, maxRestarts, m,
+                             later ? 0 : -1);
   else rk4_device(c, CGPU_TD_ORBS_LIN, state, time1, time1 + 0.5 * dt);
   rk4_device(c, CGPU_TD_NONLIN, state, time1, time1 + 1.0 * dt);
-  if (krylov > 0) sil_device(c, CGPU_TD_ORBS_LIN, state, time2, time2 + 0.5 * dt, krylov, tol, maxRestarts, m);
+  if (krylov > 0) sil_device(c, CGPU_TD_ORBS_LIN, state, time2, time2 + 0.5 * dt, krylov, tol, maxRestarts, m,
+                             later ? 1 : -1);
   else rk4_device(c, CGPU_TD_ORBS_LIN, state, time2, time2 + 0.5 * dt);
 }
 
@@ -1625,6 +1636,16 @@ int cgpu_propagate_split2(cgpu_ctx* c, cgpu_complex* state, double t0, double t1
   if (krylov_dim > 0 && tolerance == 0.0 && max_restarts == 0) {
     // fixed-order SIL: the step has no host-side decisions, replay it as one graph
     propagate_graph(c, &t0, t1 - t0, 1, krylov_dim, use_metric);
+  } else if (krylov_dim > 0 && tolerance > 0.0 && c->nb == 1 && c->silGroup > 0 && c->silFits) {
+    // the SIL steps almost always end within one launch: issue the whole step, and take it
+    // again part by part if one did not
+    c->flags_h->left[0].rem = c->flags_h->left[1].rem = 0.0;
+    split2_device(c, c->state_d, t0, t1, krylov_dim, tolerance, max_restarts, use_metric, true);
+    sync(c);
+    if (sil_unfinished(c, 0) || sil_unfinished(c, 1)) {
+      up(c, c->state_d, state, c->nS);
+      split2_device(c, c->state_d, t0, t1, krylov_dim, tolerance, max_restarts, use_metric);
+    }
   } else {
     split2_device(c, c->state_d, t0, t1, krylov_dim, tolerance, max_restarts, use_metric);
   }

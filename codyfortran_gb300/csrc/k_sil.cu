@@ -354,7 +354,8 @@ struct SilArgs {
   double tol;
   double dtSub;    // the step to try first, and the halvings that led to it
   int restarts, maxRestarts;
-  SilFlags* flags;  // host memory; what an adaptive integration (trajectory 0) leaves
+  SilFlags* flags;  // host memory: the error word, and what an adaptive integration (trajectory 0) leaves
+  int place;
   int cap, smemV;  // entries of the largest piece; basis vectors in shared memory
   int pt;          // threads per entry (4 where the pieces leave most of the block idle, else 1)
   // for the pulse gradient: a given field value, and what its reverse pass reads
@@ -375,6 +376,7 @@ template <int SIL_T, int MODE = SIL_STEP>
 __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
   constexpr int SIL_W = SIL_T / 32;
   constexpr bool KEEP = MODE != SIL_STEP;
+  const double tol = KEEP ? 0.0 : A.tol;  // the kept pass is of fixed order
   const SilBlock B = A.blk[blockIdx.x];
   const TrajShape& S = shp[B.traj];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -655,7 +657,7 @@ __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
         const double be = n1 < 0.0 ? 0.0 : sqrt(n1);
         const bool broke = be <= SIL_ZERO && !KEEP;  // the kept pass runs over all orders
         const bool last = broke || j == A.K;
-        if (A.tol > 0.0 || last) {
+        if (tol > 0.0 || last) {
           __syncthreads();
           if (wid == 0) {
             if (lane == 0) beta[j - 1] = be;
@@ -665,11 +667,10 @@ __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
             if (lane == j - 1) errEst = broke ? 0.0 : be * sqrt(fr * fr + fi * fi);
           }
           __syncthreads();
-          conv = errEst <= A.tol;
-          // not finite: no step converges from here, however short (the kept pass and the fixed
-          // orders run on)
-          bad = A.tol > 0.0 && !(fabs(nrm) + fabs(alpha[j - 1]) + be < INFINITY);
-          if (bad || (A.tol > 0.0 && conv) || last) {
+          conv = errEst <= tol;
+          // not finite: no step converges from here, however short (the fixed orders run on)
+          bad = tol > 0.0 && !(fabs(nrm) + fabs(alpha[j - 1]) + be < INFINITY);
+          if (bad || (tol > 0.0 && conv) || last) {
             mDim = j;
             it++;
             break;
@@ -678,7 +679,7 @@ __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
       }
       done = mDim == 0;
       if (!ok || done) break;
-      if (conv || bad || !(A.tol > 0.0) || fabs(dtS) <= SIL_ZERO || restarts >= A.maxRestarts) {
+      if (conv || bad || !(tol > 0.0) || fabs(dtS) <= SIL_ZERO || restarts >= A.maxRestarts) {
         for (int e = tid; e < cnt; e += SIL_T) {
           z_t acc = zmk(0.0, 0.0);
           for (int k = 0; k < mDim; k++) zfma(acc, vec(k, e), phi[k]);
@@ -705,7 +706,7 @@ __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
       notFinite = 1;
       break;
     }
-    if (!(A.tol > 0.0)) break;  // fixed order: one pass over the whole step
+    if (!(tol > 0.0)) break;  // fixed order: one pass over the whole step
     tCur += dtS;
     rem -= dtS;
     dtS = rem;
@@ -713,13 +714,14 @@ __global__ void __launch_bounds__(SIL_T, 1) k_sil(const SilArgs A, TRAJ_ARGS) {
     if (fabs(rem) > SIL_ZERO) ok = barrier();  // the neighbours' pieces of the new start
   }
   if (tid == 0) {
-    if (B.traj == 0 && B.rank == 0 && A.tol > 0.0) {
-      A.flags->warnings = warnings;
-      A.flags->t = tCur;
-      A.flags->rem = rem;
-      A.flags->dtSub = dtS;
-      A.flags->restarts = restarts;
-      A.flags->notFinite = notFinite;
+    if (B.traj == 0 && B.rank == 0 && tol > 0.0) {
+      SilLeft& left = A.flags->left[A.place];
+      left.warnings = warnings;
+      left.t = tCur;
+      left.rem = rem;
+      left.dtSub = dtS;
+      left.restarts = restarts;
+      left.notFinite = notFinite;
     }
     if (B.n > 1 && atomicAdd(bar + 1, 1u) == (unsigned)B.n - 1) {
       bar[0] = 0u;
@@ -1009,10 +1011,10 @@ static void sil_launch(cgpu_ctx* c, SilArgs& a, int mode) {
 }
 
 // SIL on OrbsLin from t over dt on a state (all trajectories), in place.  With a tolerance
-// it may leave some of dt: flags_h holds, after a synchronisation, the time reached, what is
-// left of dt, and the step and the halvings to go on with (dtSub, restarts).
+// it may leave some of dt: flags_h->left[place] holds, after a synchronisation, the time reached,
+// what is left of dt, and the step and the halvings to go on with (dtSub, restarts).
 void launch_sil(cgpu_ctx* c, z_t* state, double t, double dt, int K, double tol, int maxRestarts, double dtSub,
-                int restarts) {
+                int restarts, int place) {
   ProfScope prof(c, CGPU_KERNEL_LANCZOS);
   SilArgs a = sil_args(c, state, state, dt, K);
   a.m = c->metric_d;
@@ -1021,6 +1023,7 @@ void launch_sil(cgpu_ctx* c, z_t* state, double t, double dt, int K, double tol,
   a.tol = tol;
   a.dtSub = dtSub;
   a.restarts = restarts;
+  a.place = place;
   a.maxRestarts = maxRestarts;
   sil_launch(c, a, SIL_STEP);
 }

@@ -118,3 +118,17 @@ def test_one_krylov_vector(dt, tol):
     a, w = _engine_sil(e, st, dt, 6, tol, 0)
     e.close()
     assert np.linalg.norm(a - st) < 1e-12 * np.linalg.norm(st) and (tol == 0.0 or w == 0)
+
+
+def test_a_split_step_whose_sil_takes_several_launches():
+    """The step is issued in one piece and taken again, part by part, where a SIL half did not end
+    within a launch: hundreds of sub-steps against the oracle, then a step that ends at once."""
+    from codyfortran_gb300.engine import Engine
+    sp, o, st = _system()
+    e = Engine(sp, max_krylov=6)
+    for dt, K, tol, restarts in [(0.2, 2, 1e-9, 3), (0.01, 6, 1e-7, 4)]:
+        a = e.propagate_split2(st, 2.0, 2.0 + dt, K, tol, restarts)
+        b = o.propagate_split2(st, 2.0, 2.0 + dt, K, tol, restarts)
+        print(dt, np.linalg.norm(a - b) / np.linalg.norm(b))
+        assert np.linalg.norm(a - b) < _sub_steps(dt, restarts) * 1e-12 * np.linalg.norm(b)
+    e.close()
