@@ -540,7 +540,7 @@ void launch_fx_potentials(cgpu_ctx* c, const z_t* orbs);
 void launch_fx_split_R(cgpu_ctx* c);
 void launch_fx_Z(cgpu_ctx* c);
 void launch_fx_epilogue(cgpu_ctx* c, z_t* dOrbs, const z_t* orbs);
-void launch_fx_h2(cgpu_ctx* c);  // FillH2 with the FP64 form's slices (fxOn)
+void launch_fx_h2(cgpu_ctx* c);  // h2 of the last launch_fx_potentials, in the form's own slices
 // Tile tuner hooks of the fixed-point contractions.  A tile table t[9] holds,
 // for W = V S, Z = W R'' and h2 = S^T W in turn: N-tile width, compact (two
 // CTAs per SM) flag, K splits.  fx_tiles_get returns false outside the

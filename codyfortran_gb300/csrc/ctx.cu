@@ -446,8 +446,8 @@ void detect_shared_interaction(cgpu_ctx* c) {
 // V(longest) sum |S|, so those losses stay below about 2^-8L R sqrt(points) of it, whatever
 // the source; the same bound holds for h2 = S^T W, as |W| and its own rounding are bounded
 // by V |S| too.  FP64 sums lose 2^-53 times a factor of the same kind.  Worst point of W
-// relative to V |S| (seven sources from one point to the whole box; FP64 summed in order, 7,
-// 8, 9 slices):
+// relative to V |S|, in exact arithmetic, of six sources from one point to the whole box (FP64
+// summed in order; 7, 8, 9 slices):
 //   2801 points, R = 800 = 2^9.6       5e-15  1e-12  5e-15  9e-17
 //   2801 points, R = 8000 = 2^13       5e-15  9e-12  4e-14  2e-16
 //   2801 points, R = 80000 = 2^16.3    4e-15  8e-11  3e-13  2e-15
@@ -537,8 +537,9 @@ void build_ctx(cgpu_ctx* c, const cgpu_desc* descs, int nSys) {
     total = c->bs * (size_t)nSys + mixed_outside_bytes(c);
   };
   // The contractions run as digit slices in both fixed-point forms.  In the FP64
-  // form they do too (36 or 45 slice products on the tensor cores against the FP64
-  // pipe, several times slower on every shape measured), unless the caller asks for
+  // form they do too (a Strang step with K = 4 on 36 or 45 slice products / on the FP64
+  // pipe: 21 points, 4 orbitals 327 / 721 us, 501 x 4 379 / 4834, 2801 x 12 1178 / 17877,
+  // with nine slices 1331), unless the caller asks for
   // the FP64 pipe, the interaction's range needs more slices than there are kernels
   // for (fx_slices_fp64) or the slices' larger footprint takes more than three quarters of
   // the device (the rest is for what is allocated on first use).  That is a matter of

@@ -11,21 +11,22 @@
 //     C = 2^(ea + eb) sum_l 2^(-8(l+2)) D_l,   D_l = sum_{i+j=l} sum_k a_i[k] b_j[k].
 // Each level has its own FP32 accumulator in tensor memory (L accumulators of
 // nT columns), fed by the slice products of that level.  A slice product is an
-// integer of magnitude <= 2^14, so over a chunk of K = 256 a level sum of l + 1
-// products stays below (l + 1) 2^22: exact in FP32 for the four leading levels
-// whatever the operands, and for the others unless every digit of both rows is
-// at its extreme with one sign (then C itself is 2^6 times its terms and one
-// unit of level 4 is 2^-54 of it).  After every chunk the epilogue adds the
-// level sums to 64-bit integers, so C is the product of the truncated operands
-// whatever the summation order.  Levels l >= L are not formed; with the operand
-// truncation (2^-8L of each row maximum) they bound the error at about
-// 2^-8L max|a| max|b| sqrt(K).
+// integer of magnitude <= 2^14, so over a chunk of K a level sum of l + 1 products
+// stays below (l + 1) K 2^14: exact in FP32 up to 2^24.  K = 256 in the mixed forms:
+// the four leading levels whatever the operands, the others unless the digits of both
+// rows are near their extremes with one sign (a few units of level 4, 2^-43 of the rows'
+// maxima, then).  K = 128 in the FP64 form: eight levels whatever the operands, and the
+// ninth lies below what is kept.  After every chunk the epilogue adds the level sums to
+// 64-bit integers, so C is the product of the truncated operands whatever the summation
+// order.  Levels l >= L are not formed; with the operand truncation (2^-8L of each row
+// maximum) they bound the error at about 2^-8L max|a| max|b| sqrt(K).
 //
 // L = 4 to 6 serve the mixed_fx / mixed_fx6 forms (their Z operands with
-// max_k |x[k]| < 2^e, |d_0| <= 256: one bit more, K <= 256).  L = 7 (55 bits) is
-// the FP64 form: the FP64 pipe of this GPU does two FMA a cycle and SM
-// (1.2 TFLOP/s), 28 slice products on the tensor cores about 60 TFLOP/s of the
-// same contraction, and the sum of a row rounds once instead of K times.
+// max_k |x[k]| < 2^e, |d_0| <= 256: one bit more, K <= 256).  L = 8 and 9 are the FP64
+// form (fx_slices_fp64 in ctx.cu: how many, and why that is no less than FP64 sums keep):
+// the FP64 pipe of this GPU does two FMA a cycle and SM (1.2 TFLOP/s), 36 slice products
+// on the tensor cores about 45 TFLOP/s of the same contraction, and the sum of a row
+// rounds once instead of K times.
 //
 // Pipeline: one TMA producer thread, one MMA issuer thread, eight epilogue
 // warps (two per tensor-memory lane quarter).  Per 64-wide K block the producer
@@ -53,7 +54,7 @@
 // hands the tensor memory back; scaling and stores follow the tile's last
 // chunk.  Tiles with L nT <= half the tensor-memory columns alternate between
 // the two halves, so that the next chunk's MMAs run during the drain; wider
-// ones wait for it (about 1.5 k of 13 k cycles).  The wide configuration (two B
+// ones wait for it (about 1.5 k of 13 k cycles, of 9 k in the FP64 form).  The wide configuration (two B
 // stages, deep A ring) holds one CTA per SM; the compact one (one B stage, L A
 // stages, <= 256 TMEM columns) two.  Every wait is bounded: on expiry the
 // kernel sets an error flag, drains its copies, frees its tensor memory and

@@ -1,8 +1,10 @@
 // k_mf.cu -- interaction and mean-field kernels on the FP64 pipe.
 //
-// They serve the bf16x3 / bf16x6 forms' FillH2 and FP64 contexts whose digit
-// planes would not fit the device memory; the other FP64 contexts run the same
-// contractions on the tensor cores (k_mixed.cu, cgpu_ctx::fxOn).
+// They serve the bf16x3 / bf16x6 forms' FillH2, and every contraction of the FP64
+// contexts that ask for the FP64 pipe, whose interaction has a range that digit slices
+// do not suit (a strong damping, no softening) or whose digit planes take too much of the
+// device's memory; the other FP64 contexts run the same contractions on the tensor cores
+// (k_mixed.cu, cgpu_ctx::fx64).
 //
 // The reference loops over unordered orbital pairs and, per pair, runs an
 // O(nG^2) convolution, multiplies the potential onto every orbital and

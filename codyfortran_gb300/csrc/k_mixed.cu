@@ -17,10 +17,11 @@
 //
 // The fixed-point forms (FP64, mixed_fx, mixed_fx6) carry every operand row as L
 // base-256 digit slices under one power of two per row (k_fx.cu) and return
-// FP64 results whose only error is the operand truncation (fx_slices: at least 55
+// FP64 results whose only error is the operand truncation (fx_slices: at least 63
 // / 31 / 39 bits of each row's maximum): S and V rows for GEMM1, W rows and R''
 // rows for GEMM2, W columns for GEMM3.  FillH2 (energies) runs GEMM1 and GEMM3 with the
-// seven slices of the FP64 form in all three.  The row exponents of W come from
+// eight or nine slices of the FP64 form in all three, or on the FP64 pipe where that
+// form runs there (cgpu_ctx::fx64).  The row exponents of W come from
 // the GEMM1 epilogue, or from the reduction of its K splits.  The bf16x3 /
 // bf16x6 forms keep their own operands (k_tc.cu) and the FP64 pipe's FillH2.
 #include <cuda_bf16.h>
@@ -1056,8 +1057,8 @@ static void fx_plan(const cgpu_ctx* c, F f) {
 
 // The pieces of the correlation in the fixed-point forms, for callers that place
 // them on several streams: the pair potentials; the digits of rho^-1 rho2 (after
-// launch_rdm_inverse and, in the FP64 form, BR_SOURCES: the pair sources' scales); Z from both, dOrbs += its contraction with the orbitals; h2
-// from the potentials.
+// launch_rdm_inverse and, in the FP64 form, the pair sources' scales: BR_SOURCES); Z from
+// both, dOrbs += its contraction with the orbitals; h2 from the potentials.
 bool fx_ready(const cgpu_ctx* c) { return c->fxOn && c->mixed && c->mixed->L > 0 && c->hasInteraction; }
 
 void launch_fx_potentials(cgpu_ctx* c, const z_t* orbs) {

@@ -628,7 +628,6 @@ __global__ void k_dot_partial(z_t* __restrict__ part, const z_t* __restrict__ a,
   if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
-// dC -= (sum of partials) * C   (dot_product(coeffs, dCoeffs) = sum conj(C) dC)
 // dC -= C <C, dC> by one block (one system's up to PC_ONE coefficients: the two launches
 // of the general form took 4.3 + 4.1 us for 16 coefficients, this one 5.3; for 1296, whose
 // FP64 one SM does alone, 4.3 + 4.0 and 10.2).
@@ -658,6 +657,7 @@ __global__ void __launch_bounds__(256) k_project_coeffs_one(z_t* __restrict__ dC
   }
 }
 
+// dC -= (sum of partials) * C   (dot_product(coeffs, dCoeffs) = sum conj(C) dC)
 __global__ void k_project_coeffs_apply(z_t* __restrict__ dC, const z_t* __restrict__ C, const z_t* __restrict__ part,
                                        int nBlk, TRAJ_ARGS) {
   const TrajShape& S = shp[blockIdx.z];

@@ -45,6 +45,11 @@ extern "C" {
 #define CGPU_METHOD_MCTDHX 0
 #define CGPU_METHOD_TDCI 1
 
+/* FP64 throughout.  The contractions of ApplyCorrelationOp and FillH2 run as digit slices
+ * (see CGPU_PREC_MIXED_FX): 8 (63 bits of the row maximum) where the interaction falls by at
+ * most 2^10 from zero to the longest distance, 9 (71 bits) up to 2^16, else on the FP64 pipe.
+ * Entry by entry that leaves W, h2 and the mean field as close to the exact ones as FP64 sums
+ * do; operands below the smallest normal number count as zero. */
 #define CGPU_PREC_FP64 0
 /* Mixed: the pair-potential, correlation and h2 contractions on tcgen05 tensor cores with
  * split-bf16 operands (hi + lo, three products) and FP32 accumulation; RDMs, rho^-1,
@@ -56,13 +61,12 @@ extern "C" {
  * of two per row, in base 256: 5 slices (39 bits of the row maximum) for the contractions
  * over the grid, 4 or 5 (32, 40) for the one over orbital pairs; slice products of one
  * level summed exactly in their own FP32 tensor-memory accumulator, levels combined in
- * 64-bit integers: the contractions equal the products of the truncated operands.  The
- * FP64 form runs its contractions the same way with 7 slices (55 bits). */
+ * 64-bit integers: the contractions equal the products of the truncated operands. */
 #define CGPU_PREC_MIXED_FX 3
 /* As CGPU_PREC_MIXED_FX with 5 or 6 slices over the grid (6 up to 1024 points) and 5 or 6
  * over the pairs. */
 #define CGPU_PREC_MIXED_FX6 4
-/* As CGPU_PREC_FP64 with every contraction on the FP64 pipe (12 to 40 times slower there). */
+/* As CGPU_PREC_FP64 with every contraction on the FP64 pipe (a step takes 2 to 15 times as long). */
 #define CGPU_PREC_FP64_PIPE 5
 
 /* Time-derivative selectors (the TimeDerivative procedure pointers). */
@@ -145,9 +149,9 @@ int cgpu_configlist_tables(cgpu_ctx* ctx, int bt, int kind, int* n_conf, int* ma
                            int* n_connected, int* excited_c, int* orb_code, double* factor);
 int cgpu_synchronize(cgpu_ctx* ctx);
 /* Digit slices that carry an operand of the contractions over the grid; 0 where they do
- * not run in slices (CGPU_PREC_FP64_PIPE, _MIXED, _MIXED_X6, TDCI in FP64, no interaction,
- * and contexts whose slices would take more than three quarters of the device's memory or
- * did not find theirs free). */
+ * not run in slices: CGPU_PREC_FP64_PIPE, _MIXED, _MIXED_X6, TDCI in FP64, no interaction,
+ * an interaction of a wider range than CGPU_PREC_FP64 names, and FP64 contexts whose slices
+ * would take more than three quarters of the device's memory or did not find theirs free. */
 int cgpu_contraction_slices(const cgpu_ctx* ctx);
 /* Number of CUDA kernels this context launched since the last reset. */
 long cgpu_launch_count(cgpu_ctx* ctx, int reset);
