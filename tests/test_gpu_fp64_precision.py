@@ -4,7 +4,7 @@ In each entry, (l1 l2 | k1 k2), the error is measured in units of 2^-53 of the s
 terms' sizes, over x and y |S_l1k1(x)| V(x, y) |S_l2k2(y)|, however small it is beside other
 entries.  V's formula takes three roundings, S's two products three, W, the product and the
 result one each; twelve units cover them and the losses of the digit slices, which are chosen
-to stay below (orbitals far apart and a short softening are what they lose most on: 87 and
+to stay below (orbitals far apart and a short softening are what they lose most on: 108 and
 14000 units with seven slices).  The slices' sums do not round; on the FP64 pipe (a range of V
 that slices do not suit) two sums of all points in order may lose a unit a term.
 """
