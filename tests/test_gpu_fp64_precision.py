@@ -44,9 +44,10 @@ def _exact(sp, x, w, F):
 
 
 # range of V up to 2^10 (eight slices), up to 2^16 (nine), beyond (FP64 pipe); grids below one
-# chunk of 128 points, at its edges and of several with splits
+# chunk of 128 points, at its edges and of several with splits; up to 45 pairs (column tiles of 48)
 CASES = [(4, 4.0, 1.0, 2, 8), (25, 25.0, 1.0, 3, 8), (26, 26.0, 0.5, 3, 8), (51, 100.0, 1.0, 3, 8), (100, 100.0, 1.0, 4, 8),
-         (100, 100.0, 0.1, 3, 9), (100, 100.0, 0.01, 3, 9), (25, 25.0, 0.002, 3, 9), (100, 100.0, 0.001, 3, 0)]
+         (100, 100.0, 0.1, 3, 9), (100, 100.0, 0.01, 3, 9), (25, 25.0, 0.002, 3, 9), (100, 100.0, 0.001, 3, 0),
+         (30, 60.0, 0.05, 6, 9), (52, 60.0, 0.05, 9, 9), (512, 400.0, 0.1, 2, 9)]
 
 
 @pytest.mark.parametrize("kind", ["compact", "apart", "spread"])
@@ -77,7 +78,8 @@ def test_integrals_entry_by_entry(n_el, box, soft, n, slices, kind):
 
 @pytest.mark.parametrize("kind", ["compact", "apart"])
 @pytest.mark.parametrize("weight", [1.0, 1e-12, 1e-30])
-@pytest.mark.parametrize("n_el,box,soft,n", [(4, 4.0, 1.0, 2), (51, 100.0, 1.0, 3), (100, 100.0, 1.0, 4), (100, 100.0, 0.01, 3)])
+@pytest.mark.parametrize("n_el,box,soft,n", [(4, 4.0, 1.0, 2), (51, 100.0, 1.0, 3), (100, 100.0, 1.0, 4), (100, 100.0, 0.01, 3),
+                                             (30, 60.0, 0.05, 6), (30, 60.0, 1.0, 9)])
 def test_mean_field_entry_by_entry(n_el, box, soft, n, weight, kind):
     """dphi_j(x) in units of the sum of the sizes of its terms.  The coefficients of the pairs
     of orbitals on one side are small, so that with the sides far apart the sum lies in pairs
